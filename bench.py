@@ -453,24 +453,29 @@ def bench_gbsort(args, cfg, world, rank, local):
     msd_keys = pinfo.msd_region_keys if fused else 0
     stages = None
     if not fused and pinfo.msd_stages:
-        # keys only, most significant digit first: the top digit's histogram
-        # (K bytes a key), top split (2K), pair count (K), scan, second split
-        # (2K), local sorts (2K); the other digits' histogram and the digit
-        # passes exit at once
-        names = ["msd_top_kernel (top split)", "msd_count_kernel (pair count)", "msd_scan_kernel (group offsets)",
+        # keys only, most significant bits first: sample, group count (K bytes
+        # a key), scan, top split (2K), second split (2K), local sorts (2K);
+        # the digits' histogram and the digit passes exit at once
+        names = ["msd_count_kernel (group count)", "msd_scan_kernel (group offsets)", "msd_top_kernel (top split)",
                  "msd_second_kernel (second split)", "msd_local_kernel (local sorts)"]
-        nbytes = [2 * kbytes * n, kbytes * n, 65536 * 8, 2 * kbytes * n, 2 * kbytes * n]
+        nbytes = [kbytes * n, 65536 * 8, 2 * kbytes * n, 2 * kbytes * n, 2 * kbytes * n]
         means = [statistics.mean(p[1 + i] for p in per_kernel) for i in range(5)]
         dom = max(range(5), key=lambda i: means[i])
-        ups_ms = statistics.mean(p[0] for p in per_kernel)
+        ups_ms = None
         launch_ms, launch_bytes, kernel = means[dom], nbytes[dom], names[dom]
-        sort_bytes = n * 8 * kbytes
-        stages = {"upsweep (top digit)": round(ups_ms, 4)}
+        sort_bytes = n * 7 * kbytes
+        stages = {}
         for i in range(5):
             stages[names[i]] = {"ms": round(means[i], 4),
-                                "frac": round(nbytes[i] / (means[i] / 1e3) / 1e9 / hbm, 4) if i != 2 else None}
+                                "frac": round(nbytes[i] / (means[i] / 1e3) / 1e9 / hbm, 4) if i != 1 else None}
         rest = [statistics.mean(p[i] for p in per_kernel) for i in range(6, len(per_kernel[0]))]
-        stages["other digits' histogram + digit passes + fix-up (exit at once)"] = round(sum(rest), 4)
+        stages["digits' histogram + digit passes + fix-up (exit at once)"] = round(sum(rest), 4)
+    elif not fused and all(p[0] > sum(p[1:]) for p in per_kernel):
+        # 4-byte keys, the same way: entry 0 holds its kernels together
+        launch_ms = statistics.mean(p[0] for p in per_kernel)
+        sort_bytes = n * 7 * kbytes
+        launch_bytes, kernel, ups_ms = sort_bytes, "msd kernels (group count, two splits, local sorts)", None
+        stages = {}
     if stages is not None:
         pass
     elif fused and msd_keys:
@@ -493,7 +498,7 @@ def bench_gbsort(args, cfg, world, rank, local):
                 else "fallback 6.8 TB/s", "algorithmic_bytes_per_launch": launch_bytes,
                 "mean_launch_ms": round(launch_ms, 4), "upsweep_ms": None if ups_ms is None else round(ups_ms, 4),
                 "traffic_source": traffic_src}
-    if stages is not None:
+    if stages:
         roofline["msd_stages"] = stages
     sort_roofline = {"bytes_per_key": sort_bytes // n, "achieved": round(
         sort_bytes / (mean_sort_ms / 1e3) / 1e9, 1), "peak": hbm, "unit": "GB/s",

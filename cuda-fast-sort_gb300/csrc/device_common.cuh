@@ -140,6 +140,34 @@ __device__ __forceinline__ U twiddle_out(U t, int kind, int desc) {
     return U(y ^ (was_neg_float ? U(~U(0)) : base));
 }
 
+// The same map with its launch-uniform part worked out once: three integer
+// operations a 32-bit key each way, whatever the kind and order.
+template <class U>
+struct KeyMap {
+    U m, f;  // m: bits every key flips; f: bits that negative floats flip too
+    __device__ __forceinline__ KeyMap(int kind, int desc) {
+        const U sign = U(U(1) << (8 * sizeof(U) - 1));
+        m = U((kind == KIND_UNSIGNED ? U(0) : sign) ^ (desc ? U(~U(0)) : U(0)));
+        f = kind == KIND_FLOAT ? U(~sign) : U(0);
+    }
+    __device__ __forceinline__ static U sign_mask(U x) {
+        if constexpr (sizeof(U) == 4) return U(int32_t(x) >> 31);
+        else if constexpr (sizeof(U) == 8) {
+            const uint32_t s = uint32_t(int32_t(uint32_t(x >> 32)) >> 31);
+            return (U(s) << 32) | U(s);
+        } else {
+            const uint32_t s = uint32_t(int32_t(uint32_t(x >> (8 * sizeof(U) - 32))) >> 31);
+            const uint64_t q = (uint64_t(s) << 32) | s;
+            return (U(q) << 64) | U(q);
+        }
+    }
+    __device__ __forceinline__ U in(U x) const { return U(x ^ m ^ (f & sign_mask(x))); }
+    __device__ __forceinline__ U out(U t) const {
+        const U y = U(t ^ m);
+        return U(y ^ (f & sign_mask(y)));
+    }
+};
+
 // 8-bit digit `pass` (0 = least significant byte) of a twiddled key.
 __device__ __forceinline__ uint32_t digit_of(uint8_t x, int) { return x; }
 __device__ __forceinline__ uint32_t digit_of(uint16_t x, int pass) {

@@ -643,7 +643,7 @@ int gbsort_sort_host(int key_type, int descending, void* h_keys, void* h_values,
     // keys-only sort that goes most significant digit first on the device
     // is short enough that copy, sort, copy wins (2^26 u128: the device sort
     // takes 2 ms of the ~12 the copies take)
-    if (plan.passes >= 2 && n >= split_min_keys() && !plan.msd) {
+    if (plan.passes >= 2 && n >= split_min_keys() && !(plan.msd && plan.msd_block)) {
         SplitLayout L;
         st = split_layout(key_type, value_bytes, n, &L);
         if (st != GBSORT_OK) return st;

@@ -56,34 +56,33 @@ const KernelEntry* fused_entry_for() {
     return &e;
 }
 
-// Keys-only sorts of 8- and 16-byte keys, most significant digit first:
-// top split, pair count, scan, second split, local sorts (shape 0), local
-// sorts (shape 1), the top digit's histogram.
+// Keys-only sorts above the short range, most significant bits first: sample,
+// count, scan, top split, second split, local sorts (two sizes).
 template <int KB, int L>
 KernelEntry make_msd_local_entry() {
     using S = MsdShape<KB>;
-    using GL = MsdLocalGeom<KB, S::C_THREADS, S::C_LIPT[L]>;
-    return KernelEntry{reinterpret_cast<const void*>(&msd_local_kernel<KB, S::C_THREADS, S::C_LIPT[L],
-                                                                        S::C_MIN_CTAS[L], S::C_SPLIT_WORDS[L]>),
-                       S::C_THREADS, S::C_LIPT[L], S::C_THREADS * S::C_LIPT[L],
-                       static_cast<unsigned long>(GL::SMEM_BYTES)};
+    using GL = GroupSortGeom<KB, S::C_THREADS[L], S::C_HALO>;
+    static_assert(GL::CAP == int(msd_group_cap_of<KB>(L)), "the plan's capacity");
+    return KernelEntry{
+        reinterpret_cast<const void*>(&msd_local_kernel<KB, S::C_THREADS[L], S::C_MIN_CTAS[L], S::C_HALO>),
+        S::C_THREADS[L], GL::LIPT, GL::CAP, static_cast<unsigned long>(GL::SMEM_BYTES)};
 }
 
 template <int KB>
 const KernelEntry* msd_entries_for() {
     using S = MsdShape<KB>;
-    using GS = MsdSplitGeom<KB, S::THREADS, S::IPT>;
+    using GS = MsdSplitGeom<KB, S::THREADS, S::IPT, S::CAP>;
     static const KernelEntry e[7] = {
-        {reinterpret_cast<const void*>(&msd_top_kernel<KB, S::THREADS, S::IPT, S::MIN_CTAS>), S::THREADS, S::IPT,
-         GS::TILE, static_cast<unsigned long>(GS::SMEM_BYTES)},
-        {reinterpret_cast<const void*>(&msd_count_kernel<KB, S::THREADS, S::IPT, S::MIN_CTAS>), S::THREADS, S::IPT,
-         GS::TILE, static_cast<unsigned long>(MsdCountGeom<KB, S::THREADS, S::IPT>::SMEM_BYTES)},
-        {reinterpret_cast<const void*>(&msd_scan_kernel<KB>), MSD_SCAN_THREADS, 0, 0, 0ul},
-        {reinterpret_cast<const void*>(&msd_second_kernel<KB, S::THREADS, S::IPT, S::MIN_CTAS>), S::THREADS, S::IPT,
+        {reinterpret_cast<const void*>(&msd_sample_kernel<KB>), MSD_SAMPLE_THREADS, 0, 0, 0ul},
+        {reinterpret_cast<const void*>(&msd_count_kernel<KB>), MSD_COUNT_THREADS, 0, 0,
+         static_cast<unsigned long>(MSD_COUNT_SMEM)},
+        {reinterpret_cast<const void*>(&msd_scan_kernel<KB>), 256, 0, 0, 0ul},
+        {reinterpret_cast<const void*>(&msd_top_kernel<KB, S::THREADS, S::IPT, S::MIN_CTAS, S::CAP>), S::THREADS,
+         S::IPT, GS::TILE, static_cast<unsigned long>(GS::SMEM_BYTES)},
+        {reinterpret_cast<const void*>(&msd_second_kernel<KB, S::THREADS, S::IPT, S::MIN_CTAS, S::CAP>), S::THREADS, S::IPT,
          GS::TILE, static_cast<unsigned long>(GS::SMEM_BYTES)},
         make_msd_local_entry<KB, 0>(),
         make_msd_local_entry<KB, 1>(),
-        {reinterpret_cast<const void*>(&msd_hist_kernel<KB>), MSD_HIST_THREADS, 0, 0, 0ul},
     };
     return e;
 }

@@ -1,35 +1,36 @@
-// msd.cuh — keys-only sorts of 8- and 16-byte keys, most significant digit
-// first (sm_103a).
+// msd.cuh — keys-only sorts of 4-, 8- and 16-byte keys above the short range,
+// most significant bits first (sm_103a).
 //
-// A least-significant-digit sort of 16-byte keys makes 16 passes over the
-// data (8 for 8-byte keys), each bound by its stable rank.  Keys only, equal
-// twiddled keys are equal bytes, so the order among equal keys cannot show
-// and no step needs a stable order.  This path instead:
+// A least-significant-digit sort makes one stable pass over the data per key
+// byte, each bound by its rank.  Keys only, equal twiddled keys are equal
+// bytes, so the order among equal keys cannot show and no step needs a stable
+// order.  This path instead reads a key's leading bits as a group number
+// (8 + b2 bits, so that groups average a third to 0.72 of a local sort):
+//   sample:       4096 keys say which of their bits vary (keys of a small
+//                 range leave the leading ones alone: the group number starts
+//                 at the first that varies) and how many group bits to take;
+//                 it also clears the path's counters;
+//   count:        one read of the keys counts every group (65536 16-bit
+//                 counters fit a CTA's shared memory);
+//   scan:         group offsets, and the decision: every group fits a CTA's
+//                 local sort, or MSD_OFF;
 //   top split:    every tile counts its keys per top digit with shared
-//                 atomics, claims its places in the digit's range (exact: the
-//                 upsweep's counts) with one global atomic per digit, stages
-//                 the tile by digit and writes each digit's run — no tile
-//                 waits for another (input -> alternate buffer, twiddled);
-//   pair count:   tiles of each top bucket count the second digit into
-//                 per-(top, second) totals;
-//   scan:         one CTA turns the 65536 totals into group offsets and
-//                 decides: every group fits a CTA's local sort (MSD_OK), or
-//                 not (MSD_OFF);
-//   second split: as the top split, within each top bucket, into the groups'
-//                 exact ranges (alternate buffer -> caller's buffer);
-//   local sorts:  each CTA sorts whole groups in place in shared memory (the
-//                 bucket split of fused_short.cuh: a counting pass on the next
-//                 11-12 bits, then a comparison rank inside the sub-buckets)
-//                 and writes them untwiddled; a group with a sub-bucket too
-//                 big for the comparison rank goes back untwiddled unsorted
-//                 and turns the state to MSD_OFF.
+//                 atomics, claims its places in the digit's exact range with
+//                 one global atomic per digit, stages the tile by digit and
+//                 writes each digit's run — no tile waits for another (input
+//                 -> alternate buffer, twiddled);
+//   second split: the same inside every top bucket, by the group's b2 bits
+//                 (alternate buffer -> caller's buffer);
+//   local sorts:  each CTA sorts whole groups in place in shared memory: a
+//                 counting pass on the next 11-12 bits moves every key into
+//                 its sub-bucket (about one key each), then a few rounds of
+//                 an odd-even transposition network in registers, as many as
+//                 the largest sub-bucket holds keys, put the keys in order.
 // With MSD_OFF the least-significant-digit passes, launched after these
 // kernels, sort from the caller's buffer, which then holds the input's keys
-// in some order (untouched, or as the local sorts left them); with MSD_OK
-// they exit at once.
-// Every key is read and written three times (plus the upsweep's and the pair
-// count's reads): 16-byte keys 2^26 measured 0.38 ms per split against 0.54
-// ms per digit pass.
+// in some order (untouched, or as the local sorts left them); otherwise they
+// exit at once.
+// Every key is read four times and written three times, whatever its width.
 #pragma once
 
 #include "fused_short.cuh"
@@ -37,160 +38,553 @@
 namespace gbsort {
 
 struct MsdParams {
-    const void* keys_in;   // the top split's input: the caller's keys or the input-preserving source
+    const void* keys_in;   // the input: the caller's keys or the input-preserving source
     void* keys_a;          // the caller's buffer (second split's output, sorted in place)
     void* keys_b;          // the alternate buffer (top split's output)
-    uint64_t n;
+    uint64_t n;            // < 2^32
     int kind, desc;
-    const unsigned long long* gp_top;  // the upsweep's counts of the top digit [256]
-    uint32_t* state;       // MSD_OK / MSD_OFF, zeroed before the sort
-    uint32_t* cursor1;     // [256] claimed places per top digit, zeroed
-    uint32_t* joint;       // [256 * 256] keys per (top, second) digit, zeroed
-    uint32_t* cursor2;     // [256 * 256] claimed places per group, zeroed
-    uint32_t* offs2;       // [256 * 256] first place of every group
+    int b2_max;            // most group bits below the top digit (0 .. 8) that the counters have room for
+    uint32_t* state;       // MSD_OFF: the digit passes sort; zeroed with the control block
+    uint32_t* window;      // [2] leading bits that do not vary, group bits below the top digit (b2)
+    uint32_t* zero;        // the counters below, cleared by the first kernel
+    uint32_t zero_words;
+    uint32_t* top_counts;  // [256] keys per top digit
+    uint32_t* cursor1;     // [256] next place of every top digit
+    uint32_t* joint;       // [256 << b2_max] keys per group
+    uint32_t* cursor2;     // [256 << b2_max] next place of every group; its end after the second split
     uint32_t group_cap;    // largest group a local sort takes
     uint32_t* err;         // workspace error word
 };
 
-// The MSD path's first kernel: the top digit's counts of the input into
-// h.gp_counts (the row of digit P-1), and the clear of the status words and
-// the MSD block (h.status, h.status_bytes).  One digit needs 256 counters
-// (32 copies, one per lane: no same-word atomics), so several CTAs fit an
-// SM and keep more loads in flight than the all-digit histogram kernel
-// (one CTA of 1024 threads an SM for its 128 KB of counters).
-constexpr int MSD_HIST_THREADS = 512;
+// The leading 64 bits of a twiddled key (all of a 4-byte key's, left-aligned).
+__device__ __forceinline__ uint64_t msd_top64(uint32_t k) { return uint64_t(k) << 32; }
+__device__ __forceinline__ uint64_t msd_top64(uint64_t k) { return k; }
+__device__ __forceinline__ uint64_t msd_top64(u128 k) { return uint64_t(k >> 64); }
+
+// A key's code: the 32 bits of it after the `skip` leading ones that all keys
+// share (zeros where they run past its leading 64).
+struct MsdCode {
+    uint32_t skip, b2;
+    __device__ __forceinline__ explicit MsdCode(const MsdParams& p)
+        : skip(ld_relaxed(p.window)), b2(ld_relaxed(p.window + 1)) {}
+    __device__ __forceinline__ uint32_t operator()(uint32_t k) const { return k << skip; }
+    __device__ __forceinline__ uint32_t operator()(uint64_t k) const {
+        const uint32_t hi = uint32_t(k >> 32), lo = uint32_t(k);
+        const bool low = skip >= 32u;
+        return __funnelshift_l(low ? 0u : lo, low ? lo : hi, skip);  // (the shift wraps at 32)
+    }
+    __device__ __forceinline__ uint32_t operator()(u128 k) const { return (*this)(uint64_t(k >> 64)); }
+};
+
+// The window of the codes, from a sample; the other CTAs clear the counters.
+constexpr int MSD_SAMPLE_THREADS = 1024;
 template <int KB>
-__global__ void __launch_bounds__(MSD_HIST_THREADS, 2) msd_hist_kernel(HistParams h) {
+__global__ void __launch_bounds__(MSD_SAMPLE_THREADS) msd_sample_kernel(MsdParams p) {
     using U = typename KeyBits<KB>::U;
-    __shared__ uint32_t cnt[256 * 32];
-    const int tid = threadIdx.x, lane = tid & 31;
-    for (int i = tid; i < 256 * 32; i += MSD_HIST_THREADS) cnt[i] = 0u;
     grid_launch_dependents();
-    {
-        const uint64_t nv = h.status_bytes >> 4;
-        uint4* st = static_cast<uint4*>(h.status);
-        const uint64_t stride = uint64_t(gridDim.x) * MSD_HIST_THREADS;
-        for (uint64_t i = uint64_t(blockIdx.x) * MSD_HIST_THREADS + tid; i < nv; i += stride)
-            st[i] = make_uint4(0, 0, 0, 0);
+    grid_dependency_wait();
+    const int tid = threadIdx.x;
+    if (blockIdx.x != 0) {
+        const uint32_t stride = (gridDim.x - 1) * MSD_SAMPLE_THREADS;
+        for (uint32_t i = (blockIdx.x - 1) * MSD_SAMPLE_THREADS + tid; i < p.zero_words; i += stride) p.zero[i] = 0u;
+        return;
+    }
+    constexpr uint32_t SLOTS = 8192, NONE = 0xffffffffu;
+    __shared__ uint32_t vary[2], top, again, bins[256], seen[SLOTS];
+    if (tid < 2) vary[tid] = 0u;
+    if (tid == 0) top = again = 0u;
+    for (uint32_t i = tid; i < SLOTS; i += MSD_SAMPLE_THREADS) seen[i] = NONE;
+    if (tid < 256) bins[tid] = 0u;
+    __syncthreads();
+    const KeyMap<U> map(p.kind, p.desc);
+    const U* keys = static_cast<const U*>(p.keys_in);
+    constexpr int PER = 4;
+    const uint32_t step = uint32_t(p.n / (MSD_SAMPLE_THREADS * PER));
+    uint64_t x[PER];
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+        const uint32_t at = uint32_t(i * MSD_SAMPLE_THREADS + tid);
+        x[i] = msd_top64(map.in(keys[uint64_t(at) * step + (at * 2654435761u) % step]));
+    }
+    const uint64_t first = msd_top64(map.in(keys[0]));
+    uint64_t d = 0;
+#pragma unroll
+    for (int i = 0; i < PER; ++i) d |= x[i] ^ first;
+    const uint32_t dh = __reduce_or_sync(0xffffffffu, uint32_t(d >> 32));
+    const uint32_t dl = __reduce_or_sync(0xffffffffu, uint32_t(d));
+    if ((tid & 31) == 0) {
+        atomicOr(&vary[0], dh);
+        atomicOr(&vary[1], dl);
     }
     __syncthreads();
-    const U* keys = static_cast<const U*>(h.keys);
-    const uint64_t n = h.n;
-    auto count = [&](U k) { atomicAdd(&cnt[digit_of(twiddle_in<U>(k, h.kind, h.desc), KB - 1) * 32 + lane], 1u); };
+    const uint32_t skip = vary[0] ? __clz(vary[0]) : vary[1] ? 32u + __clz(vary[1]) : 0u;
+    uint32_t most = 0, twice = 0;
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+        const uint32_t c = uint32_t((x[i] << skip) >> 32);
+        most = max(most, c);
+        atomicAdd(&bins[c >> 24], 1u);
+        // codes met before in the sample (open addressing, half full at most)
+        uint32_t h = (c * 2654435761u) >> 19;
+        for (int probe = 0; probe < 64 && c != NONE; ++probe) {
+            uint32_t v = seen[h];
+            if (v == NONE) v = atomicCAS(&seen[h], NONE, c);
+            if (v == NONE) break;
+            if (v == c) {
+                ++twice;
+                break;
+            }
+            h = (h + 1u) & (SLOTS - 1u);
+        }
+    }
+    twice = __reduce_add_sync(0xffffffffu, twice);
+    if ((tid & 31) == 0 && twice) atomicAdd(&again, twice);
+    most = __reduce_max_sync(0xffffffffu, most);
+    if ((tid & 31) == 0) atomicMax(&top, most);
+    __syncthreads();
+    // a top digit with five times its share has groups that do not fit, and
+    // codes that repeat more than 64 times (S keys of D distinct codes meet
+    // S * S / 2 D of them again) crowd the local sorts' sub-buckets
+    const bool uneven = __syncthreads_or(tid < 256 && bins[tid] > MSD_SAMPLE_THREADS * PER / 256 * 5);
+    if (tid == 0) {
+        // the codes reach `top`: groups beyond it stay empty
+        const float used = (float(top) + 1.f) * 0x1p-24f, n = float(p.n), cap = float(p.group_cap) * used;
+        uint32_t b2 = 0;
+        while (b2 < uint32_t(p.b2_max) && n > 0.72f * cap * float(1u << b2)) ++b2;
+        constexpr float S = MSD_SAMPLE_THREADS * PER;
+        const bool crowded = again >= 16u && 2.f * float(again) * n > 64.f * S * S;
+        if (uneven || crowded || n > cap * float(1u << b2)) *p.state = MSD_OFF;
+        p.window[0] = skip;
+        p.window[1] = b2;
+    }
+}
+
+// Keys per group, one read of the input.  16-bit counters, two to a word.
+// Rounds of at most 2^14 keys a CTA: a counter that a key of the round found
+// at 2^15 or above makes the CTA move those halves to the global counts after
+// the round's barrier, so none ever passes 2^15 + 2^14.
+constexpr int MSD_COUNT_THREADS = 1024;
+constexpr int MSD_COUNT_SMEM = 32768 * 4 + 256 * 4;
+template <int KB>
+__global__ void __launch_bounds__(MSD_COUNT_THREADS, 1) msd_count_kernel(MsdParams p) {
+    using U = typename KeyBits<KB>::U;
+    extern __shared__ __align__(128) uint8_t smem[];
+    uint32_t* cnt = reinterpret_cast<uint32_t*>(smem);
+    uint32_t* rows = cnt + 32768;
+    const int tid = threadIdx.x;
+    for (uint32_t i = tid; i < (128u << p.b2_max); i += MSD_COUNT_THREADS) cnt[i] = 0u;
+    if (tid < 256) rows[tid] = 0u;
+    grid_launch_dependents();
+    grid_dependency_wait();
+    if (ld_relaxed(p.state) & MSD_OFF) return;
+    __syncthreads();
+    const MsdCode code_of(p);
+    const uint32_t b2 = code_of.b2, words = 128u << b2, shift = 24u - b2;
+    const KeyMap<U> map(p.kind, p.desc);
+    const U* keys = static_cast<const U*>(p.keys_in);
+    const uint64_t n = p.n;
     uint64_t head = ((16u - (reinterpret_cast<uintptr_t>(keys) & 15u)) & 15u) / KB;
     if (head > n) head = n;
     const uint64_t nvec = (n - head) * KB / 16;
     constexpr int PER_VEC = 16 / KB, UNROLL = 4;
-    const uint64_t gthreads = uint64_t(gridDim.x) * MSD_HIST_THREADS;
-    const uint64_t gtid = uint64_t(blockIdx.x) * MSD_HIST_THREADS + tid;
-    if (gtid < head) count(keys[gtid]);
+    static_assert(MSD_COUNT_THREADS * PER_VEC * UNROLL <= 16384, "keys a round");
+    const uint64_t gthreads = uint64_t(gridDim.x) * MSD_COUNT_THREADS;
+    const uint64_t gtid = uint64_t(blockIdx.x) * MSD_COUNT_THREADS + tid;
     const uint4* vec = reinterpret_cast<const uint4*>(keys + head);
-    uint64_t i = gtid;
-    for (; i + (UNROLL - 1) * gthreads < nvec; i += UNROLL * gthreads) {
-        uint4 v[UNROLL];
+    unsigned long long* joint = reinterpret_cast<unsigned long long*>(p.joint);
+    const U first = map.in(keys[0]);
+    U outside = U(0);  // a bit set: some key differs from the first one there
+    auto sweep = [&](auto floats) {
+        uint32_t seen = 0;
+        auto count = [&](U k) {
+            const U t = decltype(floats)::value ? map.in(k) : U(k ^ map.m);
+            outside |= t ^ first;
+            const uint32_t g = code_of(t) >> shift;
+            seen |= atomicAdd(&cnt[g >> 1], __funnelshift_l(1u, 1u, g * 16u));
+        };
+        auto settle = [&] {
+            if (__syncthreads_or(seen & 0x80008000u)) {
+                for (uint32_t i = tid; i < words; i += MSD_COUNT_THREADS) {
+                    const uint32_t w = cnt[i], lo = w & 0x8000u, hi = (w >> 16) & 0x8000u;
+                    if (lo | hi) {
+                        cnt[i] = w & 0x7fff7fffu;
+                        atomicAdd(joint + i, (unsigned long long)(lo) | (unsigned long long)(hi) << 32);
+                        if (lo) atomicAdd(p.top_counts + ((2 * i) >> b2), lo);
+                        if (hi) atomicAdd(p.top_counts + ((2 * i + 1) >> b2), hi);
+                    }
+                }
+                seen = 0;
+                __syncthreads();
+            }
+        };
+        if (gtid < head) count(keys[gtid]);
+        // the same number of rounds for every thread (the barrier in them)
+        uint64_t i0 = 0;
+        for (; i0 + UNROLL * gthreads <= nvec; i0 += UNROLL * gthreads) {
+            uint4 v[UNROLL];
 #pragma unroll
-        for (int r = 0; r < UNROLL; ++r) v[r] = __ldcs(vec + i + r * gthreads);
+            for (int r = 0; r < UNROLL; ++r) v[r] = __ldcs(vec + i0 + r * gthreads + gtid);
 #pragma unroll
-        for (int r = 0; r < UNROLL; ++r) {
+            for (int r = 0; r < UNROLL; ++r) {
+                union { uint4 q; U k[PER_VEC]; } w;
+                w.q = v[r];
+#pragma unroll
+                for (int e = 0; e < PER_VEC; ++e) count(w.k[e]);
+            }
+            settle();
+        }
+        for (uint64_t i = i0 + gtid; i < nvec; i += gthreads) {
             union { uint4 q; U k[PER_VEC]; } w;
-            w.q = v[r];
+            w.q = __ldcs(vec + i);
 #pragma unroll
             for (int e = 0; e < PER_VEC; ++e) count(w.k[e]);
         }
+        for (uint64_t j = head + nvec * PER_VEC + gtid; j < n; j += gthreads) count(keys[j]);
+    };
+    if (p.kind == KIND_FLOAT) sweep(BoolTag<true>{});
+    else sweep(BoolTag<false>{});
+    // a key that differs in the bits left out of the codes: the digit passes sort
+    const uint64_t o64 = msd_top64(outside);
+    if (__syncthreads_or(code_of.skip != 0u && (o64 >> (64u - code_of.skip)) != 0u)) {
+        if (tid == 0) atomicOr(p.state, MSD_OFF);
+        return;
     }
-    for (; i < nvec; i += gthreads) {
-        union { uint4 q; U k[PER_VEC]; } w;
-        w.q = __ldcs(vec + i);
-#pragma unroll
-        for (int e = 0; e < PER_VEC; ++e) count(w.k[e]);
+    // the CTA's counts to the global ones, two groups per 64-bit add (a
+    // group's count stays below 2^32, so the halves never carry); CTAs start
+    // at different words
+    const uint32_t rot = uint32_t((uint64_t(words) * blockIdx.x / gridDim.x) & ~31u);
+    for (uint32_t i0 = tid; i0 < words; i0 += MSD_COUNT_THREADS) {
+        uint32_t i = i0 + rot;
+        if (i >= words) i -= words;
+        const uint32_t w = cnt[i];
+        const uint32_t lo = w & 0xffffu, hi = w >> 16;
+        if (w) atomicAdd(joint + i, (unsigned long long)(lo) | (unsigned long long)(hi) << 32);
+        if (b2 >= 6) {  // a warp's 32 words lie in one row
+            const uint32_t s = __reduce_add_sync(0xffffffffu, lo + hi);
+            if ((tid & 31) == 0 && s) atomicAdd(&rows[(i * 2) >> b2], s);
+        } else if (b2 >= 1) {
+            if (w) atomicAdd(&rows[(i * 2) >> b2], lo + hi);
+        } else {
+            if (lo) atomicAdd(&rows[i * 2], lo);
+            if (hi) atomicAdd(&rows[i * 2 + 1], hi);
+        }
     }
-    for (uint64_t j = head + nvec * PER_VEC + gtid; j < n; j += gthreads) count(keys[j]);
     __syncthreads();
-    // one warp per bin: the 32 copies summed by a shuffle reduction
-    for (int bin = tid >> 5; bin < 256; bin += MSD_HIST_THREADS / 32) {
-        uint32_t c = cnt[bin * 32 + lane];
+    if (tid < 256 && rows[tid]) atomicAdd(p.top_counts + tid, rows[tid]);
+}
+
+// Group offsets, one CTA per top digit, and the decision.
+template <int KB>
+__global__ void __launch_bounds__(256) msd_scan_kernel(MsdParams p) {
+    __shared__ uint32_t scan[32], base;
+    grid_launch_dependents();
+    grid_dependency_wait();
+    if (ld_relaxed(p.state) & MSD_OFF) return;
+    const int tid = threadIdx.x;
+    const uint32_t b = blockIdx.x, b2 = ld_relaxed(p.window + 1);
+    const uint32_t ex = block_exclusive_scan_256<uint32_t>(p.top_counts[tid], scan, nullptr);
+    if (uint32_t(tid) == b) {
+        base = ex;
+        p.cursor1[b] = ex;
+    }
+    __syncthreads();
+    const bool mine = tid < (1 << b2);
+    const uint32_t c = mine ? p.joint[(b << b2) + tid] : 0u;
+    const uint32_t e2 = block_exclusive_scan_256<uint32_t>(c, scan, nullptr);
+    if (mine) p.cursor2[(b << b2) + tid] = base + e2;
+    if (__syncthreads_or(c > p.group_cap) && tid == 0) atomicOr(p.state, MSD_OFF);
+}
+
+// Shared memory of a split: the stage, in which every digit has CAP places of
+// its own for a digit of 8 bits (more for a narrower one), then u32 bins[256],
+// claims[256], counts[256], tstart, tcnt, tfirst[257], scan[32].
+// CAP is odd, so that the digits' places start on different banks, and about
+// five standard deviations above the mean of THREADS * IPT / 256 keys.
+template <int KB, int THREADS, int IPT, int CAP>
+struct MsdSplitGeom {
+    static constexpr int TILE = THREADS * IPT;
+    static constexpr int STAGE = CAP ? 256 * CAP : TILE;
+    static_assert(STAGE >= TILE && (CAP % 2 == 1 || CAP == 0), "the stage also holds a dense tile");
+    static_assert(IPT % (16 / KB) == 0, "16-byte loads");
+    static constexpr size_t WORDS_OFF = size_t(STAGE) * KB;
+    static constexpr size_t SMEM_BYTES = WORDS_OFF + (256 * 6 + 1 + 32 + 4) * 4;
+};
+
+// Keys [lo, hi) from the 16-byte aligned src into registers, by 16-byte loads:
+// key VEC * i + e of a thread is key (i * THREADS + tid) * VEC + e.  The whole
+// vectors load without branches, so that nothing waits for them here.
+template <int THREADS, class U, int N>
+__device__ __forceinline__ void load_vectors(const U* src, uint32_t lo, uint32_t hi, U (&keys)[N]) {
+    constexpr int VEC = 16 / int(sizeof(U));
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
-        if (lane == 0 && c) atomicAdd(&h.gp_counts[size_t(KB - 1) * 256 + bin], static_cast<unsigned long long>(c));
+    for (int i = 0; i < N / VEC; ++i) {
+        const uint32_t j = uint32_t(i * THREADS + threadIdx.x) * VEC;
+        union { uint4 q; U k[VEC]; } w;
+        w.q = make_uint4(0u, 0u, 0u, 0u);
+        if (j >= lo && j + VEC <= hi) w.q = __ldcs(reinterpret_cast<const uint4*>(src + j));
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) keys[i * VEC + e] = w.k[e];
+    }
+    if (VEC > 1 && ((lo | hi) & uint32_t(VEC - 1))) {  // the ragged ends
+#pragma unroll
+        for (int i = 0; i < N / VEC; ++i) {
+            const uint32_t j = uint32_t(i * THREADS + threadIdx.x) * VEC;
+            if (j + VEC > lo && j < hi && (j < lo || j + VEC > hi)) {
+#pragma unroll
+                for (int e = 0; e < VEC; ++e)
+                    if (j + e >= lo && j + e < hi) keys[i * VEC + e] = src[j + e];
+            }
+        }
     }
 }
 
-// One tile split by one digit: `cnt` keys at src (twiddled on load when
-// TWIDDLE) go to dst at base[d] + (their place among the keys of digit d
-// that every tile claims from claim[d]), d = the key's digit `q`.  No order
-// among a digit's keys.  Shared: stage (the tile), bins / delta / scan.
-template <int KB, int THREADS, int IPT, bool TWIDDLE>
-__device__ __forceinline__ void msd_load_tile(const typename KeyBits<KB>::U* src, uint32_t cnt, int kind, int desc,
+// The tile's keys [lo, hi) of THREADS * IPT from a 16-byte aligned address:
+// key VEC * i + e of a thread is key (i * THREADS + tid) * VEC + e.
+template <int KB, int THREADS, int IPT>
+__device__ __forceinline__ void msd_load_tile(const typename KeyBits<KB>::U* src, uint32_t lo, uint32_t hi,
                                               typename KeyBits<KB>::U (&keys)[IPT]) {
     using U = typename KeyBits<KB>::U;
-#pragma unroll
-    for (int u = 0; u < IPT; ++u) {
-        const uint32_t j = uint32_t(u * THREADS + threadIdx.x);
-        keys[u] = U(0);
-        if (j < cnt) keys[u] = TWIDDLE ? twiddle_in<U>(src[j], kind, desc) : src[j];
-    }
+    load_vectors<THREADS>(src, lo, hi, keys);
 }
 
-// The split of a tile whose keys are in registers (msd_load_tile's layout).
-template <int KB, int THREADS, int IPT, class Base>
-__device__ __forceinline__ void msd_split_loaded(const typename KeyBits<KB>::U (&keys)[IPT], uint32_t cnt, int q,
-                                                 uint32_t* claim, Base base, typename KeyBits<KB>::U* dst, uint64_t n,
-                                                 uint32_t* err, typename KeyBits<KB>::U* stage, uint32_t* bins,
-                                                 uint32_t* delta, uint32_t* scan) {
+// One tile (msd_load_tile's keys, mapped by in()) split by one digit (code >>
+// shift, nb values, a power of two): its keys go to dst at the places that
+// the tile claims from claim[d], one atomic per digit.  No order among a
+// digit's keys.  bins: nb zeros on entry, left so.  refill() runs when the
+// keys' registers are free.
+// Every key takes its digit's next place with one shared atomic and goes
+// there at once; a warp then writes whole digits.  A digit with more keys than
+// its places hold (uneven digits) sends the tile through a dense stage, whose
+// places need the tile's counts first.
+// What bounds it: shared-memory wavefronts, 3.5 for a warp's access to random
+// banks; this makes two such accesses a key, the dense stage three (2^28
+// 4-byte keys: 0.43 against 0.58 ms).
+template <int KB, int THREADS, int IPT, int CAP, class In, class Reload, class Refill>
+__device__ __forceinline__ void msd_split_tile(typename KeyBits<KB>::U (&keys)[IPT], uint32_t lo, uint32_t hi,
+                                               const MsdCode& code_of, uint32_t shift, uint32_t nb, uint32_t* claim,
+                                               typename KeyBits<KB>::U* dst, uint32_t n, uint32_t* err, uint8_t* smem,
+                                               In in, Reload reload, Refill refill) {
     using U = typename KeyBits<KB>::U;
-    const int tid = threadIdx.x;
-    uint32_t slot[IPT];
-    if (tid < 256) bins[tid] = 0u;
-    __syncthreads();
+    using G = MsdSplitGeom<KB, THREADS, IPT, CAP>;
+    constexpr int VEC = 16 / KB;
+    U* stage = reinterpret_cast<U*>(smem);
+    uint32_t* bins = reinterpret_cast<uint32_t*>(smem + G::WORDS_OFF);
+    uint32_t* runs = bins + 256;  // u32 pairs: a digit's first place and its keys; dense: [256] twice
+    uint32_t* scan = bins + 256 * 5 + 257;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const bool full = lo == 0u && hi == uint32_t(G::TILE);
+    const uint32_t cap = nb == 256u ? uint32_t(CAP) : (uint32_t(G::STAGE) / nb - 1u) | 1u;
+    auto digit = [&](U k) { return (code_of(k) >> shift) & (nb - 1u); };
+    auto each = [&](auto f) {
+        if (full) {
 #pragma unroll
-    for (int u = 0; u < IPT; ++u)
-        if (uint32_t(u * THREADS + tid) < cnt) slot[u] = atomicAdd(&bins[digit_of(keys[u], q)], 1u);
-    __syncthreads();
+            for (int u = 0; u < IPT; ++u) f(u);
+        } else {
+#pragma unroll
+            for (int u = 0; u < IPT; ++u) {
+                const uint32_t j = uint32_t(u / VEC * THREADS + tid) * VEC + uint32_t(u % VEC);
+                if (j >= lo && j < hi) f(u);
+            }
+        }
+    };
+    if constexpr (CAP == 0) {
+        // dense stage: slots first, places once the tile's counts are scanned
+        static_assert(IPT % 2 == 0 && G::TILE < 65536, "two slots to a register");
+        uint32_t slot[IPT / 2];
+#pragma unroll
+        for (int u = 0; u < IPT / 2; ++u) slot[u] = 0u;
+#pragma unroll
+        for (int u = 0; u < IPT; ++u) keys[u] = in(keys[u]);
+        each([&](int u) {
+            slot[u / 2] = __byte_perm(slot[u / 2], atomicAdd(&bins[digit(keys[u])], 1u), (u & 1) ? 0x5410 : 0x3254);
+        });
+        __syncthreads();
+        uint32_t c = 0, g = 0;
+        if (uint32_t(tid) < nb) {
+            c = bins[tid];
+            if (c) g = atomicAdd(claim + tid, c);
+        }
+        const uint32_t ex = block_exclusive_scan_256<uint32_t>(c, scan, nullptr);
+        if (uint32_t(tid) < nb) runs[tid] = ex;
+        __syncthreads();
+        each([&](int u) {
+            stage[runs[digit(keys[u])] + __byte_perm(slot[u / 2], 0u, (u & 1) ? 0x4432 : 0x4410)] = keys[u];
+        });
+        if (uint32_t(tid) < nb) {
+            runs[256 + tid] = g - ex;  // the claim's answer: only the write-out needs it
+            bins[tid] = 0u;
+        }
+        refill();
+        __syncthreads();
+        bool bad = false;
+        const uint32_t cnt = hi - lo;
+#pragma unroll
+        for (int u = 0; u < IPT; ++u) {  // coalesced runs, one per digit
+            const uint32_t j = uint32_t(u * THREADS + tid);
+            if (full || j < cnt) {
+                const U k = stage[j];
+                const uint32_t pos = runs[256 + digit(k)] + j;
+                if (pos < n) dst[pos] = k;
+                else bad = true;
+            }
+        }
+        if (bad) atomicOr(err, ERRBIT_BOUNDS);
+        __syncthreads();
+        return;
+    }
+    uint32_t last = 0;
+    each([&](int u) {
+        const U k = in(keys[u]);
+        const uint32_t d = digit(k);
+        const uint32_t slot = atomicAdd(&bins[d], 1u);
+        last = max(last, slot);
+        if (slot < cap) stage[d * cap + slot] = k;
+    });
+    const bool over = __syncthreads_or(last >= cap) != 0;
     uint32_t c = 0, g = 0;
-    if (tid < 256) {
+    if (uint32_t(tid) < nb) {
         c = bins[tid];
         if (c) g = atomicAdd(claim + tid, c);
+        bins[tid] = 0u;
     }
-    const uint32_t ex = block_exclusive_scan_256<uint32_t>(c, scan, nullptr);
-    if (tid < 256) bins[tid] = ex;
-    __syncthreads();
-#pragma unroll
-    for (int u = 0; u < IPT; ++u)
-        if (uint32_t(u * THREADS + tid) < cnt) stage[bins[digit_of(keys[u], q)] + slot[u]] = keys[u];
-    if (tid < 256) delta[tid] = base(tid) + g - ex;  // the claim's answer: only the write-out needs it
-    __syncthreads();
     bool bad = false;
-    for (uint32_t j = tid; j < cnt; j += THREADS) {  // coalesced runs, one per digit
-        const U k = stage[j];
-        const uint32_t pos = delta[digit_of(k, q)] + j;
-        if (pos < n) dst[pos] = k;
-        else bad = true;
+    if (!over) {
+        refill();
+        if (uint32_t(tid) < nb) {
+            if (uint64_t(g) + c > n) {
+                bad = true;
+                c = 0;
+            }
+            reinterpret_cast<uint2*>(runs)[tid] = make_uint2(g, c);
+        }
+        __syncthreads();
+        // A warp writes a digit's keys 32 at a time, four digits in flight.
+        // The digit's words reach the lanes by a broadcast read: shuffles
+        // take the same pipe, and two would be needed.
+        constexpr uint32_t WARPS = THREADS / 32, AHEAD = 4;
+        if (nb == 256u) {
+            constexpr int ROWS = (THREADS * IPT / 256 + 31) / 32;  // rows of a digit of average size
+            const U* from = stage + warp * CAP + lane;
+            const uint2* run = reinterpret_cast<const uint2*>(runs) + warp;
+#pragma unroll 1
+            for (uint32_t d0 = warp; d0 < 256u; d0 += AHEAD * WARPS) {
+                U k[AHEAD][ROWS];
+                uint2 w[AHEAD];
+                uint32_t most = 0;
+#pragma unroll
+                for (uint32_t e = 0; e < AHEAD; ++e) {
+                    w[e] = run[e * WARPS];
+                    most = max(most, w[e].y);
+#pragma unroll
+                    for (int h = 0; h < ROWS; ++h)
+                        if (lane + 32 * h < int(w[e].y)) k[e][h] = from[e * WARPS * CAP + 32 * h];
+                }
+#pragma unroll
+                for (uint32_t e = 0; e < AHEAD; ++e) {
+                    U* to = dst + (w[e].x + lane);
+#pragma unroll
+                    for (int h = 0; h < ROWS; ++h)
+                        if (lane + 32 * h < int(w[e].y)) to[32 * h] = k[e][h];
+                }
+                if (most > 32u * ROWS) {
+                    for (uint32_t e = 0; e < AHEAD; ++e) {
+                        const uint2 v = run[e * WARPS];
+                        for (uint32_t q = 32 * ROWS + lane; q < v.y; q += 32)
+                            dst[v.x + q] = from[e * WARPS * CAP + q - lane];
+                    }
+                }
+                from += AHEAD * WARPS * CAP;
+                run += AHEAD * WARPS;
+            }
+        } else {  // fewer digits: cut into parts, 256 in all
+            const uint32_t pl = 8u - (31u - __clz(nb));
+            for (uint32_t item = warp; item < 256u; item += WARPS) {
+                const uint32_t d = item >> pl, part = item & ((1u << pl) - 1u);
+                const uint2 w = reinterpret_cast<const uint2*>(runs)[d];
+                const U* from = stage + d * cap;
+#pragma unroll 2
+                for (uint32_t q = part * 32u + lane; q < w.y; q += 32u << pl) dst[w.x + q] = from[q];
+            }
+        }
+    } else {
+        __syncthreads();  // every zero of the bins is written
+        const uint32_t ex = block_exclusive_scan_256<uint32_t>(c, scan, nullptr);
+        if (uint32_t(tid) < nb) {
+            runs[tid] = ex;
+            runs[256 + tid] = g - ex;
+        }
+        reload();
+        __syncthreads();
+        each([&](int u) {
+            const U k = in(keys[u]);
+            const uint32_t d = digit(k);
+            stage[runs[d] + atomicAdd(&bins[d], 1u)] = k;
+        });
+        refill();
+        __syncthreads();
+        if (uint32_t(tid) < nb) bins[tid] = 0u;
+        const uint32_t cnt = hi - lo;
+        for (uint32_t j = tid; j < cnt; j += THREADS) {  // coalesced runs, one per digit
+            const U k = stage[j];
+            const uint32_t pos = runs[256 + digit(k)] + j;
+            if (pos < n) dst[pos] = k;
+            else bad = true;
+        }
     }
     if (bad) atomicOr(err, ERRBIT_BOUNDS);
     __syncthreads();  // the stage and the digit words are free for the next tile
 }
 
-template <int KB, int THREADS, int IPT, bool TWIDDLE, class Base>
-__device__ __forceinline__ void msd_split_tile(const typename KeyBits<KB>::U* src, uint32_t cnt, int q, int kind,
-                                               int desc, uint32_t* claim, Base base, typename KeyBits<KB>::U* dst,
-                                               uint64_t n, uint32_t* err, typename KeyBits<KB>::U* stage,
-                                               uint32_t* bins, uint32_t* delta, uint32_t* scan) {
-    typename KeyBits<KB>::U keys[IPT];
-    msd_load_tile<KB, THREADS, IPT, TWIDDLE>(src, cnt, kind, desc, keys);
-    msd_split_loaded<KB, THREADS, IPT>(keys, cnt, q, claim, base, dst, n, err, stage, bins, delta, scan);
+// Top split (8 bits), input -> alternate buffer.  Tiles start at 16-byte
+// boundaries; each CTA's next tile loads while it writes one out.
+template <int KB, int THREADS, int IPT, int MIN_CTAS, int CAP>
+__global__ void __launch_bounds__(THREADS, MIN_CTAS) msd_top_kernel(MsdParams p) {
+    using U = typename KeyBits<KB>::U;
+    using G = MsdSplitGeom<KB, THREADS, IPT, CAP>;
+    extern __shared__ __align__(128) uint8_t smem[];
+    uint32_t* bins = reinterpret_cast<uint32_t*>(smem + G::WORDS_OFF);
+    const int tid = threadIdx.x;
+    for (int i = tid; i < 256; i += THREADS) bins[i] = 0u;
+    grid_launch_dependents();
+    grid_dependency_wait();
+    if (ld_relaxed(p.state) & MSD_OFF) return;
+    const KeyMap<U> map(p.kind, p.desc);
+    const MsdCode code_of(p);
+    const U* keys_in = static_cast<const U*>(p.keys_in);
+    const uint32_t skew = uint32_t(reinterpret_cast<uintptr_t>(keys_in) & 15u) / uint32_t(KB);
+    const U* in = keys_in - skew;  // keys [skew, skew + n)
+    const uint32_t n = uint32_t(p.n), end = n + skew;
+    const uint32_t T = (end + G::TILE - 1) / G::TILE;
+    U keys[IPT];
+    auto load = [&](uint32_t t) {
+        if (t >= T) return;
+        const uint32_t b = t * uint32_t(G::TILE);
+        msd_load_tile<KB, THREADS, IPT>(in + b, b == 0u ? skew : 0u, min(end - b, uint32_t(G::TILE)), keys);
+    };
+    uint32_t t = blockIdx.x;
+    load(t);
+    __syncthreads();
+    for (; t < T; t += gridDim.x) {
+        const uint32_t b = t * uint32_t(G::TILE);
+        msd_split_tile<KB, THREADS, IPT, CAP>(
+            keys, b == 0u ? skew : 0u, min(end - b, uint32_t(G::TILE)), code_of, 24u, 256u, p.cursor1, static_cast<U*>(p.keys_b),
+            n, p.err, smem, [&](U k) { return map.in(k); }, [&] { load(t); }, [&] { load(t + gridDim.x); });
+    }
 }
 
-// Every top bucket's first key, size and first tile of the second level
-// (tiles of `tile` keys that never cross a bucket), from the upsweep's
-// counts; tfirst[256] = the number of tiles.
-__device__ __forceinline__ void msd_top_table(const unsigned long long* gp_top, uint32_t tile, uint32_t* tstart,
-                                              uint32_t* tcnt, uint32_t* tfirst, uint32_t* scan) {
+// The tiles of the second level: every top bucket's keys from the 16-byte
+// boundary at or below its first one, so that no tile crosses a bucket;
+// tfirst[256] = the number of tiles.
+__device__ __forceinline__ void msd_top_table(const uint32_t* top_counts, uint32_t tile, uint32_t vec, uint32_t skew,
+                                              uint32_t* tstart, uint32_t* tcnt, uint32_t* tfirst, uint32_t* scan) {
     const int tid = threadIdx.x;
-    const uint32_t c = (tid < 256) ? uint32_t(gp_top[tid]) : 0u;
+    const uint32_t c = (tid < 256) ? top_counts[tid] : 0u;
     const uint32_t ex = block_exclusive_scan_256<uint32_t>(c, scan, nullptr);
     __syncthreads();  // the scan words are read by every thread before the next scan writes them
     uint32_t tiles = 0;
-    const uint32_t tex = block_exclusive_scan_256<uint32_t>((c + tile - 1) / tile, scan, &tiles);
+    const uint32_t lead = (ex + skew) & (vec - 1u);
+    const uint32_t tex =
+        block_exclusive_scan_256<uint32_t>(c ? (lead + c + tile - 1) / tile : 0u, scan, &tiles);
     if (tid < 256) {
         tstart[tid] = ex;
         tcnt[tid] = c;
@@ -211,293 +605,400 @@ __device__ __forceinline__ uint32_t msd_bucket_of(const uint32_t* tfirst, uint32
     return lo;
 }
 
-template <int KB, int THREADS, int IPT>
-struct MsdSplitGeom {
-    static constexpr int TILE = THREADS * IPT;
-    static constexpr size_t STAGE_BYTES = size_t(TILE) * KB;
-    static constexpr size_t WORDS_OFF = STAGE_BYTES;  // u32 bins[256], delta[256], tstart, tcnt, tfirst[257], scan[32]
-    static constexpr size_t SMEM_BYTES = WORDS_OFF + (256 * 5 + 1 + 32 + 4) * 4;
-};
-
-// Top split.  A top bucket holding more than 256 groups' worth of keys must
-// leave some group too big for a local sort: then MSD_OFF at once.
-template <int KB, int THREADS, int IPT, int MIN_CTAS>
-__global__ void __launch_bounds__(THREADS, MIN_CTAS) msd_top_kernel(MsdParams p) {
-    using U = typename KeyBits<KB>::U;
-    using G = MsdSplitGeom<KB, THREADS, IPT>;
-    extern __shared__ __align__(128) uint8_t smem[];
-    U* stage = reinterpret_cast<U*>(smem);
-    uint32_t* bins = reinterpret_cast<uint32_t*>(smem + G::WORDS_OFF);
-    uint32_t* delta = bins + 256;
-    uint32_t* tstart = delta + 256;
-    uint32_t* scan = tstart + 256 * 3 + 1;
-    uint32_t* flag = scan + 32;
-    grid_launch_dependents();
-    grid_dependency_wait();
-    const int tid = threadIdx.x;
-    if (tid == 0) *flag = 0u;
-    const uint32_t c = (tid < 256) ? uint32_t(p.gp_top[tid]) : 0u;
-    const uint32_t ex = block_exclusive_scan_256<uint32_t>(c, scan, nullptr);
-    if (tid < 256) {
-        tstart[tid] = ex;
-        if (c > 256u * p.group_cap) atomicOr(flag, 1u);
-    }
-    __syncthreads();
-    if (*flag) {
-        if (blockIdx.x == 0 && tid == 0) *p.state = MSD_OFF;
-        return;
-    }
-    const U* in = static_cast<const U*>(p.keys_in);
-    U* out = static_cast<U*>(p.keys_b);
-    const uint64_t n = p.n;
-    const uint32_t T = uint32_t((n + G::TILE - 1) / G::TILE);
-    auto tile_cnt = [&](uint32_t t) {
-        const uint64_t base = uint64_t(t) * G::TILE;
-        return (t >= T) ? 0u : (n - base) < uint64_t(G::TILE) ? uint32_t(n - base) : uint32_t(G::TILE);
-    };
-    auto base = [&](int d) { return tstart[d]; };
-    if constexpr (KB == 8) {
-        // 8-byte keys: the CTA's next tile loads into a second register set
-        // while it splits this one (2^27 keys: 0.95 -> 0.68 ms; ncu had the
-        // split waiting on global loads, 10 long-scoreboard stalls per issue
-        // against 3 in the second split).  16-byte keys measured slower so
-        // (2^26: 0.36 -> 0.56 ms).
-        U keys[IPT];
-        uint32_t t = blockIdx.x;
-        msd_load_tile<KB, THREADS, IPT, true>(in + uint64_t(t) * G::TILE, tile_cnt(t), p.kind, p.desc, keys);
-        for (; t < T; t += gridDim.x) {
-            U next[IPT];
-            const uint32_t tn = t + gridDim.x;
-            msd_load_tile<KB, THREADS, IPT, true>(in + uint64_t(tn < T ? tn : t) * G::TILE, tile_cnt(tn), p.kind,
-                                                  p.desc, next);
-            msd_split_loaded<KB, THREADS, IPT>(keys, tile_cnt(t), KB - 1, p.cursor1, base, out, n, p.err, stage,
-                                               bins, delta, scan);
-#pragma unroll
-            for (int u = 0; u < IPT; ++u) keys[u] = next[u];
-        }
-    } else {
-        for (uint32_t t = blockIdx.x; t < T; t += gridDim.x)
-            msd_split_tile<KB, THREADS, IPT, true>(in + uint64_t(t) * G::TILE, tile_cnt(t), KB - 1, p.kind, p.desc,
-                                                   p.cursor1, base, out, n, p.err, stage, bins, delta, scan);
-    }
-}
-
-// Pair count: keys per (top, second) digit.  Its shared memory is the
-// words of the split's layout only (no stage).
-template <int KB, int THREADS, int IPT>
-struct MsdCountGeom {
-    static constexpr int TILE = THREADS * IPT;
-    static constexpr size_t WORDS_OFF = 0;
-    static constexpr size_t SMEM_BYTES = MsdSplitGeom<KB, THREADS, IPT>::SMEM_BYTES -
-                                         MsdSplitGeom<KB, THREADS, IPT>::WORDS_OFF;
-};
-template <int KB, int THREADS, int IPT, int MIN_CTAS>
-__global__ void __launch_bounds__(THREADS, MIN_CTAS) msd_count_kernel(MsdParams p) {
-    using U = typename KeyBits<KB>::U;
-    using G = MsdCountGeom<KB, THREADS, IPT>;
-    extern __shared__ __align__(128) uint8_t smem[];
-    uint32_t* bins = reinterpret_cast<uint32_t*>(smem + G::WORDS_OFF);
-    uint32_t* tstart = bins + 512;
-    uint32_t* tcnt = tstart + 256;
-    uint32_t* tfirst = tcnt + 256;
-    uint32_t* scan = tfirst + 257;
-    grid_launch_dependents();
-    grid_dependency_wait();
-    if (ld_relaxed(p.state) == MSD_OFF) return;
-    const int tid = threadIdx.x;
-    msd_top_table(p.gp_top, G::TILE, tstart, tcnt, tfirst, scan);
-    const U* keys = static_cast<const U*>(p.keys_b);
-    const uint32_t T = tfirst[256];
-    for (uint32_t t = blockIdx.x; t < T; t += gridDim.x) {
-        const uint32_t b = msd_bucket_of(tfirst, t);
-        const uint32_t off = tstart[b] + (t - tfirst[b]) * G::TILE;
-        const uint32_t end = tstart[b] + tcnt[b];
-        const uint32_t cnt = (end - off) < uint32_t(G::TILE) ? end - off : uint32_t(G::TILE);
-        U k[IPT];
-#pragma unroll
-        for (int u = 0; u < IPT; ++u) {
-            const uint32_t j = uint32_t(u * THREADS + tid);
-            k[u] = (j < cnt) ? keys[off + j] : U(0);
-        }
-        if (tid < 256) bins[tid] = 0u;
-        __syncthreads();
-#pragma unroll
-        for (int u = 0; u < IPT; ++u)
-            if (uint32_t(u * THREADS + tid) < cnt) atomicAdd(&bins[digit_of(k[u], KB - 2)], 1u);
-        __syncthreads();
-        if (tid < 256 && bins[tid]) atomicAdd(p.joint + b * 256 + tid, bins[tid]);
-        __syncthreads();
-    }
-}
-
-// Scan of the 65536 group sizes (one CTA of 1024 threads, 64 groups each)
-// and the decision.
-constexpr int MSD_SCAN_THREADS = 1024;
-template <int KB>  // (one instance per key width's translation unit)
-__global__ void __launch_bounds__(MSD_SCAN_THREADS, 1) msd_scan_kernel(MsdParams p) {
-    __shared__ uint32_t scan[32];
-    __shared__ uint32_t biggest;
-    grid_launch_dependents();
-    grid_dependency_wait();
-    if (ld_relaxed(p.state) == MSD_OFF) return;
-    const int tid = threadIdx.x;
-    if (tid == 0) biggest = 0u;
-    constexpr int PER = 65536 / MSD_SCAN_THREADS;
-    const uint4* src = reinterpret_cast<const uint4*>(p.joint) + tid * (PER / 4);
-    uint32_t c[PER];
-#pragma unroll
-    for (int i = 0; i < PER / 4; ++i) {
-        const uint4 v = src[i];
-        c[4 * i] = v.x;
-        c[4 * i + 1] = v.y;
-        c[4 * i + 2] = v.z;
-        c[4 * i + 3] = v.w;
-    }
-    uint32_t sum = 0, big = 0;
-#pragma unroll
-    for (int i = 0; i < PER; ++i) {
-        sum += c[i];
-        big = max(big, c[i]);
-    }
-    uint32_t run = block_exclusive_scan_all<MSD_SCAN_THREADS>(sum, scan);
-    big = __reduce_max_sync(0xffffffffu, big);
-    if ((tid & 31) == 0) atomicMax(&biggest, big);
-    uint4* dst = reinterpret_cast<uint4*>(p.offs2) + tid * (PER / 4);
-#pragma unroll
-    for (int i = 0; i < PER / 4; ++i) {
-        uint4 v;
-        v.x = run;
-        run += c[4 * i];
-        v.y = run;
-        run += c[4 * i + 1];
-        v.z = run;
-        run += c[4 * i + 2];
-        v.w = run;
-        run += c[4 * i + 3];
-        dst[i] = v;
-    }
-    __syncthreads();
-    if (tid == 0) *p.state = (biggest <= p.group_cap) ? MSD_OK : MSD_OFF;
-}
-
-// Second split: within every top bucket, into the groups' ranges.
-template <int KB, int THREADS, int IPT, int MIN_CTAS>
+// Second split: within every top bucket, into the groups' ranges (alternate
+// buffer -> caller's buffer).
+template <int KB, int THREADS, int IPT, int MIN_CTAS, int CAP>
 __global__ void __launch_bounds__(THREADS, MIN_CTAS) msd_second_kernel(MsdParams p) {
     using U = typename KeyBits<KB>::U;
-    using G = MsdSplitGeom<KB, THREADS, IPT>;
+    using G = MsdSplitGeom<KB, THREADS, IPT, CAP>;
+    constexpr uint32_t VEC = 16 / KB;
     extern __shared__ __align__(128) uint8_t smem[];
-    U* stage = reinterpret_cast<U*>(smem);
     uint32_t* bins = reinterpret_cast<uint32_t*>(smem + G::WORDS_OFF);
-    uint32_t* delta = bins + 256;
-    uint32_t* tstart = delta + 256;
+    uint32_t* tstart = bins + 256 * 3;
     uint32_t* tcnt = tstart + 256;
     uint32_t* tfirst = tcnt + 256;
     uint32_t* scan = tfirst + 257;
+    const int tid = threadIdx.x;
+    for (int i = tid; i < 256; i += THREADS) bins[i] = 0u;
     grid_launch_dependents();
     grid_dependency_wait();
-    if (ld_relaxed(p.state) != MSD_OK) return;
-    msd_top_table(p.gp_top, G::TILE, tstart, tcnt, tfirst, scan);
+    if (ld_relaxed(p.state) & MSD_OFF) return;
+    const MsdCode code_of(p);
+    const uint32_t b2 = code_of.b2;
     const U* in = static_cast<const U*>(p.keys_b);
-    U* out = static_cast<U*>(p.keys_a);
+    const uint32_t skew = uint32_t(reinterpret_cast<uintptr_t>(in) & 15u) / uint32_t(KB);
+    msd_top_table(p.top_counts, G::TILE, VEC, skew, tstart, tcnt, tfirst, scan);
     const uint32_t T = tfirst[256];
-    for (uint32_t t = blockIdx.x; t < T; t += gridDim.x) {
-        const uint32_t b = msd_bucket_of(tfirst, t);
-        const uint32_t off = tstart[b] + (t - tfirst[b]) * G::TILE;
-        const uint32_t end = tstart[b] + tcnt[b];
-        const uint32_t cnt = (end - off) < uint32_t(G::TILE) ? end - off : uint32_t(G::TILE);
-        const uint32_t* group_base = p.offs2 + b * 256;
-        msd_split_tile<KB, THREADS, IPT, false>(in + off, cnt, KB - 2, p.kind, p.desc, p.cursor2 + b * 256,
-                                                [&](int d) { return group_base[d]; }, out, p.n, p.err, stage, bins,
-                                                delta, scan);
+    struct Tile {
+        uint32_t b, lo, hi;
+        const U* at;
+    };
+    auto tile = [&](uint32_t t) {
+        Tile r;
+        r.b = msd_bucket_of(tfirst, t);
+        const uint32_t lead = (tstart[r.b] + skew) & (VEC - 1u);
+        const uint32_t from = (t - tfirst[r.b]) * uint32_t(G::TILE);  // from the aligned start
+        r.at = in + tstart[r.b] - lead + from;
+        r.lo = from == 0u ? lead : 0u;
+        r.hi = min(lead + tcnt[r.b] - from, uint32_t(G::TILE));
+        return r;
+    };
+    U keys[IPT];
+    uint32_t t = blockIdx.x;
+    if (t >= T) return;
+    Tile cur = tile(t);
+    msd_load_tile<KB, THREADS, IPT>(cur.at, cur.lo, cur.hi, keys);
+    for (; t < T; t += gridDim.x) {
+        Tile next = cur;
+        msd_split_tile<KB, THREADS, IPT, CAP>(
+            keys, cur.lo, cur.hi, code_of, 24u - b2, 1u << b2, p.cursor2 + (cur.b << b2), static_cast<U*>(p.keys_a),
+            uint32_t(p.n), p.err, smem, [](U k) { return k; },
+            [&] { msd_load_tile<KB, THREADS, IPT>(cur.at, cur.lo, cur.hi, keys); },
+            [&] {
+                if (t + gridDim.x < T) {
+                    next = tile(t + gridDim.x);
+                    msd_load_tile<KB, THREADS, IPT>(next.at, next.lo, next.hi, keys);
+                }
+            });
+        cur = next;
     }
 }
 
-template <int KB, int THREADS, int LIPT>
-struct MsdLocalGeom {
+// ---- local sorts ----------------------------------------------------------
+// Largest sub-bucket ranked by comparison where the network's margin is too
+// narrow (below); a larger one sends the whole sort to the digit passes.
+constexpr uint32_t MSD_RANK_MAX = 32;
+
+// Shared memory of a local sort by BINS = 16 * THREADS sub-buckets.  Keys lie
+// in chunks of 64 bytes (LIPT keys, a lane's share), 80 bytes apart: sixteen
+// bytes of padding put the chunks of eight lanes on all 32 banks.
+// HALO lanes at either end of a warp hold its neighbours' keys: after m
+// rounds of the network a key has met every key at most m places away, so a
+// warp's inner lanes end up right when m <= HALO * LIPT.
+template <int KB, int THREADS, int HALO>
+struct GroupSortGeom {
+    static constexpr int LIPT = 64 / KB;
     static constexpr int WARPS = THREADS / 32;
-    static constexpr int CTR_WORDS = 2 * WARPS * 256;  // the split's sub-buckets
-    static constexpr size_t BUF_BYTES = (size_t(THREADS) * LIPT * KB + 127) & ~size_t(127);
-    static constexpr size_t CTR_OFF = BUF_BYTES;
-    static constexpr size_t SCAN_OFF = CTR_OFF + size_t(CTR_WORDS) * 4;  // u32 [32]
+    static constexpr int BINS = 16 * THREADS;
+    static constexpr int OUT = (32 - 2 * HALO) * LIPT;  // keys a warp puts in order
+    static constexpr int PLACES = WARPS * OUT;
+    static constexpr int ALIGN = 32 / KB;               // places keep the keys' position in their 32-byte sector
+    static constexpr int CAP = PLACES - ALIGN;
+    static_assert(PLACES < 65536, "16-bit places");
+    static constexpr size_t KEYS_BYTES = size_t(PLACES / LIPT) * 80;
+    static constexpr size_t CTR_OFF = (KEYS_BYTES + 127) & ~size_t(127);  // u8 [BINS]
+    static constexpr size_t START_OFF = CTR_OFF + BINS;                   // u16 [BINS]
+    static constexpr size_t SCAN_OFF = START_OFF + size_t(BINS) * 2;      // u32 [32]
     static constexpr size_t MISC_OFF = SCAN_OFF + 128;                    // u32 [4]
     static constexpr size_t SMEM_BYTES = MISC_OFF + 16;
+    // byte address of a place
+    __device__ __forceinline__ static uint32_t at(uint32_t place) {
+        return place * uint32_t(KB) + (place & ~uint32_t(LIPT - 1)) * uint32_t(16 / LIPT);
+    }
 };
 
-// 1: each CTA pulls its next group into L2 while it sorts the current one
-// (2^26 u128 local sorts 0.795 -> 0.779 ms, 2^27 u64 1.048 -> 1.040).
-#ifndef GBSORT_MSD_LOCAL_L2
-#define GBSORT_MSD_LOCAL_L2 1
-#endif
+__device__ __forceinline__ void order_pair(uint32_t& a, uint32_t& b) {
+    const uint32_t lo = min(a, b), hi = max(a, b);
+    a = lo;
+    b = hi;
+}
+template <class U>
+__device__ __forceinline__ void order_pair(U& a, U& b) {
+    const bool sw = b < a;
+    const U lo = sw ? b : a, hi = sw ? a : b;
+    a = lo;
+    b = hi;
+}
+template <class U>
+__device__ __forceinline__ U shfl_up1(U v) {
+    if constexpr (sizeof(U) <= 8) return __shfl_up_sync(0xffffffffu, v, 1);
+    else {
+        const uint64_t lo = __shfl_up_sync(0xffffffffu, uint64_t(v), 1);
+        const uint64_t hi = __shfl_up_sync(0xffffffffu, uint64_t(v >> 64), 1);
+        return (U(hi) << 64) | U(lo);
+    }
+}
+template <class U>
+__device__ __forceinline__ U shfl_down1(U v) {
+    if constexpr (sizeof(U) <= 8) return __shfl_down_sync(0xffffffffu, v, 1);
+    else {
+        const uint64_t lo = __shfl_down_sync(0xffffffffu, uint64_t(v), 1);
+        const uint64_t hi = __shfl_down_sync(0xffffffffu, uint64_t(v >> 64), 1);
+        return (U(hi) << 64) | U(lo);
+    }
+}
 
-// Local sorts: each group (keys sharing their top two digits) sorted in
-// place; the split counts over SPLIT_WORDS sub-buckets (about twice the mean
-// group: fewer scan words per key, a comparison or two per key).
-template <int KB, int THREADS, int LIPT, int MIN_CTAS, int SPLIT_WORDS>
-__global__ void __launch_bounds__(THREADS, MIN_CTAS) msd_local_kernel(MsdParams p) {
-    using U = typename KeyBits<KB>::U;
-    using G = MsdLocalGeom<KB, THREADS, LIPT>;
-    extern __shared__ __align__(128) uint8_t smem[];
+// `rounds` rounds of odd-even transposition over the warp's 32 * LIPT keys,
+// LIPT consecutive ones per lane.
+template <class U, int LIPT>
+__device__ __forceinline__ void transposition_rounds(U (&k)[LIPT], uint32_t rounds, int lane) {
+    for (uint32_t r = 0; r < rounds; r += 2) {
+#pragma unroll
+        for (int i = 0; i + 1 < LIPT; i += 2) order_pair(k[i], k[i + 1]);
+        if (r + 1 < rounds) {
+            const U before = shfl_up1(k[LIPT - 1]), after = shfl_down1(k[0]);
+#pragma unroll
+            for (int i = 1; i + 1 < LIPT; i += 2) order_pair(k[i], k[i + 1]);
+            if (lane > 0 && before > k[0]) k[0] = before;
+            if (lane < 31 && after < k[LIPT - 1]) k[LIPT - 1] = after;
+        }
+    }
+}
+
+// Exclusive scan over the CTA with one barrier: every warp scans the warp
+// totals for itself (warp_tmp is written again only after another barrier).
+template <int THREADS>
+__device__ __forceinline__ uint32_t block_exclusive_scan_1b(uint32_t x, uint32_t* warp_tmp) {
+    constexpr int WARPS = THREADS / 32;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t v = x;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v += y;
+    }
+    if (lane == 31) warp_tmp[warp] = v;
+    __syncthreads();
+    const uint32_t before = __reduce_add_sync(0xffffffffu, lane < warp && lane < WARPS ? warp_tmp[lane] : 0u);
+    return before + v - x;
+}
+
+// Sorts the CTA's `cnt` keys, all of one group: key VEC * i + e of a thread
+// (VEC = 16 bytes' worth) is the group's key (i * THREADS + tid) * VEC + e -
+// skew when that is below cnt, else nothing.  bin(key) names its sub-bucket (monotone in the key, 0 ..
+// BINS-1).  Place p of the sorted group (p < cnt) is reported as pad + p, pad
+// < ALIGN: chunk(c0, k) hands out the LIPT keys of places c0 .. (those of
+// [pad, pad + cnt) count), one(place, key) a single key.  refill() runs when
+// the keys' registers are free.  Returns false, having called none of these,
+// when a sub-bucket is too big.
+// The counters of the sub-buckets are bytes, four to a word: one 16-byte read
+// per thread scans sixteen; a count that passes 255 loses at least 255 keys
+// from the total, which shows.  They are zero on entry and left so.
+// What bounds it: a random shared-memory access costs about 2.5 SM clocks a
+// warp; a key needs three (the counter's atomic, whose answer is its slot,
+// its sub-bucket's start, its place), and one conflict-free read.
+template <class U, int THREADS, int HALO, class Bin, class Refill, class Chunk, class One>
+__device__ __forceinline__ bool group_sort(const U (&keys)[64 / sizeof(U)], uint32_t cnt, uint32_t skew,
+                                           uint32_t pad, uint8_t* smem, Bin bin, Refill refill, Chunk chunk, One one) {
+    using G = GroupSortGeom<int(sizeof(U)), THREADS, HALO>;
+    constexpr int LIPT = G::LIPT;
+    constexpr int VEC = 16 / int(sizeof(U));
+    auto sk = [&](uint32_t place) -> U& { return *reinterpret_cast<U*>(smem + G::at(place)); };
     uint32_t* ctr = reinterpret_cast<uint32_t*>(smem + G::CTR_OFF);
+    uint16_t* start = reinterpret_cast<uint16_t*>(smem + G::START_OFF);
     uint32_t* scan = reinterpret_cast<uint32_t*>(smem + G::SCAN_OFF);
     uint32_t* misc = reinterpret_cast<uint32_t*>(smem + G::MISC_OFF);
-    grid_launch_dependents();
-    grid_dependency_wait();
-    if (ld_relaxed(p.state) != MSD_OK) return;
-    const int tid = threadIdx.x;
-    for (int i = tid; i < G::CTR_WORDS; i += THREADS) ctr[i] = 0u;
-    __syncthreads();
-    // Groups blockIdx.x, + gridDim.x, ...: the next group's size and place
-    // load one group ahead.  (Its keys too, into a second register set or
-    // into this one once the current keys sit in shared memory, measured
-    // slower: 16-byte keys 2^26 2.32 vs 2.15 ms, the extra live registers
-    // spill.)
-    U* keys = static_cast<U*>(p.keys_a);
-    U k[LIPT];
-    auto load = [&](uint32_t cnt, uint32_t off) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    uint32_t slot[(LIPT + 3) / 4];
 #pragma unroll
-        for (int u = 0; u < LIPT; ++u) {
-            const uint32_t j = uint32_t(u * THREADS + tid);
-            k[u] = (j < cnt) ? keys[off + j] : U(0);
+    for (int u = 0; u < (LIPT + 3) / 4; ++u) slot[u] = 0u;
+    // rows of VEC keys; a warp whose row lies past the group skips it
+    auto rows = [&](auto f) {
+#pragma unroll
+        for (int i = 0; i < LIPT / VEC; ++i) {
+            if (uint32_t(i * THREADS + warp * 32) * VEC >= skew + cnt) break;
+            if (i != 0 || skew == 0u || warp != 0)  // (a warp of whole vectors: no test per key)
+                if (uint32_t(i * THREADS + warp * 32 + 32) * VEC <= skew + cnt) {
+#pragma unroll
+                    for (int e = 0; e < VEC; ++e) f(i * VEC + e);
+                    continue;
+                }
+            const uint32_t j = uint32_t(i * THREADS + tid) * VEC - skew;
+#pragma unroll
+            for (int e = 0; e < VEC; ++e)
+                if (j + e < cnt) f(i * VEC + e);
         }
     };
-    uint32_t g = blockIdx.x;
-    uint32_t c = (g < 65536u) ? p.joint[g] : 0u, o = (g < 65536u) ? p.offs2[g] : 0u;
-    load(c, o);
-    while (g < 65536u) {
-        const uint32_t gn = g + gridDim.x;
-        const uint32_t cn = (gn < 65536u) ? p.joint[gn] : 0u, on = (gn < 65536u) ? p.offs2[gn] : 0u;
-#if GBSORT_MSD_LOCAL_L2
-        {  // the next group into L2 while this one sorts
-            const uintptr_t a = reinterpret_cast<uintptr_t>(keys + on) & ~uintptr_t(127);
-            const uintptr_t e = reinterpret_cast<uintptr_t>(keys + on + cn);
+    rows([&](int u) {
+        const uint32_t b = bin(keys[u]);
+        const uint32_t old = atomicAdd(reinterpret_cast<uint32_t*>(reinterpret_cast<uint8_t*>(ctr) + (b & ~3u)),
+                                       __funnelshift_l(1u, 1u, b * 8u));
+        // byte (b & 3) of old into byte (u & 3) of the slots
+        const uint32_t x = __funnelshift_r(old, old, b * 8u);
+        slot[u >> 2] = __byte_perm(slot[u >> 2], x, (u & 3) == 0 ? 0x3214 : (u & 3) == 1 ? 0x3240 : (u & 3) == 2 ? 0x3410 : 0x4210);
+    });
+    __syncthreads();
+    // scan: sixteen consecutive counters a thread
+    {
+        const uint4 c = reinterpret_cast<const uint4*>(ctr)[tid];
+        uint32_t big = __vmaxu4(__vmaxu4(c.x, c.y), __vmaxu4(c.z, c.w));
+        big = max(max(big & 0xffu, (big >> 8) & 0xffu), max((big >> 16) & 0xffu, big >> 24));
+        const uint32_t sum = __dp4a(c.x, 0x01010101u, __dp4a(c.y, 0x01010101u, __dp4a(c.z, 0x01010101u, __dp4a(c.w, 0x01010101u, 0u))));
+        big = __reduce_max_sync(0xffffffffu, big);
+        if (lane == 0 && big > 1u) atomicMax(&misc[0], big);
+        uint32_t run = block_exclusive_scan_1b<THREADS>(sum, scan);
+        if (tid == THREADS - 1 && run + sum != cnt) atomicMax(&misc[0], 256u);
+        run += pad;
+        auto pack = [&](uint32_t w, uint32_t& lo, uint32_t& hi) {
+            const uint32_t b = run + (w & 0xffu), d = b + ((w >> 8) & 0xffu), e = d + ((w >> 16) & 0xffu);
+            lo = run | b << 16;
+            hi = d | e << 16;
+            run = e + (w >> 24);
+        };
+        uint4 v0, v1;
+        pack(c.x, v0.x, v0.y);
+        pack(c.y, v0.z, v0.w);
+        pack(c.z, v1.x, v1.y);
+        pack(c.w, v1.z, v1.w);
+        reinterpret_cast<uint4*>(start)[tid * 2] = v0;
+        reinterpret_cast<uint4*>(start)[tid * 2 + 1] = v1;
+        reinterpret_cast<uint4*>(ctr)[tid] = make_uint4(0u, 0u, 0u, 0u);
+    }
+    __syncthreads();
+    const uint32_t most = misc[0];
+    if (most > MSD_RANK_MAX) {
+        __syncthreads();
+        if (tid == 0) misc[0] = 0u;
+        return false;
+    }
+    rows([&](int u) { sk(start[bin(keys[u])] + __byte_perm(slot[u >> 2], 0u, 0x4440u | (u & 3))) = keys[u]; });
+    __syncthreads();
+    if (tid == 0) misc[0] = 0u;  // read by every thread before the barrier
+    refill();
+    const uint32_t end = pad + cnt;
+    if (most <= uint32_t(HALO * LIPT)) {
+        // chunks [warp * (32 - 2 HALO), ...) and the neighbours' beyond both ends
+        const int ch = warp * (32 - 2 * HALO) + lane - HALO;
+        const int c0 = ch * LIPT;
+        if (warp * G::OUT < int(end)) {
+            U k[LIPT];
+            const bool inside = c0 >= int(pad) && uint32_t(c0 + LIPT) <= end;
+            if (c0 + LIPT <= int(pad) || c0 >= int(end)) {
+#pragma unroll
+                for (int i = 0; i < LIPT; ++i) k[i] = c0 < int(pad) ? U(0) : U(~U(0));
+            } else {
+                const uint4* q = reinterpret_cast<const uint4*>(smem + uint32_t(ch) * 80u);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    union { uint4 v; U k[16 / sizeof(U)]; } w;
+                    w.v = q[i];
+#pragma unroll
+                    for (int e = 0; e < int(16 / sizeof(U)); ++e) k[i * (16 / sizeof(U)) + e] = w.k[e];
+                }
+                if (!inside) {
+#pragma unroll
+                    for (int i = 0; i < LIPT; ++i) {
+                        if (c0 + i < int(pad)) k[i] = U(0);
+                        if (c0 + i >= int(end)) k[i] = U(~U(0));
+                    }
+                }
+            }
+            if (most > 1u) transposition_rounds<U, LIPT>(k, most, lane);
+            if (lane >= HALO && lane < 32 - HALO && c0 < int(end)) chunk(uint32_t(c0), inside, k);
+        }
+    } else {
+        // a key's place is its sub-bucket's start plus the sub-bucket's other
+        // keys below it
+        for (uint32_t i = pad + tid; i < end; i += THREADS) {
+            const U k = sk(i);
+            const uint32_t b = bin(k);
+            const uint32_t s = start[b], e = b + 1 < uint32_t(G::BINS) ? uint32_t(start[b + 1]) : end;
+            uint32_t below = 0;
+            for (uint32_t q = s; q < e; ++q) {
+                const U o = sk(q);
+                below += uint32_t(o < k || (o == k && q < i));
+            }
+            one(s + below, k);
+        }
+    }
+    return true;
+}
+
+// 32 bytes to a 32-byte aligned address.
+__device__ __forceinline__ void store_32b(void* dst, const uint4& a, const uint4& b) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "r"(a.x), "r"(a.y), "r"(a.z),
+                 "r"(a.w), "r"(b.x), "r"(b.y), "r"(b.z), "r"(b.w)
+                 : "memory");
+}
+
+// Local sorts: groups blockIdx.x, + gridDim.x, ... sorted in place.  The next
+// group's keys load while the network runs, and the one after it is pulled
+// into L2.
+template <int KB, int THREADS, int MIN_CTAS, int HALO>
+__global__ void __launch_bounds__(THREADS, MIN_CTAS) msd_local_kernel(MsdParams p) {
+    using U = typename KeyBits<KB>::U;
+    using G = GroupSortGeom<KB, THREADS, HALO>;
+    constexpr int LIPT = G::LIPT, VEC = 16 / KB;
+    extern __shared__ __align__(128) uint8_t smem[];
+    grid_launch_dependents();
+    const int tid = threadIdx.x;
+    for (int i = tid; i < G::BINS / 4; i += THREADS) reinterpret_cast<uint32_t*>(smem + G::CTR_OFF)[i] = 0u;
+    if (tid == 0) *reinterpret_cast<uint32_t*>(smem + G::MISC_OFF) = 0u;
+    grid_dependency_wait();
+    if (ld_relaxed(p.state) & MSD_OFF) return;
+    __syncthreads();
+    U* keys = static_cast<U*>(p.keys_a);
+    const MsdCode code_of(p);
+    const uint32_t groups = 256u << code_of.b2;
+    auto bounds = [&](uint32_t g, uint32_t& off, uint32_t& cnt) {
+        off = (g != 0u && g < groups) ? p.cursor2[g - 1] : 0u;
+        cnt = g < groups ? p.cursor2[g] - off : 0u;
+    };
+    // Key VEC * i + e of a thread is the group's key
+    // (i * THREADS + tid) * VEC + e - shift: 16-byte loads from the address
+    // at or below the group's start (which keys a thread has does not matter)
+    const KeyMap<U> map(p.kind, p.desc);
+    uint32_t g = blockIdx.x, off, cnt, off1, cnt1;
+    bounds(g, off, cnt);
+    bounds(g + gridDim.x, off1, cnt1);
+    U k[LIPT];
+    auto skew_of = [&](uint32_t o, uint32_t bytes) {
+        return uint32_t(reinterpret_cast<uintptr_t>(keys + o) & (bytes - 1u)) / uint32_t(KB);
+    };
+    auto index = [&](uint32_t skew, int u) { return (uint32_t(u / VEC) * THREADS + tid) * VEC + uint32_t(u % VEC) - skew; };
+    auto load = [&](uint32_t o, uint32_t c) {
+        const uint32_t skew = skew_of(o, 16);
+        load_vectors<THREADS>(const_cast<const U*>(keys) + o - skew, skew, skew + c, k);
+    };
+    load(off, cnt);
+    while (g < groups) {
+        uint32_t off2, cnt2;
+        bounds(g + 2 * gridDim.x, off2, cnt2);
+        {
+            const uintptr_t a = reinterpret_cast<uintptr_t>(keys + off2) & ~uintptr_t(127);
+            const uintptr_t e = reinterpret_cast<uintptr_t>(keys + off2 + cnt2);
             for (uintptr_t q = a + uintptr_t(tid) * 128; q < e; q += uintptr_t(THREADS) * 128)
                 asm volatile("prefetch.global.L2 [%0];" ::"l"(q));
         }
-#endif
-        if (c != 0u) {
-            U* at = keys + o;
-            static_assert(SPLIT_WORDS <= G::CTR_WORDS, "the split's counters");
-            const bool split =
-                cta_bucket_split<KB, THREADS, LIPT, SPLIT_WORDS, 8 * (KB - 2)>(k, at, c, smem, ctr, scan, misc, p.kind,
-                                                                              p.desc);
-            if (!split) {
-                // a sub-bucket too big for the comparison rank (repeated
-                // keys): the group goes back untwiddled, like every group
-                // sorted here, so the buffer holds the input's keys in some
-                // order, and the digit passes sort it (keys only: any order
-                // of the input sorts to the same bytes)
+        const uint32_t skew = skew_of(off, 16), pad = skew_of(off, 32);
+        U* dst = keys + off - pad;  // place q goes to dst[q]
+        bool sorted = true;
+        if (cnt != 0u)
+            sorted = group_sort<U, THREADS, HALO>(
+                k, cnt, skew, pad, smem,
+                [&](U x) { return __umulhi(code_of(x) << (8u + code_of.b2), uint32_t(G::BINS)); },
+                [&] { load(off1, cnt1); },
+                [&](uint32_t c0, bool inside, const U(&x)[LIPT]) {
+                    union { uint4 q[4]; U k[LIPT]; } w;
 #pragma unroll
-                for (int u = 0; u < LIPT; ++u) {
-                    const uint32_t j = uint32_t(u * THREADS + tid);
-                    if (j < c) at[j] = twiddle_out<U>(k[u], p.kind, p.desc);
-                }
-                if (tid == 0) *p.state = MSD_OFF;
-            }
+                    for (int i = 0; i < LIPT; ++i) w.k[i] = map.out(x[i]);
+                    if (inside) {
+                        store_32b(dst + c0, w.q[0], w.q[1]);
+                        store_32b(dst + c0 + LIPT / 2, w.q[2], w.q[3]);
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < LIPT; ++i)
+                            if (c0 + i >= pad && c0 + i < pad + cnt) dst[c0 + i] = w.k[i];
+                    }
+                },
+                [&](uint32_t place, U x) { dst[place] = map.out(x); });
+        if (!sorted) {
+            // repeated keys, or keys that share the sub-bucket's bits: the
+            // group goes back untwiddled, like every group sorted here, so
+            // the buffer holds the input's keys in some order, and the digit
+            // passes sort it (keys only: any order of the input sorts to the
+            // same bytes)
+#pragma unroll
+            for (int u = 0; u < LIPT; ++u)
+                if (index(skew, u) < cnt) keys[off + index(skew, u)] = map.out(k[u]);
+            if (tid == 0) atomicOr(p.state, MSD_GAVE_UP);
         }
-        load(cn, on);
-        g = gn;
-        c = cn;
-        o = on;
+        if (!sorted || cnt == 0u) load(off1, cnt1);
+        g += gridDim.x;
+        off = off1;
+        cnt = cnt1;
+        off1 = off2;
+        cnt1 = cnt2;
     }
 }
 

@@ -22,8 +22,6 @@
 //     upsweep) serves every pass; all waits are bounded by %globaltimer.
 #pragma once
 
-#include <type_traits>
-
 #include "device_common.cuh"
 #include "shapes.h"
 #include "sort_params.h"
@@ -73,9 +71,8 @@ __global__ void __launch_bounds__(HIST_THREADS, 1) upsweep_kernel(HistParams p) 
     grid_launch_dependents();  // the first pass may be scheduled; it waits for this grid
     if (p.msd_state) {  // the digit passes' histogram after the MSD kernels
         grid_dependency_wait();
-        if (ld_relaxed(p.msd_state) == MSD_OK) return;
+        if (ld_relaxed(p.msd_state) == 0u) return;
     }
-    const int dlo = p.digit_lo, dhi = p.digit_hi ? p.digit_hi : G::P;
 
     // Fused clears / copies that must precede the first pass.
     {
@@ -89,15 +86,11 @@ __global__ void __launch_bounds__(HIST_THREADS, 1) upsweep_kernel(HistParams p) 
     __syncthreads();
 
     const int kind = p.kind, desc = p.desc;
-    // every digit (the usual case, fully unrolled) or the digits in
-    // [dlo, dhi): the loop is compiled once for each
-    auto sweep = [&](auto all_digits) {
-        constexpr bool ALL = decltype(all_digits)::value;
+    {
         auto count = [&](U k) {
             const U t = twiddle_in<U>(k, kind, desc);
 #pragma unroll
-            for (int d = 0; d < G::P; ++d)
-                if (ALL || (d >= dlo && d < dhi)) atomicAdd(&cnt[(d * 256 + digit_of(t, d)) * G::COPIES + copy], 1u);
+            for (int d = 0; d < G::P; ++d) atomicAdd(&cnt[(d * 256 + digit_of(t, d)) * G::COPIES + copy], 1u);
         };
         const U* keys = static_cast<const U*>(p.keys);
         const uint64_t n = p.n;
@@ -111,7 +104,7 @@ __global__ void __launch_bounds__(HIST_THREADS, 1) upsweep_kernel(HistParams p) 
 
         if (gtid < head) count(keys[gtid]);
         const uint4* vec = reinterpret_cast<const uint4*>(keys + head);
-        constexpr int UNROLL = 4;  // (8 for the top digit alone: u64 2^27 0.19 -> 0.28 ms)
+        constexpr int UNROLL = 4;
         uint64_t i = gtid;
         for (; i + (UNROLL - 1) * gthreads < nvec; i += UNROLL * gthreads) {
             uint4 v[UNROLL];
@@ -132,13 +125,11 @@ __global__ void __launch_bounds__(HIST_THREADS, 1) upsweep_kernel(HistParams p) 
             for (int e = 0; e < PER_VEC; ++e) count(w.k[e]);
         }
         for (uint64_t j = head + nvec * PER_VEC + gtid; j < n; j += gthreads) count(keys[j]);
-    };
-    if (dlo == 0 && dhi == G::P) sweep(std::true_type{});
-    else sweep(std::false_type{});
+    }
     __syncthreads();
 
     // Reduce the copies: one warp per bin, conflict-free row read.
-    for (int bin = dlo * 256 + warp; bin < dhi * 256; bin += HIST_THREADS / 32) {
+    for (int bin = warp; bin < G::NBINS; bin += HIST_THREADS / 32) {
         uint32_t s = (lane < G::COPIES) ? cnt[bin * G::COPIES + lane] : 0u;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
@@ -235,7 +226,7 @@ __device__ __forceinline__ void onesweep_pass_body(const PassParams& p, uint8_t*
     // successor never holds slots a CTA of this pass still needs.
     grid_launch_dependents();
     grid_dependency_wait();
-    if (p.msd_state && ld_relaxed(p.msd_state) == MSD_OK) return;  // the MSD kernels sorted
+    if (p.msd_state && ld_relaxed(p.msd_state) == 0u) return;  // the MSD kernels sorted
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     // Tile position of item u of this thread: warp-striped (a warp's 32 lanes
@@ -738,7 +729,7 @@ __device__ __forceinline__ void grid_copy_bytes(void* dst, const void* src, uint
 // in the other buffer than the one it belongs in (in place: an odd count
 // left it in the alternate buffer); copy it across.  Otherwise nothing to do.
 __device__ __forceinline__ void fixup_body(const FixupParams& f) {
-    if (f.msd_state && ld_relaxed(f.msd_state) == MSD_OK) return;  // the MSD kernels sorted
+    if (f.msd_state && ld_relaxed(f.msd_state) == 0u) return;  // the MSD kernels sorted
     // the executed pass kernels left their count; none ran when the word is 0
     const uint32_t w = *f.executed;
     const int executed = (w >> 31) ? int(w & 0xFFu) : 0;

@@ -27,6 +27,7 @@ struct CtlLayout {
     size_t barrier_gen_off = 0;  // its generation word (another 128-byte line)
     size_t fill_off = 0;         // [256] fill counts of its MSD regions
     size_t overflow_off = 0;     // its region overflow flag
+    size_t msd_state_off = 0;    // outcome of the most-significant-first path, its code window [2]
     size_t bytes = 0;
     static CtlLayout make(int passes) {
         CtlLayout c;
@@ -38,21 +39,23 @@ struct CtlLayout {
         c.barrier_gen_off = align_up(c.barrier_off + 4, 128);
         c.fill_off = align_up(c.barrier_gen_off + 4, 128);
         c.overflow_off = c.fill_off + 256 * 4;
-        c.bytes = align_up(c.overflow_off + 4, 256);
+        c.msd_state_off = c.overflow_off + 4;
+        c.bytes = align_up(c.msd_state_off + 12, 256);
         return c;
     }
 };
 
-// The MSD block of a keys-only sort of 8- or 16-byte keys (offsets from
-// Plan::msd_off; msd.cuh).
+// The counters of the most-significant-first path (offsets from
+// Plan::msd_off; msd.cuh): keys per top digit, their cursors, then keys per
+// group and their cursors.  BYTES is what the size query has always held for
+// it where it has a block of its own.
 struct MsdLayout {
-    static constexpr size_t STATE = 0;
-    static constexpr size_t CURSOR1 = 256;
-    static constexpr size_t JOINT = CURSOR1 + 256 * 4;
-    static constexpr size_t CURSOR2 = JOINT + 65536 * 4;
-    static constexpr size_t ZERO_BYTES = CURSOR2 + 65536 * 4;  // cleared by the upsweep
-    static constexpr size_t OFFS2 = ZERO_BYTES;
-    static constexpr size_t BYTES = OFFS2 + 65536 * 4;
+    static constexpr size_t TOP = 0;
+    static constexpr size_t CURSOR1 = 256 * 4;
+    static constexpr size_t JOINT = 512 * 4;
+    static constexpr size_t bytes(int b2) { return JOINT + 2 * (size_t(256) << b2) * 4; }
+    static constexpr size_t BYTES = 256 + 256 * 4 + 3 * 65536 * 4;
+    static_assert(JOINT + 2 * 65536 * 4 <= BYTES, "the counters fit their block");
 };
 
 struct Plan {
@@ -78,15 +81,16 @@ struct Plan {
     // the one-launch sort's MSD regions: 256 x msd_cap keys (msd_cap 0: none)
     size_t regions_off = 0;
     uint32_t msd_cap = 0;
-    // keys-only sorts of 8- and 16-byte keys, most significant digit first
-    // (msd.cuh): kernels (top split, pair count, scan, second split, local
-    // sorts), group capacity, and the block at msd_off: state word (256 B),
-    // cursors [256], group sizes [65536], group cursors [65536] — zeroed by
-    // the upsweep — then group offsets [65536]
+    // keys-only sorts above the short range, most significant bits first
+    // (msd.cuh): kernels (sample, count, scan, top split, second split, local
+    // sorts), group capacity, most group bits below the top digit, and the place
+    // of the counters: a block of their own (msd_block), else the lookback
+    // status words, which only the digit passes use
     bool msd = false;
-    KernelEntry msd_k[5]{};
-    KernelEntry msd_hist{};  // its first kernel: the top digit's histogram
+    bool msd_block = false;
+    KernelEntry msd_k[6]{};
     uint32_t msd_group_cap = 0;
+    int msd_b2 = 0;
     size_t msd_off = 0;
     size_t total_bytes = 0;
     CtlLayout ctl{};

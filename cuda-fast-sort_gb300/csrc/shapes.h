@@ -89,45 +89,55 @@ constexpr int fused_local_tile(int kb) {
                       : FusedShape<16>::THREADS * FusedShape<16>::LIPT;
 }
 
-// Keys-only sorts of 8- and 16-byte keys, most significant digit first
-// (msd.cuh): the two splits' tiles (THREADS x IPT keys; 8-byte keys 2^27:
-// 2.95 ms with 24 keys per thread, 3.06 with 16, 3.03 with 32) and the local
-// sorts' CTAs (groups of up to C_THREADS x C_LIPT keys), for n in
-// [msd_n_min, msd_n_max] (groups of ~24 to ~2048 / ~384 to ~4096 keys;
-// outside, the digit passes).  Measured against the digit passes, CUDA
-// events, descending: 16-byte keys 2^22 0.58 vs 0.82 ms, 2^24 0.89 vs 2.46,
-// 2^26 2.11 vs 9.24; 8-byte keys 2^24 0.86 vs 0.82, 2^25 1.18 vs 1.52, 2^27
-// 2.95 vs 5.71.
-// Two local-sort shapes per width: L = 0 for groups of up to ~1024
-// (16-byte) / ~2048 (8-byte) keys on average, more CTAs per SM; L = 1 for
-// the larger groups up to msd_n_max.
+// Keys-only sorts above the short range, most significant bits first
+// (msd.cuh).
+// The two splits: THREADS x IPT keys a tile; CAP places per digit in the stage
+// (0: a dense stage).  Measured, top + second split: 4-byte keys 2^28 512 x 20
+// with 69 places 0.47 + 0.50 ms (512 x 24, 79 places 0.48 + 0.51; 256 x 24
+// dense 0.61 + 0.58: the dense stage's second random read bounds it); 8-byte
+// keys 5 x 10^7 256 x 16 dense, 4 CTAs an SM, 0.166 + 0.163 ms (512 x 12
+// with 43 places 0.177 + 0.195); 16-byte keys 2^26 512 x 6 dense 0.368 + 0.380
+// (256 x 12 0.372 + 0.383).
+// The local sorts: CTAs of C_THREADS, 64 bytes of keys a lane, C_HALO lanes of
+// margin at a warp's ends, in two sizes: L = 1 for the upper half of the range
+// of 8- and 16-byte keys, whose groups are twice as large.  Three CTAs an SM
+// keep their registers (2^28 4-byte keys: 0.88 ms, four CTAs 1.11 with spills).
 template <int KB>
 struct MsdShape {
-    static constexpr int THREADS = 256;
-    static constexpr int IPT = KB == 16 ? 12 : 24;
-    static constexpr int MIN_CTAS = 2;
-    static constexpr int C_THREADS = 256;
-    // 16-byte keys up to 2^26 (groups of up to ~1024 keys on average): 6 keys
-    // a thread, 4 CTAs an SM (2^26: local sorts 0.655 ms against 0.703 with
-    // 8 keys a thread and 3 CTAs; 1024 sub-buckets 0.694)
-    static constexpr int C_LIPT[2] = {KB == 16 ? 6 : 12, KB == 16 ? 12 : 24};
-    static constexpr int C_MIN_CTAS[2] = {KB == 16 ? 4 : 3, 2};
-    static constexpr int C_SPLIT_WORDS[2] = {KB == 16 ? 2048 : 4096, 4096};
+    static constexpr int THREADS = KB == 8 ? 256 : 512;
+    static constexpr int IPT = KB == 16 ? 6 : KB == 8 ? 16 : 20;
+    static constexpr int MIN_CTAS = KB == 8 ? 4 : 2;
+    static constexpr int CAP = KB == 4 ? 69 : 0;
+    static constexpr int C_THREADS[2] = {384, KB == 4 ? 384 : 768};
+    static constexpr int C_HALO = KB == 16 ? 2 : 1;
+    static constexpr int C_MIN_CTAS[2] = {3, KB == 4 ? 3 : 1};
 };
-// (4-byte keys measured slower this way: 2^28 u32 5.12 vs 4.11 ms, 2^25
-// 1.01 vs 0.58 — groups of 4096 keys with 16 bits left cost their local sort
-// more than the two digit passes it replaces.)
-constexpr bool msd_key_bytes(int kb) { return kb == 8 || kb == 16; }
-// (16-byte keys, descending, against the digit passes of the short shape:
-// 2^20 0.40 vs 0.32 ms, 1.5 x 2^20 0.488 vs 0.491, 2^21 0.50 vs 0.56, 3 x 2^20
-// 0.52 vs 0.74.)
-constexpr uint64_t msd_n_min(int kb) { return kb == 16 ? uint64_t(3) << 19 : uint64_t(3) << 23; }
-constexpr uint64_t msd_n_max(int kb) { return kb == 16 ? uint64_t(1) << 27 : uint64_t(1) << 28; }
-// the local-sort shape for n keys (groups of n / 65536 on average)
-constexpr int msd_local_shape(int kb, uint64_t n) { return n <= (msd_n_max(kb) >> 1) ? 0 : 1; }
+constexpr uint64_t msd_n_max(int kb) {
+    return kb == 16 ? uint64_t(1) << 27 : kb == 8 ? uint64_t(1) << 28 : uint64_t(5) << 26;
+}
+// Sizes whose size query has always held a block of its own for this path
+// (8- and 16-byte keys; elsewhere the path's counters lie in the lookback
+// status words, which it does not use, and the stage count is not reported).
+constexpr uint64_t msd_block_n_min(int kb) {
+    return kb == 16 ? uint64_t(3) << 19 : kb == 8 ? uint64_t(3) << 23 : ~uint64_t(0);
+}
+constexpr int msd_local_shape(int kb, uint64_t n) { return kb == 4 || n <= (msd_n_max(kb) >> 1) ? 0 : 1; }
+template <int KB>
+constexpr uint32_t msd_group_cap_of(int shape) {
+    using S = MsdShape<KB>;
+    return uint32_t(S::C_THREADS[shape] / 32 * (32 - 2 * S::C_HALO) * (64 / KB) - 32 / KB);
+}
 constexpr uint32_t msd_group_cap(int kb, int shape) {
-    return kb == 16 ? uint32_t(MsdShape<16>::C_THREADS * MsdShape<16>::C_LIPT[shape])
-                    : uint32_t(MsdShape<8>::C_THREADS * MsdShape<8>::C_LIPT[shape]);
+    return kb == 16 ? msd_group_cap_of<16>(shape) : kb == 8 ? msd_group_cap_of<8>(shape) : msd_group_cap_of<4>(shape);
+}
+// Most group bits below the top digit (the sample chooses how many): groups
+// average at most 0.72 of the largest a local sort takes, so that uniform keys
+// (a few standard deviations of sqrt(average)) and mildly uneven ones fit, and
+// one bit more for keys that use only part of the codes' range.
+constexpr int msd_b2_max(uint64_t n, uint32_t cap) {
+    int b2 = 1;
+    while (b2 < 8 && double(n) > 0.36 * double(cap) * double(256u << b2)) ++b2;
+    return b2;
 }
 
 // Keys per MSD region of the one-launch sort (one region per top digit):

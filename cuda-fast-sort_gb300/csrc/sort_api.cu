@@ -47,12 +47,14 @@ const KernelEntry* fused_entry_k4();
 const KernelEntry* fused_entry_k8();
 const KernelEntry* fused_entry_k16();
 
+const KernelEntry* msd_entries_k4();
 const KernelEntry* msd_entries_k8();
 const KernelEntry* msd_entries_k16();
 
-// Kernels of the MSD path of keys-only sorts (8- and 16-byte keys; msd.cuh).
+// Kernels of the most-significant-first path of keys-only sorts (msd.cuh).
 const KernelEntry* msd_entries(int kb) {
     switch (kb) {
+        case 4: return msd_entries_k4();
         case 8: return msd_entries_k8();
         case 16: return msd_entries_k16();
         default: return nullptr;
@@ -108,9 +110,8 @@ std::atomic<int> g_short_msd{[] {
     const char* v = std::getenv("GBSORT_SHORT_MSD");
     return (v && v[0] == '0') ? 0 : 1;
 }()};
-// Keys-only sorts of 8- and 16-byte keys above the short range, most
-// significant digit first (msd.cuh): on unless GBSORT_MSD=0 or switched off
-// (gbsort_set_msd).
+// Keys-only sorts above the short range, most significant bits first
+// (msd.cuh): on unless GBSORT_MSD=0 or switched off (gbsort_set_msd).
 std::atomic<int> g_msd{[] {
     const char* v = std::getenv("GBSORT_MSD");
     return (v && v[0] == '0') ? 0 : 1;
@@ -329,20 +330,29 @@ int make_plan(int key_type, size_t value_bytes, uint64_t n, Plan* plan) {
             off = align_up(off + size_t(256) * p.msd_cap * kb, 256);
         }
     }
-    // keys-only sorts of 8- and 16-byte keys above the one-launch range: the
-    // MSD block (sized whether or not the path is switched on), right after
-    // the status words so that the upsweep clears both in one sweep
-    if ((!small || n > fused_n_max(p.kb)) && p.vb == 0 && msd_key_bytes(p.kb) && n >= msd_n_min(p.kb) &&
-        n <= msd_n_max(p.kb) && msd_entries(p.kb) != nullptr) {
-        p.msd_off = off;
-        off = align_up(off + MsdLayout::BYTES, 256);
+    // keys-only sorts above the one-launch range: the most-significant-first
+    // path, its counters in a block of their own (sized whether or not the
+    // path is switched on) or in the status words.  Not floats, unless they
+    // always had that block: their leading bits are the exponent, so that most
+    // values share few groups and the path's first kernels are spent in vain
+    // (f64 N(0,1), 2.5 x 10^6 keys: 247 against 222 us).
+    const bool block = n >= msd_block_n_min(p.kb);
+    if (p.vb == 0 && n > fused_n_max(p.kb) && n <= msd_n_max(p.kb) && (block || p.kind != KIND_FLOAT) &&
+        msd_entries(p.kb) != nullptr) {
         const int shape = msd_local_shape(p.kb, n);
         p.msd_group_cap = msd_group_cap(p.kb, shape);
-        if (g_msd.load(std::memory_order_relaxed)) {
+        p.msd_b2 = msd_b2_max(n, p.msd_group_cap);
+        p.msd_block = block;
+        p.msd_off = p.status_off;
+        if (p.msd_block) {
+            p.msd_off = off;
+            off = align_up(off + MsdLayout::BYTES, 256);
+        }
+        if (g_msd.load(std::memory_order_relaxed) &&
+            (p.msd_block || MsdLayout::bytes(p.msd_b2) <= p.status_bytes)) {
             p.msd = true;
-            for (int i = 0; i < 4; ++i) p.msd_k[i] = msd_entries(p.kb)[i];
-            p.msd_k[4] = msd_entries(p.kb)[4 + shape];
-            p.msd_hist = msd_entries(p.kb)[6];
+            for (int i = 0; i < 5; ++i) p.msd_k[i] = msd_entries(p.kb)[i];
+            p.msd_k[5] = msd_entries(p.kb)[5 + shape];
         }
     }
     p.total_bytes = off;
@@ -366,10 +376,13 @@ int enqueue_sort(const Plan& plan, int descending, void* d_keys, void* d_values,
     if (st != GBSORT_OK) return st;
     st = prepare_kernel(plan.upsweep);
     if (st != GBSORT_OK) return st;
-    // the MSD path of keys-only sorts runs when all its kernels can
-    bool use_msd = plan.msd && prepare_kernel(plan.msd_hist) == GBSORT_OK;
-    for (int i = 0; use_msd && i < 5; ++i) use_msd = prepare_kernel(plan.msd_k[i]) == GBSORT_OK;
-    const int ms_stages = use_msd ? 6 : 0;  // its five kernels and the other digits' histogram
+    // the most-significant-first path of keys-only sorts runs when all its
+    // kernels can
+    bool use_msd = plan.msd;
+    for (int i = 0; use_msd && i < 6; ++i) use_msd = prepare_kernel(plan.msd_k[i]) == GBSORT_OK;
+    // its kernels are timed one by one where the plan reports them (then the
+    // digits' histogram is the last of six stages), else as part of entry 0
+    const int ms_stages = use_msd && plan.msd_block ? 6 : 0;
 
     uint8_t* ws = static_cast<uint8_t*>(d_workspace);
     // a DoubleBuffer workspace starts at the control block
@@ -408,9 +421,8 @@ int enqueue_sort(const Plan& plan, int descending, void* d_keys, void* d_values,
         return GBSORT_ERR_CUDA;
     };
 
-    // the MSD block (keys-only sorts of 8- and 16-byte keys)
     uint8_t* msd_block = use_msd ? ws + plan.msd_off - ws_base : nullptr;
-    const uint32_t* msd_state = use_msd ? reinterpret_cast<const uint32_t*>(msd_block + MsdLayout::STATE) : nullptr;
+    uint32_t* msd_state = use_msd ? reinterpret_cast<uint32_t*>(ctl + plan.ctl.msd_state_off) : nullptr;
 
     // Parameters of digit pass `pass` and of the fix-up copy.
     auto pass_params = [&](int pass) {
@@ -482,16 +494,11 @@ int enqueue_sort(const Plan& plan, int descending, void* d_keys, void* d_values,
     hp.desc = descending;
     hp.gp_counts = gp;
     hp.status = status;
-    // the MSD block's counters follow the status words: one clear for both
-    hp.status_bytes = use_msd ? plan.msd_off + MsdLayout::ZERO_BYTES - plan.status_off : plan.status_bytes;
+    hp.status_bytes = plan.status_bytes;
     hp.mirror_keys = odd ? alt_keys : nullptr;
     hp.vals = copy ? vals_src : d_values;
     hp.mirror_vals = (odd && plan.vb) ? alt_vals : nullptr;
     hp.val_bytes_total = plan.n * uint64_t(plan.vb);
-    if (use_msd) {  // the MSD path needs the top digit's counts only; the rest follow if it falls back
-        hp.digit_lo = plan.passes - 1;
-        hp.digit_hi = plan.passes;
-    }
     if (fused) {
         // Short array: the whole sort in one cooperative launch (every CTA
         // resident, or the launch fails; fused_short.cuh).
@@ -536,23 +543,10 @@ int enqueue_sort(const Plan& plan, int descending, void* d_keys, void* d_values,
         cudaGetLastError();
     }
     const uint32_t hist_ctas = upsweep_ctas(plan.n, plan.kb);
-    {
-        void* args[] = {&hp};
-        if (timed) cudaEventRecord(ev[0], stream);
-        if (use_msd) {  // the top digit alone, several CTAs an SM
-            const int occ_h = resident_ctas(plan.msd_hist);
-            const uint32_t g = uint32_t((sms > 0 ? sms : 1) * (occ_h > 0 ? occ_h : 1));
-            e = cudaLaunchKernel(plan.msd_hist.fn, dim3(g), dim3(plan.msd_hist.threads), args, 0, stream);
-        } else {
-            e = cudaLaunchKernel(plan.upsweep.fn, dim3(hist_ctas), dim3(plan.upsweep.threads), args,
-                                 plan.upsweep.smem, stream);
-        }
-        if (e != cudaSuccess) return fail("upsweep launch", e);
-        if (timed) cudaEventRecord(ev[1], stream);
-    }
+    if (timed) cudaEventRecord(ev[0], stream);
     if (use_msd) {
-        // Keys only, 8- or 16-byte keys: top split, pair count, scan, second
-        // split, local sorts (msd.cuh); the digit passes below exit at once
+        // Keys only: sample, count, scan, top split, second split, local sorts
+        // (msd.cuh); the histogram and the digit passes below exit at once
         // when these sorted, and otherwise sort from the input-preserving
         // source or from the caller's buffer, which then holds the input's
         // keys in some order (keys only: the same bytes come out).
@@ -563,34 +557,39 @@ int enqueue_sort(const Plan& plan, int descending, void* d_keys, void* d_values,
         mp.n = plan.n;
         mp.kind = plan.kind;
         mp.desc = descending;
-        mp.gp_top = gp + size_t(plan.passes - 1) * 256;
-        mp.state = reinterpret_cast<uint32_t*>(msd_block + MsdLayout::STATE);
+        mp.b2_max = plan.msd_b2;
+        mp.state = msd_state;
+        mp.window = msd_state + 1;
+        mp.zero = reinterpret_cast<uint32_t*>(msd_block);
+        mp.zero_words = uint32_t(MsdLayout::bytes(plan.msd_b2) / 4);
+        mp.top_counts = reinterpret_cast<uint32_t*>(msd_block + MsdLayout::TOP);
         mp.cursor1 = reinterpret_cast<uint32_t*>(msd_block + MsdLayout::CURSOR1);
         mp.joint = reinterpret_cast<uint32_t*>(msd_block + MsdLayout::JOINT);
-        mp.cursor2 = reinterpret_cast<uint32_t*>(msd_block + MsdLayout::CURSOR2);
-        mp.offs2 = reinterpret_cast<uint32_t*>(msd_block + MsdLayout::OFFS2);
+        mp.cursor2 = mp.joint + (size_t(256) << plan.msd_b2);
         mp.group_cap = plan.msd_group_cap;
         mp.err = err_word;
-        for (int i = 0; i < 5; ++i) {
+        for (int i = 0; i < 6; ++i) {
             const KernelEntry& k = plan.msd_k[i];
             const uint64_t full = uint64_t(sms > 0 ? sms : 1) * uint64_t(resident_ctas(k) > 0 ? resident_ctas(k) : 1);
-            const uint32_t grid = (i == 2) ? 1u : uint32_t(full);
+            const uint64_t per_top = 256;  // scan: one CTA per top digit
+            const uint64_t clear = 1 + (mp.zero_words + 4095) / 4096;  // sample: and CTAs that clear the counters
+            const uint32_t grid = uint32_t(i == 0 ? (clear < full ? clear : full) : i == 2 ? per_top : full);
             void* args[] = {&mp};
             e = launch_dependent(k.fn, grid, k.threads, k.smem, stream, args);
             if (e != cudaSuccess) return fail("msd launch", e);
-            if (timed) cudaEventRecord(ev[2 + i], stream);
+            if (timed && ms_stages) cudaEventRecord(ev[1 + i], stream);
         }
-        // the other digits' counts, for the digit passes if they sort
-        HistParams rest = hp;
-        rest.digit_lo = 0;
-        rest.digit_hi = plan.passes - 1;
-        rest.status_bytes = 0;  // cleared by the first histogram kernel
+        HistParams rest = hp;  // the digit passes' histogram, if they sort
         rest.msd_state = msd_state;
         void* args[] = {&rest};
         e = launch_dependent(plan.upsweep.fn, hist_ctas, plan.upsweep.threads, plan.upsweep.smem, stream, args);
-        if (e != cudaSuccess) return fail("histogram launch", e);
-        if (timed) cudaEventRecord(ev[2 + 5], stream);
+    } else {
+        void* args[] = {&hp};
+        e = cudaLaunchKernel(plan.upsweep.fn, dim3(hist_ctas), dim3(plan.upsweep.threads), args, plan.upsweep.smem,
+                             stream);
     }
+    if (e != cudaSuccess) return fail("upsweep launch", e);
+    if (timed) cudaEventRecord(ev[1 + ms_stages], stream);
 
     const int occ = resident_ctas(plan.pass);
     const uint64_t max_ctas = uint64_t(sms) * uint64_t(occ > 0 ? occ : 1);
@@ -1079,7 +1078,7 @@ int gbsort_plan(int key_type, size_t value_bytes, size_t n, gbsort_plan_info* ou
     out->status_word_bytes = plan.wide_status ? 8 : 4;
     out->kernel_launches = uint32_t(plan.passes + 1 + ((gbsort_get_pass_skip() && (plan.passes & 1) == 0) ? 1 : 0));
     if (plan.msd) {
-        out->msd_stages = 6;
+        out->msd_stages = plan.msd_block ? 6 : 0;
         out->kernel_launches += 6;
     }
     if (plan.fused.fn && sms > 0 && prepare_kernel(plan.fused) == GBSORT_OK && resident_ctas(plan.fused) > 0) {

@@ -5,10 +5,10 @@
 
 namespace gbsort {
 
-// Outcome of the most-significant-digit-first path of a keys-only sort
-// (msd.cuh): 0 undecided, MSD_OK the MSD kernels sort, MSD_OFF the digit
-// passes sort.
-constexpr uint32_t MSD_OK = 1u, MSD_OFF = 2u;
+// Why the digit passes sort after the most-significant-first path of a
+// keys-only sort (msd.cuh; 0: that path sorts): MSD_OFF some group is too big
+// (decided before any key moves), MSD_GAVE_UP a local sort gave up.
+constexpr uint32_t MSD_OFF = 1u, MSD_GAVE_UP = 2u;
 
 // Global-histogram upsweep (one launch per sort).
 struct HistParams {
@@ -25,11 +25,9 @@ struct HistParams {
     const void* vals;
     void* mirror_vals;
     uint64_t val_bytes_total;   // n * value bytes
-    // digits counted: [digit_lo, digit_hi), every digit when digit_hi == 0
-    int digit_lo, digit_hi;
-    // non-null: a histogram of the remaining digits for the digit passes of
-    // a keys-only sort whose MSD path may already have sorted: exits when it
-    // did (MSD_OK), waits for its predecessor kernel first
+    // non-null: the histogram for the digit passes of a keys-only sort whose
+    // MSD path may already have sorted: exits when it did (0), waits for its
+    // predecessor kernel first
     const uint32_t* msd_state;
 };
 
@@ -84,7 +82,7 @@ struct PassParams {
     const uint32_t* nonuniform_mask;
     // plain mode with skipping: receives bit 31 | number of executed passes
     uint32_t* executed;
-    // keys-only sorts with the MSD path: the pass exits when it sorted (MSD_OK)
+    // keys-only sorts with the MSD path: the pass exits when it sorted (0)
     const uint32_t* msd_state;
 };
 

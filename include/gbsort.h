@@ -476,17 +476,18 @@ int gbsort_get_short_fused(void);
 void gbsort_set_short_msd(int enable);
 int gbsort_get_short_msd(void);
 
-/* Keys-only sorts of 8- and 16-byte keys above the short range (1.5 x 2^24
- * to 2^28 keys of 8 bytes, 1.5 x 2^20 to 2^27 of 16): most significant digit
- * first —
- * a split by the top digit, a count of (top, second) digit pairs, a split by
- * the second digit into the 65536 pairs' ranges, and in-place local sorts
- * of those groups in shared memory — instead of one stable pass per key
- * byte (gbsort_plan_info.msd_stages = 6).  When a group outgrows a local
- * sort (skewed or repeated keys), the digit passes sort instead, decided on
- * the device.  The size query reserves the path's ~1 MB either way.  On by
- * default; GBSORT_MSD=0 in the environment or gbsort_set_msd(0) turns it
- * off.  Keys only, so the result is the same bytes either way. */
+/* Keys-only sorts of 4-, 8- and 16-byte keys above the short range (2^21
+ * keys, 2^20 of 16 bytes; up to 1.25 x 2^28, 2^28 and 2^27): most significant
+ * bits first — a count of the keys per leading bits, a split by the top digit,
+ * a split by the bits below it into groups of a few thousand keys, and
+ * in-place local sorts of those groups in shared memory — instead of one
+ * stable pass per key byte.  When a group outgrows a local sort (skewed or
+ * repeated keys), the digit passes sort instead, decided on the device.
+ * Where the size query holds a block of its own for the path (8-byte keys
+ * from 1.5 x 2^24, 16-byte keys from 1.5 x 2^20; ~1 MB, either way)
+ * gbsort_plan_info.msd_stages is 6.  On by default; GBSORT_MSD=0 in the
+ * environment or gbsort_set_msd(0) turns it off.  Keys only, so the result is
+ * the same bytes either way. */
 void gbsort_set_msd(int enable);
 int gbsort_get_msd(void);
 
@@ -571,14 +572,14 @@ typedef struct gbsort_plan_info {
                                  partition (each key read and written twice);
                                  0: every digit takes a pass                  */
     uint32_t msd_stages;      /* keys-only sorts of 8- and 16-byte keys above
-                                 the short range, most significant digit
-                                 first: 6 kernels (top split, pair count,
-                                 scan, second split, local sorts, and the
-                                 histogram of the other digits) run after the
-                                 top digit's histogram kernel and before the
-                                 digit passes; those and the last histogram
-                                 exit at once unless a group was too big;
-                                 0: not planned                              */
+                                 the short range, most significant bits
+                                 first: 6 kernels (group count, scan, top
+                                 split, second split, local sorts, and the
+                                 digits' histogram) run after the first one,
+                                 which samples the keys, and before the     
+                                 digit passes; those and the histogram exit
+                                 at once unless a group was too big; 0: not
+                                 planned, or not reported (4-byte keys)      */
 } gbsort_plan_info;
 
 int gbsort_plan(int key_type, size_t value_bytes, size_t n,
@@ -587,10 +588,11 @@ int gbsort_plan(int key_type, size_t value_bytes, size_t n,
 /* Same as gbsort_sort_pairs (d_values may be NULL with value_bytes 0), but
  * records a CUDA event around every kernel on `stream` and, after
  * synchronizing, writes the per-kernel device milliseconds to ms_out:
- * ms_out[0] = histogram kernel, then with the MSD path planned
- * (gbsort_plan_info.msd_stages = S = 6) ms_out[1 .. S] = its kernels (top
- * split, pair count, scan, second split, local sorts, histogram of the other
- * digits), then
+ * ms_out[0] = histogram kernel (4-byte keys going most significant bits
+ * first: with that path's kernels); where the plan reports that path
+ * (gbsort_plan_info.msd_stages = S = 6) ms_out[0] = its sample
+ * and ms_out[1 .. S] = its kernels (group count, scan, top split, second
+ * split, local sorts, digits' histogram), then
  * ms_out[1 + S + p] = digit pass p (S = 0 otherwise), and with pass skipping
  * on and an even pass count P, ms_out[1 + S + P] = the fix-up copy.  A short
  * array sorted in one launch (gbsort_set_short_fused) writes one entry, the
