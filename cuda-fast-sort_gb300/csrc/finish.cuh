@@ -1,0 +1,733 @@
+// finish.cuh — key-value sorts by their leading digits only (sm_103a).
+//
+// A stable least-significant-digit sort makes a pass over keys and values per
+// key byte.  Where the leading D bytes already cut the array into groups of a
+// few thousand pairs, the passes over the other bytes can be one local sort:
+//   sample:  4096 keys say how many leading bytes that takes (or that nothing
+//            is gained, FINISH_OFF: every digit pass runs as before);
+//   passes:  the digit passes of those bytes only (onesweep.cuh);
+//   edges:   the array, now in stable order of its leading bytes, is cut near
+//            every `chunk` pairs at the next group's start, so that windows of
+//            whole groups fit a CTA;
+//   finish:  each CTA sorts whole windows in shared memory, stable, and
+//            writes them untwiddled to the caller's buffers.
+// A window's keys keep their order by group; inside a group of m keys a key
+// goes to one of m sub-buckets by its remaining bits (about one key each), and
+// a few rounds of an odd-even transposition network over (key, place before)
+// put it in its stable place.  A group whose keys are all equal keeps its
+// order as it is, however large: an edge may cut through such a group.
+// What bounds the finish: latency (two CTAs of 384 threads an SM, 80 registers;
+// a window of 2300 pairs of 8-byte keys takes its CTA 7.7 us, of which the
+// network's instructions are a fifth); 2 x 10^7 u64 + u32 0.22 ms.
+// When that fails somewhere (a group too big after all, sub-buckets too full)
+// the window is written as it was, and every digit pass runs, from the
+// caller's buffers, which then hold the pairs untwiddled, in an order that a
+// stable sort completes.
+#pragma once
+
+#include "msd.cuh"
+
+namespace gbsort {
+
+struct FinishParams {
+    const void* keys_in;   // the input (sample only)
+    void* keys_a;          // the caller's buffers: the result
+    void* vals_a;
+    void* keys_b;          // the alternate buffers
+    void* vals_b;
+    uint64_t n;            // < 2^32
+    int kind, desc;
+    int copy;              // input-preserving: the passes end in the caller's buffers
+    uint32_t* state;       // MSD_OFF, MSD_GAVE_UP: every digit pass sorts
+    uint32_t* window;      // [2] lowest digit that the passes sort by, pairs per chunk
+    const uint32_t* executed;  // passes run (bit 31 set; 0: none)
+    uint32_t* ticket;      // the sample's CTAs, zeroed with the control block
+    uint32_t* sampled;     // [FINISH_LEVELS + 1] their counts
+    uint32_t* edges;       // [chunks + 1] first pair of every window (bit 31: the edge cuts a group)
+    uint32_t max_chunks;   // room in edges
+    uint32_t places;       // pairs a window may hold
+    uint32_t* err;
+};
+
+// ---- sample -----------------------------------------------------------------
+// CTA l counts the pairs of sampled keys that share their l + 1 leading bytes
+// (the last CTA: that are equal, which no digit tells apart), in 2^15 hashed
+// counters; S keys in groups of g make S * S * g / 2n of them.  The CTA that
+// finishes last decides.
+constexpr int FINISH_SAMPLE_THREADS = 1024;
+constexpr int FINISH_LEVELS = 6;  // leading bytes tried
+constexpr int FINISH_SAMPLE_SMEM = 32768 * 4;
+template <int KB>
+constexpr int finish_levels() { return KB - 1 < FINISH_LEVELS ? KB - 1 : FINISH_LEVELS; }
+template <int KB>
+__global__ void __launch_bounds__(FINISH_SAMPLE_THREADS) finish_sample_kernel(FinishParams p) {
+    using U = typename KeyBits<KB>::U;
+    constexpr int LEVELS = finish_levels<KB>();
+    extern __shared__ __align__(16) uint32_t cnt[];
+    __shared__ uint32_t shared_pairs, vary, ticket;
+    grid_launch_dependents();
+    grid_dependency_wait();
+    const int tid = threadIdx.x, level = blockIdx.x;
+    // more of them where a group is a smaller part of the array
+    constexpr int MOST = KB == 16 ? 8 : 16;
+    const int per = p.n >= (uint64_t(1) << 26) ? MOST : p.n >= (uint64_t(1) << 23) ? 8 : 4;
+    const float S = float(FINISH_SAMPLE_THREADS * per);
+    const KeyMap<U> map(p.kind, p.desc);
+    const U* keys = static_cast<const U*>(p.keys_in);
+    const uint32_t step = max(1u, uint32_t(p.n / uint32_t(FINISH_SAMPLE_THREADS * per)));
+    U x[MOST];
+#pragma unroll
+    for (int i = 0; i < MOST; ++i) {
+        if (i >= per) break;
+        const uint32_t at = uint32_t(i * FINISH_SAMPLE_THREADS + tid);
+        const uint64_t j = uint64_t(at) * step + (at * 2654435761u) % step;
+        x[i] = map.in(keys[j < p.n ? j : j % p.n]);
+    }
+    const U first = map.in(keys[0]);
+    for (int i = tid; i < 8192; i += FINISH_SAMPLE_THREADS) reinterpret_cast<uint4*>(cnt)[i] = make_uint4(0, 0, 0, 0);
+    if (tid == 0) shared_pairs = vary = 0u;
+    __syncthreads();
+    U d = 0;
+    uint32_t pairs = 0;
+#pragma unroll
+    for (int i = 0; i < MOST; ++i) {
+        if (i >= per) break;
+        d |= x[i] ^ first;
+        const U v = level == LEVELS ? x[i] : x[i] >> (8 * (KB - 1 - level));
+        uint64_t h = uint64_t(v);
+        if constexpr (KB == 16) h ^= uint64_t(v >> 64) * 0x9E3779B97F4A7C15ull;
+        // (splitmix64's finalizer: few distinct prefixes must not spread evenly)
+        h = (h ^ (h >> 30)) * 0xBF58476D1CE4E5B9ull;
+        h = (h ^ (h >> 27)) * 0x94D049BB133111EBull;
+        h ^= h >> 31;
+        pairs += atomicAdd(&cnt[uint32_t(h) & 32767u], 1u);  // the keys there before this one
+    }
+    uint32_t bytes = 0;  // bit q: byte q differs somewhere
+#pragma unroll
+    for (int q = 0; q < KB; ++q) bytes |= uint32_t(((d >> (8 * q)) & U(0xff)) != U(0)) << q;
+    bytes = __reduce_or_sync(0xffffffffu, bytes);
+    pairs = __reduce_add_sync(0xffffffffu, pairs);
+    if ((tid & 31) == 0) {
+        atomicOr(&vary, bytes);
+        atomicAdd(&shared_pairs, pairs);
+    }
+    __syncthreads();
+    if (tid == 0) {
+        p.sampled[level] = shared_pairs;
+        __threadfence();
+        ticket = atomicAdd(p.ticket, 1u);
+    }
+    if (tid != 0 || ticket != uint32_t(LEVELS)) return;
+    __threadfence();
+    const float n = float(p.n), places = float(p.places);
+    const float equal = float(ld_relaxed(p.sampled + LEVELS));
+    // what a pair's group by l + 1 leading bytes holds on average, and a little
+    // more than a deviation of the estimate
+    auto group_of = [&](int l) {
+        const float pairs = float(ld_relaxed(p.sampled + l));
+        return (max(0.f, pairs - equal) + 1.2f * sqrtf(pairs + equal)) * 2.f * n / (S * S);
+    };
+    // The fewest leading bytes whose groups fit, and whose next byte spreads a
+    // group's keys over its sub-buckets.  Groups of floats are uneven (the
+    // largest of N(0, 1) hold twice the average): they have to be smaller.
+    const float fits = (p.kind == KIND_FLOAT ? 0.4f : 0.84f) * places;
+    const float noise = 1.2f * sqrtf(2.f * equal) * 2.f * n / (S * S);
+    int lo = 0;
+    float group = 0.f;
+    for (int l = 0; l < LEVELS; ++l) {
+        group = group_of(l);
+        if (group <= fits && (l + 1 == LEVELS || group_of(l + 1) <= group * (1.f / 16.f) + 2.f * noise + 4.f)) {
+            lo = KB - 1 - l;
+            break;
+        }
+    }
+    // worth it when it replaces two passes or more
+    const uint32_t low = vary & ((1u << lo) - 1u);
+    uint32_t chunk = 0;
+    if (lo == 0 || __popc(low) < 2) {
+        *p.state = MSD_OFF;
+    } else {
+        // the larger the groups, the more of a window is left for the one
+        // that starts last in it (and seven deviations of a random group's
+        // size)
+        const float c = 0.98f * places - (p.kind == KIND_FLOAT ? 2.f : 1.1f) * group - 7.f * sqrtf(group);
+        chunk = uint32_t(min(max(c, 0.1f * places), 0.93f * places)) & ~31u;
+        chunk = max(chunk, (uint32_t(p.n / (p.max_chunks - 1u)) + 32u) & ~31u);
+        if (float(chunk) > 0.95f * places) *p.state = MSD_OFF;
+    }
+    p.window[0] = uint32_t(lo);
+    p.window[1] = chunk;
+}
+
+// Where the passes left the pairs: the alternate buffers after an odd count
+// in place, else the caller's.
+__device__ __forceinline__ bool finish_in_b(const FinishParams& p) {
+    const uint32_t w = ld_relaxed(p.executed);
+    return !p.copy && (w & 1u) != 0u;
+}
+
+// ---- edges ------------------------------------------------------------------
+// Edge c: the first group start at or after pair c * chunk, found by a warp in
+// three rounds of 32 reads; none within places - chunk pairs: the edge stays
+// there and cuts the group, which has to consist of equal keys.
+template <int KB>
+__global__ void __launch_bounds__(256) finish_edges_kernel(FinishParams p) {
+    using U = typename KeyBits<KB>::U;
+    grid_launch_dependents();
+    grid_dependency_wait();
+    if (ld_relaxed(p.state) & MSD_OFF) return;
+    if (!(ld_relaxed(p.executed) >> 31)) {  // the leading digits do not vary: no pass has run
+        if (threadIdx.x == 0 && blockIdx.x == 0) atomicOr(p.state, MSD_GAVE_UP);
+        return;
+    }
+    const U* keys = static_cast<const U*>(finish_in_b(p) ? p.keys_b : p.keys_a);
+    const uint32_t n = uint32_t(p.n), lo = ld_relaxed(p.window), chunk = ld_relaxed(p.window + 1);
+    const uint32_t chunks = (n + chunk - 1) / chunk;
+    const int lane = threadIdx.x & 31;
+    const uint32_t shift = 8u * lo;
+    for (uint32_t c = (blockIdx.x * 256 + threadIdx.x) >> 5; c <= chunks; c += gridDim.x * 8) {
+        if (c == 0 || c == chunks) {
+            if (lane == 0) p.edges[c] = c ? n : 0u;
+            continue;
+        }
+        const uint32_t at = c * chunk;
+        const U before = keys[at - 1];
+        const U group = before >> shift;
+        // first j in [from, from + 32 * step) with another group than `before`, by steps
+        uint32_t from = at, limit = min(at + (p.places - chunk), n - 1u);  // heads looked for in [at, limit]
+        uint32_t head = 0xffffffffu;
+        if ((keys[at] >> shift) != group) {
+            head = at;
+        } else {
+            // keys[from] is in the group; the answer, if any, is in (from, limit]
+            uint32_t span = limit - from;
+            while (span) {
+                const uint32_t step = (span + 31) / 32;
+                const uint32_t j = min(from + (lane + 1) * step, limit);
+                const uint32_t past = __ballot_sync(0xffffffffu, (keys[j] >> shift) != group);
+                if (!past) break;  // only in the first round: later ones hold the answer
+                const int l = __ffs(past) - 1;
+                const uint32_t hi = min(from + (l + 1) * step, limit);
+                const uint32_t low = from + l * step;  // in the group
+                if (hi - low <= 1u) {
+                    head = hi;
+                    break;
+                }
+                from = low;
+                limit = hi;
+                span = hi - low;
+            }
+        }
+        if (lane == 0) {
+            if (head != 0xffffffffu) {
+                p.edges[c] = head;
+            } else if (at + (p.places - chunk) >= n) {
+                p.edges[c] = n;  // the last group reaches the end of the array
+            } else {
+                p.edges[c] = at | 0x80000000u;
+                if (keys[at] != before) atomicOr(p.state, MSD_GAVE_UP);
+            }
+        }
+    }
+}
+
+// ---- finish -----------------------------------------------------------------
+// Shared memory of a window of up to CAP pairs, LIPT consecutive places (a
+// chunk) a lane, HALO lanes of margin at a warp's ends.  Chunks lie 16 bytes
+// apart from a multiple of their size, so that eight lanes' 16-byte accesses
+// meet all banks.  A pair is put in order by its key and its place before: one
+// 64-bit word for 4-byte keys, else the key and a 16-bit place, apart.
+// (64-bit words for wider keys too, of the sub-bucket and 35 bits below it,
+// with the keys fetched at the end: 2 x 10^7 8-byte keys 0.31 against 0.23 ms.)
+template <int KB, int VB, int THREADS, int LIPT_, int HALO>
+struct FinishGeom {
+    static constexpr int LIPT = LIPT_;
+    static constexpr int WARPS = THREADS / 32;
+    static constexpr int OUT = (32 - 2 * HALO) * LIPT;  // places a warp puts in order
+    static constexpr int PLACES = WARPS * OUT;
+    static constexpr int ALIGN = 32 / KB;  // places keep the result's position in its 32-byte sector
+    static constexpr int CAP = PLACES - ALIGN;
+    static_assert(PLACES < 65536, "16-bit places");
+    static_assert(LIPT * KB % 32 == 0 && LIPT % 2 == 0 && LIPT <= 16, "whole sectors a lane");
+    // sub-buckets, one per place; byte counters scanned by a thread
+    static constexpr int PER = (PLACES + THREADS * 4 - 1) / (THREADS * 4) * 4;
+    static constexpr int BINS = PER * THREADS;
+    static constexpr int EB = KB == 4 ? 8 : KB;  // bytes of a place's word or key
+    static constexpr int STRIDE = LIPT * EB + 16;
+    static constexpr size_t POS_OFF = (size_t(PLACES / LIPT) * STRIDE + 127) & ~size_t(127);  // u16, keys of 8 bytes and more
+    static constexpr size_t VALS_OFF = (POS_OFF + (KB == 4 ? 0 : size_t(PLACES) * 2) + 127) & ~size_t(127);
+    static constexpr size_t CTR_OFF = (VALS_OFF + size_t(PLACES) * VB + 127) & ~size_t(127);  // u8 [BINS]
+    static constexpr size_t START_OFF = CTR_OFF + BINS;                                       // u16 [BINS]
+    static constexpr size_t SCAN_OFF = START_OFF + size_t(BINS) * 2;                          // u32 [32]
+    static constexpr size_t MISC_OFF = SCAN_OFF + 128;                                        // u32 [4]
+    static constexpr size_t HEADS_OFF = MISC_OFF + 16;                                        // u32 [2][WARPS]
+    static constexpr size_t SMEM_BYTES = HEADS_OFF + size_t(WARPS) * 8;
+    static_assert(size_t(PLACES) <= POS_OFF, "the groups' marks lie where the keys go later");
+    __device__ __forceinline__ static uint32_t at(uint32_t place) {
+        return place * uint32_t(EB) + (place / LIPT) * 16u;
+    }
+};
+
+// A key and its place in the window before (unique, so the order is total).
+template <class U>
+struct Placed {
+    U k;
+    uint32_t j;
+    __device__ __forceinline__ static Placed make(U key, uint32_t place) { return Placed{key, place}; }
+    __device__ __forceinline__ U key() const { return k; }
+    __device__ __forceinline__ uint32_t place() const { return j; }
+};
+template <>
+struct Placed<uint32_t> {
+    uint64_t v;
+    __device__ __forceinline__ static Placed make(uint32_t key, uint32_t place) {
+        return Placed{(uint64_t(key) << 32) | place};
+    }
+    __device__ __forceinline__ uint32_t key() const { return uint32_t(v >> 32); }
+    __device__ __forceinline__ uint32_t place() const { return uint32_t(v); }
+};
+// b comes before a: one borrow chain over the words.
+__device__ __forceinline__ bool after(const Placed<uint32_t>& a, const Placed<uint32_t>& b) { return b.v < a.v; }
+__device__ __forceinline__ bool after(const Placed<uint64_t>& a, const Placed<uint64_t>& b) {
+    uint32_t r;
+    asm("{\n\t.reg .u32 t;\n\tsub.cc.u32 t, %1, %2;\n\tsubc.cc.u32 t, %3, %4;\n\tsubc.cc.u32 t, %5, %6;\n\t"
+        "subc.u32 %0, 0, 0;\n\t}"
+        : "=r"(r)
+        : "r"(b.j), "r"(a.j), "r"(uint32_t(b.k)), "r"(uint32_t(a.k)), "r"(uint32_t(b.k >> 32)),
+          "r"(uint32_t(a.k >> 32)));
+    return r != 0u;
+}
+__device__ __forceinline__ bool after(const Placed<u128>& a, const Placed<u128>& b) {
+    return b.k < a.k || (b.k == a.k && b.j < a.j);
+}
+template <class U>
+__device__ __forceinline__ void order_pair(Placed<U>& a, Placed<U>& b) {
+    const bool sw = after(a, b);
+    const Placed<U> lo = sw ? b : a, hi = sw ? a : b;
+    a = lo;
+    b = hi;
+}
+template <class U>
+__device__ __forceinline__ Placed<U> placed_up1(const Placed<U>& p) {
+    return Placed<U>::make(shfl_up1(p.key()), __shfl_up_sync(0xffffffffu, p.place(), 1));
+}
+template <class U>
+__device__ __forceinline__ Placed<U> placed_down1(const Placed<U>& p) {
+    return Placed<U>::make(shfl_down1(p.key()), __shfl_down_sync(0xffffffffu, p.place(), 1));
+}
+
+template <class U, int LIPT>
+__device__ __forceinline__ void placed_rounds(Placed<U> (&k)[LIPT], uint32_t rounds, int lane) {
+    for (uint32_t r = 0; r < rounds; r += 2) {
+#pragma unroll
+        for (int i = 0; i + 1 < LIPT; i += 2) order_pair(k[i], k[i + 1]);
+        if (r + 1 < rounds) {
+            const Placed<U> before = placed_up1(k[LIPT - 1]), next = placed_down1(k[0]);
+#pragma unroll
+            for (int i = 1; i + 1 < LIPT; i += 2) order_pair(k[i], k[i + 1]);
+            if (lane > 0 && after(before, k[0])) k[0] = before;
+            if (lane < 31 && after(k[LIPT - 1], next)) k[LIPT - 1] = next;
+        }
+    }
+}
+
+// Global to shared memory without registers in between (4, 8 or 16 bytes,
+// aligned to their size); waited for by the thread that issued it.
+template <int BYTES>
+__device__ __forceinline__ void copy_async(void* dst, const void* src) {
+    if constexpr (BYTES == 16)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(smem_u32(dst)), "l"(src), "n"(BYTES) : "memory");
+}
+__device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// Exclusive places of the sub-buckets from their byte counters (zeroed), the
+// first at `base`; misc[0] takes the largest count, or 256 when one passed 255
+// (the counts then do not add up to cnt).
+template <class F, int THREADS>
+__device__ __forceinline__ void scan_bins(uint8_t* smem, uint32_t cnt, uint32_t base) {
+    constexpr int WORDS = F::PER / 4;
+    static_assert(WORDS == 1 || WORDS == 2 || WORDS == 4, "whole vectors");
+    uint32_t* ctr = reinterpret_cast<uint32_t*>(smem + F::CTR_OFF) + threadIdx.x * WORDS;
+    uint32_t* misc = reinterpret_cast<uint32_t*>(smem + F::MISC_OFF);
+    uint32_t c[WORDS], big = 0, sum = 0;
+    if constexpr (WORDS == 4) {
+        const uint4 q = *reinterpret_cast<const uint4*>(ctr);
+        c[0] = q.x, c[1] = q.y, c[2] = q.z, c[3] = q.w;
+        *reinterpret_cast<uint4*>(ctr) = make_uint4(0u, 0u, 0u, 0u);
+    } else if constexpr (WORDS == 2) {
+        const uint2 q = *reinterpret_cast<const uint2*>(ctr);
+        c[0] = q.x, c[1] = q.y;
+        *reinterpret_cast<uint2*>(ctr) = make_uint2(0u, 0u);
+    } else {
+        c[0] = *ctr;
+        *ctr = 0u;
+    }
+#pragma unroll
+    for (int i = 0; i < WORDS; ++i) {
+        big = __vmaxu4(big, c[i]);
+        sum = __dp4a(c[i], 0x01010101u, sum);
+    }
+    big = max(max(big & 0xffu, (big >> 8) & 0xffu), max((big >> 16) & 0xffu, big >> 24));
+    big = __reduce_max_sync(0xffffffffu, big);
+    if ((threadIdx.x & 31) == 0 && big > 1u) atomicMax(&misc[0], big);
+    uint32_t run = block_exclusive_scan_1b<THREADS>(sum, reinterpret_cast<uint32_t*>(smem + F::SCAN_OFF));
+    if (threadIdx.x == THREADS - 1 && run + sum != cnt) atomicMax(&misc[0], 256u);
+    run += base;
+    uint32_t v[2 * WORDS];
+#pragma unroll
+    for (int i = 0; i < WORDS; ++i) {
+        const uint32_t b = run + (c[i] & 0xffu), d = b + ((c[i] >> 8) & 0xffu), e = d + ((c[i] >> 16) & 0xffu);
+        v[2 * i] = run | b << 16;
+        v[2 * i + 1] = d | e << 16;
+        run = e + (c[i] >> 24);
+    }
+    uint32_t* start = reinterpret_cast<uint32_t*>(smem + F::START_OFF) + threadIdx.x * 2 * WORDS;
+    if constexpr (WORDS == 1) {
+        *reinterpret_cast<uint2*>(start) = make_uint2(v[0], v[1]);
+    } else {
+#pragma unroll
+        for (int i = 0; i < WORDS / 2; ++i)
+            reinterpret_cast<uint4*>(start)[i] = make_uint4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+    }
+}
+
+template <int KB, int VB, int THREADS, int MIN_CTAS, int LIPT, int HALO>
+__global__ void __launch_bounds__(THREADS, MIN_CTAS) finish_kernel(FinishParams p) {
+    using U = typename KeyBits<KB>::U;
+    using V = typename ValBits<VB>::V;
+    using F = FinishGeom<KB, VB, THREADS, LIPT, HALO>;
+    using E = Placed<U>;
+    constexpr int WARPS = THREADS / 32, VEC = 16 / KB;
+    constexpr bool WIDE = KB > 4;
+    extern __shared__ __align__(128) uint8_t smem[];
+    uint32_t* ctr = reinterpret_cast<uint32_t*>(smem + F::CTR_OFF);
+    uint16_t* start = reinterpret_cast<uint16_t*>(smem + F::START_OFF);
+    uint32_t* misc = reinterpret_cast<uint32_t*>(smem + F::MISC_OFF);  // [0] largest sub-bucket
+    uint32_t* heads_last = reinterpret_cast<uint32_t*>(smem + F::HEADS_OFF);
+    uint32_t* heads_first = heads_last + WARPS;
+    V* sv = reinterpret_cast<V*>(smem + F::VALS_OFF);
+    uint8_t* uneven = smem;  // by a group's first place: its keys differ (before the keys are placed)
+    uint16_t* sp = reinterpret_cast<uint16_t*>(smem + F::POS_OFF);
+    auto put = [&](uint32_t place, U key, uint32_t before) {
+        if constexpr (WIDE) {
+            *reinterpret_cast<U*>(smem + F::at(place)) = key;
+            sp[place] = uint16_t(before);
+        } else {
+            *reinterpret_cast<uint64_t*>(smem + F::at(place)) = E::make(key, before).v;
+        }
+    };
+    auto get = [&](uint32_t place) {
+        if constexpr (WIDE) return E::make(*reinterpret_cast<const U*>(smem + F::at(place)), sp[place]);
+        else return E{*reinterpret_cast<const uint64_t*>(smem + F::at(place))};
+    };
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t lt = lanemask_lt();
+    grid_launch_dependents();
+    for (int i = tid; i < F::BINS / 4; i += THREADS) ctr[i] = 0u;
+    if (tid == 0) misc[0] = 0u;
+    grid_dependency_wait();
+    if ((ld_relaxed(p.state) & MSD_OFF) || !(ld_relaxed(p.executed) >> 31)) return;
+    const bool in_b = finish_in_b(p);
+    const U* keys = static_cast<const U*>(in_b ? p.keys_b : p.keys_a);
+    const V* vals = static_cast<const V*>(in_b ? p.vals_b : p.vals_a);
+    U* okeys = static_cast<U*>(p.keys_a);
+    V* ovals = static_cast<V*>(p.vals_a);
+    const uint32_t n = uint32_t(p.n), lo = ld_relaxed(p.window), chunk = ld_relaxed(p.window + 1);
+    const uint32_t chunks = (n + chunk - 1) / chunk, gshift = 8u * lo;
+    const KeyMap<U> map(p.kind, p.desc);
+    const U group_bits = U(~U(0)) << gshift;
+
+    // The CTA's windows are blockIdx.x, + gridDim.x, ...; lane l holds the
+    // edges of the l-th of the next 32, and those that are not empty (where
+    // groups are larger than a chunk many are) come one by one.
+    uint32_t batch = blockIdx.x, b0 = 0, b1 = 0, left = 0;
+    uint32_t e0 = 0, e1 = 0;
+    auto advance = [&] {  // the next window; false: none left
+        while (left == 0u) {
+            if (batch >= chunks) return false;
+            const uint64_t c = uint64_t(batch) + uint64_t(lane) * gridDim.x;
+            b0 = c < chunks ? p.edges[c] : 0u;
+            b1 = c < chunks ? p.edges[c + 1] : 0u;
+            left = __ballot_sync(0xffffffffu, ((b0 ^ b1) & 0x7fffffffu) != 0u);
+            batch = uint64_t(batch) + 32ull * gridDim.x < chunks ? batch + 32u * gridDim.x : chunks;
+        }
+        const int l = __ffs(left) - 1;
+        left &= left - 1u;
+        e0 = __shfl_sync(0xffffffffu, b0, l);
+        e1 = __shfl_sync(0xffffffffu, b1, l);
+        return true;
+    };
+    // place q of a window: the pair at s - pad + q; pad puts the lanes' chunks
+    // on 32-byte boundaries of the result
+    const uint32_t c0 = uint32_t(tid) * LIPT;
+    U k[LIPT];
+    auto pad_of = [&](uint32_t at) { return uint32_t(reinterpret_cast<uintptr_t>(okeys + at) & 31u) / uint32_t(KB); };
+    auto load = [&] {  // the window's keys, a chunk a thread
+        const uint32_t at = e0 & 0x7fffffffu, pad = pad_of(at), end = pad + (e1 & 0x7fffffffu) - at;
+        const U* kp = keys + at - pad + c0;
+        if (c0 >= pad && c0 + LIPT <= end && (reinterpret_cast<uintptr_t>(kp) & 15u) == 0u) {
+#pragma unroll
+            for (int i = 0; i < LIPT / VEC; ++i) {
+                union { uint4 q; U x[VEC]; } w;
+                w.q = reinterpret_cast<const uint4*>(kp)[i];
+#pragma unroll
+                for (int e = 0; e < VEC; ++e) k[i * VEC + e] = w.x[e];
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < LIPT; ++i) k[i] = (c0 + i >= pad && c0 + i < end) ? kp[i] : U(0);
+        }
+    };
+    bool more = advance();
+    if (more) load();
+    __syncthreads();
+    while (more) {
+        const uint32_t w0 = e0, w1 = e1;
+        const uint32_t s = w0 & 0x7fffffffu, cnt = (w1 & 0x7fffffffu) - s;
+        if (cnt > uint32_t(F::CAP)) {  // (the edges keep cnt <= CAP)
+            if (tid == 0) atomicOr(p.err, ERRBIT_BOUNDS);
+            more = advance();
+            if (more) load();
+            continue;
+        }
+        const uint32_t pad = pad_of(s), end = pad + cnt;
+        const U* kp = keys + s - pad;
+        const bool some = c0 < end && c0 + LIPT > pad;
+        const uint32_t i0 = some && c0 < pad ? pad - c0 : 0u, i1 = some ? min(end - c0, uint32_t(LIPT)) : 0u;
+        // ---- group heads: the last one at or before, the first one after
+        U prev = shfl_up1(k[LIPT - 1]);
+        if (lane == 0 && some && c0 > pad) prev = kp[c0 - 1];
+        const bool whole = i0 == 0u && i1 == uint32_t(LIPT) && c0 != pad;  // every key has one before it
+        const bool all_whole = __all_sync(0xffffffffu, whole);
+        uint32_t heads = 0;  // bit i: key i starts a group
+#pragma unroll
+        for (int i = 0; i < LIPT; ++i)
+            if (((k[i] ^ (i ? k[i ? i - 1 : 0] : prev)) & group_bits) != U(0)) heads |= 1u << i;
+        const uint32_t valid = (1u << i1) - (1u << i0);  // bit i: key i is one of the window
+        if (!all_whole) {
+            heads &= valid;
+            if (some && c0 <= pad) heads |= 1u << (pad - c0);
+        }
+        const uint32_t last = heads ? c0 + 31u - __clz(heads) : 0u;
+        const uint32_t firsth = heads ? c0 + __ffs(heads) - 1u : end;
+        const uint32_t with = __ballot_sync(0xffffffffu, heads != 0u);  // lanes with a head
+        const uint32_t under = with & lt, over = with & ~lt & ~(1u << lane);
+        uint32_t gs = __shfl_sync(0xffffffffu, last, under ? 31 - __clz(under) : 0);
+        uint32_t next = __shfl_sync(0xffffffffu, firsth, over ? __ffs(over) - 1 : 0);
+        if (lane == (with ? 31 - __clz(with) : 0)) heads_last[warp] = last;
+        if (lane == (with ? __ffs(with) - 1 : 0)) heads_first[warp] = firsth;
+        __syncthreads();
+        // the values arrive while the keys are sorted
+        if ((reinterpret_cast<uintptr_t>(vals + s - pad) & 15u) == 0u) {
+            constexpr uint32_t VVEC = 16 / VB;
+            for (uint32_t j = tid * VVEC; j < end; j += THREADS * VVEC) {
+                if (j >= pad && j + VVEC <= end) copy_async<16>(sv + j, vals + s - pad + j);
+                else
+                    for (uint32_t e = j; e < j + VVEC; ++e)
+                        if (e >= pad && e < end) copy_async<VB>(sv + e, vals + s - pad + e);
+            }
+        } else {
+            for (uint32_t j = pad + tid; j < end; j += THREADS) copy_async<VB>(sv + j, vals + s - pad + j);
+        }
+        {
+            const uint32_t l = __reduce_max_sync(0xffffffffu, lane < warp ? heads_last[lane] : 0u);
+            const uint32_t f = __reduce_min_sync(0xffffffffu, lane > warp && lane < WARPS ? heads_first[lane] : end);
+            gs = under ? gs : l;
+            next = over ? next : f;
+        }
+        // ---- count: sub-bucket and slot of every key.  First without looking
+        // whether groups consist of equal keys; when a sub-bucket then holds
+        // too many (or an edge cuts a group), again with that known: such a
+        // group's keys keep their places.
+        uint32_t where[LIPT];  // sub-bucket | slot << 16
+        // a key's bits below its group's, left-aligned in 32
+        auto below = [&](U x) {
+            if constexpr (KB == 4) return uint32_t(x) << (32u - gshift);
+            else return uint32_t((x << (8u * KB - gshift)) >> (8 * KB - 32));
+        };
+        auto take = [&](int i, uint32_t b) {
+            const uint32_t old = atomicAdd(reinterpret_cast<uint32_t*>(reinterpret_cast<uint8_t*>(ctr) + (b & ~3u)),
+                                           __funnelshift_l(1u, 1u, b * 8u));
+            where[i] = __byte_perm(b, __funnelshift_r(old, old, b * 8u), 0x5410) & 0xffffffu;
+        };
+        bool marked = ((w0 | w1) >> 31) != 0u, cut = false;
+        uint32_t most;
+        const bool all_few = __all_sync(0xffffffffu, (heads & (heads - 1u)) == 0u);  // a lane's keys: two groups at most
+        for (;;) {
+            if (marked) {
+                for (int i = tid; i < F::PLACES / 4; i += THREADS) reinterpret_cast<uint32_t*>(uneven)[i] = 0u;
+                __syncthreads();
+                uint32_t g = gs;
+#pragma unroll
+                for (int i = 0; i < LIPT; ++i) {
+                    if ((heads >> i) & 1u) g = c0 + i;
+                    else if (((valid >> i) & 1u) && k[i] != (i ? k[i ? i - 1 : 0] : prev)) uneven[g] = 1;
+                }
+                __syncthreads();
+                // an edge through a group of different keys: nothing this window can do
+                if ((w0 >> 31) && uneven[pad]) cut = true;
+                if (w1 >> 31) {  // the window's last group
+                    uint32_t last_group = 0;
+#pragma unroll
+                    for (int q = 0; q < WARPS; ++q) last_group = max(last_group, heads_last[q]);
+                    if (uneven[last_group]) cut = true;
+                }
+            }
+            if (all_whole && all_few && !marked) {
+                const int h = heads ? __ffs(heads) - 1 : LIPT;
+                const uint32_t g1 = c0 + h, m0 = (heads ? g1 : next) - gs, m1 = next - g1;
+#pragma unroll
+                for (int i = 0; i < LIPT; ++i) take(i, (i < h ? gs : g1) + __umulhi(below(k[i]), i < h ? m0 : m1));
+            } else {
+                uint32_t g = gs;
+#pragma unroll
+                for (int i = 0; i < LIPT; ++i) {
+                    if ((heads >> i) & 1u) g = c0 + i;
+                    const uint32_t rest = heads & ~((2u << i) - 1u);  // the heads after this key
+                    const uint32_t m = (rest ? c0 + __ffs(rest) - 1u : next) - g;
+                    if ((valid >> i) & 1u) take(i, marked && !uneven[g] ? c0 + i : g + __umulhi(below(k[i]), m));
+                }
+            }
+            __syncthreads();
+            scan_bins<F, THREADS>(smem, cnt, pad);
+            __syncthreads();
+            most = misc[0];
+            if (marked || most <= uint32_t(HALO * LIPT)) break;
+            marked = true;
+            __syncthreads();
+            if (tid == 0) misc[0] = 0u;
+        }
+        if (cut || most > MSD_RANK_MAX) {
+            // as it was, untwiddled (keys are in registers, values in shared memory)
+#pragma unroll
+            for (int i = 0; i < LIPT; ++i)
+                if ((valid >> i) & 1u) okeys[s - pad + c0 + i] = map.out(k[i]);
+            copy_async_wait();
+            __syncthreads();
+            for (uint32_t j = tid; j < cnt; j += THREADS) ovals[s + j] = sv[pad + j];
+            if (tid == 0) {
+                atomicOr(p.state, MSD_GAVE_UP);
+                misc[0] = 0u;
+            }
+            more = advance();
+            if (more) load();
+            __syncthreads();
+            continue;
+        }
+        auto move = [&](int i) { put(uint32_t(start[where[i] & 0xffffu]) + (where[i] >> 16), k[i], c0 + i); };
+        if (all_whole) {
+#pragma unroll
+            for (int i = 0; i < LIPT; ++i) move(i);
+        } else {
+#pragma unroll
+            for (int i = 0; i < LIPT; ++i)
+                if ((valid >> i) & 1u) move(i);
+        }
+        copy_async_wait();
+        __syncthreads();
+        if (tid == 0) misc[0] = 0u;
+        more = advance();
+        if (more) load();  // the next window's keys, while this one's are put in order
+        if (most <= uint32_t(HALO * LIPT)) {
+            // chunks [warp * (32 - 2 HALO), ...) and the neighbours' beyond both ends
+            const int ch = warp * (32 - 2 * HALO) + lane - HALO;
+            const int d0 = ch * LIPT;
+            if (warp * F::OUT < int(end)) {
+                E x[LIPT];
+                const bool inside = d0 >= int(pad) && uint32_t(d0 + LIPT) <= end;
+                const E least = E::make(U(0), 0u), greatest = E::make(U(~U(0)), 0xffffu);
+                if (d0 + LIPT <= int(pad) || d0 >= int(end)) {
+#pragma unroll
+                    for (int i = 0; i < LIPT; ++i) x[i] = d0 < int(pad) ? least : greatest;
+                } else {
+                    const uint4* q = reinterpret_cast<const uint4*>(smem + uint32_t(ch) * F::STRIDE);
+                    if constexpr (WIDE) {
+                        const uint32_t* pj = reinterpret_cast<const uint32_t*>(sp + d0);
+#pragma unroll
+                        for (int i = 0; i < LIPT / VEC; ++i) {
+                            union { uint4 v; U k[VEC]; } w;
+                            w.v = q[i];
+#pragma unroll
+                            for (int e = 0; e < VEC; ++e) {
+                                const int u = i * VEC + e;
+                                const uint32_t jj = pj[u / 2];
+                                x[u] = E::make(w.k[e], u & 1 ? jj >> 16 : jj & 0xffffu);
+                            }
+                        }
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < LIPT / 2; ++i) {
+                            union { uint4 v; E w[2]; } w;
+                            w.v = q[i];
+                            x[2 * i] = w.w[0];
+                            x[2 * i + 1] = w.w[1];
+                        }
+                    }
+                    if (!inside) {
+#pragma unroll
+                        for (int i = 0; i < LIPT; ++i) {
+                            if (d0 + i < int(pad)) x[i] = least;
+                            if (d0 + i >= int(end)) x[i] = greatest;
+                        }
+                    }
+                }
+                if (most > 1u) placed_rounds<U, LIPT>(x, most, lane);
+                if (lane >= HALO && lane < 32 - HALO && d0 < int(end)) {
+                    U* ok = okeys + s - pad + d0;
+                    V* ov = ovals + s - pad + d0;
+                    if (inside) {
+#pragma unroll
+                        for (int i = 0; i < LIPT * KB / 32; ++i) {
+                            union { uint4 q[2]; U k[32 / KB]; } y;
+#pragma unroll
+                            for (int e = 0; e < 32 / KB; ++e) y.k[e] = map.out(x[i * (32 / KB) + e].key());
+                            store_32b(ok + i * (32 / KB), y.q[0], y.q[1]);
+                        }
+                        if ((reinterpret_cast<uintptr_t>(ov) & 15u) == 0u) {
+#pragma unroll
+                            for (int i = 0; i < LIPT * VB / 16; ++i) {
+                                union { uint4 q; V v[16 / VB]; } y;
+#pragma unroll
+                                for (int e = 0; e < 16 / VB; ++e) y.v[e] = sv[x[i * (16 / VB) + e].place()];
+                                reinterpret_cast<uint4*>(ov)[i] = y.q;
+                            }
+                        } else {
+#pragma unroll
+                            for (int i = 0; i < LIPT; ++i) ov[i] = sv[x[i].place()];
+                        }
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < LIPT; ++i) {
+                            if (d0 + i >= int(pad) && d0 + i < int(end)) {
+                                ok[i] = map.out(x[i].key());
+                                ov[i] = sv[x[i].place()];
+                            }
+                        }
+                    }
+                }
+            }
+        } else {
+            // a pair's place is its sub-bucket's start plus the sub-bucket's
+            // other pairs before it; the sub-bucket of a place: the last one
+            // that starts at or before it and is not empty
+            for (uint32_t i = pad + tid; i < end; i += THREADS) {
+                uint32_t a = 0, z = F::BINS;
+                while (z - a > 1u) {
+                    const uint32_t mid = (a + z) / 2;
+                    if (start[mid] <= i) a = mid;
+                    else z = mid;
+                }
+                const uint32_t q0 = start[a], q1 = a + 1 < uint32_t(F::BINS) ? uint32_t(start[a + 1]) : end;
+                const E me = get(i);
+                uint32_t before = 0;
+                for (uint32_t q = q0; q < q1; ++q) before += after(me, get(q));
+                okeys[s - pad + q0 + before] = map.out(me.key());
+                ovals[s - pad + q0 + before] = sv[me.place()];
+            }
+        }
+    }
+}
+
+}  // namespace gbsort

@@ -3,6 +3,7 @@
 // parallel translation units.
 #pragma once
 
+#include "finish.cuh"
 #include "fused_short.cuh"
 #include "msd.cuh"
 #include "onesweep.cuh"
@@ -18,6 +19,22 @@ KernelEntry make_pass_entry() {
         reinterpret_cast<const void*>(
             &onesweep_pass_kernel<KB, VB, W, S::THREADS, S::IPT, SEG, S::MIN_CTAS, S::LOOKBACK_WINDOW>),
         S::THREADS, S::IPT, G::TILE, static_cast<unsigned long>(G::SMEM_BYTES)};
+}
+
+// Several passes in one cooperative launch: [0: 32-bit status, 1: 64-bit
+// status, 2: small-n shape] (the sorts by leading digits).
+template <int KB, int VB, class W, class S = PassShape<KB, VB>>
+KernelEntry make_multi_entry() {
+    using G = PassGeom<KB, VB, S::THREADS, S::IPT>;
+    return KernelEntry{reinterpret_cast<const void*>(&onesweep_multi_kernel<KB, VB, W, S::THREADS, S::IPT, S::MIN_CTAS,
+                                                                            S::LOOKBACK_WINDOW>),
+                       S::THREADS, S::IPT, G::TILE, static_cast<unsigned long>(G::SMEM_BYTES)};
+}
+template <int KB, int VB>
+const KernelEntry* multi_entries_of() {
+    static const KernelEntry e[3] = {make_multi_entry<KB, VB, uint32_t>(), make_multi_entry<KB, VB, uint64_t>(),
+                                     make_multi_entry<KB, VB, uint32_t, PassShapeSmall<KB, VB>>()};
+    return e;
 }
 
 // [value size][0: 32-bit status, 1: 64-bit status, 2: small-n shape (32-bit)]
@@ -83,6 +100,25 @@ const KernelEntry* msd_entries_for() {
          GS::TILE, static_cast<unsigned long>(GS::SMEM_BYTES)},
         make_msd_local_entry<KB, 0>(),
         make_msd_local_entry<KB, 1>(),
+    };
+    return e;
+}
+
+// Key-value sorts by their leading digits: sample, edges, finish (4- and
+// 8-byte values).
+template <int KB>
+const KernelEntry* finish_entries_for() {
+    using S = FinishShape<KB>;
+    using F4 = FinishGeom<KB, 4, S::THREADS, S::LIPT, S::HALO>;
+    using F8 = FinishGeom<KB, 8, S::THREADS, S::LIPT, S::HALO>;
+    static const KernelEntry e[4] = {
+        {reinterpret_cast<const void*>(&finish_sample_kernel<KB>), FINISH_SAMPLE_THREADS, 0, finish_levels<KB>() + 1,
+         static_cast<unsigned long>(FINISH_SAMPLE_SMEM)},
+        {reinterpret_cast<const void*>(&finish_edges_kernel<KB>), 256, 0, 0, 0ul},
+        {reinterpret_cast<const void*>(&finish_kernel<KB, 4, S::THREADS, S::MIN_CTAS, S::LIPT, S::HALO>), S::THREADS, F4::LIPT,
+         F4::CAP, static_cast<unsigned long>(F4::SMEM_BYTES)},
+        {reinterpret_cast<const void*>(&finish_kernel<KB, 8, S::THREADS, S::MIN_CTAS, S::LIPT, S::HALO>), S::THREADS, F8::LIPT,
+         F8::CAP, static_cast<unsigned long>(F8::SMEM_BYTES)},
     };
     return e;
 }

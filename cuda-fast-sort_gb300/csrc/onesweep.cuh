@@ -135,6 +135,9 @@ __global__ void __launch_bounds__(HIST_THREADS, 1) upsweep_kernel(HistParams p) 
         for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
         if (lane == 0 && s) atomicAdd(&p.gp_counts[bin], static_cast<unsigned long long>(s));
     }
+    // (launched beside the sample of a sort by leading digits: whatever waits
+    // for this grid finds that one complete too)
+    grid_dependency_wait();
 }
 
 
@@ -195,14 +198,34 @@ struct PassGeom {
     }
 };
 
+// Passes that do not run because one digit holds all n keys (bit q: digit q),
+// from every pass's counts; word: a shared word.
+__device__ __forceinline__ uint32_t pass_mask(const PassParams& p, uint32_t* word) {
+    const int tid = threadIdx.x;
+    if (tid == 0) *word = 0u;
+    __syncthreads();
+    if (tid < 256) {
+        uint32_t m = 0;
+        for (int q = 0; q < p.passes; ++q) m |= uint32_t(p.gp_all[size_t(q) * 256 + tid] == p.n) << q;
+        if (m) atomicOr(word, m);
+    }
+    __syncthreads();
+    return *word;
+}
+
 // One onesweep digit pass.  SEG = false: one array of n keys.  SEG = true:
 // many independent segments; global tile g is p.tiles[g] (segment, base,
 // count), each segment's first tile publishes an inclusive prefix of its own
 // so lookback chains never cross segments, and digit bases come per segment
 // from p.seg_gofs.
-// The pass as a device function, run once by the pass kernel below.
-template <int KB, int VB, class W, int THREADS, int IPT, bool SEG, int LBW>
-__device__ __forceinline__ void onesweep_pass_body(const PassParams& p, uint8_t* smem) {
+// The pass on digit `pass` as a device function.  The pass kernel below runs
+// it once.  MULTI: the kernel of several passes, which knows the passes that do
+// not run (uniform, bit q: digit q) and has the digit offsets in shared memory
+// already; final: the last pass that runs maps the keys back.  False: a copy
+// ran out of time, or (not MULTI) the pass does not run.
+template <int KB, int VB, class W, int THREADS, int IPT, bool SEG, int LBW, bool MULTI = false>
+__device__ __forceinline__ bool onesweep_pass_body(const PassParams& p, uint8_t* smem, int pass, uint32_t uniform = 0,
+                                                   bool final = true) {
     using U = typename KeyBits<KB>::U;
     using V = typename ValBits<VB>::V;
     using G = PassGeom<KB, VB, THREADS, IPT>;
@@ -217,17 +240,6 @@ __device__ __forceinline__ void onesweep_pass_body(const PassParams& p, uint8_t*
     TileInfo* info_slot = reinterpret_cast<TileInfo*>(smem + G::INFO_OFF);
     uint32_t* binb32 = reinterpret_cast<uint32_t*>(smem + G::BINB32_OFF);
     uint32_t* match_scratch = reinterpret_cast<uint32_t*>(smem + G::MATCH_OFF);
-    if constexpr (!G::HALF && rank_uses_or(IPT)) {
-        for (int i = threadIdx.x; i < G::WARPS * 256; i += THREADS) match_scratch[i] = 0u;
-    }
-    // Launched as a dependent of the previous kernel of the sort (plain mode):
-    // let the next one be scheduled, then wait for this one's inputs.  Every
-    // CTA of a pass is resident at once (grid <= SMs x occupancy), so the
-    // successor never holds slots a CTA of this pass still needs.
-    grid_launch_dependents();
-    grid_dependency_wait();
-    if (p.msd_state && ld_relaxed(p.msd_state) == 0u) return;  // the MSD kernels sorted
-
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     // Tile position of item u of this thread: warp-striped (a warp's 32 lanes
     // read 32 consecutive keys per column), or with HALF half-warp-striped
@@ -240,7 +252,7 @@ __device__ __forceinline__ void onesweep_pass_body(const PassParams& p, uint8_t*
     };
     const uint32_t T = p.num_tiles;
     const uint64_t n = p.n;
-    const int pass = p.pass, kind = p.kind, desc = p.desc;
+    const int kind = p.kind, desc = p.desc;
     const uint32_t epoch = uint32_t(pass);
     W* status = static_cast<W*>(p.status);
     const void* keys_in = p.keys_in;
@@ -250,27 +262,15 @@ __device__ __forceinline__ void onesweep_pass_body(const PassParams& p, uint8_t*
     int twiddle_load = p.twiddle_load, twiddle_store = p.twiddle_store;
     {
         if (p.skip || p.copy_keys_in) {
-            uint32_t uniform = 0;
             const uint32_t all = (p.passes >= 32) ? 0xffffffffu : ((1u << p.passes) - 1u);
-            if (p.skip) {
+            if (!MULTI && p.skip) {
                 if constexpr (SEG) {
                     // the batched scan marked every pass whose digit varies in some segment
                     uniform = ~ld_relaxed(p.nonuniform_mask) & all;
                 } else {
-                    // a pass is uniform when one digit holds all n keys
-                    uint32_t* smask = reinterpret_cast<uint32_t*>(smem + G::SKIP_OFF);
-                    if (tid == 0) *smask = 0u;
-                    __syncthreads();
-                    if (tid < 256) {
-                        uint32_t m = 0;
-                        for (int q = 0; q < p.passes; ++q)
-                            m |= uint32_t(p.gp_all[size_t(q) * 256 + tid] == n) << q;
-                        if (m) atomicOr(smask, m);
-                    }
-                    __syncthreads();
-                    uniform = *smask;
+                    uniform = pass_mask(p, reinterpret_cast<uint32_t*>(smem + G::SKIP_OFF));
                 }
-                if ((uniform >> pass) & 1u) return;  // every CTA of this pass leaves: a no-op pass
+                if ((uniform >> pass) & 1u) return false;  // every CTA of this pass leaves: a no-op pass
             }
             const int before = __popc(~uniform & ((1u << pass) - 1u));  // executed passes before this one
             const int total = __popc(~uniform & all);
@@ -289,7 +289,7 @@ __device__ __forceinline__ void onesweep_pass_body(const PassParams& p, uint8_t*
                 vals_out = from_b ? p.vals_a : p.vals_b;
             }
             twiddle_load = before == 0;
-            twiddle_store = before + 1 == total;
+            twiddle_store = before + 1 == total && final;
             if constexpr (!SEG) {
                 if (p.executed && blockIdx.x == 0 && tid == 0) *p.executed = 0x80000000u | uint32_t(total);
             }
@@ -304,13 +304,20 @@ __device__ __forceinline__ void onesweep_pass_body(const PassParams& p, uint8_t*
         mbar_init(&mbar[2], 1);
         fence_mbar_init();
     }
-    if constexpr (!SEG) {  // global exclusive digit offsets of this pass (once per CTA)
+    if constexpr (!SEG && !MULTI) {  // global exclusive digit offsets of this pass (once per CTA)
         const unsigned long long c = (tid < 256) ? p.gp_counts[tid] : 0ull;
         const unsigned long long ex = block_exclusive_scan_256<unsigned long long>(c, scan64, nullptr);
         if (tid < 256) gexcl[tid] = ex;
     }
 
     // Thread 0: describe tile t (its table entry `rec` in batched mode).
+    uint32_t* tile_counter = p.tile_counter + (MULTI ? pass - p.pass : 0);
+    // MULTI: every CTA is resident and starts at about the same time, so with
+    // few tiles a CTA the first ones need no claim (with many, claims in the
+    // order of arrival make up for it: 4 x 10^6 8-byte keys + values, three
+    // passes, 209 against 228 us)
+    const bool given = MULTI && T <= 4u * gridDim.x;
+    auto claim = [&] { return atomicAdd(tile_counter, 1u) + (given ? gridDim.x : 0u); };
     auto make_info = [&](uint32_t t, const TileRec& rec) {
         TileInfo ti{};
         ti.id = t;
@@ -380,14 +387,14 @@ __device__ __forceinline__ void onesweep_pass_body(const PassParams& p, uint8_t*
 #endif
     __syncthreads();
     if (tid == 0) {
-        const uint32_t t0 = atomicAdd(p.tile_counter, 1u);
+        const uint32_t t0 = given ? blockIdx.x : claim();
         const TileInfo i0 = make_info(t0, load_rec(t0));
         info_slot[0] = i0;
         if (t0 < T) issue_tile(i0, 0);
 #if GBSORT_TILE_LOOKAHEAD >= 3
-        id_an = t0 < T ? atomicAdd(p.tile_counter, 1u) : T;
+        id_an = t0 < T ? claim() : T;
         rec_an = load_rec(id_an);
-        id_aan = id_an < T ? atomicAdd(p.tile_counter, 1u) : T;
+        id_aan = id_an < T ? claim() : T;
 #endif
     }
     __syncthreads();
@@ -407,7 +414,7 @@ __device__ __forceinline__ void onesweep_pass_body(const PassParams& p, uint8_t*
 #if GBSORT_TILE_LOOKAHEAD >= 3
             const TileInfo ni = make_info(id_an, rec_an);
 #else  // claim the next tile only now: a CTA holds two claims at most
-            const uint32_t nid = atomicAdd(p.tile_counter, 1u);
+            const uint32_t nid = claim();
             const TileInfo ni = make_info(nid, load_rec(nid));
 #endif
             info_slot[(it + 1) & 1u] = ni;
@@ -418,7 +425,7 @@ __device__ __forceinline__ void onesweep_pass_body(const PassParams& p, uint8_t*
 #if GBSORT_TILE_LOOKAHEAD >= 3
                 rec_an = load_rec(id_aan);
                 id_an = id_aan;
-                id_aan = id_aan < T ? atomicAdd(p.tile_counter, 1u) : T;
+                id_aan = id_aan < T ? claim() : T;
 #endif
             }
         }
@@ -502,7 +509,7 @@ __device__ __forceinline__ void onesweep_pass_body(const PassParams& p, uint8_t*
                 if (next_issued) mbar_wait_bounded(&mbar[b ^ 1], (parity >> (b ^ 1)) & 1u, DRAIN_LIMIT_NS, p.err);
                 if constexpr (G::LATE) mbar_wait_bounded(&mbar[2], vparity, DRAIN_LIMIT_NS, p.err);
             }
-            return;
+            return false;
         }
         const TileInfo next_info = info_slot[(it + 1) & 1u];
 
@@ -688,7 +695,7 @@ __device__ __forceinline__ void onesweep_pass_body(const PassParams& p, uint8_t*
                     if (next_issued)
                         mbar_wait_bounded(&mbar[b ^ 1], (parity >> (b ^ 1)) & 1u, DRAIN_LIMIT_NS, p.err);
                 }
-                return;
+                return false;
             }
         } else {
             __syncthreads();
@@ -696,12 +703,93 @@ __device__ __forceinline__ void onesweep_pass_body(const PassParams& p, uint8_t*
         cur = next_info;
         ++it;
     }
+    return true;
 }
 
 template <int KB, int VB, class W, int THREADS, int IPT, bool SEG, int MIN_CTAS, int LBW>
 __global__ void __launch_bounds__(THREADS, MIN_CTAS) onesweep_pass_kernel(PassParams p) {
+    using G = PassGeom<KB, VB, THREADS, IPT>;
     extern __shared__ __align__(128) uint8_t smem[];
-    onesweep_pass_body<KB, VB, W, THREADS, IPT, SEG, LBW>(p, smem);
+    if constexpr (!G::HALF && rank_uses_or(IPT)) {
+        uint32_t* match_scratch = reinterpret_cast<uint32_t*>(smem + G::MATCH_OFF);
+        for (int i = threadIdx.x; i < G::WARPS * 256; i += THREADS) match_scratch[i] = 0u;
+    }
+    // Launched as a dependent of the previous kernel of the sort (plain mode):
+    // let the next one be scheduled, then wait for this one's inputs.  Every
+    // CTA of a pass is resident at once (grid <= SMs x occupancy), so the
+    // successor never holds slots a CTA of this pass still needs.
+    grid_launch_dependents();
+    grid_dependency_wait();
+    if (p.msd_state && ld_relaxed(p.msd_state) == 0u) return;  // the MSD kernels sorted
+    onesweep_pass_body<KB, VB, W, THREADS, IPT, SEG, LBW>(p, smem, p.pass);
+}
+
+__device__ __forceinline__ void grid_copy_bytes(void* dst, const void* src, uint64_t bytes);
+
+// Digits p.pass .. p.last_pass in one cooperative launch, a grid barrier
+// between the passes that run, then the parity fix-up.  Used where most passes
+// do not run (a launch that exits costs about 2.2 us, a barrier with the next
+// pass's start about 2 us more than a launch that overlaps its predecessor's
+// end: eight passes of 65537 8-byte keys with three that run 44 against 47 us,
+// four that all run 55 against 47).
+template <int KB, int VB, class W, int THREADS, int IPT, int MIN_CTAS, int LBW>
+__global__ void __launch_bounds__(THREADS, MIN_CTAS) onesweep_multi_kernel(PassParams p) {
+    using G = PassGeom<KB, VB, THREADS, IPT>;
+    extern __shared__ __align__(128) uint8_t smem[];
+    if constexpr (!G::HALF && rank_uses_or(IPT)) {
+        uint32_t* match_scratch = reinterpret_cast<uint32_t*>(smem + G::MATCH_OFF);
+        for (int i = threadIdx.x; i < G::WARPS * 256; i += THREADS) match_scratch[i] = 0u;
+    }
+    grid_launch_dependents();
+    grid_dependency_wait();
+    if (p.msd_state && (ld_relaxed(p.msd_state) & p.state_mask) == 0u) return;  // sorted already
+    uint32_t left_out = 0;  // digits below the leading ones
+    if (p.leading && !(ld_relaxed(p.leading) & MSD_OFF)) left_out = (1u << ld_relaxed(p.leading + 1)) - 1u;
+    const uint32_t uniform = left_out | pass_mask(p, reinterpret_cast<uint32_t*>(smem + G::SKIP_OFF));
+    const uint32_t all = (p.passes >= 32) ? 0xffffffffu : ((1u << p.passes) - 1u);
+    const int total = __popc(~uniform & all);
+    const bool to_b = !p.copy_keys_in && (total & 1) != 0;  // where the last pass leaves the result
+    const bool move = left_out == 0u && (p.copy_keys_in ? total == 0 : (total & 1) != p.want_odd);
+    auto offsets = [&](int pass) {  // the pass's digit offsets
+        const int tid = threadIdx.x;
+        const unsigned long long c = (tid < 256) ? p.gp_all[size_t(pass) * 256 + tid] : 0ull;
+        const unsigned long long ex = block_exclusive_scan_256<unsigned long long>(
+            c, reinterpret_cast<unsigned long long*>(smem + G::SCAN64_OFF), nullptr);
+        if (tid < 256) reinterpret_cast<unsigned long long*>(smem + G::GEXCL_OFF)[tid] = ex;
+    };
+    uint32_t barriers = 0;
+    if (p.clear_bytes) {
+        uint4* st = static_cast<uint4*>(p.status);
+        for (uint64_t i = uint64_t(blockIdx.x) * THREADS + threadIdx.x; i < p.clear_bytes / 16;
+             i += uint64_t(gridDim.x) * THREADS)
+            st[i] = make_uint4(0, 0, 0, 0);
+        if (!grid_barrier(p.barrier, p.barrier_gen, ++barriers, p.wait_limit_ns, p.err)) return;
+    }
+    uint32_t runs = ~uniform & all;
+    if (runs) offsets(__ffs(runs) - 1);
+    while (runs) {
+        const int pass = __ffs(runs) - 1;
+        runs &= runs - 1u;
+        if (!onesweep_pass_body<KB, VB, W, THREADS, IPT, false, LBW, true>(p, smem, pass, uniform, left_out == 0u))
+            return;
+        if (runs || move) {  // another pass, or the fix-up
+            __syncthreads();
+            if (threadIdx.x < 3) mbar_inval(reinterpret_cast<uint64_t*>(smem + G::MBAR_OFF) + threadIdx.x);
+            if (runs) offsets(__ffs(runs) - 1);
+            // the next pass's bulk copies read what the CTAs stored
+            fence_proxy_async_all();
+            if (!grid_barrier(p.barrier, p.barrier_gen, ++barriers, p.wait_limit_ns, p.err)) return;
+            fence_proxy_async_all();
+        }
+    }
+    if (move) {
+        const bool copied = p.copy_keys_in != nullptr;
+        const void* ks = copied ? p.copy_keys_in : to_b ? p.keys_b : p.keys_a;
+        const void* vs = copied ? p.copy_vals_in : to_b ? p.vals_b : p.vals_a;
+        const bool to_a = to_b || copied;
+        grid_copy_bytes(to_a ? p.keys_a : p.keys_b, ks, p.n * uint64_t(KB));
+        if constexpr (VB > 0) grid_copy_bytes(to_a ? p.vals_a : p.vals_b, vs, p.n * uint64_t(VB));
+    }
 }
 
 // Copies `bytes` from src to dst with all threads of the grid (16-byte

@@ -27,9 +27,12 @@ struct CtlLayout {
     size_t barrier_gen_off = 0;  // its generation word (another 128-byte line)
     size_t fill_off = 0;         // [256] fill counts of its MSD regions
     size_t overflow_off = 0;     // its region overflow flag
+    size_t counters2_off = 0;    // a second set of tile counters and a second grid barrier, for the
+                                 // digit passes after a sort by leading digits (0: none)
+    size_t sampled_off = 0;      // that sort's sample: ticket, [8] counts
     size_t msd_state_off = 0;    // outcome of the most-significant-first path, its code window [2]
     size_t bytes = 0;
-    static CtlLayout make(int passes) {
+    static CtlLayout make(int passes, bool finish = false) {
         CtlLayout c;
         c.gp_off = 0;
         c.counters_off = size_t(passes) * 256 * 8;
@@ -41,6 +44,11 @@ struct CtlLayout {
         c.overflow_off = c.fill_off + 256 * 4;
         c.msd_state_off = c.overflow_off + 4;
         c.bytes = align_up(c.msd_state_off + 12, 256);
+        if (finish) {
+            c.counters2_off = c.bytes;
+            c.sampled_off = c.counters2_off + 18 * 4;
+            c.bytes = align_up(c.sampled_off + 9 * 4, 256);
+        }
         return c;
     }
 };
@@ -92,6 +100,12 @@ struct Plan {
     uint32_t msd_group_cap = 0;
     int msd_b2 = 0;
     size_t msd_off = 0;
+    // key-value sorts by their leading digits (finish.cuh): sample, edges,
+    // finish, and the digit passes in one launch; the edges lie in the status
+    // words
+    bool finish = false;
+    KernelEntry multi{};
+    KernelEntry finish_k[3]{};
     size_t total_bytes = 0;
     CtlLayout ctl{};
 };

@@ -140,6 +140,21 @@ constexpr int msd_b2_max(uint64_t n, uint32_t cap) {
     return b2;
 }
 
+// Key-value sorts by their leading digits (finish.cuh): the finishing CTAs.
+// 8- and 16-byte keys with 4- or 8-byte values.  4-byte keys keep their four
+// digit passes: two of them and the finish take longer (2^26 u32 + u32 1.54
+// against 1.42 ms, finishing in CTAs of 768 threads; in 384 of 16 keys 1.84).
+template <int KB>
+struct FinishShape {
+    static constexpr int THREADS = 384;
+    static constexpr int LIPT = KB == 8 ? 8 : 4;
+    static constexpr int HALO = KB == 16 ? 2 : 1;
+    static constexpr int MIN_CTAS = 2;
+};
+constexpr bool finish_pairs(int kb, int vb) { return kb >= 8 && (vb == 4 || vb == 8); }
+constexpr uint64_t FINISH_N_MIN = 2048;  // (u64 + u32, uniform: 16385 pairs 45 us, the digit passes 78)
+constexpr uint64_t FINISH_N_MAX = (uint64_t(1) << 31) - 1;  // edges keep a flag in bit 31
+
 // Keys per MSD region of the one-launch sort (one region per top digit):
 // the mean bucket n/256 plus four of its standard deviations plus 64,
 // rounded up to 32 (uniform top digits overflow a region about once in

@@ -24,6 +24,7 @@
 #include "gbsort.h"
 #include "plan.h"
 #include "device_common.cuh"
+#include "finish.cuh"
 #include "fused_short.cuh"
 #include "msd.cuh"
 #include "onesweep.cuh"
@@ -47,6 +48,10 @@ const KernelEntry* fused_entry_k4();
 const KernelEntry* fused_entry_k8();
 const KernelEntry* fused_entry_k16();
 
+const KernelEntry* multi_entries_k8(int vb);
+const KernelEntry* multi_entries_k16(int vb);
+const KernelEntry* finish_entries_k8();
+const KernelEntry* finish_entries_k16();
 const KernelEntry* msd_entries_k4();
 const KernelEntry* msd_entries_k8();
 const KernelEntry* msd_entries_k16();
@@ -57,6 +62,15 @@ const KernelEntry* msd_entries(int kb) {
         case 4: return msd_entries_k4();
         case 8: return msd_entries_k8();
         case 16: return msd_entries_k16();
+        default: return nullptr;
+    }
+}
+
+// Kernels of the key-value sorts by leading digits (finish.cuh).
+const KernelEntry* finish_entries(int kb) {
+    switch (kb) {
+        case 8: return finish_entries_k8();
+        case 16: return finish_entries_k16();
         default: return nullptr;
     }
 }
@@ -313,7 +327,8 @@ int make_plan(int key_type, size_t value_bytes, uint64_t n, Plan* plan) {
     off = align_up(off + size_t(n) * kb, 256);
     p.alt_vals_off = off;
     off = align_up(off + size_t(n) * value_bytes, 256);
-    p.ctl = CtlLayout::make(p.passes);
+    const bool finish = finish_pairs(p.kb, p.vb) && n >= FINISH_N_MIN && n <= FINISH_N_MAX;
+    p.ctl = CtlLayout::make(p.passes, finish);
     p.ctl_off = off;
     off = align_up(off + p.ctl.bytes, 256);
     p.status_off = off;
@@ -354,6 +369,14 @@ int make_plan(int key_type, size_t value_bytes, uint64_t n, Plan* plan) {
             for (int i = 0; i < 5; ++i) p.msd_k[i] = msd_entries(p.kb)[i];
             p.msd_k[5] = msd_entries(p.kb)[5 + shape];
         }
+    }
+    if (finish && g_pass_skip.load(std::memory_order_relaxed)) {
+        p.finish = true;
+        const KernelEntry* e = finish_entries(p.kb);
+        p.finish_k[0] = e[0];
+        p.finish_k[1] = e[1];
+        p.finish_k[2] = e[p.vb == 4 ? 2 : 3];
+        p.multi = (p.kb == 8 ? multi_entries_k8(p.vb) : multi_entries_k16(p.vb))[small ? 2 : p.wide_status ? 1 : 0];
     }
     p.total_bytes = off;
     *plan = p;
@@ -422,7 +445,11 @@ int enqueue_sort(const Plan& plan, int descending, void* d_keys, void* d_values,
     };
 
     uint8_t* msd_block = use_msd ? ws + plan.msd_off - ws_base : nullptr;
-    uint32_t* msd_state = use_msd ? reinterpret_cast<uint32_t*>(ctl + plan.ctl.msd_state_off) : nullptr;
+    // (its digit passes run in one launch, which sort_timed does not use)
+    bool use_finish = plan.finish && ms == nullptr;
+    for (int i = 0; use_finish && i < 3; ++i) use_finish = prepare_kernel(plan.finish_k[i]) == GBSORT_OK;
+    use_finish = use_finish && prepare_kernel(plan.multi) == GBSORT_OK;
+    uint32_t* msd_state = use_msd || use_finish ? reinterpret_cast<uint32_t*>(ctl + plan.ctl.msd_state_off) : nullptr;
 
     // Parameters of digit pass `pass` and of the fix-up copy.
     auto pass_params = [&](int pass) {
@@ -460,7 +487,12 @@ int enqueue_sort(const Plan& plan, int descending, void* d_keys, void* d_values,
         pp.copy_keys_in = copy ? keys_src : nullptr;
         pp.copy_vals_in = copy ? vals_src : nullptr;
         pp.executed = fixup ? reinterpret_cast<uint32_t*>(ctl + plan.ctl.exec_off) : nullptr;
-        pp.msd_state = msd_state;
+        pp.msd_state = use_msd ? msd_state : nullptr;
+        pp.state_mask = MSD_OFF | MSD_GAVE_UP;
+        pp.leading = use_finish ? msd_state : nullptr;
+        pp.want_odd = alt ? (plan.passes & 1) : 0;
+        pp.barrier = reinterpret_cast<uint32_t*>(ctl + plan.ctl.barrier_off);
+        pp.barrier_gen = reinterpret_cast<uint32_t*>(ctl + plan.ctl.barrier_gen_off);
         return pp;
     };
     auto fixup_params = [&] {
@@ -476,7 +508,7 @@ int enqueue_sort(const Plan& plan, int descending, void* d_keys, void* d_values,
         fp.copy_keys_in = copy ? keys_src : nullptr;
         fp.copy_vals_in = copy ? vals_src : nullptr;
         fp.want_odd = alt ? (plan.passes & 1) : 0;
-        fp.msd_state = msd_state;
+        fp.msd_state = use_msd ? msd_state : nullptr;
         return fp;
     };
 
@@ -544,7 +576,59 @@ int enqueue_sort(const Plan& plan, int descending, void* d_keys, void* d_values,
     }
     const uint32_t hist_ctas = upsweep_ctas(plan.n, plan.kb);
     if (timed) cudaEventRecord(ev[0], stream);
-    if (use_msd) {
+    const int occ = resident_ctas(plan.pass);
+    const uint64_t max_ctas = uint64_t(sms) * uint64_t(occ > 0 ? occ : 1);
+    const uint32_t pass_ctas = uint32_t(plan.num_tiles < max_ctas ? plan.num_tiles : max_ctas);
+    // sorts by leading digits: every digit pass in one cooperative launch
+    auto launch_passes = [&](const PassParams& pp) {
+        const int occ_m = resident_ctas(plan.multi);
+        const uint64_t most = uint64_t(sms) * uint64_t(occ_m > 0 ? occ_m : 1);
+        PassParams q = pp;
+        void* args[] = {&q};
+        const cudaError_t r =
+            cudaLaunchCooperativeKernel(plan.multi.fn, dim3(uint32_t(plan.num_tiles < most ? plan.num_tiles : most)),
+                                        dim3(plan.multi.threads), args, plan.multi.smem, stream);
+        if (r != cudaSuccess) cudaGetLastError();
+        return r;
+    };
+    FinishParams fin{};
+    auto launch_finish = [&](int i, uint64_t grid) {
+        const KernelEntry& k = plan.finish_k[i];
+        const uint64_t full = uint64_t(sms > 0 ? sms : 1) * uint64_t(resident_ctas(k) > 0 ? resident_ctas(k) : 1);
+        void* args[] = {&fin};
+        return launch_dependent(k.fn, uint32_t(grid < full ? grid : full), k.threads, k.smem, stream, args);
+    };
+    if (use_finish) {
+        // Key-value pairs by their leading digits (finish.cuh): the sample,
+        // beside the histogram; the digit passes; edges and finish; and every
+        // digit pass again if that did not work out.
+        fin.keys_in = copy ? keys_src : d_keys;
+        fin.keys_a = d_keys;
+        fin.vals_a = d_values;
+        fin.keys_b = alt_keys;
+        fin.vals_b = alt_vals;
+        fin.n = plan.n;
+        fin.kind = plan.kind;
+        fin.desc = descending;
+        fin.copy = copy ? 1 : 0;
+        fin.state = msd_state;
+        fin.window = msd_state + 1;
+        fin.executed = reinterpret_cast<const uint32_t*>(ctl + plan.ctl.exec_off);
+        fin.ticket = reinterpret_cast<uint32_t*>(ctl + plan.ctl.sampled_off);
+        fin.sampled = fin.ticket + 1;
+        fin.edges = static_cast<uint32_t*>(status);
+        fin.max_chunks = uint32_t(plan.status_bytes / 4 - 2 < 0xffffffffull ? plan.status_bytes / 4 - 2 : 0xffffffffull);
+        fin.places = uint32_t(plan.finish_k[2].tile);
+        fin.err = err_word;
+        {  // an ordinary launch: the histogram, its dependent, does not wait for what came before
+            const KernelEntry& k = plan.finish_k[0];
+            void* args[] = {&fin};
+            e = cudaLaunchKernel(k.fn, dim3(k.tile), dim3(k.threads), args, k.smem, stream);
+            if (e != cudaSuccess) return fail("finish launch", e);
+        }
+        void* args[] = {&hp};
+        e = launch_dependent(plan.upsweep.fn, hist_ctas, plan.upsweep.threads, plan.upsweep.smem, stream, args);
+    } else if (use_msd) {
         // Keys only: sample, count, scan, top split, second split, local sorts
         // (msd.cuh); the histogram and the digit passes below exit at once
         // when these sorted, and otherwise sort from the input-preserving
@@ -591,15 +675,31 @@ int enqueue_sort(const Plan& plan, int descending, void* d_keys, void* d_values,
     if (e != cudaSuccess) return fail("upsweep launch", e);
     if (timed) cudaEventRecord(ev[1 + ms_stages], stream);
 
-    const int occ = resident_ctas(plan.pass);
-    const uint64_t max_ctas = uint64_t(sms) * uint64_t(occ > 0 ? occ : 1);
-    const uint32_t pass_ctas = uint32_t(plan.num_tiles < max_ctas ? plan.num_tiles : max_ctas);
-    for (int pass = 0; pass < plan.passes; ++pass) {
+    // a refused launch: every digit pass below, each in a launch of its own
+    if (use_finish && launch_passes(pass_params(0)) != cudaSuccess) use_finish = false;
+    for (int pass = 0; pass < plan.passes && !use_finish; ++pass) {
         PassParams pp = pass_params(pass);
         void* args[] = {&pp};
         e = launch_dependent(plan.pass.fn, pass_ctas, plan.pass.threads, plan.pass.smem, stream, args);
         if (e != cudaSuccess) return fail("pass launch", e);
         if (timed) cudaEventRecord(ev[2 + ms_stages + pass], stream);
+    }
+    if (use_finish) {
+        // chunks hold about places / 10 pairs at least, and a CTA of edges finds eight
+        e = launch_finish(1, plan.n / (fin.places / 11 * 8) + 1);
+        if (e == cudaSuccess) e = launch_finish(2, plan.n / (fin.places / 11) + 1);
+        if (e != cudaSuccess) return fail("finish launch", e);
+        PassParams pp = pass_params(0);
+        pp.msd_state = msd_state;
+        pp.state_mask = MSD_GAVE_UP;
+        pp.leading = nullptr;
+        pp.tile_counter = reinterpret_cast<uint32_t*>(ctl + plan.ctl.counters2_off);
+        pp.barrier = pp.tile_counter + 16;
+        pp.barrier_gen = pp.barrier + 1;
+        pp.clear_bytes = plan.status_bytes;
+        e = launch_passes(pp);
+        if (e != cudaSuccess) return fail("pass launch", e);
+        return GBSORT_OK;  // (the fix-up is part of those launches; nothing is timed)
     }
     if (fixup) {
         FixupParams fp = fixup_params();

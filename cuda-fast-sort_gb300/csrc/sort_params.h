@@ -82,8 +82,20 @@ struct PassParams {
     const uint32_t* nonuniform_mask;
     // plain mode with skipping: receives bit 31 | number of executed passes
     uint32_t* executed;
-    // keys-only sorts with the MSD path: the pass exits when it sorted (0)
+    // after a path that may already have sorted: nothing to do when its state
+    // is 0 (several passes in one launch: when none of these bits is set)
     const uint32_t* msd_state;
+    uint32_t state_mask;
+    // Several passes in one launch (plain mode, with skipping): digits pass ..
+    // passes - 1; tile_counter is the first of a counter per pass.
+    // leading, non-null: a sort by its leading digits ([0] without MSD_OFF:
+    // digits below [1] are left out, and the finish maps the keys back;
+    // finish.cuh)
+    const uint32_t* leading;
+    int want_odd;               // parity of executed passes that leaves the result where it belongs
+    uint32_t* barrier;          // grid barrier counter and generation, zeroed
+    uint32_t* barrier_gen;
+    uint64_t clear_bytes;       // status words to clear first (they hold an earlier run's)
 };
 
 // The copy home after uniform-pass skipping left an odd number of executed
