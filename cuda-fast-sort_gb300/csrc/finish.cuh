@@ -501,7 +501,9 @@ __global__ void __launch_bounds__(THREADS, MIN_CTAS) finish_kernel(FinishParams 
         if (lane == 0 && some && c0 > pad) prev = kp[c0 - 1];
         const bool whole = i0 == 0u && i1 == uint32_t(LIPT) && c0 != pad;  // every key has one before it
         const bool all_whole = __all_sync(0xffffffffu, whole);
+        const bool busy = warp * 32 * LIPT < int(end);  // the warp has keys of the window
         uint32_t heads = 0;  // bit i: key i starts a group
+        if (busy)
 #pragma unroll
         for (int i = 0; i < LIPT; ++i)
             if (((k[i] ^ (i ? k[i ? i - 1 : 0] : prev)) & group_bits) != U(0)) heads |= 1u << i;
@@ -580,7 +582,7 @@ __global__ void __launch_bounds__(THREADS, MIN_CTAS) finish_kernel(FinishParams 
                 const uint32_t g1 = c0 + h, m0 = (heads ? g1 : next) - gs, m1 = next - g1;
 #pragma unroll
                 for (int i = 0; i < LIPT; ++i) take(i, (i < h ? gs : g1) + __umulhi(below(k[i]), i < h ? m0 : m1));
-            } else {
+            } else if (busy) {
                 uint32_t g = gs;
 #pragma unroll
                 for (int i = 0; i < LIPT; ++i) {
@@ -620,7 +622,7 @@ __global__ void __launch_bounds__(THREADS, MIN_CTAS) finish_kernel(FinishParams 
         if (all_whole) {
 #pragma unroll
             for (int i = 0; i < LIPT; ++i) move(i);
-        } else {
+        } else if (busy) {
 #pragma unroll
             for (int i = 0; i < LIPT; ++i)
                 if ((valid >> i) & 1u) move(i);

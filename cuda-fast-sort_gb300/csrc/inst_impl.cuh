@@ -9,6 +9,7 @@
 #include "onesweep.cuh"
 #include "segmented.cuh"
 #include "shapes.h"
+#include "short_pairs.cuh"
 
 namespace gbsort {
 
@@ -120,6 +121,24 @@ const KernelEntry* finish_entries_for() {
         {reinterpret_cast<const void*>(&finish_kernel<KB, 8, S::THREADS, S::MIN_CTAS, S::LIPT, S::HALO>), S::THREADS, F8::LIPT,
          F8::CAP, static_cast<unsigned long>(F8::SMEM_BYTES)},
     };
+    return e;
+}
+
+// Short key-value arrays in one launch: [4- or 8-byte values][that kernel, the
+// digit passes in one launch].
+template <int KB, int VB>
+KernelEntry make_short_pairs_entry() {
+    using S = ShortPairsShape;
+    using G = ShortPairsGeom<KB, S::THREADS, S::halo(KB)>;
+    static_assert(uint32_t(G::CAP) == short_pairs_cap(KB), "the plan's capacity");
+    return KernelEntry{reinterpret_cast<const void*>(&short_pairs_kernel<KB, VB, S::THREADS, S::MIN_CTAS, S::halo(KB)>),
+                       S::THREADS, 0, G::CAP, static_cast<unsigned long>(G::SMEM_BYTES)};
+}
+template <int KB>
+const KernelEntry* short_pairs_entries_for() {
+    static const KernelEntry e[4] = {
+        make_short_pairs_entry<KB, 4>(), make_multi_entry<KB, 4, uint32_t, PassShapeSmall<KB, 4>>(),
+        make_short_pairs_entry<KB, 8>(), make_multi_entry<KB, 8, uint32_t, PassShapeSmall<KB, 8>>()};
     return e;
 }
 

@@ -67,6 +67,7 @@ struct MsdCode {
     uint32_t skip, b2;
     __device__ __forceinline__ explicit MsdCode(const MsdParams& p)
         : skip(ld_relaxed(p.window)), b2(ld_relaxed(p.window + 1)) {}
+    __device__ __forceinline__ MsdCode(uint32_t left_out, uint32_t bits) : skip(left_out), b2(bits) {}
     __device__ __forceinline__ uint32_t operator()(uint32_t k) const { return k << skip; }
     __device__ __forceinline__ uint32_t operator()(uint64_t k) const {
         const uint32_t hi = uint32_t(k >> 32), lo = uint32_t(k);

@@ -316,7 +316,7 @@ __device__ __forceinline__ bool onesweep_pass_body(const PassParams& p, uint8_t*
     // few tiles a CTA the first ones need no claim (with many, claims in the
     // order of arrival make up for it: 4 x 10^6 8-byte keys + values, three
     // passes, 209 against 228 us)
-    const bool given = MULTI && T <= 4u * gridDim.x;
+    const bool given = MULTI && T <= 2u * gridDim.x;
     auto claim = [&] { return atomicAdd(tile_counter, 1u) + (given ? gridDim.x : 0u); };
     auto make_info = [&](uint32_t t, const TileRec& rec) {
         TileInfo ti{};

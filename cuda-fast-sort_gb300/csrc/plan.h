@@ -29,10 +29,11 @@ struct CtlLayout {
     size_t overflow_off = 0;     // its region overflow flag
     size_t counters2_off = 0;    // a second set of tile counters and a second grid barrier, for the
                                  // digit passes after a sort by leading digits (0: none)
-    size_t sampled_off = 0;      // that sort's sample: ticket, [8] counts
+    size_t short_fill_off = 0;   // [1024] fill counts of a short key-value sort's regions
+    size_t sampled_off = 0;      // its sample: ticket, [8] counts
     size_t msd_state_off = 0;    // outcome of the most-significant-first path, its code window [2]
     size_t bytes = 0;
-    static CtlLayout make(int passes, bool finish = false) {
+    static CtlLayout make(int passes, bool finish = false, bool short_pairs = false) {
         CtlLayout c;
         c.gp_off = 0;
         c.counters_off = size_t(passes) * 256 * 8;
@@ -48,6 +49,10 @@ struct CtlLayout {
             c.counters2_off = c.bytes;
             c.sampled_off = c.counters2_off + 18 * 4;
             c.bytes = align_up(c.sampled_off + 9 * 4, 256);
+        }
+        if (short_pairs) {
+            c.short_fill_off = c.bytes;
+            c.bytes += 1024 * 4;
         }
         return c;
     }
@@ -106,6 +111,12 @@ struct Plan {
     bool finish = false;
     KernelEntry multi{};
     KernelEntry finish_k[3]{};
+    // short key-value arrays in one launch (short_pairs.cuh): that kernel, the
+    // digit passes after it, its regions, and their place in the workspace
+    bool short_pairs = false;
+    KernelEntry short_k[2]{};
+    int short_regions = 0;
+    size_t short_off = 0;
     size_t total_bytes = 0;
     CtlLayout ctl{};
 };

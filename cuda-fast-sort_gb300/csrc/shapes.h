@@ -142,8 +142,9 @@ constexpr int msd_b2_max(uint64_t n, uint32_t cap) {
 
 // Key-value sorts by their leading digits (finish.cuh): the finishing CTAs.
 // 8- and 16-byte keys with 4- or 8-byte values.  4-byte keys keep their four
-// digit passes: two of them and the finish take longer (2^26 u32 + u32 1.54
-// against 1.42 ms, finishing in CTAs of 768 threads; in 384 of 16 keys 1.84).
+// digit passes: two of them and the finish take longer (2^26 u32 + u32 1.51
+// against 1.42 ms, the finish 0.68 in two CTAs of 512 threads, 8 keys a lane,
+// or one of 768).
 template <int KB>
 struct FinishShape {
     static constexpr int THREADS = 384;
@@ -153,6 +154,30 @@ struct FinishShape {
 };
 constexpr bool finish_pairs(int kb, int vb) { return kb >= 8 && (vb == 4 || vb == 8); }
 constexpr uint64_t FINISH_N_MIN = 2048;  // (u64 + u32, uniform: 16385 pairs 45 us, the digit passes 78)
+// Short key-value arrays in one launch (short_pairs.cuh): regions of up to
+// `cap` words (key and index) a CTA of THREADS sorts.
+struct ShortPairsShape {
+    static constexpr int THREADS = 384;
+    static constexpr int MIN_CTAS = 3;
+    static constexpr int halo(int kb) { return kb == 8 ? 2 : 1; }
+};
+constexpr uint32_t short_pairs_cap(int kb) {
+    return (uint32_t(ShortPairsShape::THREADS / 32 * (32 - 2 * ShortPairsShape::halo(kb)) * (32 / kb)) - 8u) & ~3u;
+}
+// Regions: 256, or one or two per resident CTA of a GB300 (a region more than
+// that waits for a whole round: 10^6 pairs in 512 regions 48 us, in 456 42;
+// more regions than needed cost a global atomic each per tile: 600001 pairs in
+// 456 36 us, in 256 31), the first of these whose mean region of uniform keys
+// and six of its standard deviations fit the cap; 0: none do.
+inline int short_pairs_regions(int kb, uint64_t n) {
+    for (int regions : {256, 456, 912}) {
+        const double mean = double(n) / double(regions);
+        if (mean * 1.01 + 6.0 * std::sqrt(mean) + 8.0 <= double(short_pairs_cap(kb))) return regions;
+    }
+    return 0;
+}
+constexpr uint64_t SHORT_PAIRS_N_MIN = 2048;
+
 constexpr uint64_t FINISH_N_MAX = (uint64_t(1) << 31) - 1;  // edges keep a flag in bit 31
 
 // Keys per MSD region of the one-launch sort (one region per top digit):

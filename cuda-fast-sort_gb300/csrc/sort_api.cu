@@ -28,6 +28,7 @@
 #include "fused_short.cuh"
 #include "msd.cuh"
 #include "onesweep.cuh"
+#include "short_pairs.cuh"
 #include "sort_params.h"
 
 namespace gbsort {
@@ -48,6 +49,8 @@ const KernelEntry* fused_entry_k4();
 const KernelEntry* fused_entry_k8();
 const KernelEntry* fused_entry_k16();
 
+const KernelEntry* short_pairs_entries_k4();
+const KernelEntry* short_pairs_entries_k8();
 const KernelEntry* multi_entries_k8(int vb);
 const KernelEntry* multi_entries_k16(int vb);
 const KernelEntry* finish_entries_k8();
@@ -328,7 +331,13 @@ int make_plan(int key_type, size_t value_bytes, uint64_t n, Plan* plan) {
     p.alt_vals_off = off;
     off = align_up(off + size_t(n) * value_bytes, 256);
     const bool finish = finish_pairs(p.kb, p.vb) && n >= FINISH_N_MIN && n <= FINISH_N_MAX;
-    p.ctl = CtlLayout::make(p.passes, finish);
+    // short key-value arrays in one launch; not floats, whose leading bits are
+    // the exponent (most values share few regions)
+    const int short_regions = (p.kb == 4 || p.kb == 8) && (p.vb == 4 || p.vb == 8) && p.kind != KIND_FLOAT && small &&
+                                   n >= SHORT_PAIRS_N_MIN
+                               ? short_pairs_regions(p.kb, n)
+                               : 0;
+    p.ctl = CtlLayout::make(p.passes, finish, short_regions != 0);
     p.ctl_off = off;
     off = align_up(off + p.ctl.bytes, 256);
     p.status_off = off;
@@ -368,6 +377,17 @@ int make_plan(int key_type, size_t value_bytes, uint64_t n, Plan* plan) {
             p.msd = true;
             for (int i = 0; i < 5; ++i) p.msd_k[i] = msd_entries(p.kb)[i];
             p.msd_k[5] = msd_entries(p.kb)[5 + shape];
+        }
+    }
+    if (short_regions) {
+        p.short_off = off;
+        off = align_up(off + size_t(short_regions) * short_pairs_cap(p.kb) * 2 * kb, 256);
+        if (g_pass_skip.load(std::memory_order_relaxed)) {
+            p.short_pairs = true;
+            p.short_regions = short_regions;
+            const KernelEntry* e = p.kb == 4 ? short_pairs_entries_k4() : short_pairs_entries_k8();
+            p.short_k[0] = e[p.vb == 4 ? 0 : 2];
+            p.short_k[1] = e[p.vb == 4 ? 1 : 3];
         }
     }
     if (finish && g_pass_skip.load(std::memory_order_relaxed)) {
@@ -449,7 +469,9 @@ int enqueue_sort(const Plan& plan, int descending, void* d_keys, void* d_values,
     bool use_finish = plan.finish && ms == nullptr;
     for (int i = 0; use_finish && i < 3; ++i) use_finish = prepare_kernel(plan.finish_k[i]) == GBSORT_OK;
     use_finish = use_finish && prepare_kernel(plan.multi) == GBSORT_OK;
-    uint32_t* msd_state = use_msd || use_finish ? reinterpret_cast<uint32_t*>(ctl + plan.ctl.msd_state_off) : nullptr;
+    const bool use_short = plan.short_pairs && ms == nullptr && prepare_kernel(plan.short_k[0]) == GBSORT_OK &&
+                           prepare_kernel(plan.short_k[1]) == GBSORT_OK;
+    uint32_t* msd_state = use_msd || use_finish || use_short ? reinterpret_cast<uint32_t*>(ctl + plan.ctl.msd_state_off) : nullptr;
 
     // Parameters of digit pass `pass` and of the fix-up copy.
     auto pass_params = [&](int pass) {
@@ -575,6 +597,50 @@ int enqueue_sort(const Plan& plan, int descending, void* d_keys, void* d_values,
         cudaGetLastError();
     }
     const uint32_t hist_ctas = upsweep_ctas(plan.n, plan.kb);
+    if (use_short) {
+        // A short key-value array: one cooperative launch, and another for
+        // every digit pass in case the keys were too uneven for it.
+        ShortPairsParams sp{};
+        sp.hist = hp;
+        sp.keys_in = copy ? keys_src : d_keys;
+        sp.vals_in = copy ? vals_src : d_values;
+        sp.vals_aside = copy ? nullptr : alt_vals;
+        sp.keys_out = d_keys;
+        sp.vals_out = d_values;
+        sp.n = uint32_t(plan.n);
+        sp.kind = plan.kind;
+        sp.desc = descending;
+        sp.nb = uint32_t(plan.short_regions);
+        sp.regions = ws + plan.short_off - ws_base;
+        sp.cap = short_pairs_cap(plan.kb);
+        sp.fill = reinterpret_cast<uint32_t*>(ctl + plan.ctl.short_fill_off);
+        sp.state = msd_state;
+        sp.barrier = reinterpret_cast<uint32_t*>(ctl + plan.ctl.barrier_off);
+        sp.barrier_gen = reinterpret_cast<uint32_t*>(ctl + plan.ctl.barrier_gen_off);
+        sp.wait_limit_ns = wait_limit_ns();
+        sp.err = err_word;
+        const uint64_t most = uint64_t(sms) * uint64_t(resident_ctas(plan.short_k[0]));
+        const uint32_t grid = uint32_t(sp.nb < most ? sp.nb : most);
+        void* args[] = {&sp};
+        e = cudaLaunchCooperativeKernel(plan.short_k[0].fn, dim3(grid), dim3(plan.short_k[0].threads), args,
+                                        plan.short_k[0].smem, stream);
+        if (e == cudaSuccess) {
+            PassParams pp = pass_params(0);
+            pp.msd_state = msd_state;
+            pp.state_mask = MSD_OFF;
+            pp.leading = nullptr;
+            pp.barrier = sp.barrier_gen + 1;  // (the first kernel's barrier has its own words)
+            pp.barrier_gen = sp.barrier_gen + 2;
+            void* pargs[] = {&pp};
+            const uint64_t mostp = uint64_t(sms) * uint64_t(resident_ctas(plan.short_k[1]));
+            e = cudaLaunchCooperativeKernel(plan.short_k[1].fn,
+                                            dim3(uint32_t(plan.num_tiles < mostp ? plan.num_tiles : mostp)),
+                                            dim3(plan.short_k[1].threads), pargs, plan.short_k[1].smem, stream);
+            if (e != cudaSuccess) return fail("pass launch", e);
+            return GBSORT_OK;
+        }
+        cudaGetLastError();  // refused: the separate launches below
+    }
     if (timed) cudaEventRecord(ev[0], stream);
     const int occ = resident_ctas(plan.pass);
     const uint64_t max_ctas = uint64_t(sms) * uint64_t(occ > 0 ? occ : 1);
