@@ -1,4 +1,6 @@
-// finish.cuh — key-value sorts by their leading digits only (sm_103a).
+// finish.cuh — sorts by the keys' leading digits only (sm_103a): key-value
+// arrays of 8- and 16-byte keys, and 8-byte floats alone, whose leading bits
+// are too uneven for the splits of msd.cuh.
 //
 // A stable least-significant-digit sort makes a pass over keys and values per
 // key byte.  Where the leading D bytes already cut the array into groups of a
@@ -522,16 +524,17 @@ __global__ void __launch_bounds__(THREADS, MIN_CTAS) finish_kernel(FinishParams 
         if (lane == (with ? __ffs(with) - 1 : 0)) heads_first[warp] = firsth;
         __syncthreads();
         // the values arrive while the keys are sorted
-        if ((reinterpret_cast<uintptr_t>(vals + s - pad) & 15u) == 0u) {
-            constexpr uint32_t VVEC = 16 / VB;
+        if constexpr (VB == 0) {
+        } else if ((reinterpret_cast<uintptr_t>(vals + s - pad) & 15u) == 0u) {
+            constexpr uint32_t VVEC = 16 / (VB ? VB : 1);
             for (uint32_t j = tid * VVEC; j < end; j += THREADS * VVEC) {
                 if (j >= pad && j + VVEC <= end) copy_async<16>(sv + j, vals + s - pad + j);
                 else
                     for (uint32_t e = j; e < j + VVEC; ++e)
-                        if (e >= pad && e < end) copy_async<VB>(sv + e, vals + s - pad + e);
+                        if (e >= pad && e < end) copy_async<(VB ? VB : 4)>(sv + e, vals + s - pad + e);
             }
         } else {
-            for (uint32_t j = pad + tid; j < end; j += THREADS) copy_async<VB>(sv + j, vals + s - pad + j);
+            for (uint32_t j = pad + tid; j < end; j += THREADS) copy_async<(VB ? VB : 4)>(sv + j, vals + s - pad + j);
         }
         {
             const uint32_t l = __reduce_max_sync(0xffffffffu, lane < warp ? heads_last[lane] : 0u);
@@ -606,9 +609,12 @@ __global__ void __launch_bounds__(THREADS, MIN_CTAS) finish_kernel(FinishParams 
 #pragma unroll
             for (int i = 0; i < LIPT; ++i)
                 if ((valid >> i) & 1u) okeys[s - pad + c0 + i] = map.out(k[i]);
-            copy_async_wait();
+            if constexpr (VB > 0) {
+                copy_async_wait();
+                __syncthreads();
+                for (uint32_t j = tid; j < cnt; j += THREADS) ovals[s + j] = sv[pad + j];
+            }
             __syncthreads();
-            for (uint32_t j = tid; j < cnt; j += THREADS) ovals[s + j] = sv[pad + j];
             if (tid == 0) {
                 atomicOr(p.state, MSD_GAVE_UP);
                 misc[0] = 0u;
@@ -627,7 +633,7 @@ __global__ void __launch_bounds__(THREADS, MIN_CTAS) finish_kernel(FinishParams 
             for (int i = 0; i < LIPT; ++i)
                 if ((valid >> i) & 1u) move(i);
         }
-        copy_async_wait();
+        if constexpr (VB > 0) copy_async_wait();
         __syncthreads();
         if (tid == 0) misc[0] = 0u;
         more = advance();
@@ -687,12 +693,14 @@ __global__ void __launch_bounds__(THREADS, MIN_CTAS) finish_kernel(FinishParams 
                             for (int e = 0; e < 32 / KB; ++e) y.k[e] = map.out(x[i * (32 / KB) + e].key());
                             store_32b(ok + i * (32 / KB), y.q[0], y.q[1]);
                         }
-                        if ((reinterpret_cast<uintptr_t>(ov) & 15u) == 0u) {
+                        constexpr int VV = 16 / (VB ? VB : 16);
+                        if constexpr (VB == 0) {
+                        } else if ((reinterpret_cast<uintptr_t>(ov) & 15u) == 0u) {
 #pragma unroll
-                            for (int i = 0; i < LIPT * VB / 16; ++i) {
-                                union { uint4 q; V v[16 / VB]; } y;
+                            for (int i = 0; i < LIPT / VV; ++i) {
+                                union { uint4 q; V v[VV]; } y;
 #pragma unroll
-                                for (int e = 0; e < 16 / VB; ++e) y.v[e] = sv[x[i * (16 / VB) + e].place()];
+                                for (int e = 0; e < VV; ++e) y.v[e] = sv[x[i * VV + e].place()];
                                 reinterpret_cast<uint4*>(ov)[i] = y.q;
                             }
                         } else {
@@ -704,7 +712,7 @@ __global__ void __launch_bounds__(THREADS, MIN_CTAS) finish_kernel(FinishParams 
                         for (int i = 0; i < LIPT; ++i) {
                             if (d0 + i >= int(pad) && d0 + i < int(end)) {
                                 ok[i] = map.out(x[i].key());
-                                ov[i] = sv[x[i].place()];
+                                if constexpr (VB > 0) ov[i] = sv[x[i].place()];
                             }
                         }
                     }
@@ -726,7 +734,7 @@ __global__ void __launch_bounds__(THREADS, MIN_CTAS) finish_kernel(FinishParams 
                 uint32_t before = 0;
                 for (uint32_t q = q0; q < q1; ++q) before += after(me, get(q));
                 okeys[s - pad + q0 + before] = map.out(me.key());
-                ovals[s - pad + q0 + before] = sv[me.place()];
+                if constexpr (VB > 0) ovals[s - pad + q0 + before] = sv[me.place()];
             }
         }
     }

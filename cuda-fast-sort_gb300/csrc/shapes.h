@@ -153,6 +153,10 @@ struct FinishShape {
     static constexpr int MIN_CTAS = 2;
 };
 constexpr bool finish_pairs(int kb, int vb) { return kb >= 8 && (vb == 4 || vb == 8); }
+// 8-byte floats without values too, from here on (N(0, 1): 140001 keys 58 us,
+// the one-launch sort, whose regions overflow, 81; 1.6 x 10^7 564, eight digit
+// passes 770).
+constexpr uint64_t FINISH_KEYS_N_MIN = uint64_t(1) << 14;
 constexpr uint64_t FINISH_N_MIN = 2048;  // (u64 + u32, uniform: 16385 pairs 45 us, the digit passes 78)
 // Short key-value arrays in one launch (short_pairs.cuh): regions of up to
 // `cap` words (key and index) a CTA of THREADS sorts.

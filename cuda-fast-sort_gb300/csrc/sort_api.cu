@@ -330,7 +330,9 @@ int make_plan(int key_type, size_t value_bytes, uint64_t n, Plan* plan) {
     off = align_up(off + size_t(n) * kb, 256);
     p.alt_vals_off = off;
     off = align_up(off + size_t(n) * value_bytes, 256);
-    const bool finish = finish_pairs(p.kb, p.vb) && n >= FINISH_N_MIN && n <= FINISH_N_MAX;
+    const bool finish = ((finish_pairs(p.kb, p.vb) && n >= FINISH_N_MIN) ||
+                         (p.kb == 8 && p.vb == 0 && p.kind == KIND_FLOAT && n >= FINISH_KEYS_N_MIN)) &&
+                        n <= FINISH_N_MAX;
     // short key-value arrays in one launch; not floats, whose leading bits are
     // the exponent (most values share few regions)
     const int short_regions = (p.kb == 4 || p.kb == 8) && (p.vb == 4 || p.vb == 8) && p.kind != KIND_FLOAT && small &&
@@ -395,7 +397,7 @@ int make_plan(int key_type, size_t value_bytes, uint64_t n, Plan* plan) {
         const KernelEntry* e = finish_entries(p.kb);
         p.finish_k[0] = e[0];
         p.finish_k[1] = e[1];
-        p.finish_k[2] = e[p.vb == 4 ? 2 : 3];
+        p.finish_k[2] = e[p.vb == 4 ? 2 : p.vb == 8 ? 3 : 4];
         p.multi = (p.kb == 8 ? multi_entries_k8(p.vb) : multi_entries_k16(p.vb))[small ? 2 : p.wide_status ? 1 : 0];
     }
     p.total_bytes = off;
@@ -419,9 +421,13 @@ int enqueue_sort(const Plan& plan, int descending, void* d_keys, void* d_values,
     if (st != GBSORT_OK) return st;
     st = prepare_kernel(plan.upsweep);
     if (st != GBSORT_OK) return st;
+    // (its digit passes run in one launch, which sort_timed does not use)
+    bool use_finish = plan.finish && ms == nullptr;
+    for (int i = 0; use_finish && i < 3; ++i) use_finish = prepare_kernel(plan.finish_k[i]) == GBSORT_OK;
+    use_finish = use_finish && prepare_kernel(plan.multi) == GBSORT_OK;
     // the most-significant-first path of keys-only sorts runs when all its
     // kernels can
-    bool use_msd = plan.msd;
+    bool use_msd = plan.msd && !use_finish;
     for (int i = 0; use_msd && i < 6; ++i) use_msd = prepare_kernel(plan.msd_k[i]) == GBSORT_OK;
     // its kernels are timed one by one where the plan reports them (then the
     // digits' histogram is the last of six stages), else as part of entry 0
@@ -465,10 +471,6 @@ int enqueue_sort(const Plan& plan, int descending, void* d_keys, void* d_values,
     };
 
     uint8_t* msd_block = use_msd ? ws + plan.msd_off - ws_base : nullptr;
-    // (its digit passes run in one launch, which sort_timed does not use)
-    bool use_finish = plan.finish && ms == nullptr;
-    for (int i = 0; use_finish && i < 3; ++i) use_finish = prepare_kernel(plan.finish_k[i]) == GBSORT_OK;
-    use_finish = use_finish && prepare_kernel(plan.multi) == GBSORT_OK;
     const bool use_short = plan.short_pairs && ms == nullptr && prepare_kernel(plan.short_k[0]) == GBSORT_OK &&
                            prepare_kernel(plan.short_k[1]) == GBSORT_OK;
     uint32_t* msd_state = use_msd || use_finish || use_short ? reinterpret_cast<uint32_t*>(ctl + plan.ctl.msd_state_off) : nullptr;
@@ -536,7 +538,7 @@ int enqueue_sort(const Plan& plan, int descending, void* d_keys, void* d_values,
 
     // the one-launch short sort runs when its kernel can be made resident
     const bool fused =
-        plan.fused.fn != nullptr && prepare_kernel(plan.fused) == GBSORT_OK && resident_ctas(plan.fused) > 0;
+        !use_finish && plan.fused.fn != nullptr && prepare_kernel(plan.fused) == GBSORT_OK && resident_ctas(plan.fused) > 0;
     // (it clears its lookback status words itself, before its first pass)
     cudaError_t e = cudaMemsetAsync(ctl, 0, plan.ctl.bytes, stream);
     if (e != cudaSuccess) return fail("memset control block", e);

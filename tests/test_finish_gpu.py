@@ -94,3 +94,18 @@ def test_input_preserving_and_double_buffer(gb, cuda, oracle, kt, how):
     cuda.cuda.synchronize()
     assert gb.double_buffer_status(kt, n, dws, 4) == gb.OK
     assert _eq(from_dev(src if sel else k0, raw), ek) and _eq(from_dev(vsrc if sel else v0, vals), ev)
+
+
+@pytest.mark.parametrize("n", [16383, 16384, 70001, 300007, (1 << 21) + 1])
+@pytest.mark.parametrize("how", ["normal", "spike", "uneven", "few"])
+def test_floats_without_values(gb, cuda, oracle, n, how):
+    if how == "normal":
+        rng = np.random.default_rng(n)
+        x = rng.standard_normal(n)
+        x[rng.random(n) < 0.02] = -0.0
+        x[:5] = [np.inf, -np.inf, np.nan, 0.0, 5e-324]
+        raw = x.view(np.uint64)
+    else:
+        raw = _spread("f64", n, n, how)
+    for desc in (False, True):
+        assert _eq(gpu_sort(gb, cuda, "f64", raw, desc, garbage_workspace=True, key_offset=1), oracle.sort("f64", raw, desc))
