@@ -105,11 +105,12 @@ struct Plan {
     uint32_t msd_group_cap = 0;
     int msd_b2 = 0;
     size_t msd_off = 0;
-    // key-value sorts by their leading digits (finish.cuh): sample, edges,
-    // finish, and the digit passes in one launch; the edges lie in the status
-    // words
-    bool finish = false;
+    // the digit passes in one launch, after (or, by leading digits, in) a path
+    // that seldom needs all of them
     KernelEntry multi{};
+    // sorts by leading digits (finish.cuh): sample, edges,
+    // finish; the edges lie in the status words
+    bool finish = false;
     KernelEntry finish_k[3]{};
     // short key-value arrays in one launch (short_pairs.cuh): that kernel, the
     // digit passes after it, its regions, and their place in the workspace
