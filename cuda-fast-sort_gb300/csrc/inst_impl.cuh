@@ -76,13 +76,13 @@ const KernelEntry* fused_entry_for() {
 
 // Keys-only sorts above the short range, most significant bits first: sample,
 // count, scan, top split, second split, local sorts (two sizes).
-template <int KB, int L>
+template <int KB, int L, bool EVEN = false>
 KernelEntry make_msd_local_entry() {
     using S = MsdShape<KB>;
     using GL = GroupSortGeom<KB, S::C_THREADS[L], S::C_HALO>;
     static_assert(GL::CAP == int(msd_group_cap_of<KB>(L)), "the plan's capacity");
     return KernelEntry{
-        reinterpret_cast<const void*>(&msd_local_kernel<KB, S::C_THREADS[L], S::C_MIN_CTAS[L], S::C_HALO>),
+        reinterpret_cast<const void*>(&msd_local_kernel<KB, S::C_THREADS[L], S::C_MIN_CTAS[L], S::C_HALO, EVEN>),
         S::C_THREADS[L], GL::LIPT, GL::CAP, static_cast<unsigned long>(GL::SMEM_BYTES)};
 }
 
@@ -92,15 +92,35 @@ const KernelEntry* msd_entries_for() {
     using GS = MsdSplitGeom<KB, S::THREADS, S::IPT, S::CAP>;
     static const KernelEntry e[7] = {
         {reinterpret_cast<const void*>(&msd_sample_kernel<KB>), MSD_SAMPLE_THREADS, 0, 0, 0ul},
-        {reinterpret_cast<const void*>(&msd_count_kernel<KB>), MSD_COUNT_THREADS, 0, 0,
+        {reinterpret_cast<const void*>(&msd_count_kernel<KB, false>), MSD_COUNT_THREADS, 0, 0,
          static_cast<unsigned long>(MSD_COUNT_SMEM)},
-        {reinterpret_cast<const void*>(&msd_scan_kernel<KB>), 256, 0, 0, 0ul},
-        {reinterpret_cast<const void*>(&msd_top_kernel<KB, S::THREADS, S::IPT, S::MIN_CTAS, S::CAP>), S::THREADS,
+        {reinterpret_cast<const void*>(&msd_scan_kernel<false>), 256, 0, 0, 0ul},
+        {reinterpret_cast<const void*>(&msd_top_kernel<KB, S::THREADS, S::IPT, S::MIN_CTAS, S::CAP, false>), S::THREADS,
          S::IPT, GS::TILE, static_cast<unsigned long>(GS::SMEM_BYTES)},
-        {reinterpret_cast<const void*>(&msd_second_kernel<KB, S::THREADS, S::IPT, S::MIN_CTAS, S::CAP>), S::THREADS, S::IPT,
+        {reinterpret_cast<const void*>(&msd_second_kernel<KB, S::THREADS, S::IPT, S::MIN_CTAS, S::CAP, false>), S::THREADS, S::IPT,
          GS::TILE, static_cast<unsigned long>(GS::SMEM_BYTES)},
         make_msd_local_entry<KB, 0>(),
         make_msd_local_entry<KB, 1>(),
+    };
+    return e;
+}
+
+// The same for 4-byte floats.
+template <int KB>
+const KernelEntry* msd_even_entries_for() {
+    using S = MsdShape<KB>;
+    using GS = MsdSplitGeom<KB, S::THREADS, S::IPT, S::CAP>;
+    static const KernelEntry e[6] = {
+        {reinterpret_cast<const void*>(&msd_even_sample_kernel<KB>), MSD_SAMPLE_THREADS, 0, 0,
+         static_cast<unsigned long>(MSD_EVEN_SMEM)},
+        {reinterpret_cast<const void*>(&msd_count_kernel<KB, true>), MSD_COUNT_THREADS, 0, 0,
+         static_cast<unsigned long>(MSD_COUNT_SMEM + MsdEvenCode::BINS * 8)},
+        {reinterpret_cast<const void*>(&msd_scan_kernel<true>), 256, 0, 0, 0ul},
+        {reinterpret_cast<const void*>(&msd_top_kernel<KB, S::THREADS, S::IPT, S::MIN_CTAS, S::CAP, true>), S::THREADS,
+         S::IPT, GS::TILE, static_cast<unsigned long>(GS::EVEN_BYTES)},
+        {reinterpret_cast<const void*>(&msd_second_kernel<KB, S::THREADS, S::IPT, S::MIN_CTAS, S::CAP, true>), S::THREADS,
+         S::IPT, GS::TILE, static_cast<unsigned long>(GS::EVEN_BYTES)},
+        make_msd_local_entry<KB, 0, true>(),
     };
     return e;
 }

@@ -31,7 +31,13 @@
 // in some order (untouched, or as the local sorts left them); otherwise they
 // exit at once.
 // Every key is read four times and written three times, whatever its width.
+// 4-byte floats take it too, by a group number from the sample's distribution
+// (MsdEvenCode; 2^27 keys of N(0, 1) 1.47 ms, four digit passes 2.03; the
+// table's reads cost the count and the splits about a half: 6 * 10^7 keys
+// 80 + 160 + 185 us, unsigned keys 49 + 110 + 138).
 #pragma once
+
+#include <cooperative_groups.h>
 
 #include "fused_short.cuh"
 
@@ -53,6 +59,8 @@ struct MsdParams {
     uint32_t* joint;       // [256 << b2_max] keys per group
     uint32_t* cursor2;     // [256 << b2_max] next place of every group; its end after the second split
     uint32_t group_cap;    // largest group a local sort takes
+    uint2* table;          // floats: the code of every leading 12 bits (MsdEvenCode), then a sampled key of each
+    uint32_t* giants;      // floats: count, then group and key of every group of equal keys above group_cap
     uint32_t* err;         // workspace error word
 };
 
@@ -76,6 +84,35 @@ struct MsdCode {
     }
     __device__ __forceinline__ uint32_t operator()(u128 k) const { return (*this)(uint64_t(k >> 64)); }
 };
+
+// The code of a float.  Floats crowd into few leading bits (the exponent), so
+// their codes are the sample's distribution function instead: the leading 12
+// bits (sign, exponent, 3 bits of mantissa) name a stretch of the codes as wide
+// as the share of the sample there, {start, width}, and the 20 bits below
+// divide it evenly (both after the `skip` bits that all keys share).
+// Monotone; two keys may share a code.
+struct MsdEvenCode {
+    static constexpr uint32_t BINS = 4096;
+    const uint2* table;
+    uint32_t skip, b2;
+    __device__ __forceinline__ MsdEvenCode(const MsdParams& p, const uint2* t)
+        : table(t), skip(ld_relaxed(p.window)), b2(ld_relaxed(p.window + 1)) {}
+    __device__ __forceinline__ uint32_t operator()(uint32_t k) const {
+        const uint32_t c = k << skip;
+        const uint2 e = table[c >> 20];
+        return e.x + __umulhi(c << 12, e.y);
+    }
+    // copies the table to shared memory (the caller's barrier follows)
+    __device__ __forceinline__ static void fetch(const MsdParams& p, uint2* to) {
+        const uint4* from = reinterpret_cast<const uint4*>(p.table);
+        for (uint32_t i = threadIdx.x; i < BINS / 2; i += blockDim.x) reinterpret_cast<uint4*>(to)[i] = from[i];
+    }
+};
+template <bool EVEN>
+__device__ __forceinline__ auto msd_code(const MsdParams& p, const uint2* table) {
+    if constexpr (EVEN) return MsdEvenCode(p, table);
+    else return MsdCode(p);
+}
 
 // The window of the codes, from a sample; the other CTAs clear the counters.
 constexpr int MSD_SAMPLE_THREADS = 1024;
@@ -160,13 +197,210 @@ __global__ void __launch_bounds__(MSD_SAMPLE_THREADS) msd_sample_kernel(MsdParam
     }
 }
 
+// Exclusive scan over the CTA with one barrier: every warp scans the warp
+// totals for itself (warp_tmp is written again only after another barrier).
+template <int THREADS>
+__device__ __forceinline__ uint32_t block_exclusive_scan_1b(uint32_t x, uint32_t* warp_tmp) {
+    constexpr int WARPS = THREADS / 32;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t v = x;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v += y;
+    }
+    if (lane == 31) warp_tmp[warp] = v;
+    __syncthreads();
+    const uint32_t before = __reduce_add_sync(0xffffffffu, lane < warp && lane < WARPS ? warp_tmp[lane] : 0u);
+    return before + v - x;
+}
+
+// The codes of 4-byte floats, from 65536 keys in vectors of four spread over
+// the array: a cluster of eight CTAs samples and counts the leading 12 bits
+// (one SM alone would wait eight times as long for its gathers), its first CTA
+// lays the codes out; the other clusters clear the counters.
+// A bin with k keys of the sample gets a stretch of k + 4 sqrt(k) + 8, so that
+// neither the sample's error nor the slope of the density inside the bin makes
+// its groups too large, and in the ratio of the bin's range to the part of it
+// that the keys take; an empty one gets 1, beside another bin 4.  A bin whose sampled keys, two at least, are all equal
+// (zeros, infinities, NaNs) has a group of its own: equal keys need no sort, however
+// many they are.
+constexpr int MSD_EVEN_CLUSTER = 8;
+constexpr size_t MSD_EVEN_SMEM = 6 * MsdEvenCode::BINS * 4;
+constexpr uint32_t MSD_GIANTS = 31;
+template <int KB>
+__global__ void __cluster_dims__(MSD_EVEN_CLUSTER, 1, 1) __launch_bounds__(MSD_SAMPLE_THREADS)
+    msd_even_sample_kernel(MsdParams p) {
+    static_assert(KB == 4, "codes of 4-byte floats");
+    namespace cg = cooperative_groups;
+    constexpr uint32_t BINS = MsdEvenCode::BINS, NONE = 0xffffffffu, SLOTS = 4096;
+    constexpr int VECS = 2, PER = MSD_SAMPLE_THREADS * MSD_EVEN_CLUSTER;
+    constexpr float S = float(PER * VECS * 4);
+    extern __shared__ __align__(16) uint32_t smem_even[];
+    uint32_t* cnt = smem_even;  // keys per bin, their least and their largest
+    uint32_t* low = cnt + BINS;
+    uint32_t* high = low + BINS;
+    uint32_t* all = high + BINS;  // (first CTA) the same of the cluster
+    __shared__ uint32_t vary, again, dense, scan[2][32], total[2];
+    grid_launch_dependents();
+    grid_dependency_wait();
+    const uint32_t tid = threadIdx.x;
+    if (blockIdx.x >= MSD_EVEN_CLUSTER) {
+        const uint32_t stride = (gridDim.x - MSD_EVEN_CLUSTER) * MSD_SAMPLE_THREADS;
+        for (uint32_t i = (blockIdx.x - MSD_EVEN_CLUSTER) * MSD_SAMPLE_THREADS + tid; i < p.zero_words; i += stride)
+            p.zero[i] = 0u;
+        return;
+    }
+    cg::cluster_group cluster = cg::this_cluster();
+    const uint32_t rank = blockIdx.x;
+    const KeyMap<uint32_t> map(p.kind, p.desc);
+    const uint32_t* keys = static_cast<const uint32_t*>(p.keys_in);
+    const uint32_t head = ((16u - (reinterpret_cast<uintptr_t>(keys) & 15u)) & 15u) / 4u;
+    const uint32_t nvec = uint32_t((p.n - head) / 4u);
+    const uint32_t step = nvec / uint32_t(PER * VECS);  // (the path's arrays are 32 times as long at least)
+    uint32_t x[VECS * 4];
+#pragma unroll
+    for (int i = 0; i < VECS; ++i) {
+        const uint32_t at = (uint32_t(i) * MSD_SAMPLE_THREADS + tid) * MSD_EVEN_CLUSTER + rank;
+        const uint4 v = __ldcs(reinterpret_cast<const uint4*>(keys + head) + (at * step + (at * 2654435761u) % step));
+        x[i * 4] = map.in(v.x);
+        x[i * 4 + 1] = map.in(v.y);
+        x[i * 4 + 2] = map.in(v.z);
+        x[i * 4 + 3] = map.in(v.w);
+    }
+    const uint32_t first = map.in(keys[0]);
+    for (uint32_t i = tid; i < BINS; i += MSD_SAMPLE_THREADS) {
+        cnt[i] = high[i] = 0u;
+        low[i] = NONE;
+    }
+    if (tid == 0) vary = again = dense = 0u;
+    __syncthreads();
+    uint32_t d = 0;
+#pragma unroll
+    for (int i = 0; i < VECS * 4; ++i) d |= x[i] ^ first;
+    d = __reduce_or_sync(0xffffffffu, d);
+    if ((tid & 31u) == 0u) atomicOr(&vary, d);
+    cluster.sync();
+    d = 0;
+    for (uint32_t r = 0; r < MSD_EVEN_CLUSTER; ++r) d |= *cluster.map_shared_rank(&vary, r);
+    const uint32_t skip = d ? __clz(d) : 0u;
+#pragma unroll
+    for (int i = 0; i < VECS * 4; ++i) {
+        const uint32_t c = x[i] << skip, b = c >> 20;
+        atomicAdd(&cnt[b], 1u);
+        atomicMin(&low[b], c);
+        atomicMax(&high[b], c);
+    }
+    cluster.sync();
+    {  // every CTA merges its share of the bins into the first one's arrays
+        uint32_t* to = cluster.map_shared_rank(all, 0);
+        const uint32_t b = rank * (BINS / MSD_EVEN_CLUSTER) + tid;
+        if (tid < BINS / MSD_EVEN_CLUSTER) {
+            uint32_t k = 0, lo = NONE, hi = 0;
+#pragma unroll
+            for (uint32_t r = 0; r < MSD_EVEN_CLUSTER; ++r) {
+                k += *cluster.map_shared_rank(cnt + b, r);
+                lo = min(lo, *cluster.map_shared_rank(low + b, r));
+                hi = max(hi, *cluster.map_shared_rank(high + b, r));
+            }
+            to[b] = k;
+            to[BINS + b] = lo;
+            to[2 * BINS + b] = hi;
+        }
+    }
+    cluster.sync();  // (nobody reads the others' arrays after this)
+    if (rank != 0) return;
+    // Keys that repeat more than 32 times would crowd the local sorts'
+    // sub-buckets (those of a bin of equal keys do not matter): pairs of equal
+    // keys among 2048 of the sample.
+    for (uint32_t i = tid; i < SLOTS; i += MSD_SAMPLE_THREADS) cnt[i] = NONE;
+    __syncthreads();
+    uint32_t twice = 0;
+#pragma unroll
+    for (int i = 0; i < VECS; ++i) {
+        const uint32_t k = x[i * 4], b = (k << skip) >> 20;
+        if (all[BINS + b] == all[2 * BINS + b] || k == NONE) continue;
+        uint32_t h = (k * 2654435761u) >> 20;
+        for (int probe = 0; probe < 64; ++probe) {
+            uint32_t v = cnt[h];
+            if (v == NONE) v = atomicCAS(&cnt[h], NONE, k);
+            if (v == NONE) break;
+            if (v == k) {
+                ++twice;
+                break;
+            }
+            h = (h + 1u) & (SLOTS - 1u);
+        }
+    }
+    if (twice) atomicAdd(&again, twice);
+    // the layout: four bins a thread
+    uint32_t w[4], alone = 0, sum = 0;
+    float most = 0.f;  // keys of the sample per unit of stretch, where they lie densest
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const uint32_t b = tid * 4 + i;
+        const float k = float(all[b]);
+        const uint32_t range = all[2 * BINS + b] - all[BINS + b];
+        if (k == 0.f) w[i] = (b != 0u && all[b - 1]) || (b + 1 != BINS && all[b + 1]) ? 4u : 1u;
+        else if (range == 0u && k >= 2.f) w[i] = 0u;  // a group of its own
+        else {
+            // (the least and the largest of k even ones lie (k - 1) / (k + 1) of their range apart)
+            const float part =
+                k < 2.f ? 1.f
+                        : fminf(1.f, fmaxf((float(range) + 1.f) * 0x1p-20f * (k + 1.f) / (k - 1.f), k < 32.f ? 0.25f : 0.f));
+            const float f = k + 4.f * sqrtf(k) + 8.f;
+            w[i] = uint32_t(fminf(f / part, 8.f * S));
+            most = fmaxf(most, k / f);
+        }
+        sum += w[i];
+        alone += w[i] == 0u;
+    }
+    atomicMax(&dense, __float_as_uint(most));
+    uint32_t at = block_exclusive_scan_1b<MSD_SAMPLE_THREADS>(sum, scan[0]);
+    uint32_t alones = block_exclusive_scan_1b<MSD_SAMPLE_THREADS>(alone, scan[1]);
+    if (tid == MSD_SAMPLE_THREADS - 1) {
+        total[0] = at + sum;
+        total[1] = alones + alone;
+    }
+    __syncthreads();
+    const uint32_t W = total[0], P = total[1];
+    const float n = float(p.n), units = float(W) * __uint_as_float(dense);
+    uint32_t b2 = 0;  // groups of 0.6 of the largest at most where keys lie densest
+    auto fits = [&] {
+        const uint32_t groups = 256u << b2;
+        return groups >= 4u * P && n * units <= 0.6f * S * float(p.group_cap) * float(groups - 2u * P);
+    };
+    while (b2 < uint32_t(p.b2_max) && !fits()) ++b2;
+    const uint32_t group = 1u << (24u - b2);
+    const uint64_t scale = ((uint64_t(1) << 32) - 2ull * P * group) / W;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const uint32_t b = tid * 4 + i;
+        const uint64_t r = at * scale + 2ull * alones * group;
+        p.table[b] = w[i] == 0u ? make_uint2(uint32_t((r + group - 1u) & ~uint64_t(group - 1u)), group)
+                                : make_uint2(uint32_t(r), uint32_t(w[i] * scale));
+        // a bin of equal keys: the key
+        reinterpret_cast<uint32_t*>(p.table + BINS)[b] = (skip ? first >> (32u - skip) << (32u - skip) : 0u) | all[BINS + b] >> skip;
+        at += w[i];
+        alones += w[i] == 0u;
+    }
+    if (tid == 0) {
+        constexpr float R = MSD_SAMPLE_THREADS * VECS;
+        const bool crowded = again >= 6u && 2.f * float(again) * n > 32.f * R * R;
+        // (d == 0: equal keys, which no digit pass moves)
+        if (crowded || d == 0u || !fits()) *p.state = MSD_OFF;
+        p.window[0] = skip;
+        p.window[1] = b2;
+    }
+}
+
 // Keys per group, one read of the input.  16-bit counters, two to a word.
 // Rounds of at most 2^14 keys a CTA: a counter that a key of the round found
 // at 2^15 or above makes the CTA move those halves to the global counts after
 // the round's barrier, so none ever passes 2^15 + 2^14.
 constexpr int MSD_COUNT_THREADS = 1024;
 constexpr int MSD_COUNT_SMEM = 32768 * 4 + 256 * 4;
-template <int KB>
+template <int KB, bool EVEN>
 __global__ void __launch_bounds__(MSD_COUNT_THREADS, 1) msd_count_kernel(MsdParams p) {
     using U = typename KeyBits<KB>::U;
     extern __shared__ __align__(128) uint8_t smem[];
@@ -178,8 +412,10 @@ __global__ void __launch_bounds__(MSD_COUNT_THREADS, 1) msd_count_kernel(MsdPara
     grid_launch_dependents();
     grid_dependency_wait();
     if (ld_relaxed(p.state) & MSD_OFF) return;
+    uint2* table = reinterpret_cast<uint2*>(smem + MSD_COUNT_SMEM);
+    if constexpr (EVEN) MsdEvenCode::fetch(p, table);
     __syncthreads();
-    const MsdCode code_of(p);
+    const auto code_of = msd_code<EVEN>(p, table);
     const uint32_t b2 = code_of.b2, words = 128u << b2, shift = 24u - b2;
     const KeyMap<U> map(p.kind, p.desc);
     const U* keys = static_cast<const U*>(p.keys_in);
@@ -242,7 +478,7 @@ __global__ void __launch_bounds__(MSD_COUNT_THREADS, 1) msd_count_kernel(MsdPara
         }
         for (uint64_t j = head + nvec * PER_VEC + gtid; j < n; j += gthreads) count(keys[j]);
     };
-    if (p.kind == KIND_FLOAT) sweep(BoolTag<true>{});
+    if (EVEN || p.kind == KIND_FLOAT) sweep(BoolTag<true>{});
     else sweep(BoolTag<false>{});
     // a key that differs in the bits left out of the codes: the digit passes sort
     const uint64_t o64 = msd_top64(outside);
@@ -275,7 +511,7 @@ __global__ void __launch_bounds__(MSD_COUNT_THREADS, 1) msd_count_kernel(MsdPara
 }
 
 // Group offsets, one CTA per top digit, and the decision.
-template <int KB>
+template <bool EVEN>
 __global__ void __launch_bounds__(256) msd_scan_kernel(MsdParams p) {
     __shared__ uint32_t scan[32], base;
     grid_launch_dependents();
@@ -293,7 +529,27 @@ __global__ void __launch_bounds__(256) msd_scan_kernel(MsdParams p) {
     const uint32_t c = mine ? p.joint[(b << b2) + tid] : 0u;
     const uint32_t e2 = block_exclusive_scan_256<uint32_t>(c, scan, nullptr);
     if (mine) p.cursor2[(b << b2) + tid] = base + e2;
-    if (__syncthreads_or(c > p.group_cap) && tid == 0) atomicOr(p.state, MSD_OFF);
+    bool fits = c <= p.group_cap;
+    if constexpr (EVEN) {
+        if (!fits) {  // the group of a bin whose sampled keys were equal?
+            const uint32_t width = 1u << (24u - b2), code = ((b << b2) + tid) * width;
+            uint32_t lo = 0, hi = MsdEvenCode::BINS;  // the last bin that starts at or below it
+            while (hi - lo > 1u) {
+                const uint32_t mid = (lo + hi) / 2u;
+                if (p.table[mid].x <= code) lo = mid;
+                else hi = mid;
+            }
+            if (p.table[lo].x == code && p.table[lo].y == width) {
+                const uint32_t i = atomicAdd(p.giants, 1u);
+                if (i < MSD_GIANTS) {
+                    fits = true;
+                    p.giants[1 + 2 * i] = (b << b2) + tid;
+                    p.giants[2 + 2 * i] = reinterpret_cast<const uint32_t*>(p.table + MsdEvenCode::BINS)[lo];
+                }
+            }
+        }
+    }
+    if (__syncthreads_or(!fits) && tid == 0) atomicOr(p.state, MSD_OFF);
 }
 
 // Shared memory of a split: the stage, in which every digit has CAP places of
@@ -308,7 +564,12 @@ struct MsdSplitGeom {
     static_assert(STAGE >= TILE && (CAP % 2 == 1 || CAP == 0), "the stage also holds a dense tile");
     static_assert(IPT % (16 / KB) == 0, "16-byte loads");
     static constexpr size_t WORDS_OFF = size_t(STAGE) * KB;
-    static constexpr size_t SMEM_BYTES = WORDS_OFF + (256 * 6 + 1 + 32 + 4) * 4;
+    static constexpr int SPILL = CAP ? 512 : 0;  // keys beyond their digit's places
+    static constexpr size_t SPILL_OFF = (WORDS_OFF + (256 * 6 + 1 + 32 + 4) * 4 + 15) & ~size_t(15);
+    static constexpr size_t SMEM_BYTES = SPILL_OFF + SPILL * KB;
+    // floats: then the table of the codes
+    static constexpr size_t TABLE_OFF = (SMEM_BYTES + 15) & ~size_t(15);
+    static constexpr size_t EVEN_BYTES = TABLE_OFF + MsdEvenCode::BINS * 8;
 };
 
 // Keys [lo, hi) from the 16-byte aligned src into registers, by 16-byte loads:
@@ -354,15 +615,17 @@ __device__ __forceinline__ void msd_load_tile(const typename KeyBits<KB>::U* src
 // digit's keys.  bins: nb zeros on entry, left so.  refill() runs when the
 // keys' registers are free.
 // Every key takes its digit's next place with one shared atomic and goes
-// there at once; a warp then writes whole digits.  A digit with more keys than
-// its places hold (uneven digits) sends the tile through a dense stage, whose
-// places need the tile's counts first.
+// there at once; a warp then writes whole digits.  Keys beyond their digit's
+// places (uneven digits: a float's zeros) go to a list; more than the list
+// holds send the tile through a dense stage, whose places need the tile's
+// counts first (N(0, 1) floats with 1% zeros, 2^27: top split 606 -> 350 us
+// with the list; 2 * 10^7 row identifiers, whole sort 240 -> 225).
 // What bounds it: shared-memory wavefronts, 3.5 for a warp's access to random
 // banks; this makes two such accesses a key, the dense stage three (2^28
 // 4-byte keys: 0.43 against 0.58 ms).
-template <int KB, int THREADS, int IPT, int CAP, class In, class Reload, class Refill>
+template <int KB, int THREADS, int IPT, int CAP, class Code, class In, class Reload, class Refill>
 __device__ __forceinline__ void msd_split_tile(typename KeyBits<KB>::U (&keys)[IPT], uint32_t lo, uint32_t hi,
-                                               const MsdCode& code_of, uint32_t shift, uint32_t nb, uint32_t* claim,
+                                               const Code& code_of, uint32_t shift, uint32_t nb, uint32_t* claim,
                                                typename KeyBits<KB>::U* dst, uint32_t n, uint32_t* err, uint8_t* smem,
                                                In in, Reload reload, Refill refill) {
     using U = typename KeyBits<KB>::U;
@@ -433,15 +696,21 @@ __device__ __forceinline__ void msd_split_tile(typename KeyBits<KB>::U (&keys)[I
         __syncthreads();
         return;
     }
-    uint32_t last = 0;
+    U* spill = reinterpret_cast<U*>(smem + G::SPILL_OFF);
+    uint32_t* spilled = scan + 32;
     each([&](int u) {
         const U k = in(keys[u]);
         const uint32_t d = digit(k);
         const uint32_t slot = atomicAdd(&bins[d], 1u);
-        last = max(last, slot);
         if (slot < cap) stage[d * cap + slot] = k;
+        else {
+            const uint32_t i = atomicAdd(spilled, 1u);
+            if (i < uint32_t(G::SPILL)) spill[i] = k;
+        }
     });
-    const bool over = __syncthreads_or(last >= cap) != 0;
+    __syncthreads();
+    const uint32_t extra = *spilled;
+    const bool over = extra > uint32_t(G::SPILL);
     uint32_t c = 0, g = 0;
     if (uint32_t(tid) < nb) {
         c = bins[tid];
@@ -456,9 +725,20 @@ __device__ __forceinline__ void msd_split_tile(typename KeyBits<KB>::U (&keys)[I
                 bad = true;
                 c = 0;
             }
-            reinterpret_cast<uint2*>(runs)[tid] = make_uint2(g, c);
+            reinterpret_cast<uint2*>(runs)[tid] = make_uint2(g, min(c, cap));
         }
         __syncthreads();
+        if (extra) {  // after their digit's staged keys
+            for (uint32_t i = tid; i < extra; i += THREADS) {
+                const U k = spill[i];
+                const uint32_t d = digit(k), pos = reinterpret_cast<const uint2*>(runs)[d].x + cap + atomicAdd(&bins[d], 1u);
+                if (pos < n) dst[pos] = k;
+                else bad = true;
+            }
+            __syncthreads();
+            if (uint32_t(tid) < nb) bins[tid] = 0u;
+            if (tid == 0) *spilled = 0u;
+        }
         // A warp writes a digit's keys 32 at a time, four digits in flight.
         // The digit's words reach the lanes by a broadcast read: shuffles
         // take the same pipe, and two would be needed.
@@ -524,6 +804,7 @@ __device__ __forceinline__ void msd_split_tile(typename KeyBits<KB>::U (&keys)[I
         refill();
         __syncthreads();
         if (uint32_t(tid) < nb) bins[tid] = 0u;
+        if (tid == 0) *spilled = 0u;
         const uint32_t cnt = hi - lo;
         for (uint32_t j = tid; j < cnt; j += THREADS) {  // coalesced runs, one per digit
             const U k = stage[j];
@@ -538,7 +819,7 @@ __device__ __forceinline__ void msd_split_tile(typename KeyBits<KB>::U (&keys)[I
 
 // Top split (8 bits), input -> alternate buffer.  Tiles start at 16-byte
 // boundaries; each CTA's next tile loads while it writes one out.
-template <int KB, int THREADS, int IPT, int MIN_CTAS, int CAP>
+template <int KB, int THREADS, int IPT, int MIN_CTAS, int CAP, bool EVEN>
 __global__ void __launch_bounds__(THREADS, MIN_CTAS) msd_top_kernel(MsdParams p) {
     using U = typename KeyBits<KB>::U;
     using G = MsdSplitGeom<KB, THREADS, IPT, CAP>;
@@ -546,11 +827,14 @@ __global__ void __launch_bounds__(THREADS, MIN_CTAS) msd_top_kernel(MsdParams p)
     uint32_t* bins = reinterpret_cast<uint32_t*>(smem + G::WORDS_OFF);
     const int tid = threadIdx.x;
     for (int i = tid; i < 256; i += THREADS) bins[i] = 0u;
+    if (tid == 0) bins[256 * 5 + 257 + 32] = 0u;  // (the list's length)
     grid_launch_dependents();
     grid_dependency_wait();
     if (ld_relaxed(p.state) & MSD_OFF) return;
     const KeyMap<U> map(p.kind, p.desc);
-    const MsdCode code_of(p);
+    uint2* table = reinterpret_cast<uint2*>(smem + G::TABLE_OFF);
+    if constexpr (EVEN) MsdEvenCode::fetch(p, table);  // (the barrier below)
+    const auto code_of = msd_code<EVEN>(p, table);
     const U* keys_in = static_cast<const U*>(p.keys_in);
     const uint32_t skew = uint32_t(reinterpret_cast<uintptr_t>(keys_in) & 15u) / uint32_t(KB);
     const U* in = keys_in - skew;  // keys [skew, skew + n)
@@ -608,7 +892,7 @@ __device__ __forceinline__ uint32_t msd_bucket_of(const uint32_t* tfirst, uint32
 
 // Second split: within every top bucket, into the groups' ranges (alternate
 // buffer -> caller's buffer).
-template <int KB, int THREADS, int IPT, int MIN_CTAS, int CAP>
+template <int KB, int THREADS, int IPT, int MIN_CTAS, int CAP, bool EVEN>
 __global__ void __launch_bounds__(THREADS, MIN_CTAS) msd_second_kernel(MsdParams p) {
     using U = typename KeyBits<KB>::U;
     using G = MsdSplitGeom<KB, THREADS, IPT, CAP>;
@@ -621,10 +905,13 @@ __global__ void __launch_bounds__(THREADS, MIN_CTAS) msd_second_kernel(MsdParams
     uint32_t* scan = tfirst + 257;
     const int tid = threadIdx.x;
     for (int i = tid; i < 256; i += THREADS) bins[i] = 0u;
+    if (tid == 0) bins[256 * 5 + 257 + 32] = 0u;  // (the list's length)
     grid_launch_dependents();
     grid_dependency_wait();
     if (ld_relaxed(p.state) & MSD_OFF) return;
-    const MsdCode code_of(p);
+    uint2* table = reinterpret_cast<uint2*>(smem + G::TABLE_OFF);
+    if constexpr (EVEN) MsdEvenCode::fetch(p, table);  // (msd_top_table's barriers)
+    const auto code_of = msd_code<EVEN>(p, table);
     const uint32_t b2 = code_of.b2;
     const U* in = static_cast<const U*>(p.keys_b);
     const uint32_t skew = uint32_t(reinterpret_cast<uintptr_t>(in) & 15u) / uint32_t(KB);
@@ -744,24 +1031,6 @@ __device__ __forceinline__ void transposition_rounds(U (&k)[LIPT], uint32_t roun
             if (lane < 31 && after < k[LIPT - 1]) k[LIPT - 1] = after;
         }
     }
-}
-
-// Exclusive scan over the CTA with one barrier: every warp scans the warp
-// totals for itself (warp_tmp is written again only after another barrier).
-template <int THREADS>
-__device__ __forceinline__ uint32_t block_exclusive_scan_1b(uint32_t x, uint32_t* warp_tmp) {
-    constexpr int WARPS = THREADS / 32;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint32_t v = x;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xffffffffu, v, o);
-        if (lane >= o) v += y;
-    }
-    if (lane == 31) warp_tmp[warp] = v;
-    __syncthreads();
-    const uint32_t before = __reduce_add_sync(0xffffffffu, lane < warp && lane < WARPS ? warp_tmp[lane] : 0u);
-    return before + v - x;
 }
 
 // Sorts the CTA's `cnt` keys, all of one group: key VEC * i + e of a thread
@@ -915,7 +1184,7 @@ __device__ __forceinline__ void store_32b(void* dst, const uint4& a, const uint4
 // Local sorts: groups blockIdx.x, + gridDim.x, ... sorted in place.  The next
 // group's keys load while the network runs, and the one after it is pulled
 // into L2.
-template <int KB, int THREADS, int MIN_CTAS, int HALO>
+template <int KB, int THREADS, int MIN_CTAS, int HALO, bool EVEN>
 __global__ void __launch_bounds__(THREADS, MIN_CTAS) msd_local_kernel(MsdParams p) {
     using U = typename KeyBits<KB>::U;
     using G = GroupSortGeom<KB, THREADS, HALO>;
@@ -929,35 +1198,58 @@ __global__ void __launch_bounds__(THREADS, MIN_CTAS) msd_local_kernel(MsdParams 
     if (ld_relaxed(p.state) & MSD_OFF) return;
     __syncthreads();
     U* keys = static_cast<U*>(p.keys_a);
-    const MsdCode code_of(p);
+    // (floats: a group's keys share few bins, so the table's reads are broadcasts)
+    const auto code_of = msd_code<EVEN>(p, p.table);
     const uint32_t groups = 256u << code_of.b2;
-    auto bounds = [&](uint32_t g, uint32_t& off, uint32_t& cnt) {
-        off = (g != 0u && g < groups) ? p.cursor2[g - 1] : 0u;
-        cnt = g < groups ? p.cursor2[g] - off : 0u;
+    // The CTA's groups in turn: g, + gridDim.x, ...  Floats: two neighbours are
+    // sorted as one where they fit, since their groups, as many as the densest
+    // stretch needs, are small (6 * 10^7 keys of N(0, 1): 336 -> 243 us).
+    struct Group {
+        uint32_t off, word;  // word: its keys, below 2^16, and the leading bits that their codes share; 0: none left
+        __device__ __forceinline__ uint32_t cnt() const { return word & 0xffffu; }
+    };
+    uint32_t ahead = blockIdx.x, half = 0u;  // the next one
+    auto next_group = [&] {
+        Group r{0u, 0u};
+        if constexpr (EVEN) {
+            if (ahead * 2u < groups) {
+                const uint32_t a = ahead ? p.cursor2[ahead * 2u - 1u] : 0u, b = p.cursor2[ahead * 2u], c = p.cursor2[ahead * 2u + 1u];
+                const bool both = c - a <= p.group_cap;
+                r.off = half ? b : a;
+                uint32_t cnt = (both || half ? c : b) - r.off;
+                if (cnt > p.group_cap) cnt = 0u;  // equal keys, below
+                r.word = cnt | (8u + code_of.b2 - uint32_t(both)) << 16;
+                half = both ? 0u : half ^ 1u;
+                if (half) return r;
+            }
+        } else if (ahead < groups) {
+            r.off = ahead ? p.cursor2[ahead - 1u] : 0u;
+            r.word = (p.cursor2[ahead] - r.off) | (8u + code_of.b2) << 16;
+        }
+        ahead += gridDim.x;
+        return r;
     };
     // Key VEC * i + e of a thread is the group's key
     // (i * THREADS + tid) * VEC + e - shift: 16-byte loads from the address
     // at or below the group's start (which keys a thread has does not matter)
     const KeyMap<U> map(p.kind, p.desc);
-    uint32_t g = blockIdx.x, off, cnt, off1, cnt1;
-    bounds(g, off, cnt);
-    bounds(g + gridDim.x, off1, cnt1);
+    Group cur = next_group(), next = next_group();
     U k[LIPT];
     auto skew_of = [&](uint32_t o, uint32_t bytes) {
         return uint32_t(reinterpret_cast<uintptr_t>(keys + o) & (bytes - 1u)) / uint32_t(KB);
     };
     auto index = [&](uint32_t skew, int u) { return (uint32_t(u / VEC) * THREADS + tid) * VEC + uint32_t(u % VEC) - skew; };
-    auto load = [&](uint32_t o, uint32_t c) {
-        const uint32_t skew = skew_of(o, 16);
-        load_vectors<THREADS>(const_cast<const U*>(keys) + o - skew, skew, skew + c, k);
+    auto load = [&](const Group& f) {
+        const uint32_t skew = skew_of(f.off, 16);
+        load_vectors<THREADS>(const_cast<const U*>(keys) + f.off - skew, skew, skew + f.cnt(), k);
     };
-    load(off, cnt);
-    while (g < groups) {
-        uint32_t off2, cnt2;
-        bounds(g + 2 * gridDim.x, off2, cnt2);
+    load(cur);
+    while (cur.word != 0u) {
+        const Group later = next_group();
+        const uint32_t off = cur.off, cnt = cur.cnt();
         {
-            const uintptr_t a = reinterpret_cast<uintptr_t>(keys + off2) & ~uintptr_t(127);
-            const uintptr_t e = reinterpret_cast<uintptr_t>(keys + off2 + cnt2);
+            const uintptr_t a = reinterpret_cast<uintptr_t>(keys + later.off) & ~uintptr_t(127);
+            const uintptr_t e = reinterpret_cast<uintptr_t>(keys + later.off + later.cnt());
             for (uintptr_t q = a + uintptr_t(tid) * 128; q < e; q += uintptr_t(THREADS) * 128)
                 asm volatile("prefetch.global.L2 [%0];" ::"l"(q));
         }
@@ -967,8 +1259,8 @@ __global__ void __launch_bounds__(THREADS, MIN_CTAS) msd_local_kernel(MsdParams 
         if (cnt != 0u)
             sorted = group_sort<U, THREADS, HALO>(
                 k, cnt, skew, pad, smem,
-                [&](U x) { return __umulhi(code_of(x) << (8u + code_of.b2), uint32_t(G::BINS)); },
-                [&] { load(off1, cnt1); },
+                [&](U x) { return __umulhi(code_of(x) << (cur.word >> 16), uint32_t(G::BINS)); },
+                [&] { load(next); },
                 [&](uint32_t c0, bool inside, const U(&x)[LIPT]) {
                     union { uint4 q[4]; U k[LIPT]; } w;
 #pragma unroll
@@ -989,17 +1281,65 @@ __global__ void __launch_bounds__(THREADS, MIN_CTAS) msd_local_kernel(MsdParams 
             // the buffer holds the input's keys in some order, and the digit
             // passes sort it (keys only: any order of the input sorts to the
             // same bytes)
+            if constexpr (EVEN) {
+                // equal keys are in order, and values that the sample has
+                // missed take a bitonic network over the group, 91 steps at
+                // most, where a sort that gave up would be lost
+                U* sk = reinterpret_cast<U*>(smem);
 #pragma unroll
-            for (int u = 0; u < LIPT; ++u)
-                if (index(skew, u) < cnt) keys[off + index(skew, u)] = map.out(k[u]);
-            if (tid == 0) atomicOr(p.state, MSD_GAVE_UP);
+                for (int u = 0; u < LIPT; ++u)
+                    if (index(skew, u) < cnt) sk[index(skew, u)] = k[u];
+                __syncthreads();
+                bool differ = false;
+                for (uint32_t i = tid; i < cnt; i += THREADS) differ |= sk[i] != sk[0];
+                differ = __syncthreads_or(differ) != 0;
+                uint32_t size = 1024u;
+                static_assert(KB != 4 || 8192 * KB <= int(G::SCAN_OFF), "the group padded to a power of two");
+                while (size < cnt) size *= 2u;
+                for (uint32_t i = cnt + tid; i < size; i += THREADS) sk[i] = U(~U(0));
+                for (uint32_t run = 2; differ && run <= size; run *= 2u)
+                    for (uint32_t gap = run / 2u; gap != 0u; gap /= 2u) {
+                        __syncthreads();
+                        for (uint32_t i = tid; i < size / 2u; i += THREADS) {
+                            const uint32_t a = 2u * i - (i & (gap - 1u)), b = a + gap;
+                            U x = sk[a], y = sk[b];
+                            if ((x > y) == ((a & run) == 0u)) {
+                                sk[a] = y;
+                                sk[b] = x;
+                            }
+                        }
+                    }
+                __syncthreads();
+                for (uint32_t i = tid; i < cnt; i += THREADS) keys[off + i] = map.out(sk[i]);
+                __syncthreads();
+                for (int i = tid; i < G::BINS / 4; i += THREADS) reinterpret_cast<uint32_t*>(smem + G::CTR_OFF)[i] = 0u;
+                __syncthreads();
+            } else {
+#pragma unroll
+                for (int u = 0; u < LIPT; ++u)
+                    if (index(skew, u) < cnt) keys[off + index(skew, u)] = map.out(k[u]);
+                if (tid == 0) atomicOr(p.state, MSD_GAVE_UP);
+            }
         }
-        if (!sorted || cnt == 0u) load(off1, cnt1);
-        g += gridDim.x;
-        off = off1;
-        cnt = cnt1;
-        off1 = off2;
-        cnt1 = cnt2;
+        if (!sorted || cnt == 0u) load(next);
+        cur = next;
+        next = later;
+    }
+    if constexpr (EVEN) {
+        // groups of equal keys above the largest: every CTA takes a slice and
+        // looks whether they are
+        const uint32_t giants = min(p.giants[0], MSD_GIANTS);
+        for (uint32_t i = 0; i < giants; ++i) {
+            const uint32_t gi = p.giants[1 + 2 * i], value = p.giants[2 + 2 * i];
+            const uint32_t from = gi != 0u ? p.cursor2[gi - 1] : 0u, to = p.cursor2[gi];
+            bool d = false;
+            for (uint64_t j = uint64_t(from) + blockIdx.x * THREADS + tid; j < to; j += uint64_t(gridDim.x) * THREADS) {
+                const U x = keys[j];
+                d |= x != value;
+                keys[j] = map.out(x);
+            }
+            if (__syncthreads_or(d) && tid == 0) atomicOr(p.state, MSD_GAVE_UP);
+        }
     }
 }
 

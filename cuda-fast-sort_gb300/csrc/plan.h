@@ -69,6 +69,10 @@ struct MsdLayout {
     static constexpr size_t bytes(int b2) { return JOINT + 2 * (size_t(256) << b2) * 4; }
     static constexpr size_t BYTES = 256 + 256 * 4 + 3 * 65536 * 4;
     static_assert(JOINT + 2 * 65536 * 4 <= BYTES, "the counters fit their block");
+    // 4-byte floats: then the large groups of equal keys, cleared with the
+    // counters, and the codes' table with a sampled key of every bin
+    static constexpr size_t GIANTS_BYTES = 256;
+    static constexpr size_t even_bytes(int b2) { return bytes(b2) + GIANTS_BYTES + 4096 * 12; }
 };
 
 struct Plan {
@@ -101,6 +105,7 @@ struct Plan {
     // status words, which only the digit passes use
     bool msd = false;
     bool msd_block = false;
+    bool msd_even = false;  // 4-byte floats: codes by the sample's distribution
     KernelEntry msd_k[6]{};
     uint32_t msd_group_cap = 0;
     int msd_b2 = 0;

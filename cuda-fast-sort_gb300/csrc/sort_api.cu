@@ -57,6 +57,7 @@ const KernelEntry* multi_entries_k16(int vb);
 const KernelEntry* finish_entries_k8();
 const KernelEntry* finish_entries_k16();
 const KernelEntry* msd_entries_k4();
+const KernelEntry* msd_even_entries_k4();
 const KernelEntry* msd_entries_k8();
 const KernelEntry* msd_entries_k16();
 
@@ -359,13 +360,15 @@ int make_plan(int key_type, size_t value_bytes, uint64_t n, Plan* plan) {
     }
     // keys-only sorts above the one-launch range: the most-significant-first
     // path, its counters in a block of their own (sized whether or not the
-    // path is switched on) or in the status words.  Not floats, unless they
-    // always had that block: their leading bits are the exponent, so that most
-    // values share few groups and the path's first kernels are spent in vain
-    // (f64 N(0,1), 2.5 x 10^6 keys: 247 against 222 us).
+    // path is switched on) or in the status words.  Floats' leading bits are the
+    // exponent, so that most values share few groups: 4-byte ones have codes of
+    // their own (MsdEvenCode), the others take it only where they always had
+    // that block (f64 N(0,1), 2.5 x 10^6 keys: 247 against 222 us).
     const bool block = n >= msd_block_n_min(p.kb);
-    if (p.vb == 0 && n > fused_n_max(p.kb) && n <= msd_n_max(p.kb) && (block || p.kind != KIND_FLOAT) &&
-        msd_entries(p.kb) != nullptr) {
+    const bool even = p.kb == 4 && p.kind == KIND_FLOAT;
+    if (p.vb == 0 && n > fused_n_max(p.kb) && n <= (even ? MSD_EVEN_N_MAX : msd_n_max(p.kb)) &&
+        (!even || n >= MSD_EVEN_N_MIN) &&
+        (block || even || p.kind != KIND_FLOAT) && msd_entries(p.kb) != nullptr) {
         const int shape = msd_local_shape(p.kb, n);
         p.msd_group_cap = msd_group_cap(p.kb, shape);
         p.msd_b2 = msd_b2_max(n, p.msd_group_cap);
@@ -376,10 +379,12 @@ int make_plan(int key_type, size_t value_bytes, uint64_t n, Plan* plan) {
             off = align_up(off + MsdLayout::BYTES, 256);
         }
         if (g_msd.load(std::memory_order_relaxed) &&
-            (p.msd_block || MsdLayout::bytes(p.msd_b2) <= p.status_bytes)) {
+            (p.msd_block || (even ? MsdLayout::even_bytes(p.msd_b2) : MsdLayout::bytes(p.msd_b2)) <= p.status_bytes)) {
             p.msd = true;
-            for (int i = 0; i < 5; ++i) p.msd_k[i] = msd_entries(p.kb)[i];
-            p.msd_k[5] = msd_entries(p.kb)[5 + shape];
+            p.msd_even = even;
+            const KernelEntry* e = even ? msd_even_entries_k4() : msd_entries(p.kb);
+            for (int i = 0; i < 5; ++i) p.msd_k[i] = e[i];
+            p.msd_k[5] = e[5 + shape];
         }
     }
     if (short_regions) {
@@ -723,14 +728,23 @@ int enqueue_sort(const Plan& plan, int descending, void* d_keys, void* d_values,
         mp.cursor1 = reinterpret_cast<uint32_t*>(msd_block + MsdLayout::CURSOR1);
         mp.joint = reinterpret_cast<uint32_t*>(msd_block + MsdLayout::JOINT);
         mp.cursor2 = mp.joint + (size_t(256) << plan.msd_b2);
+        if (plan.msd_even) {
+            uint8_t* even = msd_block + MsdLayout::bytes(plan.msd_b2);
+            mp.giants = reinterpret_cast<uint32_t*>(even);
+            mp.zero_words += uint32_t(MsdLayout::GIANTS_BYTES / 4);
+            mp.table = reinterpret_cast<uint2*>(even + MsdLayout::GIANTS_BYTES);
+        }
         mp.group_cap = plan.msd_group_cap;
         mp.err = err_word;
         for (int i = 0; i < 6; ++i) {
             const KernelEntry& k = plan.msd_k[i];
             const uint64_t full = uint64_t(sms > 0 ? sms : 1) * uint64_t(resident_ctas(k) > 0 ? resident_ctas(k) : 1);
             const uint64_t per_top = 256;  // scan: one CTA per top digit
-            const uint64_t clear = 1 + (mp.zero_words + 4095) / 4096;  // sample: and CTAs that clear the counters
-            const uint32_t grid = uint32_t(i == 0 ? (clear < full ? clear : full) : i == 2 ? per_top : full);
+            // sample: and CTAs that clear the counters (floats: clusters of both)
+            const uint64_t zeros = (mp.zero_words + 4095) / 4096;
+            const uint64_t clear = plan.msd_even ? MSD_EVEN_CLUSTER + (zeros + MSD_EVEN_CLUSTER - 1) / MSD_EVEN_CLUSTER * MSD_EVEN_CLUSTER
+                                                 : 1 + zeros;
+            const uint32_t grid = uint32_t(i == 0 ? clear : i == 2 ? per_top : full);
             void* args[] = {&mp};
             e = launch_dependent(k.fn, grid, k.threads, k.smem, stream, args);
             if (e != cudaSuccess) return fail("msd launch", e);
@@ -751,8 +765,8 @@ int enqueue_sort(const Plan& plan, int descending, void* d_keys, void* d_values,
     // a refused launch: every digit pass below, each in a launch of its own
     if (use_finish && launch_passes(pass_params(0)) != cudaSuccess) use_finish = false;
     // After the MSD kernels one launch looks at their state where P passes and
-    // the fix-up each did (an exit is 2.2 us: 50M u64 keys 957 -> 948 us, 5M
-    // u32 129 -> 94); timed, and without skipping, each pass has its own.
+    // the fix-up each did (an exit is 2.2 us: 50M u64 keys 957 -> 948 us, 2^26
+    // u128 ones 1754 -> 1735); timed, and without skipping, each pass has its own.
     if (use_msd && !timed && skip && prepare_kernel(plan.multi) == GBSORT_OK &&
         launch_passes(pass_params(0)) == cudaSuccess)
         return GBSORT_OK;  // (the fix-up is part of that launch)
