@@ -32,7 +32,7 @@
 // exit at once.
 // Every key is read four times and written three times, whatever its width.
 // 4-byte floats take it too, by a group number from the sample's distribution
-// (MsdEvenCode; 2^27 keys of N(0, 1) 1.47 ms, four digit passes 2.03; the
+// (MsdEvenCode; 2^27 keys of N(0, 1) 1.50 ms, four digit passes 2.03; the
 // table's reads cost the count and the splits about a half: 6 * 10^7 keys
 // 80 + 160 + 185 us, unsigned keys 49 + 110 + 138).
 #pragma once
@@ -89,16 +89,18 @@ struct MsdCode {
 // their codes are the sample's distribution function instead: the leading 12
 // bits (sign, exponent, 3 bits of mantissa) name a stretch of the codes as wide
 // as the share of the sample there, {start, width}, and the 20 bits below
-// divide it evenly (both after the `skip` bits that all keys share).
+// divide it evenly (both after the `skip` bits that the sample's keys share; keys
+// outside their range, few if any, count as its nearest end).
 // Monotone; two keys may share a code.
 struct MsdEvenCode {
     static constexpr uint32_t BINS = 4096;
     const uint2* table;
-    uint32_t skip, b2;
+    uint32_t skip, b2, low, high;  // low, high: the range
     __device__ __forceinline__ MsdEvenCode(const MsdParams& p, const uint2* t)
-        : table(t), skip(ld_relaxed(p.window)), b2(ld_relaxed(p.window + 1)) {}
+        : table(t), skip(ld_relaxed(p.window)), b2(ld_relaxed(p.window + 1)), low(p.table[BINS + BINS / 2].x),
+          high(low | 0xffffffffu >> skip) {}
     __device__ __forceinline__ uint32_t operator()(uint32_t k) const {
-        const uint32_t c = k << skip;
+        const uint32_t c = min(max(k, low), high) << skip;
         const uint2 e = table[c >> 20];
         return e.x + __umulhi(c << 12, e.y);
     }
@@ -128,9 +130,9 @@ __global__ void __launch_bounds__(MSD_SAMPLE_THREADS) msd_sample_kernel(MsdParam
         return;
     }
     constexpr uint32_t SLOTS = 8192, NONE = 0xffffffffu;
-    __shared__ uint32_t vary[2], top, again, bins[256], seen[SLOTS];
+    __shared__ uint32_t vary[2], top, again, neighbours, bins[256], seen[SLOTS];
     if (tid < 2) vary[tid] = 0u;
-    if (tid == 0) top = again = 0u;
+    if (tid == 0) top = again = neighbours = 0u;
     for (uint32_t i = tid; i < SLOTS; i += MSD_SAMPLE_THREADS) seen[i] = NONE;
     if (tid < 256) bins[tid] = 0u;
     __syncthreads();
@@ -138,7 +140,11 @@ __global__ void __launch_bounds__(MSD_SAMPLE_THREADS) msd_sample_kernel(MsdParam
     const U* keys = static_cast<const U*>(p.keys_in);
     constexpr int PER = 4;
     const uint32_t step = uint32_t(p.n / (MSD_SAMPLE_THREADS * PER));
-    uint64_t x[PER];
+    uint64_t x[PER], y;  // y: four keys after the first of them
+    {
+        const uint64_t j = uint64_t(tid) * step + (uint32_t(tid) * 2654435761u) % step;
+        y = msd_top64(map.in(keys[j + 4u]));
+    }
 #pragma unroll
     for (int i = 0; i < PER; ++i) {
         const uint32_t at = uint32_t(i * MSD_SAMPLE_THREADS + tid);
@@ -156,6 +162,10 @@ __global__ void __launch_bounds__(MSD_SAMPLE_THREADS) msd_sample_kernel(MsdParam
     }
     __syncthreads();
     const uint32_t skip = vary[0] ? __clz(vary[0]) : vary[1] ? 32u + __clz(vary[1]) : 0u;
+    // keys in order send whole tiles to one digit: shared atomics on one
+    // address, slower than the digit passes (10^7 4-byte keys 290 and 207 us)
+    const uint32_t close = __popc(__ballot_sync(0xffffffffu, ((x[0] ^ y) << skip) >> 56 == 0u));
+    if ((tid & 31) == 0) atomicAdd(&neighbours, close);
     uint32_t most = 0, twice = 0;
 #pragma unroll
     for (int i = 0; i < PER; ++i) {
@@ -191,7 +201,7 @@ __global__ void __launch_bounds__(MSD_SAMPLE_THREADS) msd_sample_kernel(MsdParam
         while (b2 < uint32_t(p.b2_max) && n > 0.72f * cap * float(1u << b2)) ++b2;
         constexpr float S = MSD_SAMPLE_THREADS * PER;
         const bool crowded = again >= 16u && 2.f * float(again) * n > 64.f * S * S;
-        if (uneven || crowded || n > cap * float(1u << b2)) *p.state = MSD_OFF;
+        if (uneven || crowded || 2u * neighbours > uint32_t(MSD_SAMPLE_THREADS) || n > cap * float(1u << b2)) *p.state = MSD_OFF;
         p.window[0] = skip;
         p.window[1] = b2;
     }
@@ -233,7 +243,7 @@ __global__ void __cluster_dims__(MSD_EVEN_CLUSTER, 1, 1) __launch_bounds__(MSD_S
     msd_even_sample_kernel(MsdParams p) {
     static_assert(KB == 4, "codes of 4-byte floats");
     namespace cg = cooperative_groups;
-    constexpr uint32_t BINS = MsdEvenCode::BINS, NONE = 0xffffffffu, SLOTS = 4096;
+    constexpr uint32_t BINS = MsdEvenCode::BINS, NONE = 0xffffffffu, SLOTS = 8192;
     constexpr int VECS = 2, PER = MSD_SAMPLE_THREADS * MSD_EVEN_CLUSTER;
     constexpr float S = float(PER * VECS * 4);
     extern __shared__ __align__(16) uint32_t smem_even[];
@@ -241,7 +251,7 @@ __global__ void __cluster_dims__(MSD_EVEN_CLUSTER, 1, 1) __launch_bounds__(MSD_S
     uint32_t* low = cnt + BINS;
     uint32_t* high = low + BINS;
     uint32_t* all = high + BINS;  // (first CTA) the same of the cluster
-    __shared__ uint32_t vary, again, dense, scan[2][32], total[2];
+    __shared__ uint32_t vary, again, neighbours, equal, dense, scan[2][32], total[2];
     grid_launch_dependents();
     grid_dependency_wait();
     const uint32_t tid = threadIdx.x;
@@ -273,7 +283,7 @@ __global__ void __cluster_dims__(MSD_EVEN_CLUSTER, 1, 1) __launch_bounds__(MSD_S
         cnt[i] = high[i] = 0u;
         low[i] = NONE;
     }
-    if (tid == 0) vary = again = dense = 0u;
+    if (tid == 0) vary = again = neighbours = equal = dense = 0u;
     __syncthreads();
     uint32_t d = 0;
 #pragma unroll
@@ -308,19 +318,25 @@ __global__ void __cluster_dims__(MSD_EVEN_CLUSTER, 1, 1) __launch_bounds__(MSD_S
             to[2 * BINS + b] = hi;
         }
     }
-    cluster.sync();  // (nobody reads the others' arrays after this)
-    if (rank != 0) return;
-    // Keys that repeat more than 32 times would crowd the local sorts'
+    // Keys that repeat more than a dozen times would crowd the local sorts'
     // sub-buckets (those of a bin of equal keys do not matter): pairs of equal
-    // keys among 2048 of the sample.
+    // keys among half of every CTA's sample.
+    uint32_t count_in = 0;
+#pragma unroll
+    for (int i = 0; i < VECS * 4; ++i) {
+        const uint32_t b = (x[i] << skip) >> 20;
+        count_in |= uint32_t((i & 3) < 2 && low[b] != high[b] && x[i] != NONE) << i;
+    }
+    cluster.sync();  // (nobody reads the others' counts after this)
     for (uint32_t i = tid; i < SLOTS; i += MSD_SAMPLE_THREADS) cnt[i] = NONE;
     __syncthreads();
-    uint32_t twice = 0;
+    uint32_t twice = 0, runs = 0;
 #pragma unroll
-    for (int i = 0; i < VECS; ++i) {
-        const uint32_t k = x[i * 4], b = (k << skip) >> 20;
-        if (all[BINS + b] == all[2 * BINS + b] || k == NONE) continue;
-        uint32_t h = (k * 2654435761u) >> 20;
+    for (int i = 0; i < VECS * 4; ++i) {
+        const uint32_t k = x[i];
+        if (i % 4 == 0) runs += ((k ^ x[i + 1]) | (k ^ x[i + 2]) | (k ^ x[i + 3])) << skip < 1u << 24;
+        if (!(count_in >> i & 1u)) continue;
+        uint32_t h = (k * 2654435761u) >> 19;
         for (int probe = 0; probe < 64; ++probe) {
             uint32_t v = cnt[h];
             if (v == NONE) v = atomicCAS(&cnt[h], NONE, k);
@@ -332,9 +348,12 @@ __global__ void __cluster_dims__(MSD_EVEN_CLUSTER, 1, 1) __launch_bounds__(MSD_S
             h = (h + 1u) & (SLOTS - 1u);
         }
     }
-    if (twice) atomicAdd(&again, twice);
+    if (twice) atomicAdd(cluster.map_shared_rank(&again, 0), twice);
+    if (runs) atomicAdd(cluster.map_shared_rank(&neighbours, 0), runs);
+    cluster.sync();
+    if (rank != 0) return;
     // the layout: four bins a thread
-    uint32_t w[4], alone = 0, sum = 0;
+    uint32_t w[4], alone = 0, sum = 0, same = 0;
     float most = 0.f;  // keys of the sample per unit of stretch, where they lie densest
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -354,7 +373,9 @@ __global__ void __cluster_dims__(MSD_EVEN_CLUSTER, 1, 1) __launch_bounds__(MSD_S
         }
         sum += w[i];
         alone += w[i] == 0u;
+        same += w[i] == 0u ? uint32_t(k) : 0u;
     }
+    if (same) atomicAdd(&equal, same);
     atomicMax(&dense, __float_as_uint(most));
     uint32_t at = block_exclusive_scan_1b<MSD_SAMPLE_THREADS>(sum, scan[0]);
     uint32_t alones = block_exclusive_scan_1b<MSD_SAMPLE_THREADS>(alone, scan[1]);
@@ -371,6 +392,7 @@ __global__ void __cluster_dims__(MSD_EVEN_CLUSTER, 1, 1) __launch_bounds__(MSD_S
         return groups >= 4u * P && n * units <= 0.6f * S * float(p.group_cap) * float(groups - 2u * P);
     };
     while (b2 < uint32_t(p.b2_max) && !fits()) ++b2;
+    const uint32_t shared = skip ? first >> (32u - skip) << (32u - skip) : 0u;
     const uint32_t group = 1u << (24u - b2);
     const uint64_t scale = ((uint64_t(1) << 32) - 2ull * P * group) / W;
 #pragma unroll
@@ -380,15 +402,20 @@ __global__ void __cluster_dims__(MSD_EVEN_CLUSTER, 1, 1) __launch_bounds__(MSD_S
         p.table[b] = w[i] == 0u ? make_uint2(uint32_t((r + group - 1u) & ~uint64_t(group - 1u)), group)
                                 : make_uint2(uint32_t(r), uint32_t(w[i] * scale));
         // a bin of equal keys: the key
-        reinterpret_cast<uint32_t*>(p.table + BINS)[b] = (skip ? first >> (32u - skip) << (32u - skip) : 0u) | all[BINS + b] >> skip;
+        reinterpret_cast<uint32_t*>(p.table + BINS)[b] = shared | all[BINS + b] >> skip;
         at += w[i];
         alones += w[i] == 0u;
     }
     if (tid == 0) {
-        constexpr float R = MSD_SAMPLE_THREADS * VECS;
-        const bool crowded = again >= 6u && 2.f * float(again) * n > 32.f * R * R;
-        // (d == 0: equal keys, which no digit pass moves)
-        if (crowded || d == 0u || !fits()) *p.state = MSD_OFF;
+        constexpr float R = MSD_SAMPLE_THREADS * VECS * 2;  // of CLUSTER * R * R / 2 pairs
+        const bool crowded = again >= 6u && float(again) * n > 12.f * 0.5f * MSD_EVEN_CLUSTER * R * R;
+        // Keys in order send whole tiles to one digit, and so do many equal
+        // ones: shared atomics on one address, slower than the digit passes
+        // (10^7 keys in order 294 and 207 us, with 60% zeros 267 and 250).
+        // d == 0: equal keys, which no digit pass moves.
+        const bool runs_of_keys = 2u * neighbours > uint32_t(PER * VECS) || float(equal) > 0.4f * S;
+        if (crowded || runs_of_keys || d == 0u || !fits()) *p.state = MSD_OFF;
+        p.table[BINS + BINS / 2].x = shared;
         p.window[0] = skip;
         p.window[1] = b2;
     }
@@ -480,9 +507,10 @@ __global__ void __launch_bounds__(MSD_COUNT_THREADS, 1) msd_count_kernel(MsdPara
     };
     if (EVEN || p.kind == KIND_FLOAT) sweep(BoolTag<true>{});
     else sweep(BoolTag<false>{});
+    if constexpr (EVEN) __syncthreads();  // (else the barrier of the next test)
     // a key that differs in the bits left out of the codes: the digit passes sort
     const uint64_t o64 = msd_top64(outside);
-    if (__syncthreads_or(code_of.skip != 0u && (o64 >> (64u - code_of.skip)) != 0u)) {
+    if (!EVEN && __syncthreads_or(code_of.skip != 0u && (o64 >> (64u - code_of.skip)) != 0u)) {
         if (tid == 0) atomicOr(p.state, MSD_OFF);
         return;
     }

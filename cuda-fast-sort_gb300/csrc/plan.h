@@ -70,9 +70,10 @@ struct MsdLayout {
     static constexpr size_t BYTES = 256 + 256 * 4 + 3 * 65536 * 4;
     static_assert(JOINT + 2 * 65536 * 4 <= BYTES, "the counters fit their block");
     // 4-byte floats: then the large groups of equal keys, cleared with the
-    // counters, and the codes' table with a sampled key of every bin
+    // counters, and the codes' table, a sampled key of every
+    // bin, and the range of the codes
     static constexpr size_t GIANTS_BYTES = 256;
-    static constexpr size_t even_bytes(int b2) { return bytes(b2) + GIANTS_BYTES + 4096 * 12; }
+    static constexpr size_t even_bytes(int b2) { return bytes(b2) + GIANTS_BYTES + 4096 * 12 + 16; }
 };
 
 struct Plan {

@@ -564,8 +564,10 @@ typedef struct gbsort_plan_info {
     uint32_t pass_ctas;       /* persistent CTAs of the pass kernel          */
     uint32_t hist_ctas;       /* CTAs of the histogram kernel                */
     uint32_t status_word_bytes; /* 4 or 8                                    */
-    uint32_t kernel_launches; /* launches (plus one memset node) per sort;
-                                 1 when a short array sorts in one launch     */
+    uint32_t kernel_launches; /* launches (plus one memset node) of a timed
+                                 sort; 1 when a short keys-only array sorts in
+                                 one launch.  Untimed sorts make one launch of
+                                 the digit passes where a shorter path runs   */
     uint64_t workspace_bytes;
     uint32_t msd_region_keys; /* one-launch sort, most significant digit
                                  first: keys per top-digit region of its

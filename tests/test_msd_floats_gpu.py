@@ -30,6 +30,10 @@ def _values(dist, n, rng):
         x = rng.random(n, dtype=np.float32) * np.float32(900)
     elif dist == "one_exponent":
         x = rng.random(n, dtype=np.float32) + np.float32(1)
+    elif dist == "outliers":  # outside the range that the sample's keys share
+        x = rng.random(n, dtype=np.float32) + np.float32(1)
+        for i, v in enumerate((0.0, -0.0, -5.0, 1e30, np.inf, 0.25, 64.0)):
+            x[rng.integers(0, n, 1 + 3 * i)] = v
     elif dist == "exponential":
         x = rng.standard_exponential(n, dtype=np.float32)
     elif dist == "rounded":  # few values: too crowded for the local sorts
@@ -48,8 +52,8 @@ def _values(dist, n, rng):
 
 
 @pytest.mark.parametrize("desc", [False, True])
-@pytest.mark.parametrize("dist", ["normal", "special", "to_900", "one_exponent", "exponential", "rounded",
-                                  "mixed_giant", "many_giants", "crowds"])
+@pytest.mark.parametrize("dist", ["normal", "special", "to_900", "one_exponent", "outliers", "exponential",
+                                  "rounded", "mixed_giant", "many_giants", "crowds"])
 def test_distributions(gb, cuda, oracle, dist, desc):
     rng = np.random.default_rng(len(dist) + desc)
     raw = _values(dist, LEAST + 4099, rng).astype(raw_keys("f32", 1, 0).dtype)
