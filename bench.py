@@ -491,12 +491,6 @@ def bench_gbsort(args, cfg, world, rank, local):
         ups_ms = statistics.mean(p[0] for p in per_kernel)
         launch_ms = statistics.mean(statistics.mean(p[1:1 + passes]) for p in per_kernel)
         launch_bytes, kernel = n * 2 * (kbytes + vb), "onesweep_pass_kernel"
-    # launches of one untimed sort
-    sort_launches = plan.kernel_launches
-    if not vb and plan.kernel_launches > passes + 2:
-        sort_launches = 8
-    elif vb in (4, 8) and kbytes >= 8:
-        sort_launches = 6
     achieved = launch_bytes / (launch_ms / 1e3) / 1e9
     roofline = {"bound": "hbm", "kernel": kernel, "achieved": round(achieved, 1),
                 "peak": hbm, "unit": "GB/s", "frac": round(achieved / hbm, 4), "traffic": traffic,
@@ -509,6 +503,9 @@ def bench_gbsort(args, cfg, world, rank, local):
     sort_roofline = {"bytes_per_key": sort_bytes // n, "achieved": round(
         sort_bytes / (mean_sort_ms / 1e3) / 1e9, 1), "peak": hbm, "unit": "GB/s",
         "frac": round(sort_bytes / (mean_sort_ms / 1e3) / 1e9 / hbm, 4)}
+    if vb in (4, 8) and kbytes >= 8:
+        sort_roofline["note"] = ("counts a pass per key byte; the sort makes the leading ones and a finish, so fewer "
+                                 "bytes move")
 
     # comparator: CUB DeviceRadixSort (toolkit) on the same buffers, same timing
     cub = None
@@ -600,6 +597,12 @@ def bench_gbsort(args, cfg, world, rank, local):
     if rank != 0:
         return None
     plan = gbsort.plan(kt, n, vb)
+    # launches of one untimed sort
+    sort_launches = plan.kernel_launches
+    if not vb and plan.kernel_launches > passes + 2:
+        sort_launches = 8
+    elif vb in (4, 8) and kbytes >= 8:
+        sort_launches = 6
     line = {
         "metric": PLAIN_METRIC, "value": round(value, 3),
         "unit": "Gkeys/s", "n_gpus": world, "steps": args.steps, "warmup": args.warmup,
