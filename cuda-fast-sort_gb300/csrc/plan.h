@@ -126,6 +126,11 @@ struct Plan {
     size_t short_off = 0;
     size_t total_bytes = 0;
     CtlLayout ctl{};
+    // the process-wide switches as this plan found them, each read once: the
+    // kernels, their parameters and the graph's key have to agree while another
+    // thread changes them
+    bool skip = false;       // uniform-digit pass skipping
+    bool short_msd = false;  // most significant digit first inside the one-launch sort
 };
 
 // Fills *plan; returns a gbsort_status code.

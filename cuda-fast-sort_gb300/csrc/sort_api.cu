@@ -313,6 +313,8 @@ int make_plan(int key_type, size_t value_bytes, uint64_t n, Plan* plan) {
     p.kind = key_kind_of(key_type);
     p.passes = int(kb);
     p.n = n;
+    p.skip = g_pass_skip.load(std::memory_order_relaxed) != 0;
+    p.short_msd = g_short_msd.load(std::memory_order_relaxed) != 0;
     // 32-bit status words hold values < 2^(30 - log2(passes)); every published
     // value is < n (the last tile never publishes an inclusive prefix).
     const int value_bits32 = 30 - log2_exact(p.passes);
@@ -390,7 +392,7 @@ int make_plan(int key_type, size_t value_bytes, uint64_t n, Plan* plan) {
     if (short_regions) {
         p.short_off = off;
         off = align_up(off + size_t(short_regions) * short_pairs_cap(p.kb) * 2 * kb, 256);
-        if (g_pass_skip.load(std::memory_order_relaxed)) {
+        if (p.skip) {
             p.short_pairs = true;
             p.short_regions = short_regions;
             const KernelEntry* e = p.kb == 4 ? short_pairs_entries_k4() : short_pairs_entries_k8();
@@ -398,7 +400,7 @@ int make_plan(int key_type, size_t value_bytes, uint64_t n, Plan* plan) {
             p.short_k[1] = e[p.vb == 4 ? 1 : 3];
         }
     }
-    if (finish && g_pass_skip.load(std::memory_order_relaxed)) {
+    if (finish && p.skip) {
         p.finish = true;
         const KernelEntry* e = finish_entries(p.kb);
         p.finish_k[0] = e[0];
@@ -458,7 +460,7 @@ int enqueue_sort(const Plan& plan, int descending, void* d_keys, void* d_values,
     const bool odd = !copy && !alt && (plan.passes & 1) != 0;
     const int sms = device_sm_count();
 
-    const bool skip = g_pass_skip.load(std::memory_order_relaxed) != 0;
+    const bool skip = plan.skip;
     // odd pass counts start mirrored and always end at home; an
     // input-preserving sort needs the copy only when every pass was skipped;
     // a DoubleBuffer sort when the executed passes' parity differs from the
@@ -574,7 +576,7 @@ int enqueue_sort(const Plan& plan, int descending, void* d_keys, void* d_values,
         f.fixup = fixup ? 1 : 0;
         f.barrier = reinterpret_cast<uint32_t*>(ctl + plan.ctl.barrier_off);
         f.barrier_gen = reinterpret_cast<uint32_t*>(ctl + plan.ctl.barrier_gen_off);
-        f.msd = (g_short_msd.load(std::memory_order_relaxed) && plan.msd_cap) ? 1 : 0;
+        f.msd = (plan.short_msd && plan.msd_cap) ? 1 : 0;
         f.regions = ws + plan.regions_off - ws_base;
         f.region_cap = plan.msd_cap;
         f.fill = reinterpret_cast<uint32_t*>(ctl + plan.ctl.fill_off);
@@ -898,9 +900,9 @@ int launch_sort(const Plan& plan, int descending, void* keys, void* vals, void* 
     cudaGetDevice(&k.device);
     k.key_type = plan.key_type;
     k.desc = descending;
-    k.skip = g_pass_skip.load(std::memory_order_relaxed);
+    k.skip = plan.skip ? 1 : 0;
     k.fused = plan.fused.fn != nullptr;
-    k.msd = g_short_msd.load(std::memory_order_relaxed);
+    k.msd = plan.short_msd ? 1 : 0;
     k.large_msd = plan.msd ? 1 : 0;
     k.vb = size_t(plan.vb);
     k.n = plan.n;
@@ -1269,7 +1271,7 @@ int gbsort_plan(int key_type, size_t value_bytes, size_t n, gbsort_plan_info* ou
         out->hist_ctas = upsweep_ctas(plan.n, plan.kb);
     }
     out->status_word_bytes = plan.wide_status ? 8 : 4;
-    out->kernel_launches = uint32_t(plan.passes + 1 + ((gbsort_get_pass_skip() && (plan.passes & 1) == 0) ? 1 : 0));
+    out->kernel_launches = uint32_t(plan.passes + 1 + ((plan.skip && (plan.passes & 1) == 0) ? 1 : 0));
     if (plan.msd) {
         out->msd_stages = plan.msd_block ? 6 : 0;
         out->kernel_launches += 6;
@@ -1277,11 +1279,11 @@ int gbsort_plan(int key_type, size_t value_bytes, size_t n, gbsort_plan_info* ou
     if (plan.fused.fn && sms > 0 && prepare_kernel(plan.fused) == GBSORT_OK && resident_ctas(plan.fused) > 0) {
         const uint64_t fmax = uint64_t(sms) * uint64_t(resident_ctas(plan.fused));
         uint64_t want = plan.num_tiles;
-        if (g_short_msd.load(std::memory_order_relaxed) && plan.msd_cap && want < 256) want = 256;
+        if (plan.short_msd && plan.msd_cap && want < 256) want = 256;
         out->pass_ctas = uint32_t(want < fmax ? want : fmax);
         out->hist_ctas = 0;  // counted by the same launch
         out->kernel_launches = 1;
-        out->msd_region_keys = g_short_msd.load(std::memory_order_relaxed) ? plan.msd_cap : 0u;
+        out->msd_region_keys = plan.short_msd ? plan.msd_cap : 0u;
     }
     out->workspace_bytes = plan.total_bytes;
     return GBSORT_OK;
