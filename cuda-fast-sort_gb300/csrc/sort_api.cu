@@ -1167,23 +1167,29 @@ GBSORT_DEFINE_TYPED(f128, GBSORT_KEY_F128)
 #undef GBSORT_DEFINE_TYPED
 
 namespace {
-// Synchronizes `stream` and decodes the error word of a workspace whose
-// control block starts `ctl_at` bytes in.
-int read_status(const Plan& plan, size_t ctl_at, void* d_workspace, void* stream) {
-    if (d_workspace == nullptr) return GBSORT_ERR_INVALID_ARGUMENT;
-    if (plan.n == 0) return GBSORT_OK;
+// Synchronizes `stream` and reads one word of a workspace.
+int read_word(void* d_workspace, size_t at, void* stream, uint32_t* word) {
     cudaError_t e = cudaStreamSynchronize(static_cast<cudaStream_t>(stream));
     if (e != cudaSuccess) {
         set_last_error("stream sync", e);
         return GBSORT_ERR_CUDA;
     }
-    uint32_t err = 0;
-    e = cudaMemcpy(&err, static_cast<uint8_t*>(d_workspace) + ctl_at + plan.ctl.err_off, 4, cudaMemcpyDeviceToHost);
+    e = cudaMemcpy(word, static_cast<uint8_t*>(d_workspace) + at, 4, cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) {
         set_last_error("status read", e);
         return GBSORT_ERR_CUDA;
     }
-    return status_from_error_word(err);
+    return GBSORT_OK;
+}
+
+// Decodes the error word of a workspace whose control block starts `ctl_at`
+// bytes in.
+int read_status(const Plan& plan, size_t ctl_at, void* d_workspace, void* stream) {
+    if (d_workspace == nullptr) return GBSORT_ERR_INVALID_ARGUMENT;
+    if (plan.n == 0) return GBSORT_OK;
+    uint32_t err = 0;
+    const int st = read_word(d_workspace, ctl_at + plan.ctl.err_off, stream, &err);
+    return st != GBSORT_OK ? st : status_from_error_word(err);
 }
 }  // namespace
 
@@ -1197,6 +1203,18 @@ int gbsort_double_buffer_status(int key_type, size_t value_bytes, size_t n, void
     Plan plan;
     const int st = make_plan(key_type, value_bytes, n, &plan);
     return st != GBSORT_OK ? st : read_status(plan, 0, d_workspace, stream);
+}
+
+int gbsort_workspace_outcome(int key_type, size_t value_bytes, size_t n, int double_buffer, void* d_workspace,
+                             void* stream, uint32_t* outcome) {
+    Plan plan;
+    const int st = make_plan(key_type, value_bytes, n, &plan);
+    if (st != GBSORT_OK) return st;
+    if (d_workspace == nullptr || outcome == nullptr) return GBSORT_ERR_INVALID_ARGUMENT;
+    static_assert(GBSORT_OUTCOME_PASSES == MSD_OFF && GBSORT_OUTCOME_GAVE_UP == MSD_GAVE_UP, "the device's word");
+    *outcome = 0;
+    if (n == 0) return GBSORT_OK;
+    return read_word(d_workspace, (double_buffer ? 0 : plan.ctl_off) + plan.ctl.msd_state_off, stream, outcome);
 }
 
 int gbsort_workspace_reset(int key_type, size_t value_bytes, size_t n, void* d_workspace, void* stream) {

@@ -442,6 +442,19 @@ int gbsort_workspace_reset(int key_type, size_t value_bytes, size_t n,
 int gbsort_workspace_status(int key_type, size_t value_bytes, size_t n,
                             void* d_workspace, void* stream);
 
+/* Whether the last sort on this workspace was finished by the shorter path
+ * that its size and type take, where it takes one, or by the digit passes that
+ * follow it: synchronizes `stream` and writes to *outcome 0 (the planned path
+ * sorted), GBSORT_OUTCOME_PASSES (the keys were too uneven for it, found before
+ * any key moved) or GBSORT_OUTCOME_GAVE_UP (found later: the costly case).
+ * The result is the same either way; this is for tests and for tuning.
+ * double_buffer: the workspace is one of a DoubleBuffer sort. */
+#define GBSORT_OUTCOME_PASSES 1u
+#define GBSORT_OUTCOME_GAVE_UP 2u
+int gbsort_workspace_outcome(int key_type, size_t value_bytes, size_t n,
+                             int double_buffer, void* d_workspace,
+                             void* stream, uint32_t* outcome);
+
 /* Uniform-digit pass skipping (default on; GBSORT_PASS_SKIP=0 in the
  * environment turns it off at load).  A digit pass in which every key has
  * the same digit leaves the order unchanged, so the sort runs only the other
