@@ -5,8 +5,8 @@
 // A stable least-significant-digit sort makes a pass over keys and values per
 // key byte.  Where the leading D bytes already cut the array into groups of a
 // few thousand pairs, the passes over the other bytes can be one local sort:
-//   sample:  4096 keys say how many leading bytes that takes (or that nothing
-//            is gained, FINISH_OFF: every digit pass runs as before);
+//   sample:  4096 to 16384 keys say how many leading bytes that takes (or that
+//            nothing is gained, MSD_OFF: every digit pass runs as before);
 //   passes:  the digit passes of those bytes only (onesweep.cuh);
 //   edges:   the array, now in stable order of its leading bytes, is cut near
 //            every `chunk` pairs at the next group's start, so that windows of
@@ -237,10 +237,10 @@ __global__ void __launch_bounds__(256) finish_edges_kernel(FinishParams p) {
 // Shared memory of a window of up to CAP pairs, LIPT consecutive places (a
 // chunk) a lane, HALO lanes of margin at a warp's ends.  Chunks lie 16 bytes
 // apart from a multiple of their size, so that eight lanes' 16-byte accesses
-// meet all banks.  A pair is put in order by its key and its place before: one
-// 64-bit word for 4-byte keys, else the key and a 16-bit place, apart.
-// (64-bit words for wider keys too, of the sub-bucket and 35 bits below it,
-// with the keys fetched at the end: 2 x 10^7 8-byte keys 0.31 against 0.23 ms.)
+// meet all banks.  A pair is put in order by its key and its place before, a
+// 16-bit place apart from the key.
+// (64-bit words of the sub-bucket, 35 bits below it and the place, with the
+// keys fetched at the end: 2 x 10^7 8-byte keys 0.31 against 0.23 ms.)
 template <int KB, int VB, int THREADS, int LIPT_, int HALO>
 struct FinishGeom {
     static constexpr int LIPT = LIPT_;
@@ -254,10 +254,9 @@ struct FinishGeom {
     // sub-buckets, one per place; byte counters scanned by a thread
     static constexpr int PER = (PLACES + THREADS * 4 - 1) / (THREADS * 4) * 4;
     static constexpr int BINS = PER * THREADS;
-    static constexpr int EB = KB == 4 ? 8 : KB;  // bytes of a place's word or key
-    static constexpr int STRIDE = LIPT * EB + 16;
-    static constexpr size_t POS_OFF = (size_t(PLACES / LIPT) * STRIDE + 127) & ~size_t(127);  // u16, keys of 8 bytes and more
-    static constexpr size_t VALS_OFF = (POS_OFF + (KB == 4 ? 0 : size_t(PLACES) * 2) + 127) & ~size_t(127);
+    static constexpr int STRIDE = LIPT * KB + 16;
+    static constexpr size_t POS_OFF = (size_t(PLACES / LIPT) * STRIDE + 127) & ~size_t(127);  // u16
+    static constexpr size_t VALS_OFF = (POS_OFF + size_t(PLACES) * 2 + 127) & ~size_t(127);
     static constexpr size_t CTR_OFF = (VALS_OFF + size_t(PLACES) * VB + 127) & ~size_t(127);  // u8 [BINS]
     static constexpr size_t START_OFF = CTR_OFF + BINS;                                       // u16 [BINS]
     static constexpr size_t SCAN_OFF = START_OFF + size_t(BINS) * 2;                          // u32 [32]
@@ -266,7 +265,7 @@ struct FinishGeom {
     static constexpr size_t SMEM_BYTES = HEADS_OFF + size_t(WARPS) * 8;
     static_assert(size_t(PLACES) <= POS_OFF, "the groups' marks lie where the keys go later");
     __device__ __forceinline__ static uint32_t at(uint32_t place) {
-        return place * uint32_t(EB) + (place / LIPT) * 16u;
+        return place * uint32_t(KB) + (place / LIPT) * 16u;
     }
 };
 
@@ -279,17 +278,7 @@ struct Placed {
     __device__ __forceinline__ U key() const { return k; }
     __device__ __forceinline__ uint32_t place() const { return j; }
 };
-template <>
-struct Placed<uint32_t> {
-    uint64_t v;
-    __device__ __forceinline__ static Placed make(uint32_t key, uint32_t place) {
-        return Placed{(uint64_t(key) << 32) | place};
-    }
-    __device__ __forceinline__ uint32_t key() const { return uint32_t(v >> 32); }
-    __device__ __forceinline__ uint32_t place() const { return uint32_t(v); }
-};
 // b comes before a: one borrow chain over the words.
-__device__ __forceinline__ bool after(const Placed<uint32_t>& a, const Placed<uint32_t>& b) { return b.v < a.v; }
 __device__ __forceinline__ bool after(const Placed<uint64_t>& a, const Placed<uint64_t>& b) {
     uint32_t r;
     asm("{\n\t.reg .u32 t;\n\tsub.cc.u32 t, %1, %2;\n\tsubc.cc.u32 t, %3, %4;\n\tsubc.cc.u32 t, %5, %6;\n\t"
@@ -402,7 +391,6 @@ __global__ void __launch_bounds__(THREADS, MIN_CTAS) finish_kernel(FinishParams 
     using F = FinishGeom<KB, VB, THREADS, LIPT, HALO>;
     using E = Placed<U>;
     constexpr int WARPS = THREADS / 32, VEC = 16 / KB;
-    constexpr bool WIDE = KB > 4;
     extern __shared__ __align__(128) uint8_t smem[];
     uint32_t* ctr = reinterpret_cast<uint32_t*>(smem + F::CTR_OFF);
     uint16_t* start = reinterpret_cast<uint16_t*>(smem + F::START_OFF);
@@ -413,17 +401,10 @@ __global__ void __launch_bounds__(THREADS, MIN_CTAS) finish_kernel(FinishParams 
     uint8_t* uneven = smem;  // by a group's first place: its keys differ (before the keys are placed)
     uint16_t* sp = reinterpret_cast<uint16_t*>(smem + F::POS_OFF);
     auto put = [&](uint32_t place, U key, uint32_t before) {
-        if constexpr (WIDE) {
-            *reinterpret_cast<U*>(smem + F::at(place)) = key;
-            sp[place] = uint16_t(before);
-        } else {
-            *reinterpret_cast<uint64_t*>(smem + F::at(place)) = E::make(key, before).v;
-        }
+        *reinterpret_cast<U*>(smem + F::at(place)) = key;
+        sp[place] = uint16_t(before);
     };
-    auto get = [&](uint32_t place) {
-        if constexpr (WIDE) return E::make(*reinterpret_cast<const U*>(smem + F::at(place)), sp[place]);
-        else return E{*reinterpret_cast<const uint64_t*>(smem + F::at(place))};
-    };
+    auto get = [&](uint32_t place) { return E::make(*reinterpret_cast<const U*>(smem + F::at(place)), sp[place]); };
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t lt = lanemask_lt();
     grid_launch_dependents();
@@ -548,10 +529,7 @@ __global__ void __launch_bounds__(THREADS, MIN_CTAS) finish_kernel(FinishParams 
         // group's keys keep their places.
         uint32_t where[LIPT];  // sub-bucket | slot << 16
         // a key's bits below its group's, left-aligned in 32
-        auto below = [&](U x) {
-            if constexpr (KB == 4) return uint32_t(x) << (32u - gshift);
-            else return uint32_t((x << (8u * KB - gshift)) >> (8 * KB - 32));
-        };
+        auto below = [&](U x) { return uint32_t((x << (8u * KB - gshift)) >> (8 * KB - 32)); };
         auto take = [&](int i, uint32_t b) {
             const uint32_t old = atomicAdd(reinterpret_cast<uint32_t*>(reinterpret_cast<uint8_t*>(ctr) + (b & ~3u)),
                                            __funnelshift_l(1u, 1u, b * 8u));
@@ -651,26 +629,16 @@ __global__ void __launch_bounds__(THREADS, MIN_CTAS) finish_kernel(FinishParams 
                     for (int i = 0; i < LIPT; ++i) x[i] = d0 < int(pad) ? least : greatest;
                 } else {
                     const uint4* q = reinterpret_cast<const uint4*>(smem + uint32_t(ch) * F::STRIDE);
-                    if constexpr (WIDE) {
-                        const uint32_t* pj = reinterpret_cast<const uint32_t*>(sp + d0);
+                    const uint32_t* pj = reinterpret_cast<const uint32_t*>(sp + d0);
 #pragma unroll
-                        for (int i = 0; i < LIPT / VEC; ++i) {
-                            union { uint4 v; U k[VEC]; } w;
-                            w.v = q[i];
+                    for (int i = 0; i < LIPT / VEC; ++i) {
+                        union { uint4 v; U k[VEC]; } w;
+                        w.v = q[i];
 #pragma unroll
-                            for (int e = 0; e < VEC; ++e) {
-                                const int u = i * VEC + e;
-                                const uint32_t jj = pj[u / 2];
-                                x[u] = E::make(w.k[e], u & 1 ? jj >> 16 : jj & 0xffffu);
-                            }
-                        }
-                    } else {
-#pragma unroll
-                        for (int i = 0; i < LIPT / 2; ++i) {
-                            union { uint4 v; E w[2]; } w;
-                            w.v = q[i];
-                            x[2 * i] = w.w[0];
-                            x[2 * i + 1] = w.w[1];
+                        for (int e = 0; e < VEC; ++e) {
+                            const int u = i * VEC + e;
+                            const uint32_t jj = pj[u / 2];
+                            x[u] = E::make(w.k[e], u & 1 ? jj >> 16 : jj & 0xffffu);
                         }
                     }
                     if (!inside) {

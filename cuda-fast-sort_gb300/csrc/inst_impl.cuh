@@ -125,26 +125,27 @@ const KernelEntry* msd_even_entries_for() {
     return e;
 }
 
-// Key-value sorts by their leading digits: sample, edges, finish (4- and
-// 8-byte values).
-// (8-byte keys: without values too, the last entry)
+// Sorts by leading digits: sample, edges, finish (4- and 8-byte values; 8-byte
+// keys without values too).
+template <int KB, int VB>
+KernelEntry make_finish_entry() {
+    using S = FinishShape<KB>;
+    using F = FinishGeom<KB, VB, S::THREADS, S::LIPT, S::HALO>;
+    return KernelEntry{reinterpret_cast<const void*>(&finish_kernel<KB, VB, S::THREADS, S::MIN_CTAS, S::LIPT, S::HALO>),
+                       S::THREADS, F::LIPT, F::CAP, static_cast<unsigned long>(F::SMEM_BYTES)};
+}
 template <int KB>
 const KernelEntry* finish_entries_for() {
-    using S = FinishShape<KB>;
-    constexpr int VB0 = KB == 8 ? 0 : 4;
-    using F0 = FinishGeom<KB, VB0, S::THREADS, S::LIPT, S::HALO>;
-    using F4 = FinishGeom<KB, 4, S::THREADS, S::LIPT, S::HALO>;
-    using F8 = FinishGeom<KB, 8, S::THREADS, S::LIPT, S::HALO>;
     static const KernelEntry e[5] = {
         {reinterpret_cast<const void*>(&finish_sample_kernel<KB>), FINISH_SAMPLE_THREADS, 0, finish_levels<KB>() + 1,
          static_cast<unsigned long>(FINISH_SAMPLE_SMEM)},
         {reinterpret_cast<const void*>(&finish_edges_kernel<KB>), 256, 0, 0, 0ul},
-        {reinterpret_cast<const void*>(&finish_kernel<KB, 4, S::THREADS, S::MIN_CTAS, S::LIPT, S::HALO>), S::THREADS, F4::LIPT,
-         F4::CAP, static_cast<unsigned long>(F4::SMEM_BYTES)},
-        {reinterpret_cast<const void*>(&finish_kernel<KB, 8, S::THREADS, S::MIN_CTAS, S::LIPT, S::HALO>), S::THREADS, F8::LIPT,
-         F8::CAP, static_cast<unsigned long>(F8::SMEM_BYTES)},
-        {reinterpret_cast<const void*>(&finish_kernel<KB, VB0, S::THREADS, S::MIN_CTAS, S::LIPT, S::HALO>), S::THREADS,
-         F0::LIPT, F0::CAP, static_cast<unsigned long>(F0::SMEM_BYTES)},
+        make_finish_entry<KB, 4>(),
+        make_finish_entry<KB, 8>(),
+        [] {
+            if constexpr (KB == 8) return make_finish_entry<KB, 0>();
+            else return KernelEntry{};
+        }(),
     };
     return e;
 }

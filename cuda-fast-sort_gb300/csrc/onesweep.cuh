@@ -726,7 +726,7 @@ __global__ void __launch_bounds__(THREADS, MIN_CTAS) onesweep_pass_kernel(PassPa
 
 __device__ __forceinline__ void grid_copy_bytes(void* dst, const void* src, uint64_t bytes);
 
-// Digits p.pass .. p.last_pass in one cooperative launch, a grid barrier
+// Digits p.pass .. p.passes - 1 in one cooperative launch, a grid barrier
 // between the passes that run, then the parity fix-up.  Used where most passes
 // do not run (a launch that exits costs about 2.2 us, a barrier with the next
 // pass's start about 2 us more than a launch that overlaps its predecessor's

@@ -149,9 +149,9 @@ constexpr int msd_b2_max(uint64_t n, uint32_t cap) {
 
 // Key-value sorts by their leading digits (finish.cuh): the finishing CTAs.
 // 8- and 16-byte keys with 4- or 8-byte values.  4-byte keys keep their four
-// digit passes: two of them and the finish take longer (2^26 u32 + u32 1.51
-// against 1.42 ms, the finish 0.68 in two CTAs of 512 threads, 8 keys a lane,
-// or one of 768).
+// digit passes: two of them and a finish took longer (2^26 u32 + u32 1.51
+// against 1.42 ms, with a kernel for 4-byte keys that this library does not
+// hold).
 template <int KB>
 struct FinishShape {
     static constexpr int THREADS = 384;

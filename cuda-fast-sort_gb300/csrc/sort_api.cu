@@ -8,9 +8,17 @@
 //                                                 launch, pass loop, ping-pong
 //   include/rsort/detail/radix_kernel.cuh:486-607 size query, policy switch,
 //                                                 per-call graph wrapper
-// Per sort this enqueues one small memset (digit counts, tile counters,
-// error word), one upsweep launch and one persistent launch per digit pass,
-// all on the caller's stream; nothing is allocated and nothing synchronizes.
+// Per sort this enqueues one small memset (control words) and the kernels of
+// the path that its type, size and values take, all on the caller's stream;
+// nothing is allocated and nothing synchronizes:
+//   - short keys-only arrays: one cooperative launch (fused_short.cuh);
+//   - short key-value arrays: one, and one that sorts by digit passes when the
+//     keys were too uneven (short_pairs.cuh);
+//   - larger keys-only arrays of 4-, 8- and 16-byte keys: most significant bits
+//     first (msd.cuh), then the digit passes in a launch that exits;
+//   - key-value arrays of 8- and 16-byte keys, 8-byte floats: leading digits
+//     and a finish (finish.cuh), then the same;
+//   - everything else: a histogram and one launch per digit pass (onesweep.cuh).
 
 #include <atomic>
 #include <cstdio>
@@ -51,7 +59,7 @@ const KernelEntry* fused_entry_k16();
 
 const KernelEntry* short_pairs_entries_k4();
 const KernelEntry* short_pairs_entries_k8();
-const KernelEntry* multi_entries_k4(int vb);
+const KernelEntry* multi_entries_k4();  // keys only
 const KernelEntry* multi_entries_k8(int vb);
 const KernelEntry* multi_entries_k16(int vb);
 const KernelEntry* finish_entries_k8();
@@ -408,7 +416,7 @@ int make_plan(int key_type, size_t value_bytes, uint64_t n, Plan* plan) {
         p.finish_k[2] = e[p.vb == 4 ? 2 : p.vb == 8 ? 3 : 4];
     }
     if (p.msd || p.finish)
-        p.multi = (p.kb == 4   ? multi_entries_k4(p.vb)
+        p.multi = (p.kb == 4   ? multi_entries_k4()
                    : p.kb == 8 ? multi_entries_k8(p.vb)
                                : multi_entries_k16(p.vb))[small ? 2 : p.wide_status ? 1 : 0];
     p.total_bytes = off;
