@@ -44,7 +44,7 @@ struct FinishParams {
     uint32_t* window;      // [2] lowest digit that the passes sort by, pairs per chunk
     const uint32_t* executed;  // passes run (bit 31 set; 0: none)
     uint32_t* ticket;      // the sample's CTAs, zeroed with the control block
-    uint32_t* sampled;     // [FINISH_LEVELS + 1] their counts
+    uint32_t* sampled;     // [FINISH_LEVELS + 2] their counts, and the keys met twice
     uint32_t* edges;       // [chunks + 1] first pair of every window (bit 31: the edge cuts a group)
     uint32_t max_chunks;   // room in edges
     uint32_t places;       // pairs a window may hold
@@ -53,20 +53,28 @@ struct FinishParams {
 
 // ---- sample -----------------------------------------------------------------
 // CTA l counts the pairs of sampled keys that share their l + 1 leading bytes
-// (the last CTA: that are equal, which no digit tells apart), in 2^15 hashed
-// counters; S keys in groups of g make S * S * g / 2n of them.  The CTA that
-// finishes last decides.
+// (the last CTA: that are equal, which no digit tells apart), exactly, in a
+// table of 2^15 slots at most half full: 17 more bits of a prefix's hash above
+// its count.  (Counters without them met S * S / 2^16 pairs by chance, and
+// their noise hid keys that repeat a hundred times.)  S keys in groups of g
+// make S * S * g / 2n pairs.  The places are random: at even distances, keys in
+// order came one to a group and groups of any size looked like none (2 x 10^7
+// sorted u64 + u32 1.68 ms, by random places 0.60).  The CTA that finishes last
+// decides.
 constexpr int FINISH_SAMPLE_THREADS = 1024;
 constexpr int FINISH_LEVELS = 6;  // leading bytes tried
 constexpr int FINISH_SAMPLE_SMEM = 32768 * 4;
 template <int KB>
 constexpr int finish_levels() { return KB - 1 < FINISH_LEVELS ? KB - 1 : FINISH_LEVELS; }
+// Copies of a key from which on its groups have to be of one key (below).
+constexpr float FINISH_REPEATS = 12.f;
+
 template <int KB>
 __global__ void __launch_bounds__(FINISH_SAMPLE_THREADS) finish_sample_kernel(FinishParams p) {
     using U = typename KeyBits<KB>::U;
     constexpr int LEVELS = finish_levels<KB>();
     extern __shared__ __align__(16) uint32_t cnt[];
-    __shared__ uint32_t shared_pairs, vary, ticket;
+    __shared__ uint32_t shared_pairs, vary, ticket, repeats, heavy;
     grid_launch_dependents();
     grid_dependency_wait();
     const int tid = threadIdx.x, level = blockIdx.x;
@@ -76,21 +84,22 @@ __global__ void __launch_bounds__(FINISH_SAMPLE_THREADS) finish_sample_kernel(Fi
     const float S = float(FINISH_SAMPLE_THREADS * per);
     const KeyMap<U> map(p.kind, p.desc);
     const U* keys = static_cast<const U*>(p.keys_in);
-    const uint32_t step = max(1u, uint32_t(p.n / uint32_t(FINISH_SAMPLE_THREADS * per)));
     U x[MOST];
 #pragma unroll
     for (int i = 0; i < MOST; ++i) {
         if (i >= per) break;
-        const uint32_t at = uint32_t(i * FINISH_SAMPLE_THREADS + tid);
-        const uint64_t j = uint64_t(at) * step + (at * 2654435761u) % step;
-        x[i] = map.in(keys[j < p.n ? j : j % p.n]);
+        uint32_t h = uint32_t(i * FINISH_SAMPLE_THREADS + tid) * 0x9E3779B9u + 0x7F4A7C15u;
+        h = (h ^ (h >> 16)) * 0x85EBCA6Bu;  // (murmur3's finalizer)
+        h = (h ^ (h >> 13)) * 0xC2B2AE35u;
+        h ^= h >> 16;
+        x[i] = map.in(keys[(uint64_t(h) * p.n) >> 32]);
     }
     const U first = map.in(keys[0]);
     for (int i = tid; i < 8192; i += FINISH_SAMPLE_THREADS) reinterpret_cast<uint4*>(cnt)[i] = make_uint4(0, 0, 0, 0);
-    if (tid == 0) shared_pairs = vary = 0u;
+    if (tid == 0) shared_pairs = vary = repeats = heavy = 0u;
     __syncthreads();
     U d = 0;
-    uint32_t pairs = 0;
+    uint32_t pairs = 0, again = 0, more = 0;  // again, more: prefixes met for the second time, or oftener
 #pragma unroll
     for (int i = 0; i < MOST; ++i) {
         if (i >= per) break;
@@ -102,46 +111,84 @@ __global__ void __launch_bounds__(FINISH_SAMPLE_THREADS) finish_sample_kernel(Fi
         h = (h ^ (h >> 30)) * 0xBF58476D1CE4E5B9ull;
         h = (h ^ (h >> 27)) * 0x94D049BB133111EBull;
         h ^= h >> 31;
-        pairs += atomicAdd(&cnt[uint32_t(h) & 32767u], 1u);  // the keys there before this one
+        const uint32_t tag = uint32_t(h >> 32) & 0xffff8000u;
+        uint32_t slot = uint32_t(h) & 32767u;
+        for (int probe = 0; probe < 128; ++probe) {
+            const uint32_t w = atomicCAS(&cnt[slot], 0u, tag | 1u);
+            if (w == 0u) break;
+            if ((w & 0xffff8000u) == tag) {
+                const uint32_t before = atomicAdd(&cnt[slot], 1u) & 32767u;  // the keys there before this one
+                pairs += before;
+                again += before == 1u;
+                more += before > 1u;
+                break;
+            }
+            slot = (slot + 1u) & 32767u;
+        }
     }
     uint32_t bytes = 0;  // bit q: byte q differs somewhere
 #pragma unroll
     for (int q = 0; q < KB; ++q) bytes |= uint32_t(((d >> (8 * q)) & U(0xff)) != U(0)) << q;
     bytes = __reduce_or_sync(0xffffffffu, bytes);
     pairs = __reduce_add_sync(0xffffffffu, pairs);
+    again = __reduce_add_sync(0xffffffffu, again);
+    more = __reduce_add_sync(0xffffffffu, more);
     if ((tid & 31) == 0) {
         atomicOr(&vary, bytes);
         atomicAdd(&shared_pairs, pairs);
+        if (again) atomicAdd(&repeats, again);
+        if (more) atomicAdd(&heavy, more);
     }
     __syncthreads();
     if (tid == 0) {
         p.sampled[level] = shared_pairs;
+        if (level == LEVELS) p.sampled[LEVELS + 1] = repeats | heavy << 16;
         __threadfence();
         ticket = atomicAdd(p.ticket, 1u);
     }
     if (tid != 0 || ticket != uint32_t(LEVELS)) return;
     __threadfence();
-    const float n = float(p.n), places = float(p.places);
-    const float equal = float(ld_relaxed(p.sampled + LEVELS));
-    // what a pair's group by l + 1 leading bytes holds on average, and a little
-    // more than a deviation of the estimate
-    auto group_of = [&](int l) {
-        const float pairs = float(ld_relaxed(p.sampled + l));
-        return (max(0.f, pairs - equal) + 1.2f * sqrtf(pairs + equal)) * 2.f * n / (S * S);
-    };
+    const float n = float(p.n), places = float(p.places), scale = 2.f * n / (S * S);
+    uint32_t sampled[LEVELS + 2];  // (loaded at once: one by one they took half of the kernel)
+#pragma unroll
+    for (int l = 0; l < LEVELS + 2; ++l) sampled[l] = ld_relaxed(p.sampled + l);
+    const float equal = float(sampled[LEVELS]);
+    const uint32_t again_more = sampled[LEVELS + 1];
+    // Others equal to a key, on average over the keys, every key that repeats
+    // counted once (1% of zeros would make an average of thousands).
+    const float copies = float(again_more & 0xffffu) * scale;
+    const bool repeating = copies >= FINISH_REPEATS;
+    // the keys unlike a key in its group by l + 1 leading bytes, on average over
+    // the keys that are not of a few very frequent ones, and a little more than
+    // half a deviation of the estimate
+    const float rest = scale / max(0.05f, 1.f - float(again_more >> 16) / S);
+    float group_of[LEVELS];
+#pragma unroll
+    for (int l = 0; l < LEVELS; ++l) {
+        const float pairs = max(0.f, float(sampled[l]) - equal);
+        group_of[l] = (pairs + 0.6f * sqrtf(pairs + 2.f)) * rest;
+    }
     // The fewest leading bytes whose groups fit, and whose next byte spreads a
     // group's keys over its sub-buckets.  Groups of floats are uneven (the
     // largest of N(0, 1) hold twice the average): they have to be smaller.
+    // Where keys repeat, one sub-bucket takes all copies of a key: groups that
+    // are one key's keep their order instead, so that few may be of more (2 x
+    // 10^7 u64 + u32 in 40 copies 0.90 ms; two bytes fit, but leave every window
+    // crowded).
     const float fits = (p.kind == KIND_FLOAT ? 0.4f : 0.84f) * places;
-    const float noise = 1.2f * sqrtf(2.f * equal) * 2.f * n / (S * S);
     int lo = 0;
-    float group = 0.f;
+    float group = 0.f, unlike = 0.f;  // unlike: its pairs of different keys
+    bool chosen = false;
+#pragma unroll
     for (int l = 0; l < LEVELS; ++l) {
-        group = group_of(l);
-        if (group <= fits && (l + 1 == LEVELS || group_of(l + 1) <= group * (1.f / 16.f) + 2.f * noise + 4.f)) {
-            lo = KB - 1 - l;
-            break;
-        }
+        const float g = group_of[l];
+        const bool spreads = l + 1 == LEVELS || group_of[l + 1 < LEVELS ? l + 1 : l] <= g * (1.f / 16.f) + 3.f * rest + 4.f;
+        if (chosen || g > fits || !spreads) continue;
+        group = g;
+        unlike = max(0.f, float(sampled[l]) - equal);
+        lo = KB - 1 - l;
+        // (in less than half of the windows, which hold places / copies such groups)
+        chosen = !repeating || unlike * rest * 2.f * places <= copies * copies;
     }
     // worth it when it replaces two passes or more
     const uint32_t low = vary & ((1u << lo) - 1u);
@@ -151,8 +198,9 @@ __global__ void __launch_bounds__(FINISH_SAMPLE_THREADS) finish_sample_kernel(Fi
     } else {
         // the larger the groups, the more of a window is left for the one
         // that starts last in it (and seven deviations of a random group's
-        // size)
-        const float c = 0.98f * places - (p.kind == KIND_FLOAT ? 2.f : 1.1f) * group - 7.f * sqrtf(group);
+        // size; where keys repeat and groups are of more than one, two keys' copies)
+        const float lumps = repeating && unlike > 0.f ? min(2.2f * copies, 0.25f * places) : 0.f;
+        const float c = 0.98f * places - (p.kind == KIND_FLOAT ? 2.f : 1.1f) * group - 7.f * sqrtf(group) - lumps;
         chunk = uint32_t(min(max(c, 0.1f * places), 0.93f * places)) & ~31u;
         chunk = max(chunk, (uint32_t(p.n / (p.max_chunks - 1u)) + 32u) & ~31u);
         if (float(chunk) > 0.95f * places) *p.state = MSD_OFF;

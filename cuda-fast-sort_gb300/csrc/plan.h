@@ -30,7 +30,7 @@ struct CtlLayout {
     size_t counters2_off = 0;    // a second set of tile counters and a second grid barrier, for the
                                  // digit passes after a sort by leading digits (0: none)
     size_t short_fill_off = 0;   // [1024] fill counts of a short key-value sort's regions
-    size_t sampled_off = 0;      // its sample: ticket, [8] counts
+    size_t sampled_off = 0;      // its sample: ticket, [FINISH_LEVELS + 2] counts
     size_t msd_state_off = 0;    // outcome of the most-significant-first path, its code window [2]
     size_t bytes = 0;
     static CtlLayout make(int passes, bool finish = false, bool short_pairs = false) {
