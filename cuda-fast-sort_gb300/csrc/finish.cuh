@@ -21,10 +21,11 @@
 // What bounds the finish: latency (two CTAs of 384 threads an SM, 80 registers;
 // a window of 2300 pairs of 8-byte keys takes its CTA 7.7 us, of which the
 // network's instructions are a fifth); 2 x 10^7 u64 + u32 0.22 ms.
-// When that fails somewhere (a group too big after all, sub-buckets too full)
-// the window is written as it was, and every digit pass runs, from the
-// caller's buffers, which then hold the pairs untwiddled, in an order that a
-// stable sort completes.
+// A window whose sub-buckets are too full (keys that repeat inside groups of
+// different keys) is put in order by a network over all of it.
+// A group of different keys that does not fit a window leaves its windows as
+// they were, and every digit pass runs, from the caller's buffers, which then
+// hold the pairs untwiddled, in an order that a stable sort completes.
 #pragma once
 
 #include "msd.cuh"
@@ -432,6 +433,87 @@ __device__ __forceinline__ void scan_bins(uint8_t* smem, uint32_t cnt, uint32_t 
     }
 }
 
+// A window whose keys and places are in shared memory as they came, places
+// [pad, end), put in order by key and place: group by group (they are in order
+// already), a warp each, groups beyond FINISH_BY_WARP by the whole CTA.  Out of
+// line: it keeps the usual window's registers.
+constexpr uint32_t FINISH_BY_WARP = 256;
+template <int KB, int VB, int THREADS, int LIPT, int HALO>
+__device__ __noinline__ void finish_crowded(uint8_t* smem, uint32_t pad, uint32_t end, uint32_t gshift,
+                                            typename KeyBits<KB>::U* okeys, typename ValBits<VB>::V* ovals, int kind,
+                                            int desc) {
+    using U = typename KeyBits<KB>::U;
+    using V = typename ValBits<VB>::V;
+    using F = FinishGeom<KB, VB, THREADS, LIPT, HALO>;
+    constexpr uint32_t WARPS = THREADS / 32, BIG = F::PLACES / FINISH_BY_WARP + 1;
+    uint16_t* sp = reinterpret_cast<uint16_t*>(smem + F::POS_OFF);
+    uint32_t* misc = reinterpret_cast<uint32_t*>(smem + F::MISC_OFF);    // [1] groups left to the CTA
+    uint32_t* big = reinterpret_cast<uint32_t*>(smem + F::HEADS_OFF);    // their first places and ends
+    static_assert(BIG <= 2 * WARPS, "the list of groups");
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    auto key = [&](uint32_t place) -> U& { return *reinterpret_cast<U*>(smem + F::at(place)); };
+    auto group = [&](uint32_t place) { return key(place) >> gshift; };
+    auto order = [&](uint32_t a, uint32_t b) {
+        U& ka = key(a);
+        U& kb = key(b);
+        const U x = ka, y = kb;
+        const uint16_t i = sp[a], j = sp[b];
+        if (y < x || (y == x && j < i)) {
+            ka = y;
+            kb = x;
+            sp[a] = j;
+            sp[b] = i;
+        }
+    };
+    if (threadIdx.x == 0) misc[1] = 0u;
+    __syncthreads();
+    const uint32_t share = (end - pad + WARPS - 1) / WARPS;
+    const uint32_t from = pad + warp * share, to = min(from + share, end);
+    for (uint32_t i0 = from; i0 < to; i0 += 32) {
+        const uint32_t i = i0 + lane;
+        uint32_t heads = __ballot_sync(0xffffffffu, i < to && (i == pad || group(i) != group(i - 1)));
+        while (heads) {
+            const uint32_t first = i0 + __ffs(heads) - 1;
+            heads &= heads - 1u;
+            // its end, and whether it is in order as it came
+            uint32_t last = first + 1;
+            bool ordered = true;
+            for (;; last += 32) {
+                const uint32_t q = last + lane;
+                const bool in = q < end && group(q) == group(first);
+                const uint32_t out = __ballot_sync(0xffffffffu, !in);
+                ordered = __all_sync(0xffffffffu, !in || key(q) >= key(q - 1)) && ordered;
+                if (out) {
+                    last += __ffs(out) - 1;
+                    break;
+                }
+            }
+            if (ordered) continue;
+            if (last - first > FINISH_BY_WARP) {
+                if (lane == 0) big[atomicAdd(&misc[1], 1u)] = first | last << 16;
+            } else {
+                ascending_network(
+                    last - first, lane, 32u, [&](uint32_t a, uint32_t b) { order(first + a, first + b); },
+                    [] { __syncwarp(); });
+            }
+        }
+    }
+    __syncthreads();
+    const uint32_t left = misc[1];
+    for (uint32_t g = 0; g < left; ++g) {
+        const uint32_t first = big[g] & 0xffffu, last = big[g] >> 16;
+        ascending_network(
+            last - first, threadIdx.x, THREADS, [&](uint32_t a, uint32_t b) { order(first + a, first + b); },
+            [] { __syncthreads(); });
+    }
+    const KeyMap<U> map(kind, desc);
+    const V* sv = reinterpret_cast<const V*>(smem + F::VALS_OFF);
+    for (uint32_t i = pad + threadIdx.x; i < end; i += THREADS) {
+        okeys[i] = map.out(key(i));
+        if constexpr (VB > 0) ovals[i] = sv[sp[i]];
+    }
+}
+
 template <int KB, int VB, int THREADS, int MIN_CTAS, int LIPT, int HALO>
 __global__ void __launch_bounds__(THREADS, MIN_CTAS) finish_kernel(FinishParams p) {
     using U = typename KeyBits<KB>::U;
@@ -630,7 +712,7 @@ __global__ void __launch_bounds__(THREADS, MIN_CTAS) finish_kernel(FinishParams 
             __syncthreads();
             if (tid == 0) misc[0] = 0u;
         }
-        if (cut || most > MSD_RANK_MAX) {
+        if (cut) {
             // as it was, untwiddled (keys are in registers, values in shared memory)
 #pragma unroll
             for (int i = 0; i < LIPT; ++i)
@@ -651,7 +733,11 @@ __global__ void __launch_bounds__(THREADS, MIN_CTAS) finish_kernel(FinishParams 
             continue;
         }
         auto move = [&](int i) { put(uint32_t(start[where[i] & 0xffffu]) + (where[i] >> 16), k[i], c0 + i); };
-        if (all_whole) {
+        if (most > MSD_RANK_MAX) {  // (the slots of a count beyond 255 mean nothing)
+#pragma unroll
+            for (int i = 0; i < LIPT; ++i)
+                if ((valid >> i) & 1u) put(c0 + i, k[i], c0 + i);
+        } else if (all_whole) {
 #pragma unroll
             for (int i = 0; i < LIPT; ++i) move(i);
         } else if (busy) {
@@ -662,6 +748,9 @@ __global__ void __launch_bounds__(THREADS, MIN_CTAS) finish_kernel(FinishParams 
         if constexpr (VB > 0) copy_async_wait();
         __syncthreads();
         if (tid == 0) misc[0] = 0u;
+        if (most > MSD_RANK_MAX)
+            finish_crowded<KB, VB, THREADS, LIPT, HALO>(smem, pad, end, gshift, okeys + s - pad, ovals + s - pad, p.kind,
+                                                        p.desc);
         more = advance();
         if (more) load();  // the next window's keys, while this one's are put in order
         if (most <= uint32_t(HALO * LIPT)) {
@@ -734,7 +823,7 @@ __global__ void __launch_bounds__(THREADS, MIN_CTAS) finish_kernel(FinishParams 
                     }
                 }
             }
-        } else {
+        } else if (most <= MSD_RANK_MAX) {
             // a pair's place is its sub-bucket's start plus the sub-bucket's
             // other pairs before it; the sub-bucket of a place: the last one
             // that starts at or before it and is not empty

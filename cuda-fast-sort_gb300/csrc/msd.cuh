@@ -1044,6 +1044,32 @@ __device__ __forceinline__ U shfl_down1(U v) {
     }
 }
 
+// The ascending network over places 0 .. m - 1, any m, by `threads` threads:
+// order(a, b) puts the pair of places a < b in order, sync() orders one step's
+// accesses before the next's.  Every step's first half meets its second half
+// mirrored, so that all comparisons point up and places from m on, which
+// would hold greatest keys, never take part.
+template <class Order, class Sync>
+__device__ __forceinline__ void ascending_network(uint32_t m, uint32_t thread, uint32_t threads, Order order, Sync sync) {
+    uint32_t half = 1;
+    while (2u * half < m) half *= 2u;
+    if (m < 2u) return;
+    for (uint32_t size = 2; size <= 2u * half; size *= 2u) {
+        for (uint32_t i = thread; i < half; i += threads) {
+            const uint32_t in = i & (size / 2u - 1u), first = 2u * (i - in);
+            if (first + size - 1u - in < m) order(first + in, first + size - 1u - in);
+        }
+        sync();
+        for (uint32_t gap = size / 4u; gap != 0u; gap /= 2u) {
+            for (uint32_t i = thread; i < half; i += threads) {
+                const uint32_t a = 2u * i - (i & (gap - 1u));
+                if (a + gap < m) order(a, a + gap);
+            }
+            sync();
+        }
+    }
+}
+
 // `rounds` rounds of odd-even transposition over the warp's 32 * LIPT keys,
 // LIPT consecutive ones per lane.
 template <class U, int LIPT>
