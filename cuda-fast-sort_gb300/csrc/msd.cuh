@@ -1228,6 +1228,123 @@ __device__ __forceinline__ bool group_sort(const U (&keys)[64 / sizeof(U)], uint
     return true;
 }
 
+// Sub-bucket of a key in its group: the 32 bits of its code after the `shift`
+// that the group's keys share, evenly over the bins.
+template <class Code>
+struct SubBucket {
+    Code code;
+    uint32_t shift, bins;
+    template <class U>
+    __device__ __forceinline__ uint32_t operator()(U x) const { return __umulhi(code(x) << shift, bins); }
+};
+
+// A group that group_sort refuses (keys that repeat, or that share the
+// sub-bucket's bits), from global memory, sorted in place and mapped back.  The
+// same counting pass with 16-bit counters, then only sub-buckets whose keys
+// differ are put in order: small ones by comparison, larger ones by a network
+// of one warp, the largest by the CTA; equal keys, the usual crowd, need
+// nothing.  Counters and misc[0] are zero on entry and left so.
+template <class U, int THREADS, int HALO, class Bin>
+__device__ __noinline__ void group_sort_crowded(U* group, uint32_t cnt, uint8_t* smem, Bin bin, KeyMap<U> map) {
+    using G = GroupSortGeom<int(sizeof(U)), THREADS, HALO>;
+    constexpr uint32_t BY_THREAD = 16, BY_WARP = 512;
+    uint32_t* flags = reinterpret_cast<uint32_t*>(smem + G::CTR_OFF);  // a byte a sub-bucket: its keys differ
+    uint32_t* place = reinterpret_cast<uint32_t*>(smem + G::START_OFF);
+    const uint16_t* ends = reinterpret_cast<const uint16_t*>(place);
+    uint32_t* scan = reinterpret_cast<uint32_t*>(smem + G::SCAN_OFF);
+    uint32_t* misc = reinterpret_cast<uint32_t*>(smem + G::MISC_OFF);  // [1] sub-buckets left to the CTA
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    auto sk = [&](uint32_t i) -> U& { return *reinterpret_cast<U*>(smem + G::at(i)); };
+    auto first_of = [&](uint32_t b) { return b ? uint32_t(ends[b - 1]) : 0u; };
+    auto order = [&](uint32_t a, uint32_t b) {
+        const U x = sk(a), y = sk(b);
+        if (y < x) {
+            sk(a) = y;
+            sk(b) = x;
+        }
+    };
+    __syncthreads();
+    for (uint32_t i = tid; i < uint32_t(G::BINS) / 2; i += THREADS) place[i] = 0u;
+    if (tid == 0) misc[1] = 0u;
+    __syncthreads();
+    for (uint32_t i = tid; i < cnt; i += THREADS) {
+        const uint32_t b = bin(group[i]);
+        atomicAdd(&place[b >> 1], 1u << 16 * (b & 1u));
+    }
+    __syncthreads();
+    {
+        uint4 w[2] = {reinterpret_cast<uint4*>(place)[2 * tid], reinterpret_cast<uint4*>(place)[2 * tid + 1]};
+        uint32_t* c = reinterpret_cast<uint32_t*>(w);
+        uint32_t sum = 0;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) sum += (c[i] & 0xffffu) + (c[i] >> 16);
+        uint32_t run = block_exclusive_scan_1b<THREADS>(sum, scan);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const uint32_t next = run + (c[i] & 0xffffu), after = next + (c[i] >> 16);
+            c[i] = run | next << 16;
+            run = after;
+        }
+        reinterpret_cast<uint4*>(place)[2 * tid] = w[0];
+        reinterpret_cast<uint4*>(place)[2 * tid + 1] = w[1];
+    }
+    __syncthreads();
+    for (uint32_t i = tid; i < cnt; i += THREADS) {
+        const U k = group[i];
+        const uint32_t b = bin(k);
+        sk((atomicAdd(&place[b >> 1], 1u << 16 * (b & 1u)) >> 16 * (b & 1u)) & 0xffffu) = k;
+    }
+    __syncthreads();  // now a sub-bucket's word is its end
+    for (uint32_t i = tid; i < cnt; i += THREADS) {
+        const U k = sk(i);
+        const uint32_t b = bin(k);
+        if (i > first_of(b) && sk(i - 1) != k) atomicOr(&flags[b >> 2], 1u << 8 * (b & 3u));
+    }
+    __syncthreads();
+    for (uint32_t w0 = warp * 32; w0 < uint32_t(G::BINS) / 4; w0 += THREADS) {
+        const uint32_t mine = flags[w0 + lane];
+        for (uint32_t some = __ballot_sync(0xffffffffu, mine != 0u); some; some &= some - 1u) {
+            const int l = __ffs(some) - 1;
+            const uint32_t word = __shfl_sync(0xffffffffu, mine, l);
+            for (uint32_t q = 0; q < 4; ++q) {
+                if (!(word >> 8 * q & 1u)) continue;
+                const uint32_t b = (w0 + l) * 4 + q, first = first_of(b), m = ends[b] - first;
+                if (m <= BY_THREAD) continue;
+                if (m > BY_WARP) {
+                    if (lane == 0) scan[atomicAdd(&misc[1], 1u)] = b;
+                } else {
+                    ascending_network(
+                        m, lane, 32u, [&](uint32_t x, uint32_t y) { order(first + x, first + y); }, [] { __syncwarp(); });
+                }
+            }
+        }
+    }
+    static_assert(G::PLACES / BY_WARP <= 32, "the list of sub-buckets");
+    __syncthreads();
+    const uint32_t left = misc[1];
+    for (uint32_t g = 0; g < left; ++g) {
+        const uint32_t first = first_of(scan[g]), m = ends[scan[g]] - first;
+        ascending_network(
+            m, tid, THREADS, [&](uint32_t x, uint32_t y) { order(first + x, first + y); }, [] { __syncthreads(); });
+    }
+    for (uint32_t i = tid; i < cnt; i += THREADS) {
+        const U k = sk(i);
+        const uint32_t b = bin(k), first = first_of(b), m = ends[b] - first;
+        uint32_t at = i;
+        if (m <= BY_THREAD && (flags[b >> 2] >> 8 * (b & 3u) & 1u)) {
+            at = first;
+            for (uint32_t q = first; q < first + m; ++q) {
+                const U o = sk(q);
+                at += uint32_t(o < k || (o == k && q < i));
+            }
+        }
+        group[at] = map.out(k);
+    }
+    __syncthreads();
+    for (uint32_t i = tid; i < uint32_t(G::BINS) / 4; i += THREADS) flags[i] = 0u;
+    __syncthreads();
+}
+
 // 32 bytes to a 32-byte aligned address.
 __device__ __forceinline__ void store_32b(void* dst, const uint4& a, const uint4& b) {
     asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "r"(a.x), "r"(a.y), "r"(a.z),
@@ -1253,8 +1370,9 @@ __global__ void __launch_bounds__(THREADS, MIN_CTAS) msd_local_kernel(MsdParams 
     __syncthreads();
     U* keys = static_cast<U*>(p.keys_a);
     // (floats: a group's keys share few bins, so the table's reads are broadcasts)
-    const auto code_of = msd_code<EVEN>(p, p.table);
-    const uint32_t groups = 256u << code_of.b2;
+    auto code_of = msd_code<EVEN>(p, p.table);
+    using Code = decltype(code_of);
+    auto groups = [&] { return 256u << code_of.b2; };
     // The CTA's groups in turn: g, + gridDim.x, ...  Floats: two neighbours are
     // sorted as one where they fit, since their groups, as many as the densest
     // stretch needs, are small (6 * 10^7 keys of N(0, 1): 336 -> 243 us).
@@ -1266,7 +1384,7 @@ __global__ void __launch_bounds__(THREADS, MIN_CTAS) msd_local_kernel(MsdParams 
     auto next_group = [&] {
         Group r{0u, 0u};
         if constexpr (EVEN) {
-            if (ahead * 2u < groups) {
+            if (ahead * 2u < groups()) {
                 const uint32_t a = ahead ? p.cursor2[ahead * 2u - 1u] : 0u, b = p.cursor2[ahead * 2u], c = p.cursor2[ahead * 2u + 1u];
                 const bool both = c - a <= p.group_cap;
                 r.off = half ? b : a;
@@ -1276,7 +1394,7 @@ __global__ void __launch_bounds__(THREADS, MIN_CTAS) msd_local_kernel(MsdParams 
                 half = both ? 0u : half ^ 1u;
                 if (half) return r;
             }
-        } else if (ahead < groups) {
+        } else if (ahead < groups()) {
             r.off = ahead ? p.cursor2[ahead - 1u] : 0u;
             r.word = (p.cursor2[ahead] - r.off) | (8u + code_of.b2) << 16;
         }
@@ -1286,7 +1404,7 @@ __global__ void __launch_bounds__(THREADS, MIN_CTAS) msd_local_kernel(MsdParams 
     // Key VEC * i + e of a thread is the group's key
     // (i * THREADS + tid) * VEC + e - shift: 16-byte loads from the address
     // at or below the group's start (which keys a thread has does not matter)
-    const KeyMap<U> map(p.kind, p.desc);
+    KeyMap<U> map(p.kind, p.desc);
     Group cur = next_group(), next = next_group();
     U k[LIPT];
     auto skew_of = [&](uint32_t o, uint32_t bytes) {
@@ -1297,87 +1415,113 @@ __global__ void __launch_bounds__(THREADS, MIN_CTAS) msd_local_kernel(MsdParams 
         const uint32_t skew = skew_of(f.off, 16);
         load_vectors<THREADS>(const_cast<const U*>(keys) + f.off - skew, skew, skew + f.cnt(), k);
     };
+    // A group that has to go another way (crowded) leaves the loop, and what the
+    // loop knows goes through shared memory: nothing of it lives across the
+    // call, which would otherwise spill in the usual path (5 x 10^7 u64 keys, the
+    // whole sort 859 us with a call in the loop, 809 this way).  Wide keys keep
+    // the two groups ahead too, 4-byte keys find them again: each as it spills less.
+    constexpr bool KEEP = KB > 4;
+    __shared__ uint32_t left_at[8];
     load(cur);
-    while (cur.word != 0u) {
-        const Group later = next_group();
-        const uint32_t off = cur.off, cnt = cur.cnt();
-        {
-            const uintptr_t a = reinterpret_cast<uintptr_t>(keys + later.off) & ~uintptr_t(127);
-            const uintptr_t e = reinterpret_cast<uintptr_t>(keys + later.off + later.cnt());
-            for (uintptr_t q = a + uintptr_t(tid) * 128; q < e; q += uintptr_t(THREADS) * 128)
-                asm volatile("prefetch.global.L2 [%0];" ::"l"(q));
-        }
-        const uint32_t skew = skew_of(off, 16), pad = skew_of(off, 32);
-        U* dst = keys + off - pad;  // place q goes to dst[q]
-        bool sorted = true;
-        if (cnt != 0u)
-            sorted = group_sort<U, THREADS, HALO>(
-                k, cnt, skew, pad, smem,
-                [&](U x) { return __umulhi(code_of(x) << (cur.word >> 16), uint32_t(G::BINS)); },
-                [&] { load(next); },
-                [&](uint32_t c0, bool inside, const U(&x)[LIPT]) {
-                    union { uint4 q[4]; U k[LIPT]; } w;
+    for (;;) {
+        while (cur.word != 0u) {
+            const Group later = next_group();
+            const uint32_t off = cur.off, cnt = cur.cnt();
+            {
+                const uintptr_t a = reinterpret_cast<uintptr_t>(keys + later.off) & ~uintptr_t(127);
+                const uintptr_t e = reinterpret_cast<uintptr_t>(keys + later.off + later.cnt());
+                for (uintptr_t q = a + uintptr_t(tid) * 128; q < e; q += uintptr_t(THREADS) * 128)
+                    asm volatile("prefetch.global.L2 [%0];" ::"l"(q));
+            }
+            const uint32_t skew = skew_of(off, 16), pad = skew_of(off, 32);
+            U* dst = keys + off - pad;  // place q goes to dst[q]
+            bool sorted = true;
+            if (cnt != 0u)
+                sorted = group_sort<U, THREADS, HALO>(
+                    k, cnt, skew, pad, smem,
+                    SubBucket<Code>{code_of, cur.word >> 16, uint32_t(G::BINS)},
+                    [&] { load(next); },
+                    [&](uint32_t c0, bool inside, const U(&x)[LIPT]) {
+                        union { uint4 q[4]; U k[LIPT]; } w;
 #pragma unroll
-                    for (int i = 0; i < LIPT; ++i) w.k[i] = map.out(x[i]);
-                    if (inside) {
-                        store_32b(dst + c0, w.q[0], w.q[1]);
-                        store_32b(dst + c0 + LIPT / 2, w.q[2], w.q[3]);
-                    } else {
+                        for (int i = 0; i < LIPT; ++i) w.k[i] = map.out(x[i]);
+                        if (inside) {
+                            store_32b(dst + c0, w.q[0], w.q[1]);
+                            store_32b(dst + c0 + LIPT / 2, w.q[2], w.q[3]);
+                        } else {
 #pragma unroll
-                        for (int i = 0; i < LIPT; ++i)
-                            if (c0 + i >= pad && c0 + i < pad + cnt) dst[c0 + i] = w.k[i];
-                    }
-                },
-                [&](uint32_t place, U x) { dst[place] = map.out(x); });
-        if (!sorted) {
-            // repeated keys, or keys that share the sub-bucket's bits: the
-            // group goes back untwiddled, like every group sorted here, so
-            // the buffer holds the input's keys in some order, and the digit
-            // passes sort it (keys only: any order of the input sorts to the
-            // same bytes)
-            if constexpr (EVEN) {
-                // equal keys are in order, and values that the sample has
-                // missed take a bitonic network over the group, 91 steps at
-                // most, where a sort that gave up would be lost
-                U* sk = reinterpret_cast<U*>(smem);
-#pragma unroll
-                for (int u = 0; u < LIPT; ++u)
-                    if (index(skew, u) < cnt) sk[index(skew, u)] = k[u];
-                __syncthreads();
-                bool differ = false;
-                for (uint32_t i = tid; i < cnt; i += THREADS) differ |= sk[i] != sk[0];
-                differ = __syncthreads_or(differ) != 0;
-                uint32_t size = 1024u;
-                static_assert(KB != 4 || 8192 * KB <= int(G::SCAN_OFF), "the group padded to a power of two");
-                while (size < cnt) size *= 2u;
-                for (uint32_t i = cnt + tid; i < size; i += THREADS) sk[i] = U(~U(0));
-                for (uint32_t run = 2; differ && run <= size; run *= 2u)
-                    for (uint32_t gap = run / 2u; gap != 0u; gap /= 2u) {
-                        __syncthreads();
-                        for (uint32_t i = tid; i < size / 2u; i += THREADS) {
-                            const uint32_t a = 2u * i - (i & (gap - 1u)), b = a + gap;
-                            U x = sk[a], y = sk[b];
-                            if ((x > y) == ((a & run) == 0u)) {
-                                sk[a] = y;
-                                sk[b] = x;
-                            }
+                            for (int i = 0; i < LIPT; ++i)
+                                if (c0 + i >= pad && c0 + i < pad + cnt) dst[c0 + i] = w.k[i];
+                        }
+                    },
+                    [&](uint32_t place, U x) { dst[place] = map.out(x); });
+            if (!sorted) {
+                if constexpr (!EVEN) {
+                    if (tid == 0) {
+                        left_at[0] = cur.off;
+                        left_at[1] = cur.word;
+                        left_at[2] = KEEP ? ahead : ahead - 2u * gridDim.x;  // (the group after this one)
+                        if constexpr (KEEP) {
+                            left_at[3] = next.off;
+                            left_at[4] = next.word;
+                            left_at[5] = later.off;
+                            left_at[6] = later.word;
                         }
                     }
-                __syncthreads();
-                for (uint32_t i = tid; i < cnt; i += THREADS) keys[off + i] = map.out(sk[i]);
-                __syncthreads();
-                for (int i = tid; i < G::BINS / 4; i += THREADS) reinterpret_cast<uint32_t*>(smem + G::CTR_OFF)[i] = 0u;
-                __syncthreads();
-            } else {
+                    break;
+                }
+                if constexpr (EVEN) {
+                    // equal keys are in order, and values that the sample has
+                    // missed take a bitonic network over the group, 91 steps at
+                    // most, where a sort that gave up would be lost
+                    U* sk = reinterpret_cast<U*>(smem);
 #pragma unroll
-                for (int u = 0; u < LIPT; ++u)
-                    if (index(skew, u) < cnt) keys[off + index(skew, u)] = map.out(k[u]);
-                if (tid == 0) atomicOr(p.state, MSD_GAVE_UP);
+                    for (int u = 0; u < LIPT; ++u)
+                        if (index(skew, u) < cnt) sk[index(skew, u)] = k[u];
+                    __syncthreads();
+                    bool differ = false;
+                    for (uint32_t i = tid; i < cnt; i += THREADS) differ |= sk[i] != sk[0];
+                    differ = __syncthreads_or(differ) != 0;
+                    uint32_t size = 1024u;
+                    static_assert(KB != 4 || 8192 * KB <= int(G::SCAN_OFF), "the group padded to a power of two");
+                    while (size < cnt) size *= 2u;
+                    for (uint32_t i = cnt + tid; i < size; i += THREADS) sk[i] = U(~U(0));
+                    for (uint32_t run = 2; differ && run <= size; run *= 2u)
+                        for (uint32_t gap = run / 2u; gap != 0u; gap /= 2u) {
+                            __syncthreads();
+                            for (uint32_t i = tid; i < size / 2u; i += THREADS) {
+                                const uint32_t a = 2u * i - (i & (gap - 1u)), b = a + gap;
+                                U x = sk[a], y = sk[b];
+                                if ((x > y) == ((a & run) == 0u)) {
+                                    sk[a] = y;
+                                    sk[b] = x;
+                                }
+                            }
+                        }
+                    __syncthreads();
+                    for (uint32_t i = tid; i < cnt; i += THREADS) keys[off + i] = map.out(sk[i]);
+                    __syncthreads();
+                    for (int i = tid; i < G::BINS / 4; i += THREADS) reinterpret_cast<uint32_t*>(smem + G::CTR_OFF)[i] = 0u;
+                    __syncthreads();
+                }
             }
+            if (!sorted || cnt == 0u) load(next);
+            cur = next;
+            next = later;
         }
-        if (!sorted || cnt == 0u) load(next);
-        cur = next;
-        next = later;
+        if (EVEN || cur.word == 0u) break;
+        if constexpr (!EVEN) {
+            __syncthreads();
+            const volatile uint32_t* at = left_at;
+            group_sort_crowded<U, THREADS, HALO>(keys + at[0], at[1] & 0xffffu, smem,
+                                                 SubBucket<Code>{code_of, at[1] >> 16, uint32_t(G::BINS)}, map);
+            code_of = Code(p);
+            map = KeyMap<U>(p.kind, p.desc);
+            ahead = at[2];
+            cur = KEEP ? Group{at[3], at[4]} : next_group();
+            next = KEEP ? Group{at[5], at[6]} : next_group();
+            load(cur);
+        }
     }
     if constexpr (EVEN) {
         // groups of equal keys above the largest: every CTA takes a slice and

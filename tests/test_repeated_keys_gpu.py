@@ -27,3 +27,28 @@ def repeated(kt, n, seed, copies, share=1.0):
 @pytest.mark.parametrize("copies,share", [(36, 0.0005), (33, 1.0), (40, 1.0), (40, 0.5)])
 def test_crowded_windows(gb, cuda, oracle, kt, n, vb, copies, share):
     assert outcome_of(gb, cuda, oracle, kt, repeated(kt, n, copies, copies, share), vb, vb == 8) == 0
+
+
+@pytest.mark.parametrize("kt,n", [("u32", 3_000_001), ("i32", 20_000_003), ("u64", 3_000_001), ("i64", 30_000_001),
+                                  ("u128", 1_500_001), ("i128", 1_100_003)])
+@pytest.mark.parametrize("copies,share", [(33, 0.0002), (36, 0.4), (260, 0.001)])
+def test_crowded_groups(gb, cuda, oracle, kt, n, copies, share):
+    """Keys alone: sub-buckets of equal keys, beyond the byte counters too."""
+    assert outcome_of(gb, cuda, oracle, kt, repeated(kt, n, copies, copies, share), 0, copies == 36) == 0
+
+
+@pytest.mark.parametrize("kt,n", [("u32", 3_000_001), ("u64", 3_000_001), ("u128", 1_500_001)])
+@pytest.mark.parametrize("size", [12, 60, 300, 520, 900])
+def test_crowds_of_different_keys(gb, cuda, oracle, kt, n, size):
+    """Many keys that differ in their low bits only, in one sub-bucket: put in
+    order by a thread, a warp or the CTA, by their number."""
+    raw = raw_keys(kt, n, seed=size)
+    rng = np.random.default_rng(size)
+    word = raw if kt != "u128" else raw.view(np.uint64).reshape(-1, 2)[:, 1]
+    low = np.uint32(0xF) if kt == "u32" else np.uint64(0xFFFFF)
+    if kt == "u128" and size > 300:
+        pytest.skip("more than the groups of this many 16-byte keys have room for")
+    for g in range(50):
+        at = rng.integers(0, n, size)
+        word[at] = (word[at] & low) | (word[at[0]] & ~low)
+    assert outcome_of(gb, cuda, oracle, kt, raw) == 0
