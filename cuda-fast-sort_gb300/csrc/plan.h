@@ -11,7 +11,7 @@
 
 namespace gbsort {
 
-inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
+constexpr size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
 // Control block at the start of the workspace's control region:
 //   [gp_counts: passes*256 u64][tile_counters: 16 u32][err: u32][executed: u32][barrier: u32][pad]
@@ -27,13 +27,15 @@ struct CtlLayout {
     size_t barrier_gen_off = 0;  // its generation word (another 128-byte line)
     size_t fill_off = 0;         // [256] fill counts of its MSD regions
     size_t overflow_off = 0;     // its region overflow flag
-    size_t counters2_off = 0;    // a second set of tile counters and a second grid barrier, for the
-                                 // digit passes after a sort by leading digits (0: none)
-    size_t short_fill_off = 0;   // [1024] fill counts of a short key-value sort's regions
-    size_t sampled_off = 0;      // its sample: ticket, [FINISH_LEVELS + 2] counts
     size_t msd_state_off = 0;    // outcome of the most-significant-first path, its code window [2]
+    // Sorts by leading digits use the fill counts' words, which only the
+    // one-launch sort needs: a second set of tile counters [16] and a second grid
+    // barrier [2], for the digit passes after them, and the sample's ticket and
+    // [FINISH_LEVELS + 2] counts.
+    size_t counters2_off = 0;
+    size_t sampled_off = 0;
     size_t bytes = 0;
-    static CtlLayout make(int passes, bool finish = false, bool short_pairs = false) {
+    static constexpr CtlLayout make(int passes) {
         CtlLayout c;
         c.gp_off = 0;
         c.counters_off = size_t(passes) * 256 * 8;
@@ -44,16 +46,9 @@ struct CtlLayout {
         c.fill_off = align_up(c.barrier_gen_off + 4, 128);
         c.overflow_off = c.fill_off + 256 * 4;
         c.msd_state_off = c.overflow_off + 4;
+        c.counters2_off = c.fill_off;
+        c.sampled_off = c.counters2_off + 18 * 4;
         c.bytes = align_up(c.msd_state_off + 12, 256);
-        if (finish) {
-            c.counters2_off = c.bytes;
-            c.sampled_off = c.counters2_off + 18 * 4;
-            c.bytes = align_up(c.sampled_off + 9 * 4, 256);
-        }
-        if (short_pairs) {
-            c.short_fill_off = c.bytes;
-            c.bytes += 1024 * 4;
-        }
         return c;
     }
 };
@@ -119,12 +114,16 @@ struct Plan {
     bool finish = false;
     KernelEntry finish_k[3]{};
     // short key-value arrays in one launch (short_pairs.cuh): that kernel, the
-    // digit passes after it, its regions, and their place in the workspace
+    // digit passes after it, its regions, the words in each, and their place, at
+    // the end of the workspace (their fill counts lie in the status words, which
+    // only the digit passes use)
     bool short_pairs = false;
     KernelEntry short_k[2]{};
     int short_regions = 0;
+    uint32_t short_cap = 0;
     size_t short_off = 0;
-    size_t total_bytes = 0;
+    size_t min_bytes = 0;    // workspace below which a sort is refused (without regions)
+    size_t total_bytes = 0;  // what the size query asks for
     CtlLayout ctl{};
     // the process-wide switches as this plan found them, each read once: the
     // kernels, their parameters and the graph's key have to agree while another
@@ -145,6 +144,10 @@ struct AltBuffers {
     void* vals_b;
 };
 size_t double_buffer_bytes(const Plan& plan);
+
+// Makes the plan fit a workspace of `bytes` (of a DoubleBuffer sort: `alt`):
+// regions as large as there is room for, or none.  False: too small for any sort.
+bool fit_workspace(Plan* plan, size_t bytes, bool alt);
 
 // Enqueues one sort on `stream`.  `ms` (optional) receives per-kernel event
 // times after a stream sync: [upsweep, pass 0 .. pass P-1].

@@ -180,12 +180,23 @@ constexpr uint32_t short_pairs_cap(int kb) {
 // more regions than needed cost a global atomic each per tile: 600001 pairs in
 // 456 36 us, in 256 31), the first of these whose mean region of uniform keys
 // and six of its standard deviations fit the cap; 0: none do.
+inline uint32_t short_pairs_need(uint64_t n, int regions) {  // words a region has to take
+    const double mean = double(n) / double(regions);
+    return (uint32_t(mean * 1.01 + 6.0 * std::sqrt(mean) + 8.0) + 4u) & ~3u;
+}
 inline int short_pairs_regions(int kb, uint64_t n) {
-    for (int regions : {256, 456, 912}) {
-        const double mean = double(n) / double(regions);
-        if (mean * 1.01 + 6.0 * std::sqrt(mean) + 8.0 <= double(short_pairs_cap(kb))) return regions;
-    }
+    for (int regions : {256, 456, 912})
+        if (short_pairs_need(n, regions) <= short_pairs_cap(kb)) return regions;
     return 0;
+}
+// Words that the size query holds for a region: six times the mean, where the
+// cap is not nearer, so that keys whose leading bits take few values (2^16 keys
+// with 256 upper halves: six to a region somewhere) still sort here.  A
+// DoubleBuffer workspace, whose point is its size, holds what uniform keys need.
+inline uint32_t short_pairs_room(int kb, uint64_t n, int regions) {
+    const uint64_t six = (6 * n / uint64_t(regions) + 64) & ~uint64_t(3);
+    const uint32_t need = short_pairs_need(n, regions);
+    return six > short_pairs_cap(kb) ? short_pairs_cap(kb) : six < need ? need : uint32_t(six);
 }
 constexpr uint64_t SHORT_PAIRS_N_MIN = 2048;
 

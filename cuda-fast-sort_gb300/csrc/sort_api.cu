@@ -20,6 +20,7 @@
 //     and a finish (finish.cuh), then the same;
 //   - everything else: a histogram and one launch per digit pass (onesweep.cuh).
 
+#include <algorithm>
 #include <atomic>
 #include <cstdio>
 #include <cstdlib>
@@ -351,7 +352,7 @@ int make_plan(int key_type, size_t value_bytes, uint64_t n, Plan* plan) {
                                    n >= SHORT_PAIRS_N_MIN
                                ? short_pairs_regions(p.kb, n)
                                : 0;
-    p.ctl = CtlLayout::make(p.passes, finish, short_regions != 0);
+    p.ctl = CtlLayout::make(p.passes);
     p.ctl_off = off;
     off = align_up(off + p.ctl.bytes, 256);
     p.status_off = off;
@@ -397,12 +398,14 @@ int make_plan(int key_type, size_t value_bytes, uint64_t n, Plan* plan) {
             p.msd_k[5] = e[5 + shape];
         }
     }
+    p.min_bytes = off;
     if (short_regions) {
         p.short_off = off;
-        off = align_up(off + size_t(short_regions) * short_pairs_cap(p.kb) * 2 * kb, 256);
+        p.short_regions = short_regions;
+        p.short_cap = short_pairs_room(p.kb, n, short_regions);
+        off = align_up(off + size_t(short_regions) * p.short_cap * 2 * kb, 256);
         if (p.skip) {
             p.short_pairs = true;
-            p.short_regions = short_regions;
             const KernelEntry* e = p.kb == 4 ? short_pairs_entries_k4() : short_pairs_entries_k8();
             p.short_k[0] = e[p.vb == 4 ? 0 : 2];
             p.short_k[1] = e[p.vb == 4 ? 1 : 3];
@@ -424,7 +427,28 @@ int make_plan(int key_type, size_t value_bytes, uint64_t n, Plan* plan) {
     return GBSORT_OK;
 }
 
-size_t double_buffer_bytes(const Plan& plan) { return plan.total_bytes - plan.ctl_off; }
+namespace {
+size_t region_bytes(const Plan& plan, uint32_t cap) {
+    return size_t(plan.short_regions) * cap * 2 * size_t(plan.kb);
+}
+}  // namespace
+
+size_t double_buffer_bytes(const Plan& plan) {
+    const size_t regions =
+        plan.short_regions ? align_up(region_bytes(plan, short_pairs_need(plan.n, plan.short_regions)), 256) : 0;
+    return plan.min_bytes - plan.ctl_off + regions;
+}
+
+bool fit_workspace(Plan* plan, size_t bytes, bool alt) {
+    if (alt) bytes += plan->ctl_off;
+    if (bytes < plan->min_bytes) return false;
+    if (plan->short_regions) {
+        const size_t cap = (bytes - plan->min_bytes) / region_bytes(*plan, 1) & ~size_t(3);
+        plan->short_cap = uint32_t(std::min<size_t>(cap, short_pairs_cap(plan->kb)));
+        if (plan->short_cap < short_pairs_need(plan->n, plan->short_regions)) plan->short_pairs = false;
+    }
+    return true;
+}
 
 int enqueue_sort(const Plan& plan, int descending, void* d_keys, void* d_values, void* d_workspace,
                  cudaStream_t stream, float* ms, int ms_cap, int* n_ms, const void* keys_src,
@@ -559,7 +583,9 @@ int enqueue_sort(const Plan& plan, int descending, void* d_keys, void* d_values,
     const bool fused =
         !use_finish && plan.fused.fn != nullptr && prepare_kernel(plan.fused) == GBSORT_OK && resident_ctas(plan.fused) > 0;
     // (it clears its lookback status words itself, before its first pass)
-    cudaError_t e = cudaMemsetAsync(ctl, 0, plan.ctl.bytes, stream);
+    // (with a short key-value sort's fill counts, which follow it)
+    static_assert(CtlLayout::make(16).bytes % 256 == 0, "the status words start where the control block ends");
+    cudaError_t e = cudaMemsetAsync(ctl, 0, plan.ctl.bytes + (use_short ? size_t(plan.short_regions) * 4 : 0), stream);
     if (e != cudaSuccess) return fail("memset control block", e);
 
     HistParams hp{};
@@ -633,8 +659,8 @@ int enqueue_sort(const Plan& plan, int descending, void* d_keys, void* d_values,
         sp.desc = descending;
         sp.nb = uint32_t(plan.short_regions);
         sp.regions = ws + plan.short_off - ws_base;
-        sp.cap = short_pairs_cap(plan.kb);
-        sp.fill = reinterpret_cast<uint32_t*>(ctl + plan.ctl.short_fill_off);
+        sp.cap = plan.short_cap;
+        sp.fill = static_cast<uint32_t*>(status);
         sp.state = msd_state;
         sp.barrier = reinterpret_cast<uint32_t*>(ctl + plan.ctl.barrier_off);
         sp.barrier_gen = reinterpret_cast<uint32_t*>(ctl + plan.ctl.barrier_gen_off);
@@ -866,13 +892,14 @@ int check_args(int key_type, size_t value_bytes, void* d_keys, void* d_values, s
 // completes).  gbsort_graph_cache_clear() frees them all.
 struct GraphKey {
     int device, key_type, desc, skip, fused, msd, large_msd;
+    uint32_t short_cap;
     size_t vb;
     uint64_t n, wait_limit;
     const void *keys, *vals, *ws, *ksrc, *vsrc, *keys_b, *vals_b;
     cudaStream_t stream;
     auto tie() const {
-        return std::tie(device, key_type, desc, skip, fused, msd, large_msd, vb, n, wait_limit, keys, vals, ws, ksrc,
-                        vsrc, keys_b, vals_b, stream);
+        return std::tie(device, key_type, desc, skip, fused, msd, large_msd, short_cap, vb, n, wait_limit, keys, vals,
+                        ws, ksrc, vsrc, keys_b, vals_b, stream);
     }
     bool operator==(const GraphKey& o) const { return tie() == o.tie(); }
 };
@@ -912,6 +939,7 @@ int launch_sort(const Plan& plan, int descending, void* keys, void* vals, void* 
     k.fused = plan.fused.fn != nullptr;
     k.msd = plan.short_msd ? 1 : 0;
     k.large_msd = plan.msd ? 1 : 0;
+    k.short_cap = plan.short_pairs ? plan.short_cap : 0;
     k.vb = size_t(plan.vb);
     k.n = plan.n;
     k.wait_limit = wait_limit_ns();
@@ -994,7 +1022,7 @@ int sort_common(int key_type, int descending, void* d_keys, void* d_values, size
         set_last_error_text("keys and values must be aligned to their own size");
         return GBSORT_ERR_INVALID_ARGUMENT;
     }
-    if (*temp_bytes < plan.total_bytes) return GBSORT_ERR_WORKSPACE_TOO_SMALL;
+    if (!fit_workspace(&plan, *temp_bytes, false)) return GBSORT_ERR_WORKSPACE_TOO_SMALL;
     return launch_sort(plan, descending ? 1 : 0, d_keys, d_values, d_workspace, static_cast<cudaStream_t>(stream),
                        nullptr, nullptr);
 }
@@ -1035,7 +1063,7 @@ int sort_double_common(int key_type, int descending, void* keys0, void* keys1, v
         set_last_error_text("keys and values must be aligned to their own size");
         return GBSORT_ERR_INVALID_ARGUMENT;
     }
-    if (*temp_bytes < double_buffer_bytes(plan)) return GBSORT_ERR_WORKSPACE_TOO_SMALL;
+    if (!fit_workspace(&plan, *temp_bytes, true)) return GBSORT_ERR_WORKSPACE_TOO_SMALL;
     const int sel = *selector;
     void* ka = sel ? keys1 : keys0;
     void* va = value_bytes ? (sel ? vals1 : vals0) : nullptr;
@@ -1076,7 +1104,7 @@ int sort_copy_common(int key_type, int descending, const void* keys_in, void* ke
         set_last_error_text("keys and values must be aligned to their own size");
         return GBSORT_ERR_INVALID_ARGUMENT;
     }
-    if (*temp_bytes < plan.total_bytes) return GBSORT_ERR_WORKSPACE_TOO_SMALL;
+    if (!fit_workspace(&plan, *temp_bytes, false)) return GBSORT_ERR_WORKSPACE_TOO_SMALL;
     return launch_sort(plan, descending ? 1 : 0, keys_out, value_bytes ? vals_out : nullptr, d_workspace,
                        static_cast<cudaStream_t>(stream), keys_in, value_bytes ? vals_in : nullptr);
 }
@@ -1326,7 +1354,7 @@ int gbsort_sort_timed(int key_type, int descending, void* d_keys, void* d_values
         return GBSORT_OK;
     }
     if (d_keys == nullptr || d_workspace == nullptr || ms_out == nullptr) return GBSORT_ERR_INVALID_ARGUMENT;
-    if (temp_bytes < plan.total_bytes) return GBSORT_ERR_WORKSPACE_TOO_SMALL;
+    if (!fit_workspace(&plan, temp_bytes, false)) return GBSORT_ERR_WORKSPACE_TOO_SMALL;
     return enqueue_sort(plan, descending ? 1 : 0, d_keys, d_values, d_workspace,
                         static_cast<cudaStream_t>(stream), ms_out, ms_cap, n_ms);
 }

@@ -683,7 +683,8 @@ def _double_buffer_fn(value_bytes: int):
 
 
 def double_buffer_bytes(key_type, n: int, value_bytes: int = 0) -> int:
-    """Workspace bytes of the DoubleBuffer form (control words and status only)."""
+    """Workspace bytes of the DoubleBuffer form (control words and status, and for
+    short key-value arrays regions, without which they sort too)."""
     f = _double_buffer_fn(value_bytes)
     tb = ctypes.c_size_t(0)
     sel = ctypes.c_int(0)

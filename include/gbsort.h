@@ -126,10 +126,20 @@ int gbsort_sort_pairs_copy(int key_type, int descending, const void* d_keys_in,
  * (and two value buffers) of n elements; *selector (0 or 1) names the one
  * holding the input and, on return, the one holding the sorted result (it
  * flips only for 1-byte keys, whose sort is a single pass).  The passes ping-pong between the caller's buffers, so the
- * workspace holds only control words and lookback status, not n-sized
+ * workspace needs only control words and lookback status, not n-sized
  * alternate buffers (2^28 u32 keys: ~30 MB instead of ~1.1 GB).  The other
- * buffer is clobbered.  d_workspace == NULL writes the required bytes to
- * *temp_bytes (no device work).  The buffers of a pair must not overlap. */
+ * buffer is clobbered.  d_workspace == NULL writes the bytes to ask for to
+ * *temp_bytes (no device work).  The buffers of a pair must not overlap.
+ *
+ * Short key-value arrays (4- or 8-byte integer keys, 4- or 8-byte values, 2048
+ * to about 2.3 M pairs, 1.1 M of 8-byte keys) sort in one launch through
+ * regions of (key, index) words, for which the size queries hold room: this
+ * form 1.1 to 4.5 words of twice the key's size per pair (2^16 u32 + u32 pairs
+ * 0.75 MB, 10^6 9.1 MB), the other forms up to 7 (3.3 MB, 10.5 MB), so that
+ * unevenly spread keys fit too.  A workspace without that room is accepted, down
+ * to what the query says less the regions, and the digit passes sort; so the
+ * query is not monotone in n, but a workspace asked for at a larger n is never
+ * too small. */
 int gbsort_sort_keys_double_buffer(int key_type, int descending, void* d_keys0,
                                    void* d_keys1, int* selector,
                                    size_t* temp_bytes, void* d_workspace,
