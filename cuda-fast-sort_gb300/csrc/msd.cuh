@@ -163,7 +163,9 @@ __global__ void __launch_bounds__(MSD_SAMPLE_THREADS) msd_sample_kernel(MsdParam
     __syncthreads();
     const uint32_t skip = vary[0] ? __clz(vary[0]) : vary[1] ? 32u + __clz(vary[1]) : 0u;
     // keys in order send whole tiles to one digit: shared atomics on one
-    // address, slower than the digit passes (10^7 4-byte keys 290 and 207 us)
+    // address, slower than four digit passes (10^7 4-byte keys 290 and 207 us),
+    // though not than eight or sixteen (5 x 10^7 8-byte keys 1.16 and 2.13 ms,
+    // 2^24 16-byte ones 0.62 and 2.41)
     const uint32_t close = __popc(__ballot_sync(0xffffffffu, ((x[0] ^ y) << skip) >> 56 == 0u));
     if ((tid & 31) == 0) atomicAdd(&neighbours, close);
     uint32_t most = 0, twice = 0;
@@ -201,7 +203,7 @@ __global__ void __launch_bounds__(MSD_SAMPLE_THREADS) msd_sample_kernel(MsdParam
         while (b2 < uint32_t(p.b2_max) && n > 0.72f * cap * float(1u << b2)) ++b2;
         constexpr float S = MSD_SAMPLE_THREADS * PER;
         const bool crowded = again >= 16u && 2.f * float(again) * n > 64.f * S * S;
-        if (uneven || crowded || 2u * neighbours > uint32_t(MSD_SAMPLE_THREADS) || n > cap * float(1u << b2)) *p.state = MSD_OFF;
+        if (uneven || crowded || (KB == 4 && 2u * neighbours > uint32_t(MSD_SAMPLE_THREADS)) || n > cap * float(1u << b2)) *p.state = MSD_OFF;
         p.window[0] = skip;
         p.window[1] = b2;
     }
