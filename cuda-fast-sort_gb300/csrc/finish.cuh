@@ -24,8 +24,10 @@
 // A window whose sub-buckets are too full (keys that repeat inside groups of
 // different keys) is put in order by a network over all of it.
 // A group of different keys that does not fit a window leaves its windows as
-// they were, and every digit pass runs, from the caller's buffers, which then
-// hold the pairs untwiddled, in an order that a stable sort completes.
+// they were, untwiddled, and their range is sorted by all digits afterwards
+// (finish_repair_kernel; pairs in an order that a stable sort completes).
+// Where the leading digits do not vary, or those ranges are most of the array,
+// every digit pass runs, from the caller's buffers.
 #pragma once
 
 #include "msd.cuh"
@@ -41,13 +43,15 @@ struct FinishParams {
     uint64_t n;            // < 2^32
     int kind, desc;
     int copy;              // input-preserving: the passes end in the caller's buffers
-    uint32_t* state;       // MSD_OFF, MSD_GAVE_UP: every digit pass sorts
+    uint32_t* state;       // MSD_OFF, MSD_GAVE_UP: every digit pass sorts; MSD_RANGES: the list is not empty
     uint32_t* window;      // [2] lowest digit that the passes sort by, pairs per chunk
     const uint32_t* executed;  // passes run (bit 31 set; 0: none)
     uint32_t* ticket;      // the sample's CTAs, zeroed with the control block
     uint32_t* sampled;     // [FINISH_LEVELS + 2] their counts, and the keys met twice
     uint32_t* edges;       // [chunks + 1] first pair of every window (bit 31: the edge cuts a group)
-    uint32_t max_chunks;   // room in edges
+    uint32_t* seen;        // [chunks + 1] bit 1: the cut edge has different keys on its sides; bit 0: listed
+    uint32_t max_chunks;   // room in edges and seen
+    RangeList left;        // ranges that the finish leaves to sort
     uint32_t places;       // pairs a window may hold
     uint32_t* err;
 };
@@ -220,7 +224,7 @@ __device__ __forceinline__ bool finish_in_b(const FinishParams& p) {
 // ---- edges ------------------------------------------------------------------
 // Edge c: the first group start at or after pair c * chunk, found by a warp in
 // three rounds of 32 reads; none within places - chunk pairs: the edge stays
-// there and cuts the group, which has to consist of equal keys.
+// there and cuts the group, which should consist of equal keys.
 template <int KB>
 __global__ void __launch_bounds__(256) finish_edges_kernel(FinishParams p) {
     using U = typename KeyBits<KB>::U;
@@ -238,7 +242,10 @@ __global__ void __launch_bounds__(256) finish_edges_kernel(FinishParams p) {
     const uint32_t shift = 8u * lo;
     for (uint32_t c = (blockIdx.x * 256 + threadIdx.x) >> 5; c <= chunks; c += gridDim.x * 8) {
         if (c == 0 || c == chunks) {
-            if (lane == 0) p.edges[c] = c ? n : 0u;
+            if (lane == 0) {
+                p.edges[c] = c ? n : 0u;
+                p.seen[c] = 0u;
+            }
             continue;
         }
         const uint32_t at = c * chunk;
@@ -270,14 +277,16 @@ __global__ void __launch_bounds__(256) finish_edges_kernel(FinishParams p) {
             }
         }
         if (lane == 0) {
+            bool differ = false;
             if (head != 0xffffffffu) {
                 p.edges[c] = head;
             } else if (at + (p.places - chunk) >= n) {
                 p.edges[c] = n;  // the last group reaches the end of the array
             } else {
                 p.edges[c] = at | 0x80000000u;
-                if (keys[at] != before) atomicOr(p.state, MSD_GAVE_UP);
+                differ = keys[at] != before;
             }
+            p.seen[c] = differ ? 2u : 0u;
         }
     }
 }
@@ -431,6 +440,40 @@ __device__ __forceinline__ void scan_bins(uint8_t* smem, uint32_t cnt, uint32_t 
         for (int i = 0; i < WORDS / 2; ++i)
             reinterpret_cast<uint4*>(start)[i] = make_uint4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
     }
+}
+
+// Lists the windows that consecutive cut edges join, edge c one of them, once
+// (a warp; more than FINISH_FAR windows: the whole sort gives up).
+constexpr uint32_t FINISH_FAR = 16384;
+template <int KB>  // (one instance per key width's translation unit)
+__device__ __noinline__ void finish_list(const FinishParams& p, uint32_t c) {
+    const uint32_t lane = threadIdx.x & 31;
+    uint32_t first = c, last = c, steps = 0;
+    for (bool found = false; !found && steps < FINISH_FAR / 32; ++steps) {  // (edge 0 is whole)
+        const bool whole = lane < first && !(p.edges[first - 1u - lane] >> 31);
+        const uint32_t b = __ballot_sync(0xffffffffu, whole || lane >= first);
+        found = b != 0u;
+        first -= found ? uint32_t(__ffs(b)) : 32u;
+    }
+    for (bool found = false; !found && steps < 2 * (FINISH_FAR / 32); ++steps) {  // (so is the last one)
+        const bool whole = !(p.edges[last + 1u + lane] >> 31);
+        const uint32_t b = __ballot_sync(0xffffffffu, whole);
+        found = b != 0u;
+        last += found ? uint32_t(__ffs(b)) : 32u;
+    }
+    if (lane != 0) return;
+    const uint32_t begin = p.edges[first], end = p.edges[last];
+    if ((begin | end) >> 31) {  // not found so near
+        atomicOr(p.state, MSD_GAVE_UP);
+        return;
+    }
+    if (atomicOr(p.seen + first, 1u) & 1u) return;
+    const uint32_t i = atomicAdd(p.left.count, 1u);
+    if (i < p.left.most) {
+        p.left.ranges[2 * i] = begin;
+        p.left.ranges[2 * i + 1] = end - begin;
+    }
+    atomicOr(p.state, i < p.left.most ? MSD_RANGES : MSD_GAVE_UP);
 }
 
 // A window whose keys and places are in shared memory as they came, places
@@ -680,7 +723,7 @@ __global__ void __launch_bounds__(THREADS, MIN_CTAS) finish_kernel(FinishParams 
                 }
                 __syncthreads();
                 // an edge through a group of different keys: nothing this window can do
-                if ((w0 >> 31) && uneven[pad]) cut = true;
+                if ((w0 >> 31) && (uneven[pad] || (ld_relaxed(p.seen + s / chunk) & 2u))) cut = true;
                 if (w1 >> 31) {  // the window's last group
                     uint32_t last_group = 0;
 #pragma unroll
@@ -723,10 +766,8 @@ __global__ void __launch_bounds__(THREADS, MIN_CTAS) finish_kernel(FinishParams 
                 for (uint32_t j = tid; j < cnt; j += THREADS) ovals[s + j] = sv[pad + j];
             }
             __syncthreads();
-            if (tid == 0) {
-                atomicOr(p.state, MSD_GAVE_UP);
-                misc[0] = 0u;
-            }
+            if (tid == 0) misc[0] = 0u;
+            if (warp == 0) finish_list<KB>(p, (w0 >> 31 ? w0 & 0x7fffffffu : w1 & 0x7fffffffu) / chunk);  // (cut edges lie at c * chunk)
             more = advance();
             if (more) load();
             __syncthreads();

@@ -7,6 +7,7 @@
 #include "fused_short.cuh"
 #include "msd.cuh"
 #include "onesweep.cuh"
+#include "repair.cuh"
 #include "segmented.cuh"
 #include "shapes.h"
 #include "short_pairs.cuh"
@@ -133,6 +134,20 @@ KernelEntry make_finish_entry() {
     using F = FinishGeom<KB, VB, S::THREADS, S::LIPT, S::HALO>;
     return KernelEntry{reinterpret_cast<const void*>(&finish_kernel<KB, VB, S::THREADS, S::MIN_CTAS, S::LIPT, S::HALO>),
                        S::THREADS, F::LIPT, F::CAP, static_cast<unsigned long>(F::SMEM_BYTES)};
+}
+// What a finish leaves over: as the several passes' entries.
+template <int KB, int VB, class W, class S = PassShape<KB, VB>>
+KernelEntry make_repair_entry() {
+    using G = PassGeom<KB, VB, S::THREADS, S::IPT>;
+    return KernelEntry{reinterpret_cast<const void*>(&finish_repair_kernel<KB, VB, W, S::THREADS, S::IPT, S::MIN_CTAS,
+                                                                           S::LOOKBACK_WINDOW>),
+                       S::THREADS, S::IPT, G::TILE, static_cast<unsigned long>(G::SMEM_BYTES)};
+}
+template <int KB, int VB>
+const KernelEntry* repair_entries_of() {
+    static const KernelEntry e[3] = {make_repair_entry<KB, VB, uint32_t>(), make_repair_entry<KB, VB, uint64_t>(),
+                                     make_repair_entry<KB, VB, uint32_t, PassShapeSmall<KB, VB>>()};
+    return e;
 }
 template <int KB>
 const KernelEntry* finish_entries_for() {

@@ -198,15 +198,26 @@ struct PassGeom {
     }
 };
 
+// What a pass works on where that is known on the device only (in shared memory).
+struct PassView {
+    const void* keys_in;
+    void* keys_out;
+    const void* vals_in;
+    void* vals_out;
+    uint64_t n;
+    uint32_t tiles;
+    int twiddle_load, twiddle_store;
+};
+
 // Passes that do not run because one digit holds all n keys (bit q: digit q),
 // from every pass's counts; word: a shared word.
-__device__ __forceinline__ uint32_t pass_mask(const PassParams& p, uint32_t* word) {
+__device__ __forceinline__ uint32_t pass_mask(const PassParams& p, uint64_t n, uint32_t* word) {
     const int tid = threadIdx.x;
     if (tid == 0) *word = 0u;
     __syncthreads();
     if (tid < 256) {
         uint32_t m = 0;
-        for (int q = 0; q < p.passes; ++q) m |= uint32_t(p.gp_all[size_t(q) * 256 + tid] == p.n) << q;
+        for (int q = 0; q < p.passes; ++q) m |= uint32_t(p.gp_all[size_t(q) * 256 + tid] == n) << q;
         if (m) atomicOr(word, m);
     }
     __syncthreads();
@@ -221,11 +232,12 @@ __device__ __forceinline__ uint32_t pass_mask(const PassParams& p, uint32_t* wor
 // The pass on digit `pass` as a device function.  The pass kernel below runs
 // it once.  MULTI: the kernel of several passes, which knows the passes that do
 // not run (uniform, bit q: digit q) and has the digit offsets in shared memory
-// already; final: the last pass that runs maps the keys back.  False: a copy
-// ran out of time, or (not MULTI) the pass does not run.
-template <int KB, int VB, class W, int THREADS, int IPT, bool SEG, int LBW, bool MULTI = false>
+// already; final: the last pass that runs maps the keys back.  VIEW: the same,
+// on what `view` says instead of the launch's arrays.  False: a copy ran out of
+// time, or (not MULTI) the pass does not run.
+template <int KB, int VB, class W, int THREADS, int IPT, bool SEG, int LBW, bool MULTI = false, bool VIEW = false>
 __device__ __forceinline__ bool onesweep_pass_body(const PassParams& p, uint8_t* smem, int pass, uint32_t uniform = 0,
-                                                   bool final = true) {
+                                                   bool final = true, const PassView* view = nullptr) {
     using U = typename KeyBits<KB>::U;
     using V = typename ValBits<VB>::V;
     using G = PassGeom<KB, VB, THREADS, IPT>;
@@ -250,8 +262,8 @@ __device__ __forceinline__ bool onesweep_pass_body(const PassParams& p, uint8_t*
         else
             return uint32_t(warp * G::IPW + u * 32 + lane);
     };
-    const uint32_t T = p.num_tiles;
-    const uint64_t n = p.n;
+    const uint32_t T = VIEW ? view->tiles : p.num_tiles;
+    const uint64_t n = VIEW ? view->n : p.n;
     const int kind = p.kind, desc = p.desc;
     const uint32_t epoch = uint32_t(pass);
     W* status = static_cast<W*>(p.status);
@@ -260,7 +272,14 @@ __device__ __forceinline__ bool onesweep_pass_body(const PassParams& p, uint8_t*
     const void* vals_in = p.vals_in;
     void* vals_out = p.vals_out;
     int twiddle_load = p.twiddle_load, twiddle_store = p.twiddle_store;
-    {
+    if constexpr (VIEW) {
+        keys_in = view->keys_in;
+        keys_out = view->keys_out;
+        vals_in = view->vals_in;
+        vals_out = view->vals_out;
+        twiddle_load = view->twiddle_load;
+        twiddle_store = view->twiddle_store;
+    } else {
         if (p.skip || p.copy_keys_in) {
             const uint32_t all = (p.passes >= 32) ? 0xffffffffu : ((1u << p.passes) - 1u);
             if (!MULTI && p.skip) {
@@ -268,7 +287,7 @@ __device__ __forceinline__ bool onesweep_pass_body(const PassParams& p, uint8_t*
                     // the batched scan marked every pass whose digit varies in some segment
                     uniform = ~ld_relaxed(p.nonuniform_mask) & all;
                 } else {
-                    uniform = pass_mask(p, reinterpret_cast<uint32_t*>(smem + G::SKIP_OFF));
+                    uniform = pass_mask(p, n, reinterpret_cast<uint32_t*>(smem + G::SKIP_OFF));
                 }
                 if ((uniform >> pass) & 1u) return false;  // every CTA of this pass leaves: a no-op pass
             }
@@ -745,7 +764,7 @@ __global__ void __launch_bounds__(THREADS, MIN_CTAS) onesweep_multi_kernel(PassP
     if (p.msd_state && (ld_relaxed(p.msd_state) & p.state_mask) == 0u) return;  // sorted already
     uint32_t left_out = 0;  // digits below the leading ones
     if (p.leading && !(ld_relaxed(p.leading) & MSD_OFF)) left_out = (1u << ld_relaxed(p.leading + 1)) - 1u;
-    const uint32_t uniform = left_out | pass_mask(p, reinterpret_cast<uint32_t*>(smem + G::SKIP_OFF));
+    const uint32_t uniform = left_out | pass_mask(p, p.n, reinterpret_cast<uint32_t*>(smem + G::SKIP_OFF));
     const uint32_t all = (p.passes >= 32) ? 0xffffffffu : ((1u << p.passes) - 1u);
     const int total = __popc(~uniform & all);
     const bool to_b = !p.copy_keys_in && (total & 1) != 0;  // where the last pass leaves the result

@@ -30,10 +30,11 @@ struct CtlLayout {
     size_t msd_state_off = 0;    // outcome of the most-significant-first path, its code window [2]
     // Sorts by leading digits use the fill counts' words, which only the
     // one-launch sort needs: a second set of tile counters [16] and a second grid
-    // barrier [2], for the digit passes after them, and the sample's ticket and
-    // [FINISH_LEVELS + 2] counts.
+    // barrier [2], for the digit passes after them, the sample's ticket and
+    // [FINISH_LEVELS + 2] counts, and the number of ranges left to sort.
     size_t counters2_off = 0;
     size_t sampled_off = 0;
+    size_t ranges_off = 0;
     size_t bytes = 0;
     static constexpr CtlLayout make(int passes) {
         CtlLayout c;
@@ -48,6 +49,7 @@ struct CtlLayout {
         c.msd_state_off = c.overflow_off + 4;
         c.counters2_off = c.fill_off;
         c.sampled_off = c.counters2_off + 18 * 4;
+        c.ranges_off = c.sampled_off + 9 * 4;
         c.bytes = align_up(c.msd_state_off + 12, 256);
         return c;
     }
@@ -113,6 +115,7 @@ struct Plan {
     // finish; the edges lie in the status words
     bool finish = false;
     KernelEntry finish_k[3]{};
+    KernelEntry repair{};  // then: what the finish leaves over (repair.cuh)
     // short key-value arrays in one launch (short_pairs.cuh): that kernel, the
     // digit passes after it, its regions, the words in each, and their place, at
     // the end of the workspace (their fill counts lie in the status words, which

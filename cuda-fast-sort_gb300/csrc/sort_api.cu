@@ -63,6 +63,8 @@ const KernelEntry* short_pairs_entries_k8();
 const KernelEntry* multi_entries_k4();  // keys only
 const KernelEntry* multi_entries_k8(int vb);
 const KernelEntry* multi_entries_k16(int vb);
+const KernelEntry* repair_entries_k8(int vb);
+const KernelEntry* repair_entries_k16(int vb);
 const KernelEntry* finish_entries_k8();
 const KernelEntry* finish_entries_k16();
 const KernelEntry* msd_entries_k4();
@@ -417,6 +419,7 @@ int make_plan(int key_type, size_t value_bytes, uint64_t n, Plan* plan) {
         p.finish_k[0] = e[0];
         p.finish_k[1] = e[1];
         p.finish_k[2] = e[p.vb == 4 ? 2 : p.vb == 8 ? 3 : 4];
+        p.repair = (p.kb == 8 ? repair_entries_k8(p.vb) : repair_entries_k16(p.vb))[small ? 2 : p.wide_status ? 1 : 0];
     }
     if (p.msd || p.finish)
         p.multi = (p.kb == 4   ? multi_entries_k4()
@@ -467,7 +470,7 @@ int enqueue_sort(const Plan& plan, int descending, void* d_keys, void* d_values,
     // (its digit passes run in one launch, which sort_timed does not use)
     bool use_finish = plan.finish && ms == nullptr;
     for (int i = 0; use_finish && i < 3; ++i) use_finish = prepare_kernel(plan.finish_k[i]) == GBSORT_OK;
-    use_finish = use_finish && prepare_kernel(plan.multi) == GBSORT_OK;
+    use_finish = use_finish && prepare_kernel(plan.multi) == GBSORT_OK && prepare_kernel(plan.repair) == GBSORT_OK;
     // the most-significant-first path of keys-only sorts runs when all its
     // kernels can
     bool use_msd = plan.msd && !use_finish;
@@ -731,7 +734,13 @@ int enqueue_sort(const Plan& plan, int descending, void* d_keys, void* d_values,
         fin.ticket = reinterpret_cast<uint32_t*>(ctl + plan.ctl.sampled_off);
         fin.sampled = fin.ticket + 1;
         fin.edges = static_cast<uint32_t*>(status);
-        fin.max_chunks = uint32_t(plan.status_bytes / 4 - 2 < 0xffffffffull ? plan.status_bytes / 4 - 2 : 0xffffffffull);
+        // the status words hold the edges from their start and the list of ranges
+        // at their end, beyond what the passes over half of the array use
+        fin.left.most = plan.num_tiles < 4 ? 0 : uint32_t(std::min<size_t>(RANGES_MOST, plan.status_bytes / 64));
+        fin.left.count = reinterpret_cast<uint32_t*>(ctl + plan.ctl.ranges_off);
+        fin.left.ranges = reinterpret_cast<uint32_t*>(static_cast<uint8_t*>(status) + plan.status_bytes) - 2 * fin.left.most;
+        fin.max_chunks = uint32_t(std::min<size_t>((plan.status_bytes - 8 * size_t(fin.left.most)) / 8 - 2, 0x7fffffff));
+        fin.seen = fin.edges + fin.max_chunks + 2;
         fin.places = uint32_t(plan.finish_k[2].tile);
         fin.err = err_word;
         {  // an ordinary launch: the histogram, its dependent, does not wait for what came before
@@ -820,13 +829,14 @@ int enqueue_sort(const Plan& plan, int descending, void* d_keys, void* d_values,
         if (e != cudaSuccess) return fail("finish launch", e);
         PassParams pp = pass_params(0);
         pp.msd_state = msd_state;
-        pp.state_mask = MSD_GAVE_UP;
-        pp.leading = nullptr;
         pp.tile_counter = reinterpret_cast<uint32_t*>(ctl + plan.ctl.counters2_off);
         pp.barrier = pp.tile_counter + 16;
         pp.barrier_gen = pp.barrier + 1;
         pp.clear_bytes = plan.status_bytes;
-        e = launch_passes(pp);
+        const uint64_t most = uint64_t(sms) * uint64_t(resident_ctas(plan.repair));
+        void* rargs[] = {&pp, &fin.left};
+        e = cudaLaunchCooperativeKernel(plan.repair.fn, dim3(uint32_t(plan.num_tiles < most ? plan.num_tiles : most)),
+                                        dim3(plan.repair.threads), rargs, plan.repair.smem, stream);
         if (e != cudaSuccess) return fail("pass launch", e);
         return GBSORT_OK;  // (the fix-up is part of those launches; nothing is timed)
     }
@@ -1247,7 +1257,9 @@ int gbsort_workspace_outcome(int key_type, size_t value_bytes, size_t n, int dou
     const int st = make_plan(key_type, value_bytes, n, &plan);
     if (st != GBSORT_OK) return st;
     if (d_workspace == nullptr || outcome == nullptr) return GBSORT_ERR_INVALID_ARGUMENT;
-    static_assert(GBSORT_OUTCOME_PASSES == MSD_OFF && GBSORT_OUTCOME_GAVE_UP == MSD_GAVE_UP, "the device's word");
+    static_assert(GBSORT_OUTCOME_PASSES == MSD_OFF && GBSORT_OUTCOME_GAVE_UP == MSD_GAVE_UP &&
+                      GBSORT_OUTCOME_RANGES == MSD_RANGES,
+                  "the device's word");
     *outcome = 0;
     if (n == 0) return GBSORT_OK;
     return read_word(d_workspace, (double_buffer ? 0 : plan.ctl_off) + plan.ctl.msd_state_off, stream, outcome);

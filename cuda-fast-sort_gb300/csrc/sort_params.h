@@ -8,7 +8,17 @@ namespace gbsort {
 // Why the digit passes sort after the most-significant-first path of a
 // keys-only sort (msd.cuh; 0: that path sorts): MSD_OFF some group is too big
 // (decided before any key moves), MSD_GAVE_UP a local sort gave up.
-constexpr uint32_t MSD_OFF = 1u, MSD_GAVE_UP = 2u;
+// MSD_RANGES: some ranges are left to sort (finish.cuh).
+constexpr uint32_t MSD_OFF = 1u, MSD_GAVE_UP = 2u, MSD_RANGES = 4u;
+
+// Ranges of the result that a sort by leading digits leaves to sort: a list in
+// no order, of first pair and length.
+struct RangeList {
+    uint32_t* count;     // zeroed with the control block
+    uint32_t* ranges;    // [2 * most]
+    uint32_t most;
+};
+constexpr uint32_t RANGES_MOST = 1024;
 
 // Global-histogram upsweep (one launch per sort).
 struct HistParams {

@@ -222,12 +222,12 @@ def workspace_status(key_type, n: int, workspace, value_bytes: int = 0, stream=N
     return lib().gbsort_workspace_status(key_type_id(key_type), value_bytes, n, _ptr(workspace), _stream(stream))
 
 
-OUTCOME_PASSES, OUTCOME_GAVE_UP = 1, 2
+OUTCOME_PASSES, OUTCOME_GAVE_UP, OUTCOME_RANGES = 1, 2, 4
 
 
 def workspace_outcome(key_type, n: int, workspace, value_bytes: int = 0, stream=None, double_buffer: bool = False) -> int:
     """gbsort_workspace_outcome: 0 when the planned path made the last sort on
-    this workspace, else OUTCOME_PASSES or OUTCOME_GAVE_UP (bits)."""
+    this workspace, else OUTCOME_PASSES, OUTCOME_GAVE_UP or OUTCOME_RANGES (bits)."""
     f = lib().gbsort_workspace_outcome
     f.restype = ctypes.c_int
     f.argtypes = [ctypes.c_int, ctypes.c_size_t, ctypes.c_size_t, ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p,

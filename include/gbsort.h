@@ -461,6 +461,9 @@ int gbsort_workspace_status(int key_type, size_t value_bytes, size_t n,
  * double_buffer: the workspace is one of a DoubleBuffer sort. */
 #define GBSORT_OUTCOME_PASSES 1u
 #define GBSORT_OUTCOME_GAVE_UP 2u
+#define GBSORT_OUTCOME_RANGES 4u /* it sorted all but some ranges, which were
+                                    sorted by themselves (key-value sorts of 8-
+                                    and 16-byte keys, 8-byte floats) */
 int gbsort_workspace_outcome(int key_type, size_t value_bytes, size_t n,
                              int double_buffer, void* d_workspace,
                              void* stream, uint32_t* outcome);

@@ -52,3 +52,40 @@ def test_crowds_of_different_keys(gb, cuda, oracle, kt, n, size):
         at = rng.integers(0, n, size)
         word[at] = (word[at] & low) | (word[at[0]] & ~low)
     assert outcome_of(gb, cuda, oracle, kt, raw) == 0
+
+
+def heavy(kt, n, seed, shares):
+    """A few keys of a share of the array each, among keys that share their
+    leading bytes."""
+    raw = raw_keys(kt, n, seed=seed)
+    rng = np.random.default_rng(seed)
+    draw = rng.random(n)
+    at = 0.0
+    for share in shares:
+        raw[(draw >= at) & (draw < at + share)] = raw[rng.integers(0, n)]
+        at += share
+    return raw
+
+
+@pytest.mark.parametrize("kt,n,vb", [("u64", 2_500_001, 4), ("i64", 9_000_011, 8), ("f64", 70_001, 4), ("f64", 600_011, 0),
+                                     ("u128", 100_003, 4), ("i128", 700_001, 8)])
+@pytest.mark.parametrize("shares", [(0.02,), (0.001, 0.01, 0.1), tuple([0.004] * 60), (0.45,), (0.7, 0.1)])
+def test_heavy_keys(gb, cuda, oracle, kt, n, vb, shares):
+    """Groups beyond a window that hold other keys too: their ranges are sorted by
+    themselves, in all three forms of the call."""
+    raw = heavy(kt, n, n % 97, shares)
+    for api, desc in (("inplace", False), ("copy", True), ("buffers", False)):
+        outcome = outcome_of(gb, cuda, oracle, kt, raw, vb, desc, api)
+        assert outcome in (0, gb.OUTCOME_RANGES) or max(shares) > 0.5  # (more than half: all of it again)
+
+
+def test_few_keys_of_very_many(gb, cuda, oracle):
+    """Half of the array in one group of two keys: too much to take apart."""
+    n = 3_000_001
+    raw = raw_keys("u64", n, seed=2)
+    raw[: 2 * n // 3] = 0x1234567800000000
+    raw[: 2 * n // 3: 3] = 0x1234567800000001
+    raw = raw[np.random.default_rng(2).permutation(n)]
+    outcome_of(gb, cuda, oracle, "u64", raw, 4)
+    outcome_of(gb, cuda, oracle, "u64", raw, 8, True, "copy")
+    outcome_of(gb, cuda, oracle, "u64", raw, 4, False, "buffers")
