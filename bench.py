@@ -450,6 +450,7 @@ def bench_gbsort(args, cfg, world, rank, local):
     mean_sort_ms = total_ms / args.steps
     fused = all(len(p) == 1 for p in per_kernel)  # the whole short sort in one launch
     pinfo = gbsort.plan(kt, n, vb)
+    route = gbsort.route(kt, n, vb)
     msd_keys = pinfo.msd_region_keys if fused else 0
     stages = None
     if not fused and pinfo.msd_stages:
@@ -470,7 +471,7 @@ def bench_gbsort(args, cfg, world, rank, local):
                                 "frac": round(nbytes[i] / (means[i] / 1e3) / 1e9 / hbm, 4) if i != 1 else None}
         rest = [statistics.mean(p[i] for p in per_kernel) for i in range(6, len(per_kernel[0]))]
         stages["digits' histogram + digit passes + fix-up (exit at once)"] = round(sum(rest), 4)
-    elif not fused and all(p[0] > sum(p[1:]) for p in per_kernel):
+    elif not fused and route.timed_path == gbsort.PATH_MSD:
         # 4-byte keys, the same way: entry 0 holds its kernels together
         launch_ms = statistics.mean(p[0] for p in per_kernel)
         sort_bytes = n * 7 * kbytes
@@ -503,9 +504,10 @@ def bench_gbsort(args, cfg, world, rank, local):
     sort_roofline = {"bytes_per_key": sort_bytes // n, "achieved": round(
         sort_bytes / (mean_sort_ms / 1e3) / 1e9, 1), "peak": hbm, "unit": "GB/s",
         "frac": round(sort_bytes / (mean_sort_ms / 1e3) / 1e9 / hbm, 4)}
-    if vb in (4, 8) and kbytes >= 8:
-        sort_roofline["note"] = ("counts a pass per key byte; the sort makes the leading ones and a finish, so fewer "
-                                 "bytes move")
+    if route.path != route.timed_path:
+        roofline["note"] = ("of the digit-pass path, whose kernels can be timed one by one; the timed value is of "
+                            "another path")
+        sort_roofline["note"] = "counts a pass per key byte; the path that sorts moves fewer bytes"
 
     # comparator: CUB DeviceRadixSort (toolkit) on the same buffers, same timing
     cub = None
@@ -597,12 +599,7 @@ def bench_gbsort(args, cfg, world, rank, local):
     if rank != 0:
         return None
     plan = gbsort.plan(kt, n, vb)
-    # launches of one untimed sort
-    sort_launches = plan.kernel_launches
-    if not vb and plan.kernel_launches > passes + 2:
-        sort_launches = 8
-    elif vb in (4, 8) and kbytes >= 8:
-        sort_launches = 6
+    sort_launches = gbsort.route(kt, n, vb).kernel_launches  # of one untimed sort
     line = {
         "metric": PLAIN_METRIC, "value": round(value, 3),
         "unit": "Gkeys/s", "n_gpus": world, "steps": args.steps, "warmup": args.warmup,
@@ -631,7 +628,7 @@ def bench_gbsort(args, cfg, world, rank, local):
                              "keys-only arrays: one launch; larger keys-only ones: the six MSD kernels, the "
                              "histogram and one launch of all digit passes (both exit at once); 8- and 16-byte "
                              "keys with values: sample, histogram, leading passes, edges, finish and a launch "
-                             "that exits; plus one memset",
+                             "that exits; short integer pairs: two; plus one memset",
         "sorted_check": ok,
     }
     return line

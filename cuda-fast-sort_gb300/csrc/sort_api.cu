@@ -1355,6 +1355,37 @@ int gbsort_plan(int key_type, size_t value_bytes, size_t n, gbsort_plan_info* ou
     return GBSORT_OK;
 }
 
+int gbsort_route(int key_type, size_t value_bytes, size_t n, gbsort_route_info* out) {
+    if (out == nullptr) return GBSORT_ERR_INVALID_ARGUMENT;
+    Plan plan;
+    const int st = make_plan(key_type, value_bytes, n, &plan);
+    if (st != GBSORT_OK) return st;
+    std::memset(out, 0, sizeof(*out));
+    // as enqueue_sort chooses
+    const uint32_t passes = uint32_t(plan.passes) + 1u + (plan.skip && (plan.passes & 1) == 0 ? 1u : 0u);
+    out->path = plan.fused.fn && !plan.finish ? GBSORT_PATH_ONE_LAUNCH
+                : plan.short_pairs            ? GBSORT_PATH_SHORT_PAIRS
+                : plan.finish                 ? GBSORT_PATH_LEADING_DIGITS
+                : plan.msd                    ? GBSORT_PATH_MSD
+                                              : GBSORT_PATH_PASSES;
+    switch (out->path) {
+        case GBSORT_PATH_ONE_LAUNCH: out->kernel_launches = 1; break;
+        case GBSORT_PATH_SHORT_PAIRS: out->kernel_launches = 2; break;
+        // sample, histogram, leading passes, edges, finish, what it leaves over
+        case GBSORT_PATH_LEADING_DIGITS: out->kernel_launches = 6; break;
+        // its six kernels, histogram, digit passes (in one launch when they may skip)
+        case GBSORT_PATH_MSD: out->kernel_launches = plan.skip ? 8u : 6u + passes; break;
+        default: out->kernel_launches = passes;
+    }
+    out->timed_path = plan.fused.fn ? GBSORT_PATH_ONE_LAUNCH : plan.msd ? GBSORT_PATH_MSD : GBSORT_PATH_PASSES;
+    out->timed_kernel_launches = plan.fused.fn ? 1u : plan.msd ? 6u + passes : passes;
+    out->workspace_bytes = plan.total_bytes;
+    out->workspace_min_bytes = plan.min_bytes;
+    out->double_buffer_bytes = double_buffer_bytes(plan);
+    out->double_buffer_min_bytes = plan.min_bytes - plan.ctl_off;
+    return GBSORT_OK;
+}
+
 int gbsort_sort_timed(int key_type, int descending, void* d_keys, void* d_values, size_t value_bytes,
                       void* d_workspace, size_t temp_bytes, size_t n, void* stream, float* ms_out, int ms_cap,
                       int* n_ms) {

@@ -261,6 +261,25 @@ def plan(key_type, n: int, value_bytes: int = 0) -> Plan:
     return Plan(*(getattr(info, f) for f, _ in PlanInfo._fields_))
 
 
+PATH_PASSES, PATH_ONE_LAUNCH, PATH_SHORT_PAIRS, PATH_MSD, PATH_LEADING_DIGITS = range(5)
+
+
+class RouteInfo(ctypes.Structure):
+    _fields_ = [(f, ctypes.c_uint32) for f in ("path", "kernel_launches", "timed_path", "timed_kernel_launches")] + [
+        (f, ctypes.c_uint64) for f in ("workspace_bytes", "workspace_min_bytes", "double_buffer_bytes",
+                                       "double_buffer_min_bytes")]
+
+
+def route(key_type, n: int, value_bytes: int = 0) -> RouteInfo:
+    """gbsort_route: the path of a sort (PATH_*), its launches, its workspace sizes."""
+    f = lib().gbsort_route
+    f.restype = ctypes.c_int
+    f.argtypes = [ctypes.c_int, ctypes.c_size_t, ctypes.c_size_t, ctypes.POINTER(RouteInfo)]
+    info = RouteInfo()
+    _check(f(key_type_id(key_type), value_bytes, n, ctypes.byref(info)), "route")
+    return info
+
+
 def generate(dist: int, key_bytes: int, out, n: int, seed: int, stream=None) -> None:
     _check(lib().gbsort_generate(dist, key_bytes, _ptr(out), n, seed, _stream(stream)), "generate")
 

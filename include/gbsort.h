@@ -592,8 +592,7 @@ typedef struct gbsort_plan_info {
     uint32_t status_word_bytes; /* 4 or 8                                    */
     uint32_t kernel_launches; /* launches (plus one memset node) of a timed
                                  sort; 1 when a short keys-only array sorts in
-                                 one launch.  Untimed sorts make one launch of
-                                 the digit passes where a shorter path runs   */
+                                 one launch (gbsort_route: of an untimed one) */
     uint64_t workspace_bytes;
     uint32_t msd_region_keys; /* one-launch sort, most significant digit
                                  first: keys per top-digit region of its
@@ -607,11 +606,33 @@ typedef struct gbsort_plan_info {
                                  which samples the keys, and before the     
                                  digit passes; those and the histogram exit
                                  at once unless a group was too big; 0: not
-                                 planned, or not reported (4-byte keys)      */
+                                 planned, or not reported (4-byte keys).  Of
+                                 a timed sort, as all of this                */
 } gbsort_plan_info;
 
 int gbsort_plan(int key_type, size_t value_bytes, size_t n,
                 gbsort_plan_info* out);
+
+/* The path that a sort with a workspace of the queried size takes under the
+ * switches as they are, and the kernels that it launches (one memset more); the
+ * path and the kernels of gbsort_sort_timed, which keeps key-value sorts and
+ * 8-byte floats on kernels that it can time one by one; and the workspace sizes:
+ * what the queries ask for, and what is accepted at least.  A path that finds
+ * the keys too uneven ends in the digit passes (gbsort_workspace_outcome). */
+#define GBSORT_PATH_PASSES 0u         /* histogram, a pass per key byte, fix-up */
+#define GBSORT_PATH_ONE_LAUNCH 1u     /* short keys-only array                  */
+#define GBSORT_PATH_SHORT_PAIRS 2u    /* short key-value array: one launch, and
+                                         one that exits                         */
+#define GBSORT_PATH_MSD 3u            /* keys only, most significant bits first */
+#define GBSORT_PATH_LEADING_DIGITS 4u /* leading digits, then a stable finish   */
+typedef struct gbsort_route_info {
+    uint32_t path, kernel_launches;
+    uint32_t timed_path, timed_kernel_launches;
+    uint64_t workspace_bytes, workspace_min_bytes;
+    uint64_t double_buffer_bytes, double_buffer_min_bytes;
+} gbsort_route_info;
+int gbsort_route(int key_type, size_t value_bytes, size_t n,
+                 gbsort_route_info* out);
 
 /* Same as gbsort_sort_pairs (d_values may be NULL with value_bytes 0), but
  * records a CUDA event around every kernel on `stream` and, after
