@@ -25,7 +25,7 @@
 // different keys) is put in order by a network over all of it.
 // A group of different keys that does not fit a window leaves its windows as
 // they were, untwiddled, and their range is sorted by all digits afterwards
-// (finish_repair_kernel; pairs in an order that a stable sort completes).
+// (sort_ranges; pairs in an order that a stable sort completes).
 // Where the leading digits do not vary, or those ranges are most of the array,
 // every digit pass runs, from the caller's buffers.
 #pragma once
@@ -119,7 +119,8 @@ __global__ void __launch_bounds__(FINISH_SAMPLE_THREADS) finish_sample_kernel(Fi
         const uint32_t tag = uint32_t(h >> 32) & 0xffff8000u;
         uint32_t slot = uint32_t(h) & 32767u;
         for (int probe = 0; probe < 128; ++probe) {
-            const uint32_t w = atomicCAS(&cnt[slot], 0u, tag | 1u);
+            uint32_t w = cnt[slot];  // (one atomic a key where all share a prefix)
+            if (w == 0u) w = atomicCAS(&cnt[slot], 0u, tag | 1u);
             if (w == 0u) break;
             if ((w & 0xffff8000u) == tag) {
                 const uint32_t before = atomicAdd(&cnt[slot], 1u) & 32767u;  // the keys there before this one

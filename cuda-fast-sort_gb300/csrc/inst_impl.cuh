@@ -6,8 +6,8 @@
 #include "finish.cuh"
 #include "fused_short.cuh"
 #include "msd.cuh"
+#include "multi.cuh"
 #include "onesweep.cuh"
-#include "repair.cuh"
 #include "segmented.cuh"
 #include "shapes.h"
 #include "short_pairs.cuh"
@@ -24,18 +24,24 @@ KernelEntry make_pass_entry() {
 }
 
 // Several passes in one cooperative launch: [0: 32-bit status, 1: 64-bit
-// status, 2: small-n shape] (the sorts by leading digits).
-template <int KB, int VB, class W, class S = PassShape<KB, VB>>
+// status, 2: small-n shape], then those that follow a path which may leave
+// ranges to sort.
+template <int KB, int VB, class W, class S = PassShape<KB, VB>, bool LEFT = false>
 KernelEntry make_multi_entry() {
     using G = PassGeom<KB, VB, S::THREADS, S::IPT>;
     return KernelEntry{reinterpret_cast<const void*>(&onesweep_multi_kernel<KB, VB, W, S::THREADS, S::IPT, S::MIN_CTAS,
-                                                                            S::LOOKBACK_WINDOW>),
+                                                                            S::LOOKBACK_WINDOW, LEFT>),
                        S::THREADS, S::IPT, G::TILE, static_cast<unsigned long>(G::SMEM_BYTES)};
 }
 template <int KB, int VB>
 const KernelEntry* multi_entries_of() {
-    static const KernelEntry e[3] = {make_multi_entry<KB, VB, uint32_t>(), make_multi_entry<KB, VB, uint64_t>(),
-                                     make_multi_entry<KB, VB, uint32_t, PassShapeSmall<KB, VB>>()};
+    using S = PassShape<KB, VB>;
+    using T = PassShapeSmall<KB, VB>;
+    static const KernelEntry e[6] = {
+        make_multi_entry<KB, VB, uint32_t>(), make_multi_entry<KB, VB, uint64_t>(),
+        make_multi_entry<KB, VB, uint32_t, T>(),
+        make_multi_entry<KB, VB, uint32_t, S, true>(), make_multi_entry<KB, VB, uint64_t, S, true>(),
+        make_multi_entry<KB, VB, uint32_t, T, true>()};
     return e;
 }
 
@@ -91,7 +97,7 @@ template <int KB>
 const KernelEntry* msd_entries_for() {
     using S = MsdShape<KB>;
     using GS = MsdSplitGeom<KB, S::THREADS, S::IPT, S::CAP>;
-    static const KernelEntry e[7] = {
+    static const KernelEntry e[8] = {
         {reinterpret_cast<const void*>(&msd_sample_kernel<KB>), MSD_SAMPLE_THREADS, 0, 0, 0ul},
         {reinterpret_cast<const void*>(&msd_count_kernel<KB, false>), MSD_COUNT_THREADS, 0, 0,
          static_cast<unsigned long>(MSD_COUNT_SMEM)},
@@ -102,6 +108,7 @@ const KernelEntry* msd_entries_for() {
          GS::TILE, static_cast<unsigned long>(GS::SMEM_BYTES)},
         make_msd_local_entry<KB, 0>(),
         make_msd_local_entry<KB, 1>(),
+        {reinterpret_cast<const void*>(&msd_map_ranges_kernel<KB>), 256, 0, 0, 0ul},
     };
     return e;
 }
@@ -134,20 +141,6 @@ KernelEntry make_finish_entry() {
     using F = FinishGeom<KB, VB, S::THREADS, S::LIPT, S::HALO>;
     return KernelEntry{reinterpret_cast<const void*>(&finish_kernel<KB, VB, S::THREADS, S::MIN_CTAS, S::LIPT, S::HALO>),
                        S::THREADS, F::LIPT, F::CAP, static_cast<unsigned long>(F::SMEM_BYTES)};
-}
-// What a finish leaves over: as the several passes' entries.
-template <int KB, int VB, class W, class S = PassShape<KB, VB>>
-KernelEntry make_repair_entry() {
-    using G = PassGeom<KB, VB, S::THREADS, S::IPT>;
-    return KernelEntry{reinterpret_cast<const void*>(&finish_repair_kernel<KB, VB, W, S::THREADS, S::IPT, S::MIN_CTAS,
-                                                                           S::LOOKBACK_WINDOW>),
-                       S::THREADS, S::IPT, G::TILE, static_cast<unsigned long>(G::SMEM_BYTES)};
-}
-template <int KB, int VB>
-const KernelEntry* repair_entries_of() {
-    static const KernelEntry e[3] = {make_repair_entry<KB, VB, uint32_t>(), make_repair_entry<KB, VB, uint64_t>(),
-                                     make_repair_entry<KB, VB, uint32_t, PassShapeSmall<KB, VB>>()};
-    return e;
 }
 template <int KB>
 const KernelEntry* finish_entries_for() {

@@ -7,7 +7,6 @@ const KernelEntry* upsweep_entry_k8() { return upsweep_entry_for<8>(); }
 const KernelEntry* fused_entry_k8() { return fused_entry_for<8>(); }
 const KernelEntry* msd_entries_k8() { return msd_entries_for<8>(); }
 const KernelEntry* multi_entries_k8(int vb) { return vb == 4 ? multi_entries_of<8, 4>() : vb == 8 ? multi_entries_of<8, 8>() : multi_entries_of<8, 0>(); }
-const KernelEntry* repair_entries_k8(int vb) { return vb == 4 ? repair_entries_of<8, 4>() : vb == 8 ? repair_entries_of<8, 8>() : repair_entries_of<8, 0>(); }
 const KernelEntry* finish_entries_k8() { return finish_entries_for<8>(); }
 const KernelEntry* short_pairs_entries_k8() { return short_pairs_entries_for<8>(); }
 const KernelEntry* seg_entries_k8() { return seg_entries_for<8>(); }

@@ -59,6 +59,7 @@ struct MsdParams {
     uint32_t* joint;       // [256 << b2_max] keys per group
     uint32_t* cursor2;     // [256 << b2_max] next place of every group; its end after the second split
     uint32_t group_cap;    // largest group a local sort takes
+    RangeList left;        // groups above group_cap, sorted by a later launch
     uint2* table;          // floats: the code of every leading 12 bits (MsdEvenCode), then a sampled key of each
     uint32_t* giants;      // floats: count, then group and key of every group of equal keys above group_cap
     uint32_t* err;         // workspace error word
@@ -130,11 +131,12 @@ __global__ void __launch_bounds__(MSD_SAMPLE_THREADS) msd_sample_kernel(MsdParam
         return;
     }
     constexpr uint32_t SLOTS = 8192, NONE = 0xffffffffu;
-    __shared__ uint32_t vary[2], top, again, neighbours, bins[256], seen[SLOTS];
+    __shared__ uint32_t vary[2], top, again, fresh, neighbours, bins[256], seen[SLOTS], met[2][SLOTS / 32];
     if (tid < 2) vary[tid] = 0u;
-    if (tid == 0) top = again = neighbours = 0u;
+    if (tid == 0) top = again = fresh = neighbours = 0u;
     for (uint32_t i = tid; i < SLOTS; i += MSD_SAMPLE_THREADS) seen[i] = NONE;
-    if (tid < 256) bins[tid] = 0u;
+    if (tid < 256) bins[tid] = met[0][tid] = met[1][tid] = 0u;
+    static_assert(SLOTS / 32 == 256, "two bits a slot");
     __syncthreads();
     const KeyMap<U> map(p.kind, p.desc);
     const U* keys = static_cast<const U*>(p.keys_in);
@@ -168,33 +170,44 @@ __global__ void __launch_bounds__(MSD_SAMPLE_THREADS) msd_sample_kernel(MsdParam
     // 2^24 16-byte ones 0.62 and 2.41)
     const uint32_t close = __popc(__ballot_sync(0xffffffffu, ((x[0] ^ y) << skip) >> 56 == 0u));
     if ((tid & 31) == 0) atomicAdd(&neighbours, close);
-    uint32_t most = 0, twice = 0;
+    uint32_t most = 0, twice = 0, distinct = 0;
 #pragma unroll
     for (int i = 0; i < PER; ++i) {
         const uint32_t c = uint32_t((x[i] << skip) >> 32);
         most = max(most, c);
-        atomicAdd(&bins[c >> 24], 1u);
-        // codes met before in the sample (open addressing, half full at most)
+        // Codes met before in the sample (open addressing, half full at most):
+        // those met twice, not oftener, are counted, and none counts again in its
+        // digit: a few very frequent keys are no matter, their groups are sorted
+        // apart.
         uint32_t h = (c * 2654435761u) >> 19;
+        bool first_met = true;
         for (int probe = 0; probe < 64 && c != NONE; ++probe) {
             uint32_t v = seen[h];
             if (v == NONE) v = atomicCAS(&seen[h], NONE, c);
             if (v == NONE) break;
             if (v == c) {
-                ++twice;
+                first_met = false;
+                const uint32_t bit = 1u << (h & 31u);
+                if (!(atomicOr(&met[0][h >> 5], bit) & bit)) ++twice;
+                else if (!(atomicOr(&met[1][h >> 5], bit) & bit)) --twice;
                 break;
             }
             h = (h + 1u) & (SLOTS - 1u);
         }
+        if (first_met) atomicAdd(&bins[c >> 24], 1u);
+        distinct += first_met;
     }
     twice = __reduce_add_sync(0xffffffffu, twice);
+    distinct = __reduce_add_sync(0xffffffffu, distinct);
     if ((tid & 31) == 0 && twice) atomicAdd(&again, twice);
+    if ((tid & 31) == 0) atomicAdd(&fresh, distinct);
     most = __reduce_max_sync(0xffffffffu, most);
     if ((tid & 31) == 0) atomicMax(&top, most);
     __syncthreads();
-    // a top digit with five times its share has groups that do not fit, and
-    // codes that repeat more than 64 times (S keys of D distinct codes meet
-    // S * S / 2 D of them again) crowd the local sorts' sub-buckets
+    // a top digit with five times its share has groups that do not fit, as have
+    // very frequent keys of more than a quarter of the array, and codes that
+    // repeat more than 64 times (S keys of D distinct codes meet S * S / 2 D of
+    // them again) crowd the local sorts' sub-buckets
     const bool uneven = __syncthreads_or(tid < 256 && bins[tid] > MSD_SAMPLE_THREADS * PER / 256 * 5);
     if (tid == 0) {
         // the codes reach `top`: groups beyond it stay empty
@@ -203,7 +216,7 @@ __global__ void __launch_bounds__(MSD_SAMPLE_THREADS) msd_sample_kernel(MsdParam
         while (b2 < uint32_t(p.b2_max) && n > 0.72f * cap * float(1u << b2)) ++b2;
         constexpr float S = MSD_SAMPLE_THREADS * PER;
         const bool crowded = again >= 16u && 2.f * float(again) * n > 64.f * S * S;
-        if (uneven || crowded || (KB == 4 && 2u * neighbours > uint32_t(MSD_SAMPLE_THREADS)) || n > cap * float(1u << b2)) *p.state = MSD_OFF;
+        if (uneven || crowded || 4u * fresh < 3u * uint32_t(S) || (KB == 4 && 2u * neighbours > uint32_t(MSD_SAMPLE_THREADS)) || n > cap * float(1u << b2)) *p.state = MSD_OFF;
         p.window[0] = skip;
         p.window[1] = b2;
     }
@@ -576,6 +589,17 @@ __global__ void __launch_bounds__(256) msd_scan_kernel(MsdParams p) {
                     p.giants[1 + 2 * i] = (b << b2) + tid;
                     p.giants[2 + 2 * i] = reinterpret_cast<const uint32_t*>(p.table + MsdEvenCode::BINS)[lo];
                 }
+            }
+        }
+    }
+    if constexpr (!EVEN) {
+        if (!fits) {  // left to be sorted by itself, while such groups are a quarter of the array at most
+            const uint32_t i = atomicAdd(p.left.count, 1u), all = atomicAdd(p.left.count + 1, c) + c;
+            if (i < p.left.most && all <= uint32_t(p.n / 4)) {
+                p.left.ranges[2 * i] = base + e2;
+                p.left.ranges[2 * i + 1] = c;
+                atomicOr(p.state, MSD_RANGES);
+                fits = true;
             }
         }
     }
@@ -1398,7 +1422,8 @@ __global__ void __launch_bounds__(THREADS, MIN_CTAS) msd_local_kernel(MsdParams 
             }
         } else if (ahead < groups()) {
             r.off = ahead ? p.cursor2[ahead - 1u] : 0u;
-            r.word = (p.cursor2[ahead] - r.off) | (8u + code_of.b2) << 16;
+            // (above the largest: one of the ranges left)
+            r.word = min(p.cursor2[ahead] - r.off, 0xffffu) | (8u + code_of.b2) << 16;
         }
         ahead += gridDim.x;
         return r;
@@ -1429,6 +1454,7 @@ __global__ void __launch_bounds__(THREADS, MIN_CTAS) msd_local_kernel(MsdParams 
         while (cur.word != 0u) {
             const Group later = next_group();
             const uint32_t off = cur.off, cnt = cur.cnt();
+            const bool some = cnt - 1u < p.group_cap;
             {
                 const uintptr_t a = reinterpret_cast<uintptr_t>(keys + later.off) & ~uintptr_t(127);
                 const uintptr_t e = reinterpret_cast<uintptr_t>(keys + later.off + later.cnt());
@@ -1438,7 +1464,7 @@ __global__ void __launch_bounds__(THREADS, MIN_CTAS) msd_local_kernel(MsdParams 
             const uint32_t skew = skew_of(off, 16), pad = skew_of(off, 32);
             U* dst = keys + off - pad;  // place q goes to dst[q]
             bool sorted = true;
-            if (cnt != 0u)
+            if (some)
                 sorted = group_sort<U, THREADS, HALO>(
                     k, cnt, skew, pad, smem,
                     SubBucket<Code>{code_of, cur.word >> 16, uint32_t(G::BINS)},
@@ -1507,7 +1533,7 @@ __global__ void __launch_bounds__(THREADS, MIN_CTAS) msd_local_kernel(MsdParams 
                     __syncthreads();
                 }
             }
-            if (!sorted || cnt == 0u) load(next);
+            if (!sorted || !some) load(next);
             cur = next;
             next = later;
         }
@@ -1540,6 +1566,21 @@ __global__ void __launch_bounds__(THREADS, MIN_CTAS) msd_local_kernel(MsdParams 
             }
             if (__syncthreads_or(d) && tid == 0) atomicOr(p.state, MSD_GAVE_UP);
         }
+    }
+}
+
+// The groups above the largest, mapped back unsorted: only where the launch that
+// sorts them is refused, and the digit passes sort everything instead.
+template <int KB>
+__global__ void __launch_bounds__(256) msd_map_ranges_kernel(MsdParams p) {
+    using U = typename KeyBits<KB>::U;
+    if (ld_relaxed(p.state) & MSD_OFF) return;
+    const KeyMap<U> map(p.kind, p.desc);
+    const uint32_t ranges = min(ld_relaxed(p.left.count), p.left.most);
+    for (uint32_t i = 0; i < ranges; ++i) {
+        U* keys = static_cast<U*>(p.keys_a) + p.left.ranges[2 * i];
+        for (uint32_t j = blockIdx.x * 256 + threadIdx.x; j < p.left.ranges[2 * i + 1]; j += gridDim.x * 256)
+            keys[j] = map.out(keys[j]);
     }
 }
 

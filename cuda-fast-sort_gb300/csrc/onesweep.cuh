@@ -71,7 +71,7 @@ __global__ void __launch_bounds__(HIST_THREADS, 1) upsweep_kernel(HistParams p) 
     grid_launch_dependents();  // the first pass may be scheduled; it waits for this grid
     if (p.msd_state) {  // the digit passes' histogram after the MSD kernels
         grid_dependency_wait();
-        if (ld_relaxed(p.msd_state) == 0u) return;
+        if (!(ld_relaxed(p.msd_state) & MSD_PASSES)) return;
     }
 
     // Fused clears / copies that must precede the first pass.
@@ -739,76 +739,8 @@ __global__ void __launch_bounds__(THREADS, MIN_CTAS) onesweep_pass_kernel(PassPa
     // successor never holds slots a CTA of this pass still needs.
     grid_launch_dependents();
     grid_dependency_wait();
-    if (p.msd_state && ld_relaxed(p.msd_state) == 0u) return;  // the MSD kernels sorted
+    if (p.msd_state && !(ld_relaxed(p.msd_state) & MSD_PASSES)) return;  // the MSD kernels sorted
     onesweep_pass_body<KB, VB, W, THREADS, IPT, SEG, LBW>(p, smem, p.pass);
-}
-
-__device__ __forceinline__ void grid_copy_bytes(void* dst, const void* src, uint64_t bytes);
-
-// Digits p.pass .. p.passes - 1 in one cooperative launch, a grid barrier
-// between the passes that run, then the parity fix-up.  Used where most passes
-// do not run (a launch that exits costs about 2.2 us, a barrier with the next
-// pass's start about 2 us more than a launch that overlaps its predecessor's
-// end: eight passes of 65537 8-byte keys with three that run 44 against 47 us,
-// four that all run 55 against 47).
-template <int KB, int VB, class W, int THREADS, int IPT, int MIN_CTAS, int LBW>
-__global__ void __launch_bounds__(THREADS, MIN_CTAS) onesweep_multi_kernel(PassParams p) {
-    using G = PassGeom<KB, VB, THREADS, IPT>;
-    extern __shared__ __align__(128) uint8_t smem[];
-    if constexpr (!G::HALF && rank_uses_or(IPT)) {
-        uint32_t* match_scratch = reinterpret_cast<uint32_t*>(smem + G::MATCH_OFF);
-        for (int i = threadIdx.x; i < G::WARPS * 256; i += THREADS) match_scratch[i] = 0u;
-    }
-    grid_launch_dependents();
-    grid_dependency_wait();
-    if (p.msd_state && (ld_relaxed(p.msd_state) & p.state_mask) == 0u) return;  // sorted already
-    uint32_t left_out = 0;  // digits below the leading ones
-    if (p.leading && !(ld_relaxed(p.leading) & MSD_OFF)) left_out = (1u << ld_relaxed(p.leading + 1)) - 1u;
-    const uint32_t uniform = left_out | pass_mask(p, p.n, reinterpret_cast<uint32_t*>(smem + G::SKIP_OFF));
-    const uint32_t all = (p.passes >= 32) ? 0xffffffffu : ((1u << p.passes) - 1u);
-    const int total = __popc(~uniform & all);
-    const bool to_b = !p.copy_keys_in && (total & 1) != 0;  // where the last pass leaves the result
-    const bool move = left_out == 0u && (p.copy_keys_in ? total == 0 : (total & 1) != p.want_odd);
-    auto offsets = [&](int pass) {  // the pass's digit offsets
-        const int tid = threadIdx.x;
-        const unsigned long long c = (tid < 256) ? p.gp_all[size_t(pass) * 256 + tid] : 0ull;
-        const unsigned long long ex = block_exclusive_scan_256<unsigned long long>(
-            c, reinterpret_cast<unsigned long long*>(smem + G::SCAN64_OFF), nullptr);
-        if (tid < 256) reinterpret_cast<unsigned long long*>(smem + G::GEXCL_OFF)[tid] = ex;
-    };
-    uint32_t barriers = 0;
-    if (p.clear_bytes) {
-        uint4* st = static_cast<uint4*>(p.status);
-        for (uint64_t i = uint64_t(blockIdx.x) * THREADS + threadIdx.x; i < p.clear_bytes / 16;
-             i += uint64_t(gridDim.x) * THREADS)
-            st[i] = make_uint4(0, 0, 0, 0);
-        if (!grid_barrier(p.barrier, p.barrier_gen, ++barriers, p.wait_limit_ns, p.err)) return;
-    }
-    uint32_t runs = ~uniform & all;
-    if (runs) offsets(__ffs(runs) - 1);
-    while (runs) {
-        const int pass = __ffs(runs) - 1;
-        runs &= runs - 1u;
-        if (!onesweep_pass_body<KB, VB, W, THREADS, IPT, false, LBW, true>(p, smem, pass, uniform, left_out == 0u))
-            return;
-        if (runs || move) {  // another pass, or the fix-up
-            __syncthreads();
-            if (threadIdx.x < 3) mbar_inval(reinterpret_cast<uint64_t*>(smem + G::MBAR_OFF) + threadIdx.x);
-            if (runs) offsets(__ffs(runs) - 1);
-            // the next pass's bulk copies read what the CTAs stored
-            fence_proxy_async_all();
-            if (!grid_barrier(p.barrier, p.barrier_gen, ++barriers, p.wait_limit_ns, p.err)) return;
-            fence_proxy_async_all();
-        }
-    }
-    if (move) {
-        const bool copied = p.copy_keys_in != nullptr;
-        const void* ks = copied ? p.copy_keys_in : to_b ? p.keys_b : p.keys_a;
-        const void* vs = copied ? p.copy_vals_in : to_b ? p.vals_b : p.vals_a;
-        const bool to_a = to_b || copied;
-        grid_copy_bytes(to_a ? p.keys_a : p.keys_b, ks, p.n * uint64_t(KB));
-        if constexpr (VB > 0) grid_copy_bytes(to_a ? p.vals_a : p.vals_b, vs, p.n * uint64_t(VB));
-    }
 }
 
 // Copies `bytes` from src to dst with all threads of the grid (16-byte
@@ -836,7 +768,7 @@ __device__ __forceinline__ void grid_copy_bytes(void* dst, const void* src, uint
 // in the other buffer than the one it belongs in (in place: an odd count
 // left it in the alternate buffer); copy it across.  Otherwise nothing to do.
 __device__ __forceinline__ void fixup_body(const FixupParams& f) {
-    if (f.msd_state && ld_relaxed(f.msd_state) == 0u) return;  // the MSD kernels sorted
+    if (f.msd_state && !(ld_relaxed(f.msd_state) & MSD_PASSES)) return;  // the MSD kernels sorted
     // the executed pass kernels left their count; none ran when the word is 0
     const uint32_t w = *f.executed;
     const int executed = (w >> 31) ? int(w & 0xFFu) : 0;

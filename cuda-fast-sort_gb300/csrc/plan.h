@@ -8,6 +8,7 @@
 #include <cuda_runtime.h>
 
 #include "shapes.h"
+#include "sort_params.h"
 
 namespace gbsort {
 
@@ -31,7 +32,8 @@ struct CtlLayout {
     // Sorts by leading digits use the fill counts' words, which only the
     // one-launch sort needs: a second set of tile counters [16] and a second grid
     // barrier [2], for the digit passes after them, the sample's ticket and
-    // [FINISH_LEVELS + 2] counts, and the number of ranges left to sort.
+    // [FINISH_LEVELS + 2] counts, and the number and the total of the ranges left
+    // to sort (keys-only sorts above the short range, too).
     size_t counters2_off = 0;
     size_t sampled_off = 0;
     size_t ranges_off = 0;
@@ -111,11 +113,11 @@ struct Plan {
     // the digit passes in one launch, after (or, by leading digits, in) a path
     // that seldom needs all of them
     KernelEntry multi{};
+    KernelEntry after{};  // the same after a path that may have left ranges to sort
     // sorts by leading digits (finish.cuh): sample, edges,
     // finish; the edges lie in the status words
     bool finish = false;
     KernelEntry finish_k[3]{};
-    KernelEntry repair{};  // then: what the finish leaves over (repair.cuh)
     // short key-value arrays in one launch (short_pairs.cuh): that kernel, the
     // digit passes after it, its regions, the words in each, and their place, at
     // the end of the workspace (their fill counts lie in the status words, which
@@ -133,6 +135,11 @@ struct Plan {
     // thread changes them
     bool skip = false;       // uniform-digit pass skipping
     bool short_msd = false;  // most significant digit first inside the one-launch sort
+
+    uint32_t ranges_most() const {  // room in the list of ranges left to sort
+        const size_t most = status_bytes / 64;
+        return num_tiles < 4 ? 0u : uint32_t(most < RANGES_MOST ? most : RANGES_MOST);
+    }
 };
 
 // Fills *plan; returns a gbsort_status code.

@@ -36,6 +36,7 @@
 #include "finish.cuh"
 #include "fused_short.cuh"
 #include "msd.cuh"
+#include "multi.cuh"
 #include "onesweep.cuh"
 #include "short_pairs.cuh"
 #include "sort_params.h"
@@ -63,8 +64,6 @@ const KernelEntry* short_pairs_entries_k8();
 const KernelEntry* multi_entries_k4();  // keys only
 const KernelEntry* multi_entries_k8(int vb);
 const KernelEntry* multi_entries_k16(int vb);
-const KernelEntry* repair_entries_k8(int vb);
-const KernelEntry* repair_entries_k16(int vb);
 const KernelEntry* finish_entries_k8();
 const KernelEntry* finish_entries_k16();
 const KernelEntry* msd_entries_k4();
@@ -392,7 +391,7 @@ int make_plan(int key_type, size_t value_bytes, uint64_t n, Plan* plan) {
             off = align_up(off + MsdLayout::BYTES, 256);
         }
         if (g_msd.load(std::memory_order_relaxed) &&
-            (p.msd_block || (even ? MsdLayout::even_bytes(p.msd_b2) : MsdLayout::bytes(p.msd_b2)) <= p.status_bytes)) {
+            (p.msd_block || (even ? MsdLayout::even_bytes(p.msd_b2) : MsdLayout::bytes(p.msd_b2)) + 8 * size_t(RANGES_MOST) <= p.status_bytes)) {
             p.msd = true;
             p.msd_even = even;
             const KernelEntry* e = even ? msd_even_entries_k4() : msd_entries(p.kb);
@@ -419,12 +418,15 @@ int make_plan(int key_type, size_t value_bytes, uint64_t n, Plan* plan) {
         p.finish_k[0] = e[0];
         p.finish_k[1] = e[1];
         p.finish_k[2] = e[p.vb == 4 ? 2 : p.vb == 8 ? 3 : 4];
-        p.repair = (p.kb == 8 ? repair_entries_k8(p.vb) : repair_entries_k16(p.vb))[small ? 2 : p.wide_status ? 1 : 0];
     }
-    if (p.msd || p.finish)
-        p.multi = (p.kb == 4   ? multi_entries_k4()
-                   : p.kb == 8 ? multi_entries_k8(p.vb)
-                               : multi_entries_k16(p.vb))[small ? 2 : p.wide_status ? 1 : 0];
+    if (p.msd || p.finish) {
+        const KernelEntry* e = p.kb == 4   ? multi_entries_k4()
+                               : p.kb == 8 ? multi_entries_k8(p.vb)
+                                           : multi_entries_k16(p.vb);
+        const int shape = small ? 2 : p.wide_status ? 1 : 0;
+        p.multi = e[shape];
+        p.after = e[p.msd_even ? shape : 3 + shape];  // (4-byte floats leave none)
+    }
     p.total_bytes = off;
     *plan = p;
     return GBSORT_OK;
@@ -470,11 +472,12 @@ int enqueue_sort(const Plan& plan, int descending, void* d_keys, void* d_values,
     // (its digit passes run in one launch, which sort_timed does not use)
     bool use_finish = plan.finish && ms == nullptr;
     for (int i = 0; use_finish && i < 3; ++i) use_finish = prepare_kernel(plan.finish_k[i]) == GBSORT_OK;
-    use_finish = use_finish && prepare_kernel(plan.multi) == GBSORT_OK && prepare_kernel(plan.repair) == GBSORT_OK;
+    use_finish = use_finish && prepare_kernel(plan.multi) == GBSORT_OK && prepare_kernel(plan.after) == GBSORT_OK;
     // the most-significant-first path of keys-only sorts runs when all its
     // kernels can
     bool use_msd = plan.msd && !use_finish;
     for (int i = 0; use_msd && i < 6; ++i) use_msd = prepare_kernel(plan.msd_k[i]) == GBSORT_OK;
+    use_msd = use_msd && prepare_kernel(plan.after) == GBSORT_OK;
     // its kernels are timed one by one where the plan reports them (then the
     // digits' histogram is the last of six stages), else as part of entry 0
     const int ms_stages = use_msd && plan.msd_block ? 6 : 0;
@@ -521,6 +524,13 @@ int enqueue_sort(const Plan& plan, int descending, void* d_keys, void* d_values,
                            prepare_kernel(plan.short_k[1]) == GBSORT_OK;
     uint32_t* msd_state = use_msd || use_finish || use_short ? reinterpret_cast<uint32_t*>(ctl + plan.ctl.msd_state_off) : nullptr;
 
+    // the list of ranges left to sort lies at the end of the status words, beyond
+    // what passes over half of the array use
+    RangeList left{};
+    left.most = plan.ranges_most();
+    left.count = reinterpret_cast<uint32_t*>(ctl + plan.ctl.ranges_off);
+    left.ranges = reinterpret_cast<uint32_t*>(static_cast<uint8_t*>(status) + plan.status_bytes) - 2 * left.most;
+
     // Parameters of digit pass `pass` and of the fix-up copy.
     auto pass_params = [&](int pass) {
         // Even passes read the user's buffer unless the mirror made the
@@ -558,7 +568,7 @@ int enqueue_sort(const Plan& plan, int descending, void* d_keys, void* d_values,
         pp.copy_vals_in = copy ? vals_src : nullptr;
         pp.executed = fixup ? reinterpret_cast<uint32_t*>(ctl + plan.ctl.exec_off) : nullptr;
         pp.msd_state = use_msd ? msd_state : nullptr;
-        pp.state_mask = MSD_OFF | MSD_GAVE_UP;
+        pp.state_mask = MSD_PASSES | MSD_RANGES;
         pp.leading = use_finish ? msd_state : nullptr;
         pp.want_odd = alt ? (plan.passes & 1) : 0;
         pp.barrier = reinterpret_cast<uint32_t*>(ctl + plan.ctl.barrier_off);
@@ -697,18 +707,19 @@ int enqueue_sort(const Plan& plan, int descending, void* d_keys, void* d_values,
     const uint32_t pass_ctas = uint32_t(plan.num_tiles < max_ctas ? plan.num_tiles : max_ctas);
     // every digit pass in one cooperative launch, where most often none or few
     // of them run
-    auto launch_passes = [&](const PassParams& pp) {
-        const int occ_m = resident_ctas(plan.multi);
+    auto launch_passes = [&](const KernelEntry& k, const PassParams& pp) {
+        const int occ_m = resident_ctas(k);
         const uint64_t most = uint64_t(sms) * uint64_t(occ_m > 0 ? occ_m : 1);
         PassParams q = pp;
         void* args[] = {&q};
         const cudaError_t r =
-            cudaLaunchCooperativeKernel(plan.multi.fn, dim3(uint32_t(plan.num_tiles < most ? plan.num_tiles : most)),
-                                        dim3(plan.multi.threads), args, plan.multi.smem, stream);
+            cudaLaunchCooperativeKernel(k.fn, dim3(uint32_t(plan.num_tiles < most ? plan.num_tiles : most)),
+                                        dim3(k.threads), args, k.smem, stream);
         if (r != cudaSuccess) cudaGetLastError();
         return r;
     };
     FinishParams fin{};
+    MsdParams mp{};
     auto launch_finish = [&](int i, uint64_t grid) {
         const KernelEntry& k = plan.finish_k[i];
         const uint64_t full = uint64_t(sms > 0 ? sms : 1) * uint64_t(resident_ctas(k) > 0 ? resident_ctas(k) : 1);
@@ -734,12 +745,8 @@ int enqueue_sort(const Plan& plan, int descending, void* d_keys, void* d_values,
         fin.ticket = reinterpret_cast<uint32_t*>(ctl + plan.ctl.sampled_off);
         fin.sampled = fin.ticket + 1;
         fin.edges = static_cast<uint32_t*>(status);
-        // the status words hold the edges from their start and the list of ranges
-        // at their end, beyond what the passes over half of the array use
-        fin.left.most = plan.num_tiles < 4 ? 0 : uint32_t(std::min<size_t>(RANGES_MOST, plan.status_bytes / 64));
-        fin.left.count = reinterpret_cast<uint32_t*>(ctl + plan.ctl.ranges_off);
-        fin.left.ranges = reinterpret_cast<uint32_t*>(static_cast<uint8_t*>(status) + plan.status_bytes) - 2 * fin.left.most;
-        fin.max_chunks = uint32_t(std::min<size_t>((plan.status_bytes - 8 * size_t(fin.left.most)) / 8 - 2, 0x7fffffff));
+        fin.left = left;
+        fin.max_chunks = uint32_t(std::min<size_t>((plan.status_bytes - 8 * size_t(left.most)) / 8 - 2, 0x7fffffff));
         fin.seen = fin.edges + fin.max_chunks + 2;
         fin.places = uint32_t(plan.finish_k[2].tile);
         fin.err = err_word;
@@ -757,7 +764,6 @@ int enqueue_sort(const Plan& plan, int descending, void* d_keys, void* d_values,
         // when these sorted, and otherwise sort from the input-preserving
         // source or from the caller's buffer, which then holds the input's
         // keys in some order (keys only: the same bytes come out).
-        MsdParams mp{};
         mp.keys_in = copy ? keys_src : d_keys;
         mp.keys_a = d_keys;
         mp.keys_b = alt_keys;
@@ -780,6 +786,8 @@ int enqueue_sort(const Plan& plan, int descending, void* d_keys, void* d_values,
             mp.table = reinterpret_cast<uint2*>(even + MsdLayout::GIANTS_BYTES);
         }
         mp.group_cap = plan.msd_group_cap;
+        mp.left = left;
+        if (timed || !skip) mp.left.most = 0;  // (they are sorted by the launch of all digit passes only)
         mp.err = err_word;
         for (int i = 0; i < 6; ++i) {
             const KernelEntry& k = plan.msd_k[i];
@@ -808,13 +816,34 @@ int enqueue_sort(const Plan& plan, int descending, void* d_keys, void* d_values,
     if (timed) cudaEventRecord(ev[1 + ms_stages], stream);
 
     // a refused launch: every digit pass below, each in a launch of its own
-    if (use_finish && launch_passes(pass_params(0)) != cudaSuccess) use_finish = false;
+    if (use_finish && launch_passes(plan.multi, pass_params(0)) != cudaSuccess) use_finish = false;
     // After the MSD kernels one launch looks at their state where P passes and
     // the fix-up each did (an exit is 2.2 us: 50M u64 keys 957 -> 948 us, 2^26
     // u128 ones 1754 -> 1735); timed, and without skipping, each pass has its own.
-    if (use_msd && !timed && skip && prepare_kernel(plan.multi) == GBSORT_OK &&
-        launch_passes(pass_params(0)) == cudaSuccess)
-        return GBSORT_OK;  // (the fix-up is part of that launch)
+    if (use_msd && !timed && skip) {
+        PassParams pp = pass_params(0);
+        pp.left = left;
+        pp.left.twiddled = 1;
+        if (launch_passes(plan.after, pp) == cudaSuccess) return GBSORT_OK;  // (the fix-up is part of that launch)
+        // A refused launch: ranges that the local sorts have left depend on it,
+        // so every digit pass runs, each in a launch of its own, from what the
+        // caller's buffer holds (any order of the input sorts to the same bytes).
+        static_assert((0x02020202u & MSD_PASSES) != 0u, "the state as the digit passes read it");
+        e = cudaSuccess;
+        if (!plan.msd_even) {
+            void* margs[] = {&mp};
+            const KernelEntry& k = msd_entries(plan.kb)[7];
+            e = cudaLaunchKernel(k.fn, dim3(uint32_t(sms > 0 ? sms : 1)), dim3(k.threads), margs, 0, stream);
+        }
+        if (e == cudaSuccess) e = cudaMemsetAsync(msd_state, 2, 4, stream);
+        if (e == cudaSuccess) e = cudaMemsetAsync(gp, 0, size_t(plan.passes) * 256 * 8, stream);
+        HistParams again = hp;
+        void* hargs[] = {&again};
+        if (e == cudaSuccess)
+            e = cudaLaunchKernel(plan.upsweep.fn, dim3(hist_ctas), dim3(plan.upsweep.threads), hargs, plan.upsweep.smem,
+                                 stream);
+        if (e != cudaSuccess) return fail("upsweep launch", e);
+    }
     for (int pass = 0; pass < plan.passes && !use_finish; ++pass) {
         PassParams pp = pass_params(pass);
         void* args[] = {&pp};
@@ -829,14 +858,14 @@ int enqueue_sort(const Plan& plan, int descending, void* d_keys, void* d_values,
         if (e != cudaSuccess) return fail("finish launch", e);
         PassParams pp = pass_params(0);
         pp.msd_state = msd_state;
+        pp.state_mask = MSD_GAVE_UP | MSD_RANGES;
+        pp.leading = nullptr;
+        pp.left = left;
         pp.tile_counter = reinterpret_cast<uint32_t*>(ctl + plan.ctl.counters2_off);
         pp.barrier = pp.tile_counter + 16;
         pp.barrier_gen = pp.barrier + 1;
         pp.clear_bytes = plan.status_bytes;
-        const uint64_t most = uint64_t(sms) * uint64_t(resident_ctas(plan.repair));
-        void* rargs[] = {&pp, &fin.left};
-        e = cudaLaunchCooperativeKernel(plan.repair.fn, dim3(uint32_t(plan.num_tiles < most ? plan.num_tiles : most)),
-                                        dim3(plan.repair.threads), rargs, plan.repair.smem, stream);
+        e = launch_passes(plan.after, pp);
         if (e != cudaSuccess) return fail("pass launch", e);
         return GBSORT_OK;  // (the fix-up is part of those launches; nothing is timed)
     }

@@ -8,15 +8,17 @@ namespace gbsort {
 // Why the digit passes sort after the most-significant-first path of a
 // keys-only sort (msd.cuh; 0: that path sorts): MSD_OFF some group is too big
 // (decided before any key moves), MSD_GAVE_UP a local sort gave up.
-// MSD_RANGES: some ranges are left to sort (finish.cuh).
+// MSD_RANGES: some ranges are left to sort (multi.cuh).
 constexpr uint32_t MSD_OFF = 1u, MSD_GAVE_UP = 2u, MSD_RANGES = 4u;
+constexpr uint32_t MSD_PASSES = MSD_OFF | MSD_GAVE_UP;  // the digit passes sort everything
 
-// Ranges of the result that a sort by leading digits leaves to sort: a list in
-// no order, of first pair and length.
+// Ranges of the result that a path leaves to sort: a list in no order, of first
+// place and length.
 struct RangeList {
-    uint32_t* count;     // zeroed with the control block
+    uint32_t* count;     // [2] their number, and (keys alone) their total; zeroed with the control block
     uint32_t* ranges;    // [2 * most]
     uint32_t most;
+    int twiddled;        // their keys are not mapped back yet
 };
 constexpr uint32_t RANGES_MOST = 1024;
 
@@ -106,6 +108,7 @@ struct PassParams {
     uint32_t* barrier;          // grid barrier counter and generation, zeroed
     uint32_t* barrier_gen;
     uint64_t clear_bytes;       // status words to clear first (they hold an earlier run's)
+    RangeList left;             // MSD_RANGES
 };
 
 // The copy home after uniform-pass skipping left an odd number of executed

@@ -89,3 +89,14 @@ def test_few_keys_of_very_many(gb, cuda, oracle):
     outcome_of(gb, cuda, oracle, "u64", raw, 4)
     outcome_of(gb, cuda, oracle, "u64", raw, 8, True, "copy")
     outcome_of(gb, cuda, oracle, "u64", raw, 4, False, "buffers")
+
+
+@pytest.mark.parametrize("kt,n", [("u32", 3_000_001), ("i32", 12_000_017), ("u64", 2_500_001), ("i64", 26_000_003),
+                                  ("u128", 1_200_007), ("i128", 5_000_011)])
+@pytest.mark.parametrize("shares", [(0.01,), (0.002, 0.03, 0.1), tuple([0.003] * 50)])
+def test_heavy_keys_alone(gb, cuda, oracle, kt, n, shares):
+    """Groups beyond a local sort: they are sorted by themselves, in all three
+    forms of the call."""
+    raw = heavy(kt, n, n % 89, shares)
+    for api, desc in (("inplace", False), ("copy", True), ("buffers", False)):
+        assert outcome_of(gb, cuda, oracle, kt, raw, 0, desc, api) == gb.OUTCOME_RANGES
