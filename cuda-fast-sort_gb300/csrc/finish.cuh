@@ -75,7 +75,7 @@ constexpr int finish_levels() { return KB - 1 < FINISH_LEVELS ? KB - 1 : FINISH_
 constexpr float FINISH_REPEATS = 12.f;
 
 template <int KB>
-__global__ void __launch_bounds__(FINISH_SAMPLE_THREADS) finish_sample_kernel(FinishParams p) {
+__global__ void __launch_bounds__(FINISH_SAMPLE_THREADS, 1) finish_sample_kernel(FinishParams p) {
     using U = typename KeyBits<KB>::U;
     constexpr int LEVELS = finish_levels<KB>();
     extern __shared__ __align__(16) uint32_t cnt[];
@@ -105,6 +105,7 @@ __global__ void __launch_bounds__(FINISH_SAMPLE_THREADS) finish_sample_kernel(Fi
     __syncthreads();
     U d = 0;
     uint32_t pairs = 0, again = 0, more = 0;  // again, more: prefixes met for the second time, or oftener
+    uint32_t at[MOST];
 #pragma unroll
     for (int i = 0; i < MOST; ++i) {
         if (i >= per) break;
@@ -116,10 +117,17 @@ __global__ void __launch_bounds__(FINISH_SAMPLE_THREADS) finish_sample_kernel(Fi
         h = (h ^ (h >> 30)) * 0xBF58476D1CE4E5B9ull;
         h = (h ^ (h >> 27)) * 0x94D049BB133111EBull;
         h ^= h >> 31;
-        const uint32_t tag = uint32_t(h >> 32) & 0xffff8000u;
-        uint32_t slot = uint32_t(h) & 32767u;
+        at[i] = (uint32_t(h >> 32) & 0xffff8000u) | (uint32_t(h) & 32767u);  // tag | slot
+    }
+    uint32_t there[MOST];  // (every key's first look at once)
+#pragma unroll
+    for (int i = 0; i < MOST; ++i) there[i] = i < per ? cnt[at[i] & 32767u] : 0u;
+#pragma unroll
+    for (int i = 0; i < MOST; ++i) {
+        if (i >= per) break;
+        const uint32_t tag = at[i] & 0xffff8000u;
+        uint32_t slot = at[i] & 32767u, w = there[i];
         for (int probe = 0; probe < 128; ++probe) {
-            uint32_t w = cnt[slot];  // (one atomic a key where all share a prefix)
             if (w == 0u) w = atomicCAS(&cnt[slot], 0u, tag | 1u);
             if (w == 0u) break;
             if ((w & 0xffff8000u) == tag) {
@@ -130,6 +138,7 @@ __global__ void __launch_bounds__(FINISH_SAMPLE_THREADS) finish_sample_kernel(Fi
                 break;
             }
             slot = (slot + 1u) & 32767u;
+            w = cnt[slot];
         }
     }
     uint32_t bytes = 0;  // bit q: byte q differs somewhere
@@ -181,7 +190,9 @@ __global__ void __launch_bounds__(FINISH_SAMPLE_THREADS) finish_sample_kernel(Fi
     // are one key's keep their order instead, so that few may be of more (2 x
     // 10^7 u64 + u32 in 40 copies 0.90 ms; two bytes fit, but leave every window
     // crowded).
-    const float fits = (p.kind == KIND_FLOAT ? 0.4f : 0.84f) * places;
+    // 16-byte keys' windows hold half as many: a pass more is cheaper than windows
+    // half full (2^25 u128 + u32: three bytes 2.03 ms, two, groups of 512, 2.07).
+    const float fits = (p.kind == KIND_FLOAT ? 0.4f : KB == 16 ? 0.36f : 0.84f) * places;
     int lo = 0;
     float group = 0.f, unlike = 0.f;  // unlike: its pairs of different keys
     bool chosen = false;
