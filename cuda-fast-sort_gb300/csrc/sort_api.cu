@@ -145,6 +145,17 @@ std::atomic<int> g_msd{[] {
     const char* v = std::getenv("GBSORT_MSD");
     return (v && v[0] == '0') ? 0 : 1;
 }()};
+// Short key-value arrays in one launch (short_pairs.cuh), and sorts by leading
+// digits (finish.cuh): on unless GBSORT_SHORT_PAIRS=0, GBSORT_LEADING_DIGITS=0 or
+// switched off.
+std::atomic<int> g_short_pairs{[] {
+    const char* v = std::getenv("GBSORT_SHORT_PAIRS");
+    return (v && v[0] == '0') ? 0 : 1;
+}()};
+std::atomic<int> g_leading{[] {
+    const char* v = std::getenv("GBSORT_LEADING_DIGITS");
+    return (v && v[0] == '0') ? 0 : 1;
+}()};
 // Uniform-digit pass skipping: on unless GBSORT_PASS_SKIP=0 or switched off.
 std::atomic<int> g_pass_skip{[] {
     const char* v = std::getenv("GBSORT_PASS_SKIP");
@@ -405,14 +416,14 @@ int make_plan(int key_type, size_t value_bytes, uint64_t n, Plan* plan) {
         p.short_regions = short_regions;
         p.short_cap = short_pairs_room(p.kb, n, short_regions);
         off = align_up(off + size_t(short_regions) * p.short_cap * 2 * kb, 256);
-        if (p.skip) {
+        if (p.skip && g_short_pairs.load(std::memory_order_relaxed)) {
             p.short_pairs = true;
             const KernelEntry* e = p.kb == 4 ? short_pairs_entries_k4() : short_pairs_entries_k8();
             p.short_k[0] = e[p.vb == 4 ? 0 : 2];
             p.short_k[1] = e[p.vb == 4 ? 1 : 3];
         }
     }
-    if (finish && p.skip) {
+    if (finish && p.skip && g_leading.load(std::memory_order_relaxed)) {
         p.finish = true;
         const KernelEntry* e = finish_entries(p.kb);
         p.finish_k[0] = e[0];
@@ -930,14 +941,14 @@ int check_args(int key_type, size_t value_bytes, void* d_keys, void* d_values, s
 // graph, if any, is destroyed; one still running is freed by CUDA when it
 // completes).  gbsort_graph_cache_clear() frees them all.
 struct GraphKey {
-    int device, key_type, desc, skip, fused, msd, large_msd;
+    int device, key_type, desc, skip, fused, msd, large_msd, finish;
     uint32_t short_cap;
     size_t vb;
     uint64_t n, wait_limit;
     const void *keys, *vals, *ws, *ksrc, *vsrc, *keys_b, *vals_b;
     cudaStream_t stream;
     auto tie() const {
-        return std::tie(device, key_type, desc, skip, fused, msd, large_msd, short_cap, vb, n, wait_limit, keys, vals,
+        return std::tie(device, key_type, desc, skip, fused, msd, large_msd, finish, short_cap, vb, n, wait_limit, keys, vals,
                         ws, ksrc, vsrc, keys_b, vals_b, stream);
     }
     bool operator==(const GraphKey& o) const { return tie() == o.tie(); }
@@ -978,6 +989,7 @@ int launch_sort(const Plan& plan, int descending, void* keys, void* vals, void* 
     k.fused = plan.fused.fn != nullptr;
     k.msd = plan.short_msd ? 1 : 0;
     k.large_msd = plan.msd ? 1 : 0;
+    k.finish = plan.finish ? 1 : 0;
     k.short_cap = plan.short_pairs ? plan.short_cap : 0;
     k.vb = size_t(plan.vb);
     k.n = plan.n;
@@ -1339,6 +1351,10 @@ void gbsort_set_pass_skip(int enable) { g_pass_skip.store(enable ? 1 : 0, std::m
 int gbsort_get_pass_skip(void) { return g_pass_skip.load(std::memory_order_relaxed); }
 void gbsort_set_msd(int enable) { g_msd.store(enable ? 1 : 0, std::memory_order_relaxed); }
 int gbsort_get_msd(void) { return g_msd.load(std::memory_order_relaxed); }
+void gbsort_set_short_pairs(int enable) { g_short_pairs.store(enable ? 1 : 0, std::memory_order_relaxed); }
+int gbsort_get_short_pairs(void) { return g_short_pairs.load(std::memory_order_relaxed); }
+void gbsort_set_leading_digits(int enable) { g_leading.store(enable ? 1 : 0, std::memory_order_relaxed); }
+int gbsort_get_leading_digits(void) { return g_leading.load(std::memory_order_relaxed); }
 void gbsort_set_short_fused(int enable) { g_short_fused.store(enable ? 1 : 0, std::memory_order_relaxed); }
 int gbsort_get_short_fused(void) { return g_short_fused.load(std::memory_order_relaxed); }
 void gbsort_set_short_msd(int enable) { g_short_msd.store(enable ? 1 : 0, std::memory_order_relaxed); }

@@ -663,6 +663,25 @@ def get_msd() -> bool:
     return bool(f())
 
 
+def _switch(name: str, enable) -> bool:
+    l = lib()
+    s, g = getattr(l, f"gbsort_set_{name}"), getattr(l, f"gbsort_get_{name}")
+    s.restype, s.argtypes, g.restype = None, [ctypes.c_int], ctypes.c_int
+    if enable is not None:
+        s(int(enable))
+    return bool(g())
+
+
+def short_pairs(enable=None) -> bool:
+    """Short key-value arrays in one launch: switches it on or off, or reads the switch."""
+    return _switch("short_pairs", enable)
+
+
+def leading_digits(enable=None) -> bool:
+    """Sorts by leading digits and a finish: switches them on or off, or reads the switch."""
+    return _switch("leading_digits", enable)
+
+
 def sort_copy(keys_in, keys_out, n: int, key_type, workspace, workspace_bytes: int, *, values_in=None,
               values_out=None, value_bytes: int = 0, descending: bool = False, stream=None) -> None:
     """Input-preserving sort (gbsort_sort_keys_copy / gbsort_sort_pairs_copy):

@@ -34,3 +34,37 @@ def test_switches_change_the_path_not_the_sizes(gb):
     finally:
         gb.set_pass_skip(True)
         gb.set_msd(True)
+
+
+def test_each_path_of_pairs_alone(gb):
+    """Short pairs and leading digits switch off one by one; sizes stay."""
+    short, wide = ("u64", 1_000_003, 4), ("u64", 1 << 24, 4)
+    sizes = [gb.temp_bytes(*c) for c in (short, wide)]
+    assert gb.short_pairs() and gb.leading_digits()
+    try:
+        gb.short_pairs(False)
+        assert gb.route(*short).path == gb.PATH_LEADING_DIGITS and gb.route(*wide).path == gb.PATH_LEADING_DIGITS
+        gb.leading_digits(False)
+        assert gb.route(*short).path == gb.route(*wide).path == gb.PATH_PASSES
+        gb.short_pairs(True)
+        assert gb.route(*short).path == gb.PATH_SHORT_PAIRS
+        assert [gb.temp_bytes(*c) for c in (short, wide)] == sizes
+    finally:
+        gb.short_pairs(True)
+        gb.leading_digits(True)
+
+
+@pytest.mark.gpu
+def test_switched_off_they_sort_the_same(gb, cuda, oracle):
+    from _oracle import raw_keys
+    from test_outcome_gpu import outcome_of
+
+    for short, wide in ((False, True), (True, False), (False, False)):
+        gb.short_pairs(short)
+        gb.leading_digits(wide)
+        try:
+            for kt, n, vb in (("u32", 70_001, 4), ("u64", 300_007, 8), ("f64", 20_001, 0), ("u128", 20_001, 4)):
+                outcome_of(gb, cuda, oracle, kt, raw_keys(kt, n, seed=1), vb, True)
+        finally:
+            gb.short_pairs(True)
+            gb.leading_digits(True)
