@@ -119,14 +119,9 @@ __global__ void __launch_bounds__(FINISH_SAMPLE_THREADS, 1) finish_sample_kernel
         h ^= h >> 31;
         at[i] = (uint32_t(h >> 32) & 0xffff8000u) | (uint32_t(h) & 32767u);  // tag | slot
     }
-    uint32_t there[MOST];  // (every key's first look at once)
-#pragma unroll
-    for (int i = 0; i < MOST; ++i) there[i] = i < per ? cnt[at[i] & 32767u] : 0u;
-#pragma unroll
-    for (int i = 0; i < MOST; ++i) {
-        if (i >= per) break;
-        const uint32_t tag = at[i] & 0xffff8000u;
-        uint32_t slot = at[i] & 32767u, w = there[i];
+    auto meet = [&](uint32_t key, uint32_t w) {  // w: what its slot held at the first look
+        const uint32_t tag = key & 0xffff8000u;
+        uint32_t slot = key & 32767u;
         for (int probe = 0; probe < 128; ++probe) {
             if (w == 0u) w = atomicCAS(&cnt[slot], 0u, tag | 1u);
             if (w == 0u) break;
@@ -140,6 +135,18 @@ __global__ void __launch_bounds__(FINISH_SAMPLE_THREADS, 1) finish_sample_kernel
             slot = (slot + 1u) & 32767u;
             w = cnt[slot];
         }
+    };
+    // (a key a thread first: a prefix that many share then takes one atomic a
+    // key; then every other key's first look at once)
+    meet(at[0], cnt[at[0] & 32767u]);
+    __syncthreads();
+    uint32_t there[MOST];
+#pragma unroll
+    for (int i = 1; i < MOST; ++i) there[i] = i < per ? cnt[at[i] & 32767u] : 0u;
+#pragma unroll
+    for (int i = 1; i < MOST; ++i) {
+        if (i >= per) break;
+        meet(at[i], there[i]);
     }
     uint32_t bytes = 0;  // bit q: byte q differs somewhere
 #pragma unroll

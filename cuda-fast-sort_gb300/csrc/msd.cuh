@@ -1274,7 +1274,7 @@ template <class U, int THREADS, int HALO, class Bin>
 __device__ __noinline__ void group_sort_crowded(U* group, uint32_t cnt, uint8_t* smem, Bin bin, KeyMap<U> map) {
     using G = GroupSortGeom<int(sizeof(U)), THREADS, HALO>;
     constexpr uint32_t BY_THREAD = 16, BY_WARP = 512;
-    uint32_t* flags = reinterpret_cast<uint32_t*>(smem + G::CTR_OFF);  // a byte a sub-bucket: its keys differ
+    uint32_t* flags = reinterpret_cast<uint32_t*>(smem + G::CTR_OFF);  // a byte a sub-bucket whose keys differ: 1 large, 2 small
     uint32_t* place = reinterpret_cast<uint32_t*>(smem + G::START_OFF);
     const uint16_t* ends = reinterpret_cast<const uint16_t*>(place);
     uint32_t* scan = reinterpret_cast<uint32_t*>(smem + G::SCAN_OFF);
@@ -1323,19 +1323,19 @@ __device__ __noinline__ void group_sort_crowded(U* group, uint32_t cnt, uint8_t*
     __syncthreads();  // now a sub-bucket's word is its end
     for (uint32_t i = tid; i < cnt; i += THREADS) {
         const U k = sk(i);
-        const uint32_t b = bin(k);
-        if (i > first_of(b) && sk(i - 1) != k) atomicOr(&flags[b >> 2], 1u << 8 * (b & 3u));
+        const uint32_t b = bin(k), first = first_of(b);
+        if (i > first && sk(i - 1) != k)
+            atomicOr(&flags[b >> 2], (ends[b] - first > BY_THREAD ? 1u : 2u) << 8 * (b & 3u));
     }
     __syncthreads();
     for (uint32_t w0 = warp * 32; w0 < uint32_t(G::BINS) / 4; w0 += THREADS) {
         const uint32_t mine = flags[w0 + lane];
-        for (uint32_t some = __ballot_sync(0xffffffffu, mine != 0u); some; some &= some - 1u) {
+        for (uint32_t some = __ballot_sync(0xffffffffu, (mine & 0x01010101u) != 0u); some; some &= some - 1u) {
             const int l = __ffs(some) - 1;
             const uint32_t word = __shfl_sync(0xffffffffu, mine, l);
             for (uint32_t q = 0; q < 4; ++q) {
                 if (!(word >> 8 * q & 1u)) continue;
                 const uint32_t b = (w0 + l) * 4 + q, first = first_of(b), m = ends[b] - first;
-                if (m <= BY_THREAD) continue;
                 if (m > BY_WARP) {
                     if (lane == 0) scan[atomicAdd(&misc[1], 1u)] = b;
                 } else {
@@ -1357,7 +1357,7 @@ __device__ __noinline__ void group_sort_crowded(U* group, uint32_t cnt, uint8_t*
         const U k = sk(i);
         const uint32_t b = bin(k), first = first_of(b), m = ends[b] - first;
         uint32_t at = i;
-        if (m <= BY_THREAD && (flags[b >> 2] >> 8 * (b & 3u) & 1u)) {
+        if (flags[b >> 2] >> 8 * (b & 3u) & 2u) {
             at = first;
             for (uint32_t q = first; q < first + m; ++q) {
                 const U o = sk(q);
