@@ -12,8 +12,9 @@
 //                 it also clears the path's counters;
 //   count:        one read of the keys counts every group (65536 16-bit
 //                 counters fit a CTA's shared memory);
-//   scan:         group offsets, and the decision: every group fits a CTA's
-//                 local sort, or MSD_OFF;
+//   scan:         group offsets, and the decision: a group that does not fit a
+//                 CTA's local sort is left out of them (MSD_RANGES), and with
+//                 more than a quarter of the keys in such groups MSD_OFF;
 //   top split:    every tile counts its keys per top digit with shared
 //                 atomics, claims its places in the digit's exact range with
 //                 one global atomic per digit, stages the tile by digit and
@@ -25,8 +26,11 @@
 //                 counting pass on the next 11-12 bits moves every key into
 //                 its sub-bucket (about one key each), then a few rounds of
 //                 an odd-even transposition network in registers, as many as
-//                 the largest sub-bucket holds keys, put the keys in order.
-// With MSD_OFF the least-significant-digit passes, launched after these
+//                 the largest sub-bucket holds keys, put the keys in order;
+//                 a group with a sub-bucket of more keys than that can take
+//                 is sorted another way (group_sort_crowded).
+// The groups left out are sorted by themselves by the launch that follows
+// (multi.cuh).  With MSD_OFF the least-significant-digit passes, launched after these
 // kernels, sort from the caller's buffer, which then holds the input's keys
 // in some order (untouched, or as the local sorts left them); otherwise they
 // exit at once.

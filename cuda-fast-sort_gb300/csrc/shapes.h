@@ -122,9 +122,8 @@ constexpr uint64_t msd_block_n_min(int kb) {
     return kb == 16 ? uint64_t(3) << 19 : kb == 8 ? uint64_t(3) << 23 : ~uint64_t(0);
 }
 // 4-byte floats: from here on (N(0, 1), against four digit passes: 5 * 10^6 128
-// and 127 us, 10^7 183 and 207, 6 * 10^7 745 and 945; values of one exponent,
-// which three passes sort, even out near 1.5 * 10^7: 10^7 177 and 160, 6 * 10^7
-// 750 and 925), and as long as 65536 groups hold them (MsdEvenCode's stretches
+// and 127 us, 10^7 183 and 207, 6 * 10^7 745 and 945; values of one exponent
+// 10^7 177 and 220, 6 * 10^7, where they are sent back, 1087 and 1020), and as long as 65536 groups hold them (MsdEvenCode's stretches
 // take about a quarter more of the codes than even keys do).
 constexpr uint64_t MSD_EVEN_N_MIN = uint64_t(1) << 23;
 constexpr uint64_t MSD_EVEN_N_MAX = uint64_t(9) << 24;

@@ -7,7 +7,8 @@ namespace gbsort {
 
 // Why the digit passes sort after the most-significant-first path of a
 // keys-only sort (msd.cuh; 0: that path sorts): MSD_OFF some group is too big
-// (decided before any key moves), MSD_GAVE_UP a local sort gave up.
+// (decided before any key moves), MSD_GAVE_UP a group of floats that should
+// have been equal was not, or a sort by leading digits could not finish.
 // MSD_RANGES: some ranges are left to sort (multi.cuh).
 constexpr uint32_t MSD_OFF = 1u, MSD_GAVE_UP = 2u, MSD_RANGES = 4u;
 constexpr uint32_t MSD_PASSES = MSD_OFF | MSD_GAVE_UP;  // the digit passes sort everything

@@ -507,8 +507,10 @@ int gbsort_get_short_msd(void);
  * bits first — a count of the keys per leading bits, a split by the top digit,
  * a split by the bits below it into groups of a few thousand keys, and
  * in-place local sorts of those groups in shared memory — instead of one
- * stable pass per key byte.  When a group outgrows a local sort (skewed or
- * repeated keys), the digit passes sort instead, decided on the device.
+ * stable pass per key byte.  Groups that outgrow a local sort (very frequent
+ * keys) are sorted by themselves afterwards; with more than a quarter of the
+ * keys in such groups (skewed keys), or most keys repeated, the digit passes
+ * sort instead, decided on the device.
  * Where the size query holds a block of its own for the path (8-byte keys
  * from 1.5 x 2^24, 16-byte keys from 1.5 x 2^20; ~1 MB, either way)
  * gbsort_plan_info.msd_stages is 6.  On by default; GBSORT_MSD=0 in the
